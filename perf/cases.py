@@ -228,7 +228,7 @@ def _room(case):
         return {"triangles": (4096 * case["pairs"], 3, np.int32)}
     if kind == "process":
         return {"vertices": (1 << 16, 3, np.float64), "triangles": (1 << 17, 3, np.int32),
-                "counts": (case["parts"], 2, np.int64)}
+                "counts": (256, 2, np.int64)}
     return {}
 
 
