@@ -157,7 +157,7 @@ struct visacd_ctx {
   int64_t last_vis_certified = 0, last_vis_trace_steps = 0;  // of the last visibility call
   int clip_nv = 0;
   int32_t sdf_nv = 0, sdf_nt = 0;                 // last SDF remesh result (device-resident)
-  void* clip_ptrs[7] = {nullptr};
+  void* clip_ptrs[6] = {nullptr};
   // Per-kernel timing: events recorded around each launch when timing is on.
   struct Pending {
     int kernel;
