@@ -1,6 +1,8 @@
 // Linear BVH over a triangle mesh, built entirely on the device.
 //
 // Replaces the OptiX GAS build of the reference (lib/src/intersections.cpp:131-180).
+// Up to kOrderMax triangles (every part and cage of a decomposition): two
+// launches and no wait (order.cu). Larger meshes:
 //  1. tri_prep: per triangle centroid, conservatively widened AABB, index check.
 //  2. morton: Morton code of the centroid, 10 to 21 bits per axis by triangle
 //     count (morton_bits), sorted on exactly those bits.
@@ -12,9 +14,8 @@
 //  6. node_layout: traversal records of 64 bytes (both child boxes with each
 //     axis stored as a (lo, hi) pair for packed f32x2 slab tests, + child ids)
 //     and leaf triangles of 48 bytes (3 vertices, vertex ids in .w).
-#include <atomic>
-
 #include "bvh.cuh"
+#include "order.cuh"
 
 namespace vgpu {
 
@@ -258,57 +259,6 @@ __global__ void fit_kernel(const int2* __restrict__ child, const int* __restrict
   }
 }
 
-// The same fit for trees of up to kFitSmallMax leaves in one CTA: the
-// topology (children, parents), the internal boxes, heights and arrival
-// counters live in shared memory, so a level costs shared-memory latency
-// instead of L2 round trips; the boxes go to global memory at the end. Boxes
-// are minima and maxima of the children's, so they equal fit_kernel's.
-constexpr int kFitSmallMax = 4096;
-constexpr size_t kFitSmallBytesPerNode = 6 * 4 + 4 + 4 + 8 + 4;
-
-__global__ void __launch_bounds__(1024) fit_small_kernel(const int2* __restrict__ child,
-                                                         const int* __restrict__ parent_int,
-                                                         const int* __restrict__ parent_leaf,
-                                                         const float* __restrict__ leafbox,
-                                                         float* __restrict__ nodebox, int32_t n,
-                                                         BuildCounters* __restrict__ c) {
-  extern __shared__ __align__(16) unsigned char fit_smem[];
-  const int ni = n - 1;
-  int2* ch_s = reinterpret_cast<int2*>(fit_smem);
-  float* nb = reinterpret_cast<float*>(ch_s + ni);
-  unsigned* vis = reinterpret_cast<unsigned*>(nb + 6 * ni);
-  int* hgt = reinterpret_cast<int*>(vis + ni);
-  int* par = hgt + ni;
-  for (int i = threadIdx.x; i < ni; i += blockDim.x) {
-    ch_s[i] = child[i];
-    par[i] = parent_int[i];
-    vis[i] = 0u;
-  }
-  __syncthreads();
-  for (int s = threadIdx.x; s < n; s += blockDim.x) {
-    int node = parent_leaf[s];
-    for (int guard = 0; node >= 0 && guard < n + 1; ++guard) {
-      __threadfence_block();
-      if (atomicAdd(&vis[node], 1u) == 0u) break;
-      __threadfence_block();
-      const int2 ch = ch_s[node];
-      const int h = 1 + max(ch.x < 0 ? 0 : hgt[ch.x], ch.y < 0 ? 0 : hgt[ch.y]);
-      hgt[node] = h;
-      if (node == 0) atomicMax(&c->depth, h);
-      const float* lb = ch.x < 0 ? &leafbox[6 * (int64_t)(~ch.x)] : &nb[6 * ch.x];
-      const float* rb = ch.y < 0 ? &leafbox[6 * (int64_t)(~ch.y)] : &nb[6 * ch.y];
-#pragma unroll
-      for (int a = 0; a < 3; ++a) {
-        nb[6 * node + a] = fminf(lb[a], rb[a]);
-        nb[6 * node + 3 + a] = fmaxf(lb[3 + a], rb[3 + a]);
-      }
-      node = par[node];
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 6 * ni; i += blockDim.x) nodebox[i] = nb[i];
-}
-
 __global__ void node_layout_kernel(const int2* __restrict__ child,
                                    const float* __restrict__ leafbox,
                                    const float* __restrict__ nodebox, int32_t n_internal,
@@ -326,14 +276,59 @@ __global__ void node_layout_kernel(const int2* __restrict__ child,
   }
 }
 
-// Single-triangle mesh: one internal node whose two children are that leaf
-// (the duplicate test is harmless and keeps the traversal branch-free).
-__global__ void single_node_kernel(const float* __restrict__ leafbox, float4* __restrict__ nodes) {
-  const float* lb = leafbox;
-  nodes[0] = make_float4(lb[0], lb[3], lb[1], lb[4]);
-  nodes[1] = make_float4(lb[2], lb[5], lb[0], lb[3]);
-  nodes[2] = make_float4(lb[1], lb[4], lb[2], lb[5]);
-  nodes[3] = make_float4(__int_as_float(~0), __int_as_float(~0), 0.f, 0.f);
+// The one-launch build (order.cu). Host input was checked by the caller, so
+// nothing has to come back; device input is checked by the kernel.
+static int bvh_build_fast(visacd_ctx* ctx, const float* dv, int32_t nv, const uint32_t* dt, int32_t nt, bool check,
+                          visacd_bvh* b) {
+  const int n_int = nt > 1 ? nt - 1 : 1;
+  const size_t o_tris = ((size_t)n_int * 64 + 255) & ~size_t(255);
+  const size_t o_head = o_tris + (((size_t)nt * 48 + 255) & ~size_t(255));
+  char* mem = nullptr;
+  if (cudaMallocAsync((void**)&mem, o_head + sizeof(BvhHead), ctx->stream) != cudaSuccess) {
+    cudaGetLastError();
+    set_error("bvh_build: device allocation failed");
+    return VISACD_ERR_NO_MEMORY;
+  }
+  b->stream = ctx->stream;
+  b->nodes = reinterpret_cast<float4*>(mem);
+  b->tris = reinterpret_cast<float4*>(mem + o_tris);
+  b->head = mem + o_head;
+  VTRY(ensure_slot(ctx, kSlotTmpTris, order_scratch(nt, true)));
+  OrderJob j = {};
+  j.verts = dv;
+  j.tris = dt;
+  j.nv = nv;
+  j.n = nt;
+  j.bits = morton_bits(nt);
+  j.head = reinterpret_cast<BvhHead*>(b->head);
+  j.leaves = b->tris;
+  order_carve(j, slot<char>(ctx, kSlotTmpTris));
+  VTRY(order_run(ctx, &j, 1));
+  VTRY(order_nodes(ctx, j, b->nodes));
+  // Every step down the tree lengthens the common prefix of (code, position).
+  int len = 0;
+  while ((1 << len) < nt) ++len;
+  b->depth = 3 * j.bits + len;
+  if (!check) return VISACD_OK;
+  BvhHead* h = nullptr;
+  VTRY(pinned(ctx, sizeof(BvhHead), (void**)&h));
+  VCUDA(cudaMemcpyAsync(h, b->head, sizeof(BvhHead), cudaMemcpyDeviceToHost, ctx->stream));
+  VCUDA(stream_wait(ctx));
+  VCHECK(!h->bad, VISACD_ERR_INVALID_ARG, "bvh_build: a triangle references a vertex index >= %d", nv);
+  memcpy(b->tri_bounds, h->tb, sizeof(b->tri_bounds));
+  b->head_read = true;
+  return VISACD_OK;
+}
+
+int bvh_head(visacd_ctx* ctx, visacd_bvh* b) {
+  if (b->head_read || !b->head) return VISACD_OK;
+  BvhHead* h = nullptr;
+  VTRY(pinned(ctx, sizeof(BvhHead), (void**)&h));
+  VCUDA(cudaMemcpyAsync(h, b->head, sizeof(BvhHead), cudaMemcpyDeviceToHost, ctx->stream));
+  VCUDA(stream_wait(ctx));
+  memcpy(b->tri_bounds, h->tb, sizeof(b->tri_bounds));
+  b->head_read = true;
+  return VISACD_OK;
 }
 
 int bvh_build(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* tris, int32_t nt,
@@ -359,6 +354,11 @@ int bvh_build(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* t
   const float* dv = verts;
   const uint32_t* dt = tris;
   if (!device_ptrs) {
+    if (!indices_in_range(reinterpret_cast<const int32_t*>(tris), 3LL * nt, nv)) {
+      delete b;
+      set_error("bvh_build: a triangle references a vertex index >= %d", nv);
+      return VISACD_ERR_INVALID_ARG;
+    }
     VTRY(ensure_slot(ctx, kSlotBuildVerts, (size_t)nv * 12));
     VTRY(ensure_slot(ctx, kSlotBuildTris, (size_t)nt * 12));
     Stager up(ctx);
@@ -368,7 +368,19 @@ int bvh_build(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* t
     dv = slot<float>(ctx, kSlotBuildVerts);
     dt = slot<uint32_t>(ctx, kSlotBuildTris);
   }
-  const int n_int = nt > 1 ? nt - 1 : 1;
+  if (nt <= kOrderMax) {
+    const int rc = bvh_build_fast(ctx, dv, nv, dt, nt, device_ptrs != 0, b);
+    if (rc != VISACD_OK) {
+      if (b->nodes) cudaFreeAsync(b->nodes, ctx->stream);
+      delete b;
+      return rc;
+    }
+    b->ctx = ctx;
+    ctx->bvhs.push_back(b);
+    *out = b;
+    return VISACD_OK;
+  }
+  const int n_int = nt - 1;
   // Scratch: centroids, keys x2, vals x2, child, parents, boxes, visits, counters.
   size_t off = 0;
   auto carve = [&](size_t bytes) {
@@ -423,51 +435,38 @@ int bvh_build(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* t
   VLAUNCH(ctx, kKMorton, g, 256, 0, morton_kernel, cent, nt, cnt, mb, keys, vals);
   VTRY(radix_sort_u64(ctx, keys, vals, keys2, vals2, nt, 3 * mb));
 
-  size_t bytes_nodes = (size_t)n_int * 64, bytes_tris = (size_t)nt * 48;
   b->stream = ctx->stream;
-  cudaError_t e1 = cudaMallocAsync((void**)&b->nodes, bytes_nodes, ctx->stream);
-  cudaError_t e2 = e1 == cudaSuccess ? cudaMallocAsync((void**)&b->tris, bytes_tris, ctx->stream) : e1;
-  if (e1 != cudaSuccess || e2 != cudaSuccess) {
+  const size_t o_tris = ((size_t)n_int * 64 + 255) & ~size_t(255);
+  char* mem = nullptr;
+  if (cudaMallocAsync((void**)&mem, o_tris + (size_t)nt * 48, ctx->stream) != cudaSuccess) {
     cudaGetLastError();
-    if (b->nodes) cudaFreeAsync(b->nodes, ctx->stream);
     delete b;
     set_error("bvh_build: device allocation failed");
     return VISACD_ERR_NO_MEMORY;
   }
+  b->nodes = reinterpret_cast<float4*>(mem);
+  b->tris = reinterpret_cast<float4*>(mem + o_tris);
   VLAUNCH(ctx, kKNodeLayout, g, 256, 0, leaf_kernel, dv, nv, dt, vals, nt, cnt, b->tris, leafbox);
-  if (nt == 1) {
-    VLAUNCH(ctx, kKNodeLayout, 1, 1, 0, single_node_kernel, leafbox, b->nodes);
-  } else {
-    const unsigned gi = grid_for(n_int, 256, 8LL * ctx->sm_count);
-    VLAUNCH(ctx, kKKarras, gi, 256, 0, karras_kernel, keys, nt, child, pint, pleaf);
-    if (nt <= kFitSmallMax) {
-      const size_t fit_smem = (size_t)n_int * kFitSmallBytesPerNode;
-      static std::atomic<bool> fit_attr_set[64];
-      if (ctx->device < 0 || ctx->device >= 64 || !fit_attr_set[ctx->device].load()) {
-        VCUDA(cudaFuncSetAttribute(fit_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                   (int)(kFitSmallMax * kFitSmallBytesPerNode)));
-        if (ctx->device >= 0 && ctx->device < 64) fit_attr_set[ctx->device].store(true);
-      }
-      VLAUNCH(ctx, kKFit, 1, 1024, fit_smem, fit_small_kernel, child, pint, pleaf, leafbox, nodebox, nt, cnt);
-    } else {
-      VLAUNCH(ctx, kKFit, g, 256, 0, fit_kernel, child, pint, pleaf, leafbox, nodebox, visits, height, nt,
-            cnt);
-    }
-    VLAUNCH(ctx, kKNodeLayout, gi, 256, 0, node_layout_kernel, child, leafbox, nodebox, n_int,
-            b->nodes);
-  }
+  const unsigned gi = grid_for(n_int, 256, 8LL * ctx->sm_count);
+  VLAUNCH(ctx, kKKarras, gi, 256, 0, karras_kernel, keys, nt, child, pint, pleaf);
+  VLAUNCH(ctx, kKFit, g, 256, 0, fit_kernel, child, pint, pleaf, leafbox, nodebox, visits, height, nt, cnt);
+  VLAUNCH(ctx, kKNodeLayout, gi, 256, 0, node_layout_kernel, child, leafbox, nodebox, n_int, b->nodes);
   VCUDA(cudaMemcpyAsync(hcnt, cnt, sizeof(BuildCounters), cudaMemcpyDeviceToHost, ctx->stream));
   VCUDA(stream_wait(ctx));
   if (hcnt->bad_index) {
     cudaFreeAsync(b->nodes, ctx->stream);
-    cudaFreeAsync(b->tris, ctx->stream);
     delete b;
     set_error("bvh_build: a triangle references a vertex index >= %d", nv);
     return VISACD_ERR_INVALID_ARG;
   }
-  b->depth = nt == 1 ? 1 : hcnt->depth;
-  b->amax = __uint_as_float_host(hcnt->amax);
-  for (int a = 0; a < 6; ++a) b->tri_bounds[a] = hcnt->tb[a];
+  b->depth = hcnt->depth;
+  b->depth_exact = true;
+  for (int a = 0; a < 6; ++a) {
+    // (order-preserving unsigned values)
+    const unsigned u = (hcnt->tb[a] & 0x80000000u) ? (hcnt->tb[a] & 0x7fffffffu) : ~hcnt->tb[a];
+    memcpy(&b->tri_bounds[a], &u, 4);
+  }
+  b->head_read = true;
   b->ctx = ctx;
   ctx->bvhs.push_back(b);
   *out = b;
@@ -476,7 +475,6 @@ int bvh_build(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* t
 
 void bvh_detach(visacd_bvh* b) {
   if (b->nodes) cudaFreeAsync(b->nodes, b->stream);
-  if (b->tris) cudaFreeAsync(b->tris, b->stream);
   if (b->free_lb) cudaFreeAsync(b->free_lb, b->stream);
   if (b->free_arr && b->ctx && !b->ctx->grid_arr) {
     // Kept on the context for the next grid of this size: work queued on the
@@ -496,6 +494,7 @@ void bvh_detach(visacd_bvh* b) {
   b->free_tex = 0;
   b->free_arr = nullptr;
   b->nodes = b->tris = nullptr;
+  b->head = nullptr;
   b->free_lb = nullptr;
   b->ctx = nullptr;
   b->stream = nullptr;
@@ -526,6 +525,31 @@ extern "C" int visacd_bvh_destroy(visacd_bvh* b) {
 extern "C" int visacd_bvh_info(const visacd_bvh* b, int32_t* n_tris, int32_t* depth) {
   VCHECK(b, VISACD_ERR_INVALID_ARG, "bvh_info: null bvh");
   if (n_tris) *n_tris = b->nt;
-  if (depth) *depth = b->depth;
+  if (depth) {
+    // A one-launch build knows only a bound: the depth is taken from the
+    // records when it is asked for.
+    visacd_bvh* m = const_cast<visacd_bvh*>(b);
+    if (!m->depth_exact && m->nodes && m->nt > 0) {
+      const int ni = m->nt > 1 ? m->nt - 1 : 1;
+      std::vector<float4> rec((size_t)ni * 4);
+      VCUDA(cudaSetDevice(m->device));
+      VCUDA(cudaMemcpyAsync(rec.data(), m->nodes, (size_t)ni * 64, cudaMemcpyDeviceToHost, m->stream));
+      VCUDA(cudaStreamSynchronize(m->stream));
+      std::vector<std::pair<int, int>> todo(1, {0, 1});
+      int deepest = 0;
+      while (!todo.empty()) {
+        const auto [node, d] = todo.back();
+        todo.pop_back();
+        deepest = std::max(deepest, d);
+        int child[2];
+        memcpy(child, &rec[4 * (size_t)node + 3], sizeof(child));
+        for (int c : child)
+          if (c >= 0) todo.push_back({c, d + 1});
+      }
+      m->depth = deepest;
+      m->depth_exact = true;
+    }
+    *depth = m->depth;
+  }
   return VISACD_OK;
 }

@@ -15,11 +15,13 @@ struct visacd_bvh {
   int device = 0;
   int32_t nt = 0;
   int32_t nv = 0;
-  int32_t depth = 0;
-  float amax = 0.f;  // largest |vertex coordinate|
-  // Bounds of the triangles' vertices as order-preserving unsigned values
-  // (min xyz, max xyz), read back with the build's counters.
-  unsigned tri_bounds[6] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0u, 0u, 0u};
+  int32_t depth = 0;         // the tree's depth, or a bound of it (depth_exact)
+  bool depth_exact = false;
+  // Bounds of the triangles' vertices (min xyz, max xyz), on the host once
+  // bvh_head() has read them (builds in one launch leave them on the device).
+  bool head_read = false;
+  float tri_bounds[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+  void* head = nullptr;      // device BvhHead, part of the nodes' allocation
   float4* nodes = nullptr;
   float4* tris = nullptr;
   visacd_ctx* ctx = nullptr;       // owning context (null once it is destroyed)
@@ -36,17 +38,18 @@ struct visacd_bvh {
 
 namespace vgpu {
 
-inline float __uint_as_float_host(unsigned u) {
-  float f;
-  memcpy(&f, &u, 4);
-  return f;
-}
-
 int bvh_build(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* tris, int32_t nt,
               int device_ptrs, visacd_bvh** out);
 // Frees a BVH's device memory when its context goes away (the handle itself
 // stays valid until visacd_bvh_destroy, and is rejected by queries).
 void bvh_detach(visacd_bvh* b);
+// Reads the BVH's head to the host (waits for the stream; once per BVH).
+int bvh_head(visacd_ctx* ctx, visacd_bvh* b);
+// A build may still be running on its context's stream: a call on another
+// stream waits for that one first.
+inline void bvh_settle(visacd_ctx* ctx, const visacd_bvh* b) {
+  if (b && b->ctx && b->stream != ctx->stream) cudaStreamSynchronize(b->stream);
+}
 // Builds the BVH's free-space grid (once; a BVH whose grid would not be
 // usable keeps none), its resolution sized for a call over `pairs` pairs. Uses the context's counter slot and pinned staging
 // buffer (waits for the stream first), so it runs before a call takes them.

@@ -94,6 +94,7 @@ enum CtxSlot {
   kSlotVisKeysAlt,
   kSlotVisPerm,
   kSlotVisPermAlt,
+  kSlotVisOrder,
   kSlotVisRank,
   kSlotBitset,
   kSlotWordCounts,
@@ -137,6 +138,7 @@ struct visacd_ctx {
   size_t h_pinned_cap = 0;
   void* h_upload = nullptr;          // pinned upload buffer (Stager)
   size_t h_upload_cap = 0;
+  size_t h_upload_used = 0;          // bytes handed out since the stream was last waited for
   int64_t launches = 0;
   int64_t last_n_edges = 0;
   bool timing = false;
@@ -242,22 +244,23 @@ int pinned(visacd_ctx* ctx, size_t bytes, void** out);
 // Host-to-device uploads of one call through the context's pinned upload
 // buffer: a host memcpy into pinned memory, then an asynchronous DMA from it,
 // so contexts driven by several host threads do not contend on the driver's
-// pageable-copy staging. reserve(total) first waits for the context stream
-// (the previous call's DMAs may still read the buffer) and grows it; put()
-// places each array at the next 64-byte boundary.
+// pageable-copy staging. reserve(total) takes the next piece of the buffer;
+// only when it does not fit does it wait for the context stream (earlier DMAs
+// may still read the buffer) and start over, growing the buffer if needed.
+// put() places each array at the next 64-byte boundary.
 class Stager {
  public:
   explicit Stager(visacd_ctx* ctx) : ctx_(ctx) {}
   int reserve(size_t total_bytes, int arrays);
   int put(void* dst, const void* src, size_t bytes);
-  // The pinned buffer itself (after reserve): filled in the device layout and
-  // sent with one copy.
-  char* host() { return static_cast<char*>(ctx_->h_upload); }
+  // The reserved pinned piece itself (after reserve): filled in the device
+  // layout and sent with one copy.
+  char* host() { return static_cast<char*>(ctx_->h_upload) + base_; }
   int copy(void* dst, size_t bytes);
 
  private:
   visacd_ctx* ctx_;
-  size_t used_ = 0, cap_ = 0;
+  size_t base_ = 0, used_ = 0, cap_ = 0;
 };
 
 template <class T>
@@ -282,6 +285,7 @@ inline bool indices_in_range(const int32_t* p, int64_t n, int64_t bound) {
 // event, which leaves the cores to the other host threads when many
 // contexts share the machine (process_batch workers).
 inline cudaError_t stream_wait(visacd_ctx* ctx) {
+  ctx->h_upload_used = 0;  // every upload is through
   if (ctx->blocking_wait && ctx->wait_event) {
     cudaError_t e = cudaEventRecord(ctx->wait_event, ctx->stream);
     return e != cudaSuccess ? e : cudaEventSynchronize(ctx->wait_event);

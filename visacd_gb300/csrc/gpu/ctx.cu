@@ -153,21 +153,26 @@ int pinned(visacd_ctx* ctx, size_t bytes, void** out) {
 }
 
 int Stager::reserve(size_t total_bytes, int arrays) {
-  const size_t need = total_bytes + 64 * (size_t)(arrays + 1);
-  VCUDA(stream_wait(ctx_));
-  if (need > ctx_->h_upload_cap) {
-    if (ctx_->h_upload) cudaFreeHost(ctx_->h_upload);
-    ctx_->h_upload = nullptr;
-    ctx_->h_upload_cap = 0;
-    const size_t want = need + need / 4;
-    cudaError_t e = cudaMallocHost(&ctx_->h_upload, want);
-    if (e != cudaSuccess) {
-      cudaGetLastError();
-      set_error("cudaMallocHost(%zu) failed: %s", want, cudaGetErrorString(e));
-      return VISACD_ERR_NO_MEMORY;
+  const size_t need = (total_bytes + 64 * (size_t)(arrays + 1) + 63) & ~size_t(63);
+  if (ctx_->h_upload_used + need > ctx_->h_upload_cap) {
+    VCUDA(stream_wait(ctx_));
+    if (need > ctx_->h_upload_cap) {
+      if (ctx_->h_upload) cudaFreeHost(ctx_->h_upload);
+      ctx_->h_upload = nullptr;
+      ctx_->h_upload_cap = 0;
+      // Room for a few calls' uploads in flight while they are small.
+      const size_t want = need <= (size_t)1 << 20 ? 4 * need : need + need / 4;
+      cudaError_t e = cudaMallocHost(&ctx_->h_upload, want);
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        set_error("cudaMallocHost(%zu) failed: %s", want, cudaGetErrorString(e));
+        return VISACD_ERR_NO_MEMORY;
+      }
+      ctx_->h_upload_cap = want;
     }
-    ctx_->h_upload_cap = want;
   }
+  base_ = ctx_->h_upload_used;
+  ctx_->h_upload_used += need;
   used_ = 0;
   cap_ = need;
   return VISACD_OK;
@@ -176,7 +181,7 @@ int Stager::reserve(size_t total_bytes, int arrays) {
 int Stager::put(void* dst, const void* src, size_t bytes) {
   if (bytes == 0) return VISACD_OK;
   VCHECK(used_ + bytes <= cap_, VISACD_ERR_INVALID_ARG, "upload larger than reserved");
-  char* h = static_cast<char*>(ctx_->h_upload) + used_;
+  char* h = host() + used_;
   std::memcpy(h, src, bytes);
   VCUDA(cudaMemcpyAsync(dst, h, bytes, cudaMemcpyHostToDevice, ctx_->stream));
   used_ += (bytes + 63) & ~size_t(63);
@@ -185,7 +190,7 @@ int Stager::put(void* dst, const void* src, size_t bytes) {
 
 int Stager::copy(void* dst, size_t bytes) {
   VCHECK(bytes <= cap_, VISACD_ERR_INVALID_ARG, "upload larger than reserved");
-  if (bytes) VCUDA(cudaMemcpyAsync(dst, ctx_->h_upload, bytes, cudaMemcpyHostToDevice, ctx_->stream));
+  if (bytes) VCUDA(cudaMemcpyAsync(dst, host(), bytes, cudaMemcpyHostToDevice, ctx_->stream));
   return VISACD_OK;
 }
 

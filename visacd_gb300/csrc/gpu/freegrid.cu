@@ -269,16 +269,12 @@ int free_grid_build(visacd_ctx* ctx, visacd_bvh* b, int64_t pairs) {
   if (b->free_built) return VISACD_OK;
   b->free_built = true;  // also when the grid is not usable: then it is not retried
   if (b->nt <= 0) return VISACD_OK;
-  // Bounding box of the triangles, read back with the BVH build's counters
-  // (order-preserving unsigned values).
-  const unsigned* h = b->tri_bounds;
+  // Bounding box of the triangles.
+  VTRY(bvh_head(ctx, b));
   float lo[3], hi[3];
   for (int a = 0; a < 3; ++a) {
-    const unsigned ol = h[a], oh = h[3 + a];
-    const unsigned bl = (ol & 0x80000000u) ? (ol & 0x7fffffffu) : ~ol;
-    const unsigned bh = (oh & 0x80000000u) ? (oh & 0x7fffffffu) : ~oh;
-    lo[a] = __uint_as_float_host(bl);
-    hi[a] = __uint_as_float_host(bh);
+    lo[a] = b->tri_bounds[a];
+    hi[a] = b->tri_bounds[3 + a];
     if (!std::isfinite(lo[a]) || !std::isfinite(hi[a]) || !(hi[a] >= lo[a])) return VISACD_OK;
   }
   const float ext = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));

@@ -26,6 +26,7 @@
 //    popcount / scan / emit pass compacts it into the row-major edge list.
 #include <math.h>
 
+#include "order.cuh"
 #include "traverse.cuh"
 
 namespace vgpu {
@@ -572,35 +573,93 @@ static int choose_vis_variant(visacd_ctx* ctx, int32_t n, bool masked, const vis
   return kDefaultVisVariant;
 }
 
-// Morton order of n device points into perm (sorted position -> vertex).
-int vis_morton_order(visacd_ctx* ctx, const float* d_pts, int32_t n, uint32_t* perm) {
-  if (n <= 0) return VISACD_OK;
-  VTRY(ensure_slot(ctx, kSlotCounters, sizeof(VisCounters)));
+// Morton orders of points above kOrderMax: the general sort. perm: sorted
+// position -> vertex.
+static int points_order_large(visacd_ctx* ctx, const float* d_pts, int32_t n, VisCounters* cnt, uint32_t* perm) {
   VTRY(ensure_slot(ctx, kSlotVisKeys, (size_t)n * 8));
   VTRY(ensure_slot(ctx, kSlotVisKeysAlt, (size_t)n * 8));
   VTRY(ensure_slot(ctx, kSlotVisPermAlt, (size_t)n * 4));
-  VisCounters* cnt = slot<VisCounters>(ctx, kSlotCounters);
-  VisCounters* h = nullptr;
-  VTRY(pinned(ctx, sizeof(VisCounters), (void**)&h));
-  memset(h, 0, sizeof(VisCounters));
-  for (int a = 0; a < 3; ++a) {
-    h->pmin[a] = 0xffffffffu;
-    h->pmax[a] = 0u;
-  }
-  VCUDA(cudaMemcpyAsync(cnt, h, sizeof(VisCounters), cudaMemcpyHostToDevice, ctx->stream));
   uint64_t* keys = slot<uint64_t>(ctx, kSlotVisKeys);
   const unsigned gp = grid_for(n, 256, 4LL * ctx->sm_count);
+  // The ordered bounds start at (max, 0); the rest of the counters is zero.
+  VCUDA(cudaMemsetAsync(cnt->pmin, 0xff, sizeof(cnt->pmin), ctx->stream));
+  VCUDA(cudaMemsetAsync(cnt->pmax, 0, sizeof(cnt->pmax), ctx->stream));
   VLAUNCH(ctx, kKVisPrep, gp, 256, 0, point_bounds_kernel, d_pts, n, cnt);
   VLAUNCH(ctx, kKVisPrep, gp, 256, 0, point_morton_kernel, d_pts, n, cnt, morton_bits(n), keys, perm);
-  VTRY(radix_sort_u64(ctx, keys, perm, slot<uint64_t>(ctx, kSlotVisKeysAlt),
-                      slot<uint32_t>(ctx, kSlotVisPermAlt), n, 3 * morton_bits(n)));
+  return radix_sort_u64(ctx, keys, perm, slot<uint64_t>(ctx, kSlotVisKeysAlt),
+                        slot<uint32_t>(ctx, kSlotVisPermAlt), n, 3 * morton_bits(n));
+}
+
+// The Morton orders of several point sets (the parts of a call), and for the
+// masked ones their new points in order and every point's rank among them
+// (rows and rank sized n each). Sets up to kOrderMax share one launch; its
+// scratch is `scratch` (points_scratch bytes).
+struct PointOrder {
+  const float* pts;
+  int32_t n;
+  uint32_t* perm;
+  const uint8_t* is_new;  // null: no mask
+  uint32_t* rows;
+  int32_t* rank;
+};
+static size_t points_scratch(const PointOrder* o, int count) {
+  size_t b = 256;
+  for (int k = 0; k < count; ++k)
+    if (o[k].n > 1 && o[k].n <= kOrderMax) b += order_scratch(o[k].n, false);
+  return b;
+}
+static int points_order(visacd_ctx* ctx, const PointOrder* o, int count, char* scratch, VisCounters* cnt) {
+  std::vector<OrderJob> jobs;
+  for (int k = 0; k < count; ++k) {
+    const PointOrder& q = o[k];
+    if (q.n < 2) continue;
+    if (q.n <= kOrderMax) {
+      OrderJob j = {};
+      j.verts = q.pts;
+      j.nv = j.n = q.n;
+      j.bits = morton_bits(q.n);
+      order_carve(j, scratch);
+      scratch += order_scratch(q.n, false);
+      j.v0 = q.perm;
+      j.is_new = q.is_new;
+      j.rows = q.rows;
+      j.rank = q.rank;
+      jobs.push_back(j);
+      continue;
+    }
+    VTRY(points_order_large(ctx, q.pts, q.n, cnt, q.perm));
+    if (q.is_new) {
+      const unsigned gp = grid_for(q.n, 256, 4LL * ctx->sm_count);
+      VTRY(ensure_slot(ctx, kSlotWordCounts, (size_t)q.n * 4));
+      VTRY(ensure_slot(ctx, kSlotWordOffsets, (size_t)(q.n + 1) * 8));
+      uint32_t* flags = slot<uint32_t>(ctx, kSlotWordCounts);
+      uint64_t* off = slot<uint64_t>(ctx, kSlotWordOffsets);
+      VLAUNCH(ctx, kKVisPrep, gp, 256, 0, new_flags_kernel, q.perm, q.is_new, q.n, flags);
+      VTRY(exclusive_scan_u32_to_u64(ctx, flags, off, q.n));
+      VLAUNCH(ctx, kKVisPrep, gp, 256, 0, new_rows_kernel, q.perm, flags, off, q.n, q.rows, q.rank);
+    }
+  }
+  return jobs.empty() ? VISACD_OK : order_run(ctx, jobs.data(), (int)jobs.size());
+}
+
+// Morton order of n device points into perm; synchronizes.
+int vis_morton_order(visacd_ctx* ctx, const float* d_pts, int32_t n, uint32_t* perm) {
+  if (n <= 0) return VISACD_OK;
+  const PointOrder o = {d_pts, n, perm, nullptr, nullptr, nullptr};
+  VTRY(ensure_slot(ctx, kSlotCounters, sizeof(VisCounters)));
+  VTRY(ensure_slot(ctx, kSlotVisOrder, points_scratch(&o, 1)));
+  if (n == 1) {
+    VCUDA(cudaMemsetAsync(perm, 0, 4, ctx->stream));
+  } else {
+    VTRY(points_order(ctx, &o, 1, slot<char>(ctx, kSlotVisOrder), slot<VisCounters>(ctx, kSlotCounters)));
+  }
   VCUDA(stream_wait(ctx));
   return VISACD_OK;
 }
 
 static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint8_t* d_new,
                       const visacd_bvh* self_bvh, const visacd_bvh* cage_bvh, int64_t* n_edges,
-                      visacd_vis_stats* stats, int64_t pairs) {
+                      visacd_vis_stats* stats, int64_t pairs, int32_t n_new) {
   // The cage's free-space grid, for calls with many pairs (`pairs`: the
   // call's pair count, or a bound of it): built once per cage BVH, before this
   // call's counters take the shared scratch and staging buffers.
@@ -608,16 +667,7 @@ static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint
   if (use_grid) VTRY(free_grid_build(ctx, const_cast<visacd_bvh*>(cage_bvh), pairs));
   VTRY(ensure_slot(ctx, kSlotCounters, sizeof(VisCounters)));
   VisCounters* cnt = slot<VisCounters>(ctx, kSlotCounters);
-  VisCounters init;
-  memset(&init, 0, sizeof(init));
-  for (int a = 0; a < 3; ++a) {
-    init.pmin[a] = 0xffffffffu;
-    init.pmax[a] = 0u;
-  }
-  VisCounters* h = nullptr;
-  VTRY(pinned(ctx, sizeof(VisCounters), (void**)&h));
-  *h = init;
-  VCUDA(cudaMemcpyAsync(cnt, h, sizeof(VisCounters), cudaMemcpyHostToDevice, ctx->stream));
+  VCUDA(cudaMemsetAsync(cnt, 0, sizeof(VisCounters), ctx->stream));
   ctx->last_n_edges = 0;
 
   const int64_t np = (int64_t)n * (n - 1) / 2;
@@ -627,18 +677,17 @@ static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint
     if (stats) memset(stats, 0, sizeof(*stats));
     return VISACD_OK;
   }
-  // Morton order of the points.
-  VTRY(ensure_slot(ctx, kSlotVisKeys, (size_t)n * 8));
-  VTRY(ensure_slot(ctx, kSlotVisKeysAlt, (size_t)n * 8));
+  // Morton order of the points; rows: the new ones in order.
   VTRY(ensure_slot(ctx, kSlotVisPerm, (size_t)n * 4));
-  VTRY(ensure_slot(ctx, kSlotVisPermAlt, (size_t)n * 4));
-  uint64_t* keys = slot<uint64_t>(ctx, kSlotVisKeys);
   uint32_t* perm = slot<uint32_t>(ctx, kSlotVisPerm);
-  const unsigned gp = grid_for(n, 256, 4LL * ctx->sm_count);
-  VLAUNCH(ctx, kKVisPrep, gp, 256, 0, point_bounds_kernel, d_pts, n, cnt);
-  VLAUNCH(ctx, kKVisPrep, gp, 256, 0, point_morton_kernel, d_pts, n, cnt, morton_bits(n), keys, perm);
-  VTRY(radix_sort_u64(ctx, keys, perm, slot<uint64_t>(ctx, kSlotVisKeysAlt),
-                      slot<uint32_t>(ctx, kSlotVisPermAlt), n, 3 * morton_bits(n)));
+  PointOrder order = {d_pts, n, perm, d_new, nullptr, nullptr};
+  if (d_new) {
+    VTRY(ensure_slot(ctx, kSlotVisRank, (size_t)n * 4 + (size_t)n * 4 + 256));
+    order.rows = slot<uint32_t>(ctx, kSlotVisRank);
+    order.rank = reinterpret_cast<int32_t*>(order.rows + ((n + 63) & ~63));
+  }
+  VTRY(ensure_slot(ctx, kSlotVisOrder, points_scratch(&order, 1)));
+  VTRY(points_order(ctx, &order, 1, slot<char>(ctx, kSlotVisOrder), cnt));
 
   const int variant = choose_vis_variant(ctx, n, d_new != nullptr, self_bvh, cage_bvh);
   const int TR = kVisVariants[variant].tr, TC = 32 / TR;
@@ -650,26 +699,18 @@ static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint
   P.nc = n;
   P.ntc = (n + TC - 1) / TC;
   if (d_new) {
-    // Rows: new vertices in Morton order (compaction by scan).
-    VTRY(ensure_slot(ctx, kSlotWordCounts, (size_t)n * 4));
-    VTRY(ensure_slot(ctx, kSlotWordOffsets, (size_t)(n + 1) * 8));
-    VTRY(ensure_slot(ctx, kSlotVisRank, (size_t)n * 4 + (size_t)n * 4 + 256));
-    uint32_t* flags = slot<uint32_t>(ctx, kSlotWordCounts);
-    uint64_t* off = slot<uint64_t>(ctx, kSlotWordOffsets);
-    uint32_t* rows = slot<uint32_t>(ctx, kSlotVisRank);
-    int32_t* newrank = reinterpret_cast<int32_t*>(rows + ((n + 63) & ~63));
-    VLAUNCH(ctx, kKVisPrep, gp, 256, 0, new_flags_kernel, perm, d_new, n, flags);
-    VTRY(exclusive_scan_u32_to_u64(ctx, flags, off, n));
-    VLAUNCH(ctx, kKVisPrep, gp, 256, 0, new_rows_kernel, perm, flags, off, n, rows, newrank);
-    uint64_t* hn = nullptr;
-    VTRY(pinned(ctx, 8, (void**)&hn));
-    VCUDA(cudaMemcpyAsync(hn, off + n, 8, cudaMemcpyDeviceToHost, ctx->stream));
-    VCUDA(stream_wait(ctx));
-    P.rows = rows;
-    P.nr = (int32_t)*hn;
+    if (n_new < 0) {  // the mask is on the device: its count with it
+      std::vector<uint8_t> mask((size_t)n);
+      VCUDA(cudaMemcpyAsync(mask.data(), d_new, (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
+      VCUDA(stream_wait(ctx));
+      n_new = 0;
+      for (uint8_t m : mask) n_new += m != 0;
+    }
+    P.rows = order.rows;
+    P.nr = n_new;
     P.triangular = 0;
     P.is_new = d_new;
-    P.newrank = newrank;
+    P.newrank = order.rank;
     P.ntr = (P.nr + TR - 1) / TR;
     P.total_tiles = (unsigned long long)P.ntr * (unsigned long long)P.ntc;
   } else {
@@ -677,13 +718,15 @@ static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint
     P.nr = n;
     P.triangular = 1;
     P.ntr = (n + TR - 1) / TR;
-    VTRY(ensure_slot(ctx, kSlotVisRowTiles, (size_t)P.ntr * 4 + (size_t)(P.ntr + 1) * 8 + 256));
-    uint32_t* rc = slot<uint32_t>(ctx, kSlotVisRowTiles);
-    uint64_t* rs = reinterpret_cast<uint64_t*>(rc + ((P.ntr + 63) & ~63LL));
-    VLAUNCH(ctx, kKVisPrep, grid_for(P.ntr, 256, 4LL * ctx->sm_count), 256, 0,
-            tile_row_counts_kernel, P.ntr, P.ntc, TR, TC, rc);
-    VTRY(exclusive_scan_u32_to_u64(ctx, rc, rs, P.ntr));
-    P.row_start = reinterpret_cast<const unsigned long long*>(rs);
+    if (TR < TC) {  // shapes whose tile rows have no closed form (tile_of)
+      VTRY(ensure_slot(ctx, kSlotVisRowTiles, (size_t)P.ntr * 4 + (size_t)(P.ntr + 1) * 8 + 256));
+      uint32_t* rc = slot<uint32_t>(ctx, kSlotVisRowTiles);
+      uint64_t* rs = reinterpret_cast<uint64_t*>(rc + ((P.ntr + 63) & ~63LL));
+      VLAUNCH(ctx, kKVisPrep, grid_for(P.ntr, 256, 4LL * ctx->sm_count), 256, 0,
+              tile_row_counts_kernel, P.ntr, P.ntc, TR, TC, rc);
+      VTRY(exclusive_scan_u32_to_u64(ctx, rc, rs, P.ntr));
+      P.row_start = reinterpret_cast<const unsigned long long*>(rs);
+    }
     // The same total as the device scan, counted here (no read-back).
     unsigned long long total = 0;
     for (int64_t r = 0; r < P.ntr; ++r) {
@@ -736,6 +779,7 @@ static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint
   VLAUNCH(ctx, kKBitPopc, gw, 256, 0, bit_popc_kernel, P.bitset, nw, wc);
   VTRY(exclusive_scan_u32_to_u64(ctx, wc, wo, nw));
   // Counters and the status word in one wait.
+  VisCounters* h = nullptr;
   uint32_t* hs = nullptr;
   VTRY(pinned(ctx, sizeof(VisCounters) + 64, (void**)&h));
   hs = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(h) + ((sizeof(VisCounters) + 15) & ~size_t(15)));
@@ -813,11 +857,6 @@ __global__ void multi_part_offsets_kernel(const unsigned long long* __restrict__
   for (int p = threadIdx.x; p <= n_parts; p += blockDim.x) out[p] = off[word_start[p]];
 }
 
-// Rows of a masked part (new vertices in Morton order) and their count.
-__global__ void copy_count_kernel(const uint64_t* __restrict__ off, int32_t n, int32_t* __restrict__ out) {
-  *out = (int32_t)off[n];
-}
-
 int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* pts, const int32_t* n_pts,
                           const uint8_t* const* is_new, const visacd_bvh* const* self_bvhs,
                           const visacd_bvh* const* cage_bvhs, int64_t* n_edges, visacd_vis_stats* stats) {
@@ -829,12 +868,14 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
   // before this call takes the shared scratch and staging buffers.
   // A part's pairs: all of them, or (masked) those with a new endpoint.
   std::vector<int64_t> part_pairs(n_parts, 0);
+  std::vector<int32_t> nr(n_parts, 0);  // new points of the masked parts
   for (int p = 0; p < n_parts; ++p) {
     const int64_t n = std::max(n_pts[p], 0);
     int64_t pairs = n * (n > 0 ? n - 1 : 0) / 2;
     if (is_new && is_new[p] && pts[p]) {
       int64_t k = 0;
       for (int64_t v = 0; v < n; ++v) k += is_new[p][v] != 0;
+      nr[p] = (int32_t)k;
       pairs -= (n - k) * (n - k - 1) / 2;
     }
     part_pairs[p] = pairs;
@@ -851,10 +892,9 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
   // Layout of the per-part arrays in one buffer (256-byte aligned pieces).
   auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
   std::vector<size_t> o_pts(n_parts), o_mask(n_parts), o_perm(n_parts), o_rows(n_parts),
-      o_rank(n_parts), o_rs(n_parts);
+      o_rank(n_parts);
   std::vector<int64_t> ntr_tri(n_parts, 0);
-  size_t total = al(sizeof(int32_t) * (size_t)n_parts);  // masked row counts
-  const size_t o_nr = 0;
+  size_t total = 0;
   unsigned long long words = 0;
   std::vector<unsigned long long> word_start(n_parts + 1);
   for (int p = 0; p < n_parts; ++p) {
@@ -863,6 +903,8 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
     const visacd_bvh* cb = cage_bvhs[p];
     VCHECK(n >= 0 && (n == 0 || pts[p]) && sb && cb, VISACD_ERR_INVALID_ARG, "visibility_batch: bad part %d", p);
     VCHECK(n <= (1 << 24), VISACD_ERR_INVALID_ARG, "visibility_batch: part %d has n = %d above 2^24", p, n);
+    bvh_settle(ctx, sb);
+    bvh_settle(ctx, cb);
     VCHECK(sb->ctx && cb->ctx && sb->device == ctx->device && cb->device == ctx->device,
            VISACD_ERR_INVALID_ARG, "visibility_batch: part %d BVH is not on this context's device", p);
     VCHECK(sb->depth <= kStack && cb->depth <= kStack, VISACD_ERR_INVALID_ARG,
@@ -876,7 +918,6 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
     o_rows[p] = total; total += al((size_t)std::max(n, 1) * 4);
     o_rank[p] = total; total += al((size_t)std::max(n, 1) * 4);
     ntr_tri[p] = (n + TR - 1) / TR;
-    o_rs[p] = total;   total += al((size_t)(ntr_tri[p] + 1) * 8);
     word_start[p] = words;
     const unsigned long long np = (unsigned long long)n * (unsigned long long)(n > 0 ? n - 1 : 0) / 2;
     words += (np + 31) / 32;
@@ -892,73 +933,33 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
   total += al(8 * (size_t)(n_parts + 1));
   VTRY(ensure_slot(ctx, kSlotVisMulti, total));
   char* base = slot<char>(ctx, kSlotVisMulti);
-  // Upload points, masks and the triangular tile-row starts.
+  // Upload points and masks.
   {
     size_t up_bytes = 0;
-    for (int p = 0; p < n_parts; ++p) up_bytes += (size_t)n_pts[p] * 13 + (size_t)(ntr_tri[p] + 1) * 8;
+    for (int p = 0; p < n_parts; ++p) up_bytes += (size_t)n_pts[p] * 13;
     Stager up(ctx);
-    VTRY(up.reserve(up_bytes + 8 * (size_t)(n_parts + 1), 3 * n_parts + 1));
-    std::vector<uint64_t> rs;
+    VTRY(up.reserve(up_bytes + 8 * (size_t)(n_parts + 1), 2 * n_parts + 1));
     for (int p = 0; p < n_parts; ++p) {
       const int32_t n = n_pts[p];
       if (n) VTRY(up.put(base + o_pts[p], pts[p], (size_t)n * 12));
       if (n && is_new && is_new[p]) VTRY(up.put(base + o_mask[p], is_new[p], (size_t)n));
-      const int64_t ntr = ntr_tri[p], ntc = (n + TC - 1) / TC;
-      rs.assign((size_t)ntr + 1, 0);
-      for (int64_t r = 0; r < ntr; ++r) {
-        const int64_t c = ntc - (r * TR) / TC;
-        rs[r + 1] = rs[r] + (uint64_t)(c > 0 ? c : 0);
-      }
-      VTRY(up.put(base + o_rs[p], rs.data(), rs.size() * 8));
     }
     VTRY(up.put(base + o_words, word_start.data(), 8 * (size_t)(n_parts + 1)));
   }
-  // Morton order of each part; rows and ranks of the masked ones.
-  int32_t* d_nr = reinterpret_cast<int32_t*>(base + o_nr);
-  for (int p = 0; p < n_parts; ++p) {
-    const int32_t n = n_pts[p];
-    if (n < 2) continue;
-    const float* dp = reinterpret_cast<const float*>(base + o_pts[p]);
-    uint32_t* perm = reinterpret_cast<uint32_t*>(base + o_perm[p]);
-    VTRY(ensure_slot(ctx, kSlotCounters, sizeof(VisCounters)));
-    VTRY(ensure_slot(ctx, kSlotVisKeys, (size_t)n * 8));
-    VTRY(ensure_slot(ctx, kSlotVisKeysAlt, (size_t)n * 8));
-    VTRY(ensure_slot(ctx, kSlotVisPermAlt, (size_t)n * 4));
-    VisCounters* cnt = slot<VisCounters>(ctx, kSlotCounters);
-    VisCounters* h = nullptr;
-    VTRY(pinned(ctx, sizeof(VisCounters), (void**)&h));
-    memset(h, 0, sizeof(VisCounters));
-    for (int a = 0; a < 3; ++a) {
-      h->pmin[a] = 0xffffffffu;
-      h->pmax[a] = 0u;
-    }
-    VCUDA(cudaMemcpyAsync(cnt, h, sizeof(VisCounters), cudaMemcpyHostToDevice, ctx->stream));
-    uint64_t* keys = slot<uint64_t>(ctx, kSlotVisKeys);
-    const unsigned gp = grid_for(n, 256, 4LL * ctx->sm_count);
-    VLAUNCH(ctx, kKVisPrep, gp, 256, 0, point_bounds_kernel, dp, n, cnt);
-    VLAUNCH(ctx, kKVisPrep, gp, 256, 0, point_morton_kernel, dp, n, cnt, morton_bits(n), keys, perm);
-    VTRY(radix_sort_u64(ctx, keys, perm, slot<uint64_t>(ctx, kSlotVisKeysAlt),
-                        slot<uint32_t>(ctx, kSlotVisPermAlt), n, 3 * morton_bits(n)));
-    if (is_new && is_new[p]) {
-      VTRY(ensure_slot(ctx, kSlotWordCounts, (size_t)n * 4));
-      VTRY(ensure_slot(ctx, kSlotWordOffsets, (size_t)(n + 1) * 8));
-      uint32_t* flags = slot<uint32_t>(ctx, kSlotWordCounts);
-      uint64_t* off = slot<uint64_t>(ctx, kSlotWordOffsets);
-      const uint8_t* dm = reinterpret_cast<const uint8_t*>(base + o_mask[p]);
-      VLAUNCH(ctx, kKVisPrep, gp, 256, 0, new_flags_kernel, perm, dm, n, flags);
-      VTRY(exclusive_scan_u32_to_u64(ctx, flags, off, n));
-      VLAUNCH(ctx, kKVisPrep, gp, 256, 0, new_rows_kernel, perm, flags, off, n,
-              reinterpret_cast<uint32_t*>(base + o_rows[p]), reinterpret_cast<int32_t*>(base + o_rank[p]));
-      VLAUNCH(ctx, kKVisPrep, 1, 1, 0, copy_count_kernel, off, n, d_nr + p);
-    }
-  }
-  std::vector<int32_t> nr(n_parts, 0);
+  // Morton orders of the parts; rows and ranks of the masked ones.
   {
-    int32_t* h = nullptr;
-    VTRY(pinned(ctx, 4 * (size_t)n_parts, (void**)&h));
-    VCUDA(cudaMemcpyAsync(h, d_nr, 4 * (size_t)n_parts, cudaMemcpyDeviceToHost, ctx->stream));
-    VCUDA(stream_wait(ctx));
-    memcpy(nr.data(), h, 4 * (size_t)n_parts);
+    std::vector<PointOrder> order(n_parts);
+    for (int p = 0; p < n_parts; ++p) {
+      const bool masked = is_new && is_new[p];
+      order[p] = {reinterpret_cast<const float*>(base + o_pts[p]), n_pts[p],
+                  reinterpret_cast<uint32_t*>(base + o_perm[p]),
+                  masked ? reinterpret_cast<const uint8_t*>(base + o_mask[p]) : nullptr,
+                  reinterpret_cast<uint32_t*>(base + o_rows[p]), reinterpret_cast<int32_t*>(base + o_rank[p])};
+    }
+    VTRY(ensure_slot(ctx, kSlotCounters, sizeof(VisCounters)));
+    VTRY(ensure_slot(ctx, kSlotVisOrder, points_scratch(order.data(), n_parts)));
+    VTRY(points_order(ctx, order.data(), n_parts, slot<char>(ctx, kSlotVisOrder),
+                      slot<VisCounters>(ctx, kSlotCounters)));
   }
   // Part descriptors and the global work numbering.
   VTRY(ensure_slot(ctx, kSlotBitset, (size_t)std::max<unsigned long long>(words, 1) * 4));
@@ -991,7 +992,6 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
       P.nr = n;
       P.triangular = 1;
       P.ntr = ntr_tri[p];
-      P.row_start = reinterpret_cast<const unsigned long long*>(base + o_rs[p]);
       unsigned long long t = 0;
       for (int64_t r = 0; r < P.ntr; ++r) {
         const int64_t c = P.ntc - (r * TR) / TC;
@@ -1123,9 +1123,13 @@ int visibility_impl(visacd_ctx* ctx, const float* pts, int32_t n, const uint8_t*
   const float* d_pts = pts;
   const uint8_t* d_new = is_new;
   int64_t pairs = (int64_t)n * (n > 0 ? n - 1 : 0) / 2;
+  int32_t n_new = -1;
+  bvh_settle(ctx, self_bvh);
+  bvh_settle(ctx, cage_bvh);
   if (is_new && !device_ptrs) {
     int64_t k = 0;
     for (int32_t v = 0; v < n; ++v) k += is_new[v] != 0;
+    n_new = (int32_t)k;
     pairs -= ((int64_t)n - k) * ((int64_t)n - k - 1) / 2;
   }
   if (!device_ptrs && n > 0) {
@@ -1140,7 +1144,7 @@ int visibility_impl(visacd_ctx* ctx, const float* pts, int32_t n, const uint8_t*
       d_new = slot<uint8_t>(ctx, kSlotMask);
     }
   }
-  return vis_device(ctx, d_pts, n, d_new, self_bvh, cage_bvh, n_edges, stats, pairs);
+  return vis_device(ctx, d_pts, n, d_new, self_bvh, cage_bvh, n_edges, stats, pairs, n_new);
 }
 
 }  // namespace vgpu
