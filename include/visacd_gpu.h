@@ -69,7 +69,7 @@ typedef struct {
   int64_t n_edges;        /* visibility edges: cage hit and no self hit */
   int64_t self_hits;      /* pairs whose segment leaves the cage and crosses the part */
   int64_t cage_hits;      /* pairs whose segment leaves the cage (tested first) */
-  int64_t fp64_rechecks;  /* segment-triangle tests re-decided in FP64 */
+  int64_t fp64_rechecks;  /* segment-triangle tests FP32 left open (decided in double-float or FP64) */
   int64_t degenerate;     /* pairs with coincident endpoints (never edges) */
   int64_t node_visits;    /* BVH node records fetched (per warp packet) */
   int64_t tri_tests;      /* segment-triangle tests started (per segment) */
@@ -140,11 +140,13 @@ int visacd_measure_tex_peak(visacd_ctx* ctx, double* coherent_gfetch, double* di
 
 /* ---- BVH ---------------------------------------------------------------- */
 /* Linear BVH over a triangle mesh: 63-bit Morton codes of triangle centroids,
-   LSD radix sort, Karras (2012) hierarchy, bottom-up AABB fit. verts is nv x 3
+   LSD radix sort, Karras (2012) hierarchy, box fit. verts is nv x 3
    float32, tris is nt x 3 uint32 (indices < nv, else VISACD_ERR_INVALID_ARG).
    device_ptrs selects host or device input. The BVH keeps the vertex indices
    of every triangle so a visibility query can skip triangles incident to the
-   segment's endpoints. Synchronizes. */
+   segment's endpoints. Host input is copied before the call returns and the
+   build is left on the context's stream (calls that use the BVH wait for it);
+   device input is read before the call returns. */
 int visacd_bvh_build(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* tris,
                      int32_t nt, int device_ptrs, visacd_bvh** out);
 int visacd_bvh_destroy(visacd_bvh* bvh);
@@ -157,7 +159,8 @@ int visacd_bvh_info(const visacd_bvh* bvh, int32_t* n_tris, int32_t* depth);
    visibility edge iff the segment hits cage_bvh and does not hit self_bvh,
    where triangles of self_bvh incident to i or j are skipped (the end-vertex
    policy). Segment-triangle tests run in FP32 with a rigorous rounding bound;
-   tests inside the bound are re-decided in FP64. Edges are kept on the device
+   tests inside the bound are re-decided in higher precision, as FP64 decides
+   them. Edges are kept on the device
    in row-major (i, j) order; fetch them with visacd_visibility_edges*.
    Returns the edge count in *n_edges. Synchronizes. */
 int visacd_visibility(visacd_ctx* ctx, const float* pts, int32_t n, const uint8_t* is_new,

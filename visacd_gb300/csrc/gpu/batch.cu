@@ -28,12 +28,7 @@ struct BatchPart {
   const uint32_t* perm;
   const unsigned long long* row_start;
   unsigned long long tile_begin;
-  const float4* self_nodes;
-  const float4* self_tris;
-  int self_nt;
-  const float4* cage_nodes;
-  const float4* cage_tris;
-  int cage_nt;
+  TileMesh mesh;
   unsigned long long word_begin;
   unsigned long long nwords;
   int plane_begin;
@@ -61,7 +56,8 @@ __global__ void __launch_bounds__(kVisThreads, 6)
                             BatchCounters* __restrict__ cnt, unsigned* __restrict__ status) {
   constexpr int TC = 32 / TR;
   const int lane = threadIdx.x & 31;
-  unsigned rechecks = 0, status_bits = 0, visits = 0, tri_tests = 0;
+  __shared__ unsigned long long sums[kVisThreads / 32][kSums];  // (a batch reports no work counters)
+  unsigned status_bits = 0;
   for (int guard = 0; guard < (1 << 30); ++guard) {
     unsigned long long w = 0;
     if (lane == 0) w = atomicAdd(&cnt->work, 1ull);
@@ -92,19 +88,9 @@ __global__ void __launch_bounds__(kVisThreads, 6)
       p = make_float3(P.pts[3 * (int64_t)i], P.pts[3 * (int64_t)i + 1], P.pts[3 * (int64_t)i + 2]);
       q = make_float3(P.pts[3 * (int64_t)j], P.pts[3 * (int64_t)j + 1], P.pts[3 * (int64_t)j + 2]);
     }
-    Seg s;
-    make_seg(s, p, q, (int)i, (int)j);
-    bool active = valid && seg_len(s) > 0.f;
-    if (!__ballot_sync(0xffffffffu, active)) continue;
-    // The cage first; the self test only for segments that leave it.
-    s.exclude = false;
-    const bool cage_hit = packet_any_hit(P.cage_nodes, P.cage_tris, P.cage_nt, s, P.pts, active,
-                                         rechecks, status_bits, visits, tri_tests);
-    active = active && cage_hit;
-    s.exclude = true;
-    const bool self_hit = packet_any_hit(P.self_nodes, P.self_tris, P.self_nt, s, P.pts, active,
-                                         rechecks, status_bits, visits, tri_tests);
-    if (active && !self_hit) {
+    const bool active = valid && seg_length(__fsub_rn(q.x, p.x), __fsub_rn(q.y, p.y), __fsub_rn(q.z, p.z)) > 0.f;
+    if (!__any_sync(0xffffffffu, active)) continue;
+    if (trace_tile(P.mesh, P.pts, i, j, p, q, active, sums[threadIdx.x >> 5], status_bits) == 1u) {
       const int64_t k = row_start(i, P.n) + (int64_t)(j - i - 1);
       atomicOr(&bitset[P.word_begin + (k >> 5)], 1u << (k & 31));
     }
@@ -565,12 +551,7 @@ extern "C" int visacd_batch_create(visacd_ctx* ctx, int32_t n_parts, const float
     word_start[p] = b->total_words;
     P.nwords = (np + 31) / 32;
     b->total_words += P.nwords;
-    P.self_nodes = self_bvhs[p]->nodes;
-    P.self_tris = self_bvhs[p]->tris;
-    P.self_nt = self_bvhs[p]->nt;
-    P.cage_nodes = cage_bvhs[p]->nodes;
-    P.cage_tris = cage_bvhs[p]->tris;
-    P.cage_nt = cage_bvhs[p]->nt;
+    P.mesh = tile_mesh(ctx, self_bvhs[p], cage_bvhs[p]);
     P.plane_begin = (int)b->total_planes;
     plane_start[p] = (int)b->total_planes;
     P.P = n_planes[p];

@@ -11,9 +11,9 @@
 //     BVHs, octrees and k-d trees" — each internal node finds its key range and
 //     split from common-prefix lengths (ties broken by sorted position).
 //  5. aabb_fit: bottom-up union with one atomic arrival counter per node.
-//  6. node_layout: traversal records of 64 bytes (both child boxes with each
-//     axis stored as a (lo, hi) pair for packed f32x2 slab tests, + child ids)
-//     and leaf triangles of 48 bytes (3 vertices, vertex ids in .w).
+//  6. node_layout: traversal records of 64 bytes (centre and half extents of
+//     both child boxes + child ids) and leaf triangles of 48 bytes (3
+//     vertices, vertex ids in .w).
 #include "bvh.cuh"
 #include "order.cuh"
 
@@ -268,11 +268,7 @@ __global__ void node_layout_kernel(const int2* __restrict__ child,
     int2 ch = child[i];
     const float* lb = ch.x < 0 ? &leafbox[6 * (int64_t)(~ch.x)] : &nodebox[6 * (int64_t)ch.x];
     const float* rb = ch.y < 0 ? &leafbox[6 * (int64_t)(~ch.y)] : &nodebox[6 * (int64_t)ch.y];
-    // (lo, hi) per axis side by side: the traversal reads them as f32x2 pairs.
-    nodes[4 * (int64_t)i + 0] = make_float4(lb[0], lb[3], lb[1], lb[4]);
-    nodes[4 * (int64_t)i + 1] = make_float4(lb[2], lb[5], rb[0], rb[3]);
-    nodes[4 * (int64_t)i + 2] = make_float4(rb[1], rb[4], rb[2], rb[5]);
-    nodes[4 * (int64_t)i + 3] = make_float4(__int_as_float(ch.x), __int_as_float(ch.y), 0.f, 0.f);
+    node_record(nodes, i, lb, rb, ch.x, ch.y);
   }
 }
 
@@ -438,7 +434,8 @@ int bvh_build(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* t
   b->stream = ctx->stream;
   const size_t o_tris = ((size_t)n_int * 64 + 255) & ~size_t(255);
   char* mem = nullptr;
-  if (cudaMallocAsync((void**)&mem, o_tris + (size_t)nt * 48, ctx->stream) != cudaSuccess) {
+  const size_t o_head = o_tris + (((size_t)nt * 48 + 255) & ~size_t(255));
+  if (cudaMallocAsync((void**)&mem, o_head + sizeof(BvhHead), ctx->stream) != cudaSuccess) {
     cudaGetLastError();
     delete b;
     set_error("bvh_build: device allocation failed");
@@ -446,6 +443,9 @@ int bvh_build(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* t
   }
   b->nodes = reinterpret_cast<float4*>(mem);
   b->tris = reinterpret_cast<float4*>(mem + o_tris);
+  b->head = mem + o_head;
+  VCUDA(cudaMemcpyAsync(&reinterpret_cast<BvhHead*>(b->head)->amax, &cnt->amax, 4, cudaMemcpyDeviceToDevice,
+                        ctx->stream));
   VLAUNCH(ctx, kKNodeLayout, g, 256, 0, leaf_kernel, dv, nv, dt, vals, nt, cnt, b->tris, leafbox);
   const unsigned gi = grid_for(n_int, 256, 8LL * ctx->sm_count);
   VLAUNCH(ctx, kKKarras, gi, 256, 0, karras_kernel, keys, nt, child, pint, pleaf);

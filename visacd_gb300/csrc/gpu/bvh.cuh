@@ -5,10 +5,11 @@
 
 #include "common.cuh"
 
-// Node record (64 bytes, 4 x float4), each axis a (lo, hi) pair:
-//   [0] L.lo.x L.hi.x L.lo.y L.hi.y
-//   [1] L.lo.z L.hi.z R.lo.x R.hi.x
-//   [2] R.lo.y R.hi.y R.lo.z R.hi.z
+// Node record (64 bytes, 4 x float4): centre c and half extents e of both
+// children's boxes, then the children.
+//   [0] L.c.x L.c.y L.c.z L.e.x
+//   [1] L.e.y L.e.z R.c.x R.c.y
+//   [2] R.c.z R.e.x R.e.y R.e.z
 //   [3] left  right  (int bits; >= 0 internal node, < 0 leaf ~sorted_triangle)
 // Leaf triangle record (48 bytes, 3 x float4): vertex xyz + vertex index bits.
 struct visacd_bvh {
@@ -37,6 +38,32 @@ struct visacd_bvh {
 };
 
 namespace vgpu {
+
+#ifdef __CUDACC__
+// The record of a node whose children's boxes are (lo xyz, hi xyz): c - e and
+// c + e enclose them (e rounded up).
+__device__ __forceinline__ void node_record(float4* __restrict__ nodes, int64_t i, const float* l, const float* r,
+                                            int left, int right) {
+  float lc[3], le[3], rc[3], re[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    lc[a] = 0.5f * l[a] + 0.5f * l[3 + a];
+    le[a] = fmaxf(__fsub_ru(l[3 + a], lc[a]), __fsub_ru(lc[a], l[a]));
+    rc[a] = 0.5f * r[a] + 0.5f * r[3 + a];
+    re[a] = fmaxf(__fsub_ru(r[3 + a], rc[a]), __fsub_ru(rc[a], r[a]));
+  }
+  nodes[4 * i + 0] = make_float4(lc[0], lc[1], lc[2], le[0]);
+  nodes[4 * i + 1] = make_float4(le[1], le[2], rc[0], rc[1]);
+  nodes[4 * i + 2] = make_float4(rc[2], re[0], re[1], re[2]);
+  nodes[4 * i + 3] = make_float4(__int_as_float(left), __int_as_float(right), 0.f, 0.f);
+}
+#endif
+
+// Device address of a mesh's largest |coordinate| (for a mesh without
+// triangles a word that is never needed).
+inline const float* bvh_amax(const visacd_ctx* ctx, const visacd_bvh* b) {
+  return b->head ? reinterpret_cast<const float*>(b->head) + 6 : reinterpret_cast<const float*>(ctx->d_status);
+}
 
 int bvh_build(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* tris, int32_t nt,
               int device_ptrs, visacd_bvh** out);

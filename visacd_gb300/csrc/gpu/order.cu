@@ -7,8 +7,8 @@
 // separate launches the same steps took 8 (up to 32,768 triangles) to 20
 // launches plus a read-back the host waited for, and the sort ran on one SM.
 // A cluster of 8 CTAs cuts the sort's serial chain by 8 and needs no spin
-// barrier; a single CTA serves up to kOrderSmall primitives, where the cluster
-// barrier costs more than it saves.
+// barrier; a single CTA serves up to kOrderSmall primitives and ranks the keys
+// by counting up to kOrderRank (no passes).
 //
 // The sort is stable on exactly the Morton bits and starts from index order, so
 // the order is that of radix_sort_u64 on the same codes.
@@ -29,7 +29,8 @@ namespace {
 constexpr int kOrderThreads = 1024;
 constexpr int kOrderWarps = kOrderThreads / 32;
 constexpr int kOrderCluster = 8;
-constexpr int kOrderSmall = 2048;
+constexpr int kOrderSmall = 2048;  // primitives one CTA serves
+constexpr int kOrderRank = 512;    // of those, ranked by counting instead of sorted
 
 struct OrderArgs {
   OrderJob job[kOrderMaxJobs];
@@ -90,26 +91,70 @@ __device__ __forceinline__ void warp_unions(const float (&b)[6], float (&pre)[6]
   }
 }
 
-// Exclusive prefix over the block's first 256 threads' values.
-__device__ __forceinline__ uint32_t prefix256(uint32_t v, uint32_t* wsum) {
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint32_t x = v;
+// Group g of 1024 leaves in order, by a block of 1024 threads: the leaf
+// records, their boxes and the tables of unions; one run of 32 per warp.
+__device__ __forceinline__ void order_leaves(const OrderJob& J, int g, float amax, float (&sum)[kOrderWarps][6]) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = 1024 * g + (int)threadIdx.x;
+  const float pad = amax * 1.9073486e-6f + 1e-30f;  // 2^-19 * max|coord|
+  float b[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
+  if (i < J.n) {
+    const uint32_t t = __ldcg(&J.v0[i]);
 #pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-    if (lane >= o) x += y;
+    for (int k = 0; k < 3; ++k) {
+      const uint32_t id = J.tris[3 * (int64_t)t + k];
+      const uint32_t vi = id < (uint32_t)J.nv ? id : 0u;
+      const float x = J.verts[3 * (int64_t)vi], y = J.verts[3 * (int64_t)vi + 1], z = J.verts[3 * (int64_t)vi + 2];
+      J.leaves[3 * (int64_t)i + k] = make_float4(x, y, z, __int_as_float((int)id));
+      b[0] = fminf(b[0], x);
+      b[1] = fminf(b[1], y);
+      b[2] = fminf(b[2], z);
+      b[3] = fmaxf(b[3], x);
+      b[4] = fmaxf(b[4], y);
+      b[5] = fmaxf(b[5], z);
+    }
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      b[a] -= pad;
+      b[3 + a] += pad;
+    }
+    box_store(J.box + 6 * (int64_t)i, b);
   }
-  if (warp < 8 && lane == 31) wsum[warp] = x;
+  float pre[6], suf[6];
+  warp_unions(b, pre, suf);
+  if (i < J.n) {
+    box_store(J.pre + 6 * (int64_t)i, pre);
+    box_store(J.suf + 6 * (int64_t)i, suf);
+  }
+  __syncthreads();  // the sums of a previous group are read
+  if (lane == 31) {
+#pragma unroll
+    for (int a = 0; a < 6; ++a) sum[warp][a] = pre[a];
+  }
   __syncthreads();
-  uint32_t before = 0;
-  for (int w = 0; w < 8; ++w)
-    if (w < warp) before += wsum[w];
-  return before + x - v;
+  if (warp == 0) {
+#pragma unroll
+    for (int a = 0; a < 6; ++a) b[a] = sum[lane][a];
+    warp_unions(b, pre, suf);
+    const int r = 32 * g + lane;
+    if (32 * r < J.n) {
+      box_store(J.bpre + 6 * (int64_t)r, pre);
+      box_store(J.bsuf + 6 * (int64_t)r, suf);
+    }
+    if (lane == 31) box_store(J.group + 6 * (int64_t)g, pre);
+  }
+}
+
+// The leaves of a job a cluster sorted: one block per group (inside the
+// cluster the groups would run one after another, 6.6 us each).
+__global__ void __launch_bounds__(kOrderThreads) order_leaves_kernel(const __grid_constant__ OrderJob J) {
+  __shared__ float sum[kOrderWarps][6];
+  order_leaves(J, (int)blockIdx.x, J.head->amax, sum);
 }
 
 __global__ void __launch_bounds__(kOrderThreads) order_kernel(const __grid_constant__ OrderArgs A) {
-  __shared__ uint32_t cnt[kOrderWarps][256];
+  __shared__ __align__(16) uint32_t cnt[kOrderWarps][256];
   __shared__ float red[kOrderWarps][14];
+  __shared__ float sum[kOrderWarps][6];
   __shared__ float bnd[14];
   __shared__ uint32_t wsum[kOrderWarps];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -129,11 +174,17 @@ __global__ void __launch_bounds__(kOrderThreads) order_kernel(const __grid_const
   }
   s[12] = s[13] = 0.f;
   if (is_tri) {
-    for (int64_t i = (int64_t)rank * kOrderThreads + tid; i < 3LL * J.nv; i += (int64_t)C * kOrderThreads) {
-      const float x = fabsf(J.verts[i]);
-      if (x < INFINITY) s[12] = fmaxf(s[12], x);
+    const int64_t m = 3LL * J.nv, step = (int64_t)C * kOrderThreads;
+    for (int64_t i = (int64_t)rank * kOrderThreads + tid; i < m; i += 4 * step) {
+      float x[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) x[q] = i + q * step < m ? fabsf(J.verts[i + q * step]) : 0.f;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        if (x[q] < INFINITY) s[12] = fmaxf(s[12], x[q]);
     }
   }
+#pragma unroll 2
   for (int i = c0 + tid; i < c1; i += kOrderThreads) {
     float c[3];
     if (is_tri) {
@@ -225,123 +276,147 @@ __global__ void __launch_bounds__(kOrderThreads) order_kernel(const __grid_const
     }
   }
   __syncthreads();
-  // ---- stable LSD passes: warp w owns a contiguous run of the CTA's chunk.
   const int run = (c1 - c0 + kOrderWarps - 1) / kOrderWarps;
   const int b0 = min(c1, c0 + warp * run), b1 = min(c1, b0 + run);
   const unsigned lt = (1u << lane) - 1u;
-  uint32_t* my = cnt[warp];
-  for (int p = 0; p < passes; ++p) {
-    const int shift = 8 * p;
-    uint32_t* hist = J.hist + (size_t)(p & 1) * C * 256;
-    for (int d = lane; d < 256; d += 32) my[d] = 0;
-    __syncwarp();
-    for (int i = b0 + lane; i < b1; i += 32) atomicAdd(&my[(__ldcg(&ks[i]) >> shift) & 255u], 1u);
+  if (n <= kOrderRank) {
+    // ---- small jobs: every key's rank is the number of keys before it in
+    // (key, index) order, counted over the keys in shared memory.
+    uint32_t* sk = &cnt[0][0];
+    const int pad = (n + 3) & ~3;
+    const uint32_t own = tid < n ? __ldcg(&ks[tid]) : 0xffffffffu;
+    if (tid < pad) sk[tid] = own;
     __syncthreads();
-    uint32_t tot = 0;
-    if (tid < 256) {
-      for (int w = 0; w < kOrderWarps; ++w) tot += cnt[w][tid];
-      if (C > 1) hist[rank * 256 + tid] = tot;
-    }
-    uint32_t all = tot, before = 0;
-    if (C > 1) {
-      cluster_barrier();
-      if (tid < 256) {
-        all = 0;
-        for (int r = 0; r < C; ++r) {
-          const uint32_t h = r == rank ? tot : __ldcg(&hist[r * 256 + tid]);
-          if (r < rank) before += h;
-          all += h;
-        }
+    if (32 * warp < n) {
+      int rk = 0;
+      for (int j = 0; j < pad; j += 4) {
+        // (the padding keys are above every key)
+        const uint4 o = *reinterpret_cast<const uint4*>(sk + j);
+        rk += (o.x < own || (o.x == own && j < tid)) + (o.y < own || (o.y == own && j + 1 < tid)) +
+              (o.z < own || (o.z == own && j + 2 < tid)) + (o.w < own || (o.w == own && j + 3 < tid));
+      }
+      // (every key was read before the barrier: source and destination may be
+      // the same buffer)
+      if (tid < n) {
+        J.k0[rk] = own;
+        J.v0[rk] = (uint32_t)tid;
       }
     }
-    const uint32_t first = prefix256(tid < 256 ? all : 0u, wsum);
-    if (tid < 256) {
-      uint32_t at = first + before;
-      for (int w = 0; w < kOrderWarps; ++w) {
-        const uint32_t c = cnt[w][tid];
-        cnt[w][tid] = at;
-        at += c;
-      }
-    }
+    vs = J.v0;
     __syncthreads();
-    for (int base = b0; base < b1; base += 32) {
-      const int i = base + lane;
-      const bool valid = i < b1;
-      const uint32_t k = valid ? __ldcg(&ks[i]) : 0u, v = valid ? __ldcg(&vs[i]) : 0u;
-      const uint32_t digit = valid ? (k >> shift) & 255u : 0xffffffffu;
-      const unsigned peers = __match_any_sync(0xffffffffu, digit);
-      if (valid) {
-        const uint32_t pos = my[digit] + __popc(peers & lt);
-        kd[pos] = k;
-        vd[pos] = v;
-      }
-      __syncwarp();
-      if (valid && (peers & lt) == 0) my[digit] += __popc(peers);
-      __syncwarp();
-    }
-    if (C > 1) cluster_barrier();
-    else __syncthreads();
-    uint32_t* t = ks;
-    ks = kd;
-    kd = t;
-    t = vs;
-    vs = vd;
-    vd = t;
-  }
-  if (is_tri) {
-    // ---- leaves in order and the tables of unions, 1024 leaves (one group)
-    // at a time, one run of 32 per warp.
-    const float pad = bnd[12] * 1.9073486e-6f + 1e-30f;  // 2^-19 * max|coord|
-    __shared__ float rb[kOrderWarps][6];
-    for (int g0 = rank * 1024; g0 < n; g0 += C * 1024) {
-      const int i = g0 + tid;
-      float b[6] = {INFINITY, INFINITY, INFINITY, -INFINITY, -INFINITY, -INFINITY};
-      if (i < n) {
-        const uint32_t t = __ldcg(&vs[i]);
+  } else {
+    // ---- stable LSD passes: warp w owns a contiguous run of the CTA's chunk,
+    // kept in registers over a pass when it fits (up to 65536 primitives).
+    constexpr int kHold = 8;
+    uint32_t* my = cnt[warp];
+    for (int p = 0; p < passes; ++p) {
+      const int shift = 8 * p;
+      uint32_t* hist = J.hist + (size_t)(p & 1) * C * 256;
+      const bool hold = run <= 32 * kHold;
+      uint32_t hk[kHold], hv[kHold];
+      if (hold) {
 #pragma unroll
-        for (int k = 0; k < 3; ++k) {
-          const uint32_t id = J.tris[3 * (int64_t)t + k];
-          const uint32_t vi = id < (uint32_t)J.nv ? id : 0u;
-          const float x = J.verts[3 * (int64_t)vi], y = J.verts[3 * (int64_t)vi + 1], z = J.verts[3 * (int64_t)vi + 2];
-          J.leaves[3 * (int64_t)i + k] = make_float4(x, y, z, __int_as_float((int)id));
-          b[0] = fminf(b[0], x);
-          b[1] = fminf(b[1], y);
-          b[2] = fminf(b[2], z);
-          b[3] = fmaxf(b[3], x);
-          b[4] = fmaxf(b[4], y);
-          b[5] = fmaxf(b[5], z);
+        for (int q = 0; q < kHold; ++q) {
+          const int i = b0 + 32 * q + lane;
+          hk[q] = i < b1 ? __ldcg(&ks[i]) : 0u;
+          hv[q] = i < b1 ? __ldcg(&vs[i]) : 0u;
         }
-#pragma unroll
-        for (int a = 0; a < 3; ++a) {
-          b[a] -= pad;
-          b[3 + a] += pad;
-        }
-        box_store(J.box + 6 * (int64_t)i, b);
       }
-      float pre[6], suf[6];
-      warp_unions(b, pre, suf);
-      if (i < n) {
-        box_store(J.pre + 6 * (int64_t)i, pre);
-        box_store(J.suf + 6 * (int64_t)i, suf);
-      }
-      __syncthreads();  // rb of the previous group is read
-      if (lane == 31) {
+      for (int d = lane; d < 256; d += 32) my[d] = 0;
+      __syncwarp();
+      if (hold) {
 #pragma unroll
-        for (int a = 0; a < 6; ++a) rb[warp][a] = pre[a];
+        for (int q = 0; q < kHold; ++q)
+          if (b0 + 32 * q + lane < b1) atomicAdd(&my[(hk[q] >> shift) & 255u], 1u);
+      } else {
+        for (int i = b0 + lane; i < b1; i += 32) atomicAdd(&my[(__ldcg(&ks[i]) >> shift) & 255u], 1u);
       }
       __syncthreads();
-      if (warp == 0) {
+      // Digit d's count over the warps: four threads a digit, eight warps each.
+      const int d = tid >> 2, w0 = (tid & 3) * 8;
+      uint32_t part = 0;
 #pragma unroll
-        for (int a = 0; a < 6; ++a) b[a] = rb[lane][a];
-        warp_unions(b, pre, suf);
-        const int r = (g0 >> 5) + lane;
-        if (32 * r < n) {
-          box_store(J.bpre + 6 * (int64_t)r, pre);
-          box_store(J.bsuf + 6 * (int64_t)r, suf);
-        }
-        if (lane == 31) box_store(J.group + 6 * (int64_t)(g0 >> 10), pre);
+      for (int w = 0; w < 8; ++w) part += cnt[w0 + w][d];
+      uint32_t upto = part;  // inclusive over the four
+      {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, upto, 1, 4);
+        if ((tid & 3) >= 1) upto += y;
+        const uint32_t z = __shfl_up_sync(0xffffffffu, upto, 2, 4);
+        if ((tid & 3) >= 2) upto += z;
       }
+      const uint32_t tot = __shfl_sync(0xffffffffu, upto, 3, 4);
+      uint32_t all = tot, before = 0;
+      if (C > 1) {
+        if ((tid & 3) == 0) hist[rank * 256 + d] = tot;
+        cluster_barrier();
+        // Counts of this digit in all CTAs: two ranks a thread of the four.
+        all = 0;
+        for (int r = tid & 3; r < C; r += 4) {
+          const uint32_t h = __ldcg(&hist[r * 256 + d]);
+          all += h;
+          if (r < rank) before += h;
+        }
+        all += __shfl_xor_sync(0xffffffffu, all, 1);
+        all += __shfl_xor_sync(0xffffffffu, all, 2);
+        before += __shfl_xor_sync(0xffffffffu, before, 1);
+        before += __shfl_xor_sync(0xffffffffu, before, 2);
+      }
+      // Exclusive prefix over the digits (a digit's four threads hold the same).
+      uint32_t x = (tid & 3) == 0 ? all : 0u;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+      }
+      if (lane == 31) wsum[warp] = x;
+      x = __shfl_sync(0xffffffffu, x, lane & ~3);  // through the digit's first thread
+      __syncthreads();
+      uint32_t first = lane < warp ? wsum[lane] : 0u;
+#pragma unroll
+      for (int o = 16; o; o >>= 1) first += __shfl_xor_sync(0xffffffffu, first, o);
+      uint32_t at = first + x - all + before + upto - part;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) {
+        const uint32_t c = cnt[w0 + w][d];
+        cnt[w0 + w][d] = at;
+        at += c;
+      }
+      __syncthreads();
+      auto place = [&](bool valid, uint32_t k, uint32_t v) {
+        const uint32_t digit = valid ? (k >> shift) & 255u : 0xffffffffu;
+        const unsigned peers = __match_any_sync(0xffffffffu, digit);
+        if (valid) {
+          const uint32_t pos = my[digit] + __popc(peers & lt);
+          kd[pos] = k;
+          vd[pos] = v;
+        }
+        __syncwarp();
+        if (valid && (peers & lt) == 0) my[digit] += __popc(peers);
+        __syncwarp();
+      };
+      if (hold) {
+#pragma unroll
+        for (int q = 0; q < kHold; ++q)
+          if (b0 + 32 * q < b1) place(b0 + 32 * q + lane < b1, hk[q], hv[q]);
+      } else {
+        for (int base = b0; base < b1; base += 32) {
+          const int i = base + lane;
+          place(i < b1, i < b1 ? __ldcg(&ks[i]) : 0u, i < b1 ? __ldcg(&vs[i]) : 0u);
+        }
+      }
+      if (C > 1) cluster_barrier();
+      else __syncthreads();
+      uint32_t* t = ks;
+      ks = kd;
+      kd = t;
+      t = vs;
+      vs = vd;
+      vd = t;
     }
+  }
+  if (is_tri) {
+    if (C == 1)
+      for (int g = 0; 1024 * g < n; ++g) order_leaves(J, g, bnd[12], sum);
   } else if (J.is_new) {
     // ---- the new points in order (rows), and every point's rank among them.
     int c = 0;
@@ -424,15 +499,6 @@ __device__ __forceinline__ int key_delta(const uint32_t* __restrict__ k, int n, 
   return __clz(a ^ b);
 }
 
-__device__ __forceinline__ void node_store(float4* __restrict__ nodes, int i, const float (&l)[6], const float (&r)[6],
-                                           int left, int right) {
-  // (lo, hi) per axis side by side: the traversal reads them as f32x2 pairs.
-  nodes[4 * (int64_t)i + 0] = make_float4(l[0], l[3], l[1], l[4]);
-  nodes[4 * (int64_t)i + 1] = make_float4(l[2], l[5], r[0], r[3]);
-  nodes[4 * (int64_t)i + 2] = make_float4(r[1], r[4], r[2], r[5]);
-  nodes[4 * (int64_t)i + 3] = make_float4(__int_as_float(left), __int_as_float(right), 0.f, 0.f);
-}
-
 // Internal node i of Karras (2012): its range from the common-prefix lengths,
 // its split, both children's boxes and the traversal record, one thread each.
 __global__ void __launch_bounds__(128) order_nodes_kernel(const __grid_constant__ OrderJob J,
@@ -443,7 +509,7 @@ __global__ void __launch_bounds__(128) order_nodes_kernel(const __grid_constant_
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       float b[6];
       order_box(J, 0, 0, b);
-      node_store(nodes, 0, b, b, ~0, ~0);
+      node_record(nodes, 0, b, b, ~0, ~0);
     }
     return;
   }
@@ -467,7 +533,7 @@ __global__ void __launch_bounds__(128) order_nodes_kernel(const __grid_constant_
     float lb[6], rb[6];
     order_box(J, lo, gamma, lb);
     order_box(J, gamma + 1, hi, rb);
-    node_store(nodes, i, lb, rb, lo == gamma ? ~gamma : gamma, hi == gamma + 1 ? ~(gamma + 1) : gamma + 1);
+    node_record(nodes, i, lb, rb, lo == gamma ? ~gamma : gamma, hi == gamma + 1 ? ~(gamma + 1) : gamma + 1);
   }
 }
 
@@ -541,6 +607,8 @@ int order_run(visacd_ctx* ctx, const OrderJob* jobs, int n_jobs) {
 }
 
 int order_nodes(visacd_ctx* ctx, const OrderJob& j, float4* nodes) {
+  if (j.n > kOrderSmall)
+    VLAUNCH(ctx, kKNodeLayout, (unsigned)((j.n + 1023) / 1024), kOrderThreads, 0, order_leaves_kernel, j);
   VLAUNCH(ctx, kKKarras, grid_for(j.n > 1 ? j.n - 1 : 1, 128, 32LL * ctx->sm_count), 128, 0, order_nodes_kernel, j,
           nodes);
   return VISACD_OK;

@@ -17,15 +17,13 @@ __global__ void seg_tri_kernel(const float* __restrict__ seg, const float* __res
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < S; k += (int64_t)gridDim.x * blockDim.x) {
     const float* sp = seg + 6 * k;
     const float* t = tri + 9 * k;
-    Seg s;
-    make_seg(s, make_float3(sp[0], sp[1], sp[2]), make_float3(sp[3], sp[4], sp[5]), -1, -1);
-    s.exclude = false;
+    const float3 p = make_float3(sp[0], sp[1], sp[2]), q = make_float3(sp[3], sp[4], sp[5]);
     const float4 a = make_float4(t[0], t[1], t[2], 0.f), b = make_float4(t[3], t[4], t[5], 0.f),
                  c = make_float4(t[6], t[7], t[8], 0.f);
-    int r = tri_test32(s, a, b, c);
+    int r = tri_test32(p, q, a, b, c);
     if (r == 2) {
       ++rechecks;
-      r = tri_test64(sp[0], sp[1], sp[2], sp[3], sp[4], sp[5], a, b, c) ? 1 : 0;
+      r = tri_recheck(p.x, p.y, p.z, q.x, q.y, q.z, a, b, c) ? 1 : 0;
     }
     out[k] = (uint8_t)r;
   }

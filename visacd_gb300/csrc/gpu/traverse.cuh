@@ -82,12 +82,15 @@ __device__ __forceinline__ bool trace_free(const FreeGridView& g, float px, floa
   return false;
 }
 
+// What the traversal keeps of a lane's segment p -> q (d = q - p rounded): per
+// axis 1 / d, |1 / d| and -p / d. A box test is then three FMAs per axis; the
+// points themselves are read again at the (few) leaf tests, which leaves the
+// registers to the traversal.
 struct Seg {
-  unsigned long long ox2, oy2, oz2;  // (o, o) pairs for packed slab tests
-  unsigned long long ix2, iy2, iz2;  // (1/d, 1/d) pairs
-  float dx, dy, dz;
-  float kw;      // Ew = kw * L^2
-  int vi, vj;    // endpoint vertex ids (q = pts[vj])
+  float ix, iy, iz;
+  float ax, ay, az;
+  float nx, ny, nz;
+  int vi, vj;    // endpoint vertex ids (p = pts[vi], q = pts[vj])
   bool exclude;  // skip triangles incident to vi or vj (self test)
 };
 
@@ -111,76 +114,69 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
   return r;
 }
 
-__device__ __forceinline__ unsigned long long pk2(float a, float b) {
-  unsigned long long r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
-  return r;
-}
-__device__ __forceinline__ float lo2(unsigned long long v) {
-  float a, b;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-  return a;
-}
-__device__ __forceinline__ void up2(unsigned long long v, float& a, float& b) {
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(v));
-}
-__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-__device__ __forceinline__ unsigned long long mul2(unsigned long long a, unsigned long long b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
-  return r;
-}
-
 __device__ __forceinline__ float inv_guard(float d) {
   float ad = fabsf(d);
   float g = ad < 1e-30f ? copysignf(1e-30f, d) : d;
   return __frcp_rn(g);
 }
 
+__device__ __forceinline__ float edge_factor(float dx, float dy, float dz) {
+  const float d1 = fabsf(dx) + fabsf(dy) + fabsf(dz);
+  return 17.0f * kU * d1 * (1.0f + 4.0f * kU);
+}
+__device__ __forceinline__ float seg_length(float dx, float dy, float dz) {
+  return __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
+}
+
 __device__ __forceinline__ void make_seg(Seg& s, float3 p, float3 q, int vi, int vj) {
-  s.ox2 = pk2(p.x, p.x);
-  s.oy2 = pk2(p.y, p.y);
-  s.oz2 = pk2(p.z, p.z);
-  s.dx = __fsub_rn(q.x, p.x);
-  s.dy = __fsub_rn(q.y, p.y);
-  s.dz = __fsub_rn(q.z, p.z);
-  float ix = inv_guard(s.dx), iy = inv_guard(s.dy), iz = inv_guard(s.dz);
-  s.ix2 = pk2(ix, ix);
-  s.iy2 = pk2(iy, iy);
-  s.iz2 = pk2(iz, iz);
-  float d1 = fabsf(s.dx) + fabsf(s.dy) + fabsf(s.dz);
-  s.kw = 17.0f * kU * d1 * (1.0f + 4.0f * kU);
+  s.ix = inv_guard(__fsub_rn(q.x, p.x));
+  s.iy = inv_guard(__fsub_rn(q.y, p.y));
+  s.iz = inv_guard(__fsub_rn(q.z, p.z));
+  s.ax = fabsf(s.ix);
+  s.ay = fabsf(s.iy);
+  s.az = fabsf(s.iz);
+  s.nx = -(p.x * s.ix);
+  s.ny = -(p.y * s.iy);
+  s.nz = -(p.z * s.iz);
   s.vi = vi;
   s.vj = vj;
   s.exclude = true;
 }
 
-__device__ __forceinline__ float seg_len(const Seg& s) {
-  return __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(s.dx, s.dx), __fmul_rn(s.dy, s.dy)),
-                              __fmul_rn(s.dz, s.dz)));
+// Conservative slab test of the segment (t in [0, 1]) against the box with
+// centre c and half extents e. Leaf boxes are widened by 2^-19 of the mesh's
+// largest |coordinate| M, 32 units of FP32 rounding; with |p|, |q| <= 4 M the
+// test's own error is below 21 units (in position: one of |p| for p / d, one
+// each of the two FMA results, one of |x - p| for 1 / d), so no slack is
+// needed. box_hit_wide serves points farther out.
+__device__ __forceinline__ bool box_hit(const Seg& s, float cx, float cy, float cz, float ex, float ey, float ez) {
+  const float tx = fmaf(cx, s.ix, s.nx), ty = fmaf(cy, s.iy, s.ny), tz = fmaf(cz, s.iz, s.nz);
+  const float tn = max3f(fmaf(-ex, s.ax, tx), fmaf(-ey, s.ay, ty), fmaxf(fmaf(-ez, s.az, tz), 0.f));
+  const float tf = min3f(fmaf(ex, s.ax, tx), fmaf(ey, s.ay, ty), fminf(fmaf(ez, s.az, tz), 1.f));
+  return tn <= tf;
 }
-
-// Conservative slab test of the segment (t in [0, 1]) against a box given as
-// (lo, hi) pairs per axis; one packed sub + mul per axis.
-__device__ __forceinline__ bool box_hit(const Seg& s, unsigned long long bx, unsigned long long by,
-                                        unsigned long long bz) {
-  float t0x, t1x, t0y, t1y, t0z, t1z;
-  up2(mul2(sub2(bx, s.ox2), s.ix2), t0x, t1x);
-  up2(mul2(sub2(by, s.oy2), s.iy2), t0y, t1y);
-  up2(mul2(sub2(bz, s.oz2), s.iz2), t0z, t1z);
-  float tn = max3f(fminf(t0x, t1x), fminf(t0y, t1y), fmaxf(fminf(t0z, t1z), 0.f));
+__device__ __forceinline__ bool box_hit_wide(const Seg& s, const float3& p, float cx, float cy, float cz, float ex,
+                                             float ey, float ez) {
+  const float t0x = __fmul_rn(__fsub_rn(__fsub_rd(cx, ex), p.x), s.ix), t1x = __fmul_rn(__fsub_rn(__fadd_ru(cx, ex), p.x), s.ix);
+  const float t0y = __fmul_rn(__fsub_rn(__fsub_rd(cy, ey), p.y), s.iy), t1y = __fmul_rn(__fsub_rn(__fadd_ru(cy, ey), p.y), s.iy);
+  const float t0z = __fmul_rn(__fsub_rn(__fsub_rd(cz, ez), p.z), s.iz), t1z = __fmul_rn(__fsub_rn(__fadd_ru(cz, ez), p.z), s.iz);
+  const float tn = max3f(fminf(t0x, t1x), fminf(t0y, t1y), fmaxf(fminf(t0z, t1z), 0.f));
   float tf = min3f(fmaxf(t0x, t1x), fmaxf(t0y, t1y), fminf(fmaxf(t0z, t1z), 1.f));
   tf = fmaf(fabsf(tf), 4e-6f, tf);
   return tn <= tf;
 }
+// Whether box_hit serves a segment against a mesh whose largest |coordinate|
+// is amax (also false for coordinates that are not finite).
+__device__ __forceinline__ bool box_test_holds(float3 p, float3 q, float amax) {
+  const float m = fmaxf(fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fmaxf(fabsf(p.z), fabsf(q.x))),
+                        fmaxf(fabsf(q.y), fabsf(q.z)));
+  // (fmax drops NaNs: those fail the sum)
+  return amax <= 1e7f && m <= 4.f * amax && fabsf(p.x + p.y + p.z + q.x + q.y + q.z) < INFINITY;
+}
 
 // FP64 segment-triangle decision from the FP32 inputs; identical formula to the
 // oracle. Explicit round-to-nearest intrinsics keep contraction out.
-static __device__ __noinline__ bool tri_test64(float ox, float oy, float oz, float qx, float qy, float qz,
+static __device__ bool tri_test64(float ox, float oy, float oz, float qx, float qy, float qz,
                                         float4 a, float4 b, float4 c) {
   double Ax = __dsub_rn(a.x, ox), Ay = __dsub_rn(a.y, oy), Az = __dsub_rn(a.z, oz);
   double Bx = __dsub_rn(b.x, ox), By = __dsub_rn(b.y, oy), Bz = __dsub_rn(b.z, oz);
@@ -211,9 +207,99 @@ static __device__ __noinline__ bool tri_test64(float ox, float oy, float oz, flo
   return lhs <= rhs && vol >= det;
 }
 
-// FP32 filter: 1 certain hit, 0 certain miss, 2 undecided (needs FP64).
-__device__ __forceinline__ int tri_test32(const Seg& s, float4 a, float4 b, float4 c) {
-  const float ox = lo2(s.ox2), oy = lo2(s.oy2), oz = lo2(s.oz2);
+// ---- double-float arithmetic: a value as the unevaluated sum h + l of two
+// FP32 numbers (about 46 bits). GB300 does about two FP64 operations per clock
+// and SM, so the tests the FP32 filter leaves open go through these first.
+struct DF {
+  float h, l;
+};
+// a - b, exactly (Knuth's two-sum).
+__device__ __forceinline__ DF df_diff(float a, float b) {
+  const float s = __fsub_rn(a, b), t = __fsub_rn(s, a);
+  return {s, __fsub_rn(__fsub_rn(a, __fsub_rn(s, t)), __fadd_rn(b, t))};
+}
+__device__ __forceinline__ DF df_norm(float h, float l) {  // |h| >= |l| or h == 0
+  const float s = __fadd_rn(h, l);
+  return {s, __fsub_rn(l, __fsub_rn(s, h))};
+}
+// x y within 2^-44 |x y|.
+__device__ __forceinline__ DF df_mul(DF x, DF y) {
+  const float p = __fmul_rn(x.h, y.h);
+  const float e = __fmaf_rn(x.h, y.l, __fmaf_rn(x.l, y.h, __fmaf_rn(x.h, y.h, -p)));
+  return df_norm(p, e);
+}
+// x + y within 2^-44 (|x| + |y|).
+__device__ __forceinline__ DF df_add(DF x, DF y) {
+  const float s = __fadd_rn(x.h, y.h), t = __fsub_rn(s, x.h);
+  const float e = __fadd_rn(__fsub_rn(x.h, __fsub_rn(s, t)), __fsub_rn(y.h, t));
+  return df_norm(s, __fadd_rn(e, __fadd_rn(x.l, y.l)));
+}
+__device__ __forceinline__ DF df_neg(DF x) { return {-x.h, -x.l}; }
+// a b - c d, and the product of the vectors a . b.
+__device__ __forceinline__ DF df_det(DF a, DF b, DF c, DF d) { return df_add(df_mul(a, b), df_neg(df_mul(c, d))); }
+__device__ __forceinline__ DF df_dot(DF ax, DF ay, DF az, DF bx, DF by, DF bz) {
+  return df_add(df_add(df_mul(ax, bx), df_mul(ay, by)), df_mul(az, bz));
+}
+
+// The segment-triangle decision in double-float: 1 hit, 0 miss, 2 undecided.
+// With L the largest component of the vertex vectors and |D| the 1-norm of the
+// direction, the differences are exact, a component of a cross product is
+// within 2^-42 L^2, an edge function within 2.5 x 2^-42 |D| L^2 and the volume
+// within 2^-40 L^3; the bounds below are four times that, far above the FP64
+// formula's own rounding (2^-49), so a sign beyond them is the sign FP64 finds.
+// Sizes outside 2^-20 .. 2^20 (where low parts could underflow) stay undecided.
+static __device__ int tri_filter_df(float ox, float oy, float oz, float qx, float qy, float qz, float4 a, float4 b,
+                                    float4 c) {
+  const DF Ax = df_diff(a.x, ox), Ay = df_diff(a.y, oy), Az = df_diff(a.z, oz);
+  const DF Bx = df_diff(b.x, ox), By = df_diff(b.y, oy), Bz = df_diff(b.z, oz);
+  const DF Cx = df_diff(c.x, ox), Cy = df_diff(c.y, oy), Cz = df_diff(c.z, oz);
+  const DF Dx = df_diff(qx, ox), Dy = df_diff(qy, oy), Dz = df_diff(qz, oz);
+  const float L = fmaxf(fmaxf(fmaxf(fabsf(Ax.h), fabsf(Ay.h)), fmaxf(fabsf(Az.h), fabsf(Bx.h))),
+                        fmaxf(fmaxf(fmaxf(fabsf(By.h), fabsf(Bz.h)), fmaxf(fabsf(Cx.h), fabsf(Cy.h))), fabsf(Cz.h)));
+  const float d1 = fabsf(Dx.h) + fabsf(Dy.h) + fabsf(Dz.h);
+  if (!(L >= 9.5367432e-7f && L <= 1048576.f && d1 >= 9.5367432e-7f && d1 <= 1048576.f)) return 2;
+  const DF BCx = df_det(By, Cz, Bz, Cy), BCy = df_det(Bz, Cx, Bx, Cz), BCz = df_det(Bx, Cy, By, Cx);
+  const DF Wa = df_dot(Dx, Dy, Dz, BCx, BCy, BCz);
+  const DF Wb = df_dot(Dx, Dy, Dz, df_det(Cy, Az, Cz, Ay), df_det(Cz, Ax, Cx, Az), df_det(Cx, Ay, Cy, Ax));
+  const DF Wc = df_dot(Dx, Dy, Dz, df_det(Ay, Bz, Az, By), df_det(Az, Bx, Ax, Bz), df_det(Ax, By, Ay, Bx));
+  const float Ew = 9.0949470e-13f * 2.5f * d1 * L * L;  // 4 x 2.5 x 2^-42
+  const float mx = fmaxf(Wa.h, fmaxf(Wb.h, Wc.h)), mn = fminf(Wa.h, fminf(Wb.h, Wc.h));
+  if (mx > Ew && mn < -Ew) return 0;
+  const bool pos = mn > Ew, neg = mx < -Ew;
+  if (!(pos || neg)) return 2;
+  DF det = df_add(df_add(Wa, Wb), Wc), vol = df_dot(Ax, Ay, Az, BCx, BCy, BCz);
+  if (neg) {
+    det = df_neg(det);
+    vol = df_neg(vol);
+  }
+  const float Ev = 3.6379788e-12f * L * L * L;  // 4 x 2^-40
+  const float Ed = 4.0f * Ew;
+  // vol <= det
+  const float g1 = df_add(det, df_neg(vol)).h;
+  const float e1 = Ed + Ev + 1e-6f * fabsf(g1);
+  // vol |D| >= tmin det; |D| in FP32, within 2^-21
+  const float dx = Dx.h, dy = Dy.h, dz = Dz.h;
+  const float len = __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
+  const float g2 = vol.h * len - kTmin * det.h;
+  const float e2 = Ev * len + kTmin * Ed + 1e-6f * (fabsf(vol.h) * len + kTmin * fabsf(det.h));
+  if (g1 < -e1 || g2 < -e2) return 0;
+  if (g1 > e1 && g2 > e2) return 1;
+  return 2;
+}
+
+// A test the FP32 filter left open: double-float, then FP64. The answer is the
+// FP64 formula's.
+static __device__ __noinline__ bool tri_recheck(float ox, float oy, float oz, float qx, float qy, float qz, float4 a,
+                                                float4 b, float4 c) {
+  const int r = tri_filter_df(ox, oy, oz, qx, qy, qz, a, b, c);
+  return r == 2 ? tri_test64(ox, oy, oz, qx, qy, qz, a, b, c) : r == 1;
+}
+
+// FP32 filter of the segment p -> q: 1 certain hit, 0 certain miss, 2
+// undecided (tri_recheck).
+__device__ __forceinline__ int tri_test32(float3 p, float3 q, float4 a, float4 b, float4 c) {
+  const float ox = p.x, oy = p.y, oz = p.z;
+  const float dx = __fsub_rn(q.x, p.x), dy = __fsub_rn(q.y, p.y), dz = __fsub_rn(q.z, p.z);
   float Ax = __fsub_rn(a.x, ox), Ay = __fsub_rn(a.y, oy), Az = __fsub_rn(a.z, oz);
   float Bx = __fsub_rn(b.x, ox), By = __fsub_rn(b.y, oy), Bz = __fsub_rn(b.z, oz);
   float Cx = __fsub_rn(c.x, ox), Cy = __fsub_rn(c.y, oy), Cz = __fsub_rn(c.z, oz);
@@ -222,11 +308,11 @@ __device__ __forceinline__ int tri_test32(const Seg& s, float4 a, float4 b, floa
   float BCx = By * Cz - Bz * Cy, BCy = Bz * Cx - Bx * Cz, BCz = Bx * Cy - By * Cx;
   float CAx = Cy * Az - Cz * Ay, CAy = Cz * Ax - Cx * Az, CAz = Cx * Ay - Cy * Ax;
   float ABx = Ay * Bz - Az * By, ABy = Az * Bx - Ax * Bz, ABz = Ax * By - Ay * Bx;
-  float Wa = s.dx * BCx + s.dy * BCy + s.dz * BCz;
-  float Wb = s.dx * CAx + s.dy * CAy + s.dz * CAz;
-  float Wc = s.dx * ABx + s.dy * ABy + s.dz * ABz;
+  float Wa = dx * BCx + dy * BCy + dz * BCz;
+  float Wb = dx * CAx + dy * CAy + dz * CAz;
+  float Wc = dx * ABx + dy * ABy + dz * ABz;
   float L2 = L * L;
-  float Ew = s.kw * L2;
+  float Ew = edge_factor(dx, dy, dz) * L2;
   float mx = max3f(Wa, Wb, Wc), mn = min3f(Wa, Wb, Wc);
   if (mx > Ew && mn < -Ew) return 0;  // edge functions of strictly opposite sign
   bool allpos = mn > Ew, allneg = mx < -Ew;
@@ -238,7 +324,7 @@ __device__ __forceinline__ int tri_test32(const Seg& s, float4 a, float4 b, floa
   float Edet = 3.0f * Ew + 2.02f * kU * det_s;
   float g1 = det_s - vol_s;
   float e1 = Edet + Ev + 2.0f * kU * fabsf(g1);
-  const float len = seg_len(s);
+  const float len = seg_length(dx, dy, dz);
   float g2 = vol_s * len - kTmin * det_s;
   float e2 = (Ev + 6.0f * kU * fabsf(vol_s)) * len + kTmin * (Edet + 2.0f * kU * det_s) +
              2.0f * kU * fabsf(g2);
@@ -255,11 +341,13 @@ __device__ __forceinline__ bool leaf_hit(const float4* __restrict__ tris, int le
     if (ia == s.vi || ia == s.vj || ib == s.vi || ib == s.vj || ic == s.vi || ic == s.vj)
       return false;
   }
-  int r = tri_test32(s, a, b, c);
+  const float* pp = pts + 3 * (int64_t)s.vi;
+  const float* qq = pts + 3 * (int64_t)s.vj;
+  const float3 p = make_float3(pp[0], pp[1], pp[2]), q = make_float3(qq[0], qq[1], qq[2]);
+  const int r = tri_test32(p, q, a, b, c);
   if (r == 2) {
     ++rechecks;
-    const float* q = pts + 3 * (int64_t)s.vj;
-    return tri_test64(lo2(s.ox2), lo2(s.oy2), lo2(s.oz2), q[0], q[1], q[2], a, b, c);
+    return tri_recheck(p.x, p.y, p.z, q.x, q.y, q.z, a, b, c);
   }
   return r == 1;
 }
@@ -276,10 +364,11 @@ __device__ __forceinline__ bool leaf_hit(const float4* __restrict__ tris, int le
 // records fetched. `status_bits` collects stack-overflow / iteration-overrun
 // conditions (the lane is then reported as hit and the call fails on the
 // host).
-static __device__ bool packet_any_hit(const float4* __restrict__ nodes, const float4* __restrict__ tris,
-                                      int nt, const Seg& s, const float* __restrict__ pts, bool active,
-                                      unsigned& rechecks, unsigned& status_bits, unsigned& visits,
-                                      unsigned& tri_tests) {
+template <bool WIDE>
+static __device__ __forceinline__ bool packet_hits(const float4* __restrict__ nodes, const float4* __restrict__ tris,
+                                                   int nt, const Seg& s, const float* __restrict__ pts, bool active,
+                                                   unsigned& rechecks, unsigned& status_bits, unsigned& visits,
+                                                   unsigned& tri_tests) {
   static_assert(kStack == 64, "two stack registers per lane");
   const unsigned full = 0xffffffffu;
   bool hit = false;
@@ -290,41 +379,41 @@ static __device__ bool packet_any_hit(const float4* __restrict__ nodes, const fl
   int node = 0, sp = 0;
   const int max_iter = 4 * nt + 64;
   for (int it = 0; it < max_iter; ++it) {
-    const ulonglong2* nd = reinterpret_cast<const ulonglong2*>(nodes) + 4 * node;
-    const ulonglong2 n0 = __ldg(nd), n1 = __ldg(nd + 1), n2 = __ldg(nd + 2);
+    const float4* nd = nodes + 4 * node;
+    const float4 n0 = __ldg(nd), n1 = __ldg(nd + 1), n2 = __ldg(nd + 2);
     const int2 lr = __ldg(reinterpret_cast<const int2*>(nd + 3));
     const int l = lr.x, r = lr.y;
-    const bool hl = active && box_hit(s, n0.x, n0.y, n1.x);
-    const bool hr = active && box_hit(s, n1.y, n2.x, n2.y);
+    bool hl, hr;
+    if (WIDE) {
+      const float* pp = pts + 3 * (int64_t)s.vi;
+      const float3 p = make_float3(pp[0], pp[1], pp[2]);
+      hl = active && box_hit_wide(s, p, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y);
+      hr = active && box_hit_wide(s, p, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w);
+    } else {
+      hl = active && box_hit(s, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y);
+      hr = active && box_hit(s, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w);
+    }
     const unsigned bl = __ballot_sync(full, hl);
     const unsigned br = __ballot_sync(full, hr);
     int next = -1;
-    bool leaf = false;
-    if (bl) {
-      if (l < 0) {
-        leaf = true;
-        if (hl) {
+    const bool leaf = (bl && l < 0) || (br && r < 0);
+    if (leaf) {
+      // (one copy of the triangle test: two would cost registers)
+#pragma unroll 1
+      for (int k = 0; k < 2; ++k) {
+        const int child = k ? r : l;
+        if (child < 0 && active && (k ? hr : hl)) {
           ++tri_tests;
-          if (leaf_hit(tris, ~l, s, pts, rechecks)) {
+          if (leaf_hit(tris, ~child, s, pts, rechecks)) {
             hit = true;
             active = false;
           }
         }
-      } else {
-        next = l;
       }
     }
-    if (br) {
-      if (r < 0) {
-        leaf = true;
-        if (hr && active) {
-          ++tri_tests;
-          if (leaf_hit(tris, ~r, s, pts, rechecks)) {
-            hit = true;
-            active = false;
-          }
-        }
-      } else if (next < 0) {
+    if (bl && l >= 0) next = l;
+    if (br && r >= 0) {
+      if (next < 0) {
         next = r;
       } else {
         if (sp >= kStack) {
@@ -357,6 +446,82 @@ static __device__ bool packet_any_hit(const float4* __restrict__ nodes, const fl
   visits += max_iter;
   status_bits |= kStatusTraversalOverrun;
   return true;
+}
+
+static __device__ __noinline__ bool packet_hits_wide(const float4* __restrict__ nodes,
+                                                     const float4* __restrict__ tris, int nt, Seg s,
+                                                     const float* __restrict__ pts, bool active, unsigned* counts) {
+  return packet_hits<true>(nodes, tris, nt, s, pts, active, counts[0], counts[1], counts[2], counts[3]);
+}
+
+// What a tile is traced against: [0] the cage, [1] the part.
+struct TileMesh {
+  const float4* nodes[2];
+  const float4* tris[2];
+  int32_t nt[2];
+  const float* amax[2];  // the meshes' largest |coordinate|
+};
+
+inline TileMesh tile_mesh(const visacd_ctx* ctx, const visacd_bvh* part, const visacd_bvh* cage) {
+  TileMesh m;
+  const visacd_bvh* b[2] = {cage, part};
+  for (int k = 0; k < 2; ++k) {
+    m.nodes[k] = b[k]->nodes;
+    m.tris[k] = b[k]->tris;
+    m.nt[k] = b[k]->nt;
+    m.amax[k] = bvh_amax(ctx, b[k]);
+  }
+  return m;
+}
+
+// A warp's totals of a launch, in shared memory (in registers they would be
+// spilled inside the traversal).
+enum { kSumPairs, kSumEdges, kSumSelf, kSumCage, kSumDegenerate, kSumRechecks, kSumVisits, kSumTests, kSums };
+
+// The warp's segments (pts[i] -> pts[j], i < j, on active lanes) against the
+// cage, then those that leave it against the part. Few segments leave the
+// cage (most vertex pairs of a part are interior chords, which cross neither
+// surface), so the second test runs for few. Bit 0: hits the cage; bit 1: hits
+// the part as well (1 alone: an edge). sum: the warp's totals.
+static __device__ __forceinline__ unsigned trace_tile(const TileMesh& M, const float* __restrict__ pts, uint32_t i,
+                                                      uint32_t j, float3 p, float3 q, bool active,
+                                                      unsigned long long* sum, unsigned& status_bits) {
+  Seg s;
+  make_seg(s, p, q, (int)i, (int)j);
+  unsigned h = 0, rechecks = 0, visits = 0, tests = 0;
+  const bool holds[2] = {!active || box_test_holds(p, q, *M.amax[0]), !active || box_test_holds(p, q, *M.amax[1])};
+#pragma unroll 1
+  for (int k = 0; k < 2; ++k) {
+    s.exclude = k == 1;
+    bool hit;
+    if (__all_sync(0xffffffffu, k ? holds[1] : holds[0])) {
+      hit = packet_hits<false>(k ? M.nodes[1] : M.nodes[0], k ? M.tris[1] : M.tris[0], k ? M.nt[1] : M.nt[0], s, pts,
+                               active, rechecks, status_bits, visits, tests);
+    } else {
+      unsigned counts[4] = {0, 0, 0, 0};
+      hit = packet_hits_wide(k ? M.nodes[1] : M.nodes[0], k ? M.tris[1] : M.tris[0], k ? M.nt[1] : M.nt[0], s, pts,
+                             active, counts);
+      rechecks += counts[0];
+      status_bits |= counts[1];
+      visits += counts[2];
+      tests += counts[3];
+    }
+    active = active && hit;
+    if (active) h |= 1u << k;
+    if (!__any_sync(0xffffffffu, active)) break;
+  }
+  const unsigned cage = __ballot_sync(0xffffffffu, h & 1u), self = __ballot_sync(0xffffffffu, h & 2u);
+  rechecks = __reduce_add_sync(0xffffffffu, rechecks);
+  tests = __reduce_add_sync(0xffffffffu, tests);
+  if ((threadIdx.x & 31) == 0) {
+    sum[kSumEdges] += __popc(cage & ~self);
+    sum[kSumSelf] += __popc(self);
+    sum[kSumCage] += __popc(cage);
+    sum[kSumRechecks] += rechecks;
+    sum[kSumVisits] += visits;
+    sum[kSumTests] += tests;
+  }
+  return h;
 }
 
 __device__ __forceinline__ int64_t row_start(int64_t i, int64_t n) {

@@ -13,14 +13,20 @@
 //    warp start and end close together (coherent traversal, dynamic balance).
 //  * Warp-packet any-hit traversal of a 64-byte-node LBVH (both child boxes per
 //    node): the warp follows one path (ballot of per-lane box tests), node
-//    records are broadcast loads, a per-warp stack lives in shared memory; the
+//    records are broadcast loads, the stack lives in registers; the
 //    cage test runs first and the self test only for lanes whose segment
 //    leaves the cage (few: most vertex pairs of a part are interior chords,
 //    which cross neither surface).
 //  * Segment-triangle test: edge functions W = D.(B x C), ... relative to the
 //    origin in FP32 with an a-priori rounding bound (8 roundings per term,
 //    bounded by 17u |D|_1 L^2). Only tests whose signs fall inside the bound
-//    are re-decided in FP64 (the same formula as the oracle).
+//    are re-decided: in double-float, and in FP64 (the oracle's formula) where
+//    that is open too. FP64 runs at about two operations per clock and SM, and
+//    segments inside a cut plane put many tests inside the bound: the two
+//    halves of a torus (4.5M pairs, 6.9M such tests) went from 6.45 to 4.32
+//    ms, a cut blob (0.15M of them) from 2.43 to 2.24 ms.
+//  * Box test: centre and half extents, three FMAs per axis and box, with the
+//    leaf boxes' widening covering its rounding (traverse.cuh).
 //  * Self-test end-vertex policy: triangles incident to i or j are skipped.
 //  * Results land in a bitset over the reference's linear pair index; a
 //    popcount / scan / emit pass compacts it into the row-major edge list.
@@ -44,12 +50,7 @@ struct VisParams {
   int triangular;          // 1: rows == cols and pairs with row < col
   const uint8_t* is_new;   // masked mode
   const int32_t* newrank;  // masked mode: position of a new vertex in rows, else INT_MAX
-  const float4* self_nodes;
-  const float4* self_tris;
-  int32_t self_nt;
-  const float4* cage_nodes;
-  const float4* cage_tris;
-  int32_t cage_nt;
+  TileMesh mesh;           // the cage and the part
   uint32_t* bitset;
   VisCounters* cnt;
   unsigned* status;
@@ -109,12 +110,6 @@ __global__ void tile_row_counts_kernel(int64_t ntr, int64_t ntc, int TR, int TC,
   }
 }
 
-// Per-lane counters of a visibility launch, reduced over the warp at the end.
-struct VisLaneCounters {
-  unsigned long long pairs = 0, edges = 0, self = 0, cage = 0, deg = 0;
-  unsigned rechecks = 0, status_bits = 0, visits = 0, tri_tests = 0;
-};
-
 // The pair of `lane` in tile w of P's tile space (original vertex ids i < j),
 // or valid = false. The walk and the traversal kernels share it, so a tile's
 // lane means the same pair in both.
@@ -153,73 +148,52 @@ __device__ __forceinline__ bool lane_pair(const VisParams& P, unsigned long long
 // pair and degenerate counts, and `done` marks the lanes it settled: they
 // take no part.
 template <int TR>
-__device__ __forceinline__ void vis_tile(const VisParams& P, unsigned long long w, int lane,
-                                         VisLaneCounters& c, bool walked, uint32_t done) {
-  const int64_t n = P.n;
+__device__ __forceinline__ void vis_tile(const VisParams& P, unsigned long long w, int lane, unsigned long long* sum,
+                                         unsigned& status_bits, bool walked, uint32_t done) {
   uint32_t i, j;
   const bool mine = !((done >> lane) & 1u);
   const bool valid = lane_pair<TR>(P, w, lane, i, j) && mine;
-  Seg s;
   float3 p = make_float3(0.f, 0.f, 0.f), q = make_float3(0.f, 0.f, 0.f);
+  bool active = false;
   if (valid) {
-    if (!walked) ++c.pairs;
     p = make_float3(P.pts[3 * (int64_t)i], P.pts[3 * (int64_t)i + 1], P.pts[3 * (int64_t)i + 2]);
     q = make_float3(P.pts[3 * (int64_t)j], P.pts[3 * (int64_t)j + 1], P.pts[3 * (int64_t)j + 2]);
+    // coincident endpoints (or NaN): never an edge
+    active = seg_length(__fsub_rn(q.x, p.x), __fsub_rn(q.y, p.y), __fsub_rn(q.z, p.z)) > 0.f;
   }
-  make_seg(s, p, q, (int)i, (int)j);
-  bool active = valid;
-  if (valid && !(seg_len(s) > 0.f)) {  // coincident endpoints (or NaN): never an edge
-    ++c.deg;
-    active = false;
+  const unsigned nv = __popc(__ballot_sync(0xffffffffu, valid)), na = __popc(__ballot_sync(0xffffffffu, active));
+  if (lane == 0) {
+    if (!walked) sum[kSumPairs] += nv;
+    sum[kSumDegenerate] += nv - na;
   }
-  if (!__ballot_sync(0xffffffffu, active)) return;
-  // The cage first: few segments leave it, so the self test runs for few.
-  s.exclude = false;
-  const bool cage_hit = packet_any_hit(P.cage_nodes, P.cage_tris, P.cage_nt, s, P.pts, active,
-                                       c.rechecks, c.status_bits, c.visits, c.tri_tests);
-  if (active && cage_hit) ++c.cage;
-  active = active && cage_hit;
-  s.exclude = true;
-  const bool self_hit = packet_any_hit(P.self_nodes, P.self_tris, P.self_nt, s, P.pts, active,
-                                       c.rechecks, c.status_bits, c.visits, c.tri_tests);
-  if (active && self_hit) ++c.self;
-  if (active && !self_hit) {
-    ++c.edges;
-    const int64_t k = row_start(i, n) + (int64_t)(j - i - 1);
+  if (!na) return;
+  if (trace_tile(P.mesh, P.pts, i, j, p, q, active, sum, status_bits) == 1u) {
+    const int64_t k = row_start(i, P.n) + (int64_t)(j - i - 1);
     atomicOr(&P.bitset[k >> 5], 1u << (k & 31));
   }
 }
 
 __device__ __forceinline__ void vis_flush_counters(VisCounters* cnt, unsigned* status, int lane,
-                                                   VisLaneCounters& c) {
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    c.pairs += __shfl_xor_sync(0xffffffffu, c.pairs, o);
-    c.edges += __shfl_xor_sync(0xffffffffu, c.edges, o);
-    c.self += __shfl_xor_sync(0xffffffffu, c.self, o);
-    c.cage += __shfl_xor_sync(0xffffffffu, c.cage, o);
-    c.deg += __shfl_xor_sync(0xffffffffu, c.deg, o);
-    c.rechecks += __shfl_xor_sync(0xffffffffu, c.rechecks, o);
-    c.tri_tests += __shfl_xor_sync(0xffffffffu, c.tri_tests, o);
-    c.status_bits |= __shfl_xor_sync(0xffffffffu, c.status_bits, o);
-  }
+                                                   const unsigned long long* sum, unsigned status_bits) {
+  status_bits = __reduce_or_sync(0xffffffffu, status_bits);
   if (lane == 0) {
-    atomicAdd(&cnt->pairs, c.pairs);
-    atomicAdd(&cnt->edges, c.edges);
-    atomicAdd(&cnt->self_hits, c.self);
-    atomicAdd(&cnt->cage_hits, c.cage);
-    atomicAdd(&cnt->degenerate, c.deg);
-    atomicAdd(&cnt->rechecks, (unsigned long long)c.rechecks);
-    atomicAdd(&cnt->node_visits, (unsigned long long)c.visits);
-    atomicAdd(&cnt->tri_tests, (unsigned long long)c.tri_tests);
-    if (c.status_bits) atomicOr(status, c.status_bits);
+    unsigned long long* const to[kSums] = {&cnt->pairs,      &cnt->edges,    &cnt->self_hits,   &cnt->cage_hits,
+                                           &cnt->degenerate, &cnt->rechecks, &cnt->node_visits, &cnt->tri_tests};
+#pragma unroll
+    for (int k = 0; k < kSums; ++k)
+      if (sum[k]) atomicAdd(to[k], sum[k]);
+    if (status_bits) atomicOr(status, status_bits);
   }
 }
 
 template <int TR, int MINB>
 __global__ void __launch_bounds__(kVisThreads, MINB) visibility_kernel(VisParams P) {
   const int lane = threadIdx.x & 31;
-  VisLaneCounters c;
+  __shared__ unsigned long long sums[kVisThreads / 32][kSums];
+  unsigned long long* sum = sums[threadIdx.x >> 5];
+  if (lane < kSums) sum[lane] = 0;
+  __syncwarp();
+  unsigned status_bits = 0;
   // After a walk only the tiles it left are traversed (their count is on the
   // device, written by the walk kernel before this launch).
   const unsigned long long items = P.pend_tiles ? P.cnt->pending : P.total_tiles;
@@ -229,11 +203,11 @@ __global__ void __launch_bounds__(kVisThreads, MINB) visibility_kernel(VisParams
     w = __shfl_sync(0xffffffffu, w, 0);
     if (w >= items) break;
     if (P.pend_tiles)
-      vis_tile<TR>(P, P.pend_tiles[w], lane, c, true, P.pend_done[w]);
+      vis_tile<TR>(P, P.pend_tiles[w], lane, sum, status_bits, true, P.pend_done[w]);
     else
-      vis_tile<TR>(P, w, lane, c, false, 0u);
+      vis_tile<TR>(P, w, lane, sum, status_bits, false, 0u);
   }
-  vis_flush_counters(P.cnt, P.status, lane, c);
+  vis_flush_counters(P.cnt, P.status, lane, sum, status_bits);
 }
 
 // The free-space walk over P's tile space, before the traversal kernel. It
@@ -314,7 +288,11 @@ __global__ void __launch_bounds__(kVisThreads, MINB)
                             unsigned* __restrict__ status, const unsigned long long* __restrict__ pend_tiles,
                             const uint32_t* __restrict__ pend_done) {
   const int lane = threadIdx.x & 31;
-  VisLaneCounters c;
+  __shared__ unsigned long long sums[kVisThreads / 32][kSums];
+  unsigned long long* sum = sums[threadIdx.x >> 5];
+  if (lane < kSums) sum[lane] = 0;
+  __syncwarp();
+  unsigned status_bits = 0;
   const unsigned long long items = pend_tiles ? cnt->pending : total_tiles;
   for (int guard = 0; guard < (1 << 30); ++guard) {
     unsigned long long w = 0;
@@ -324,13 +302,13 @@ __global__ void __launch_bounds__(kVisThreads, MINB)
     if (pend_tiles) {
       const unsigned long long g = pend_tiles[w];
       const int p = part_of(tile_start, n_parts, g);
-      vis_tile<TR>(parts[p], g - tile_start[p], lane, c, true, pend_done[w]);
+      vis_tile<TR>(parts[p], g - tile_start[p], lane, sum, status_bits, true, pend_done[w]);
     } else {
       const int p = part_of(tile_start, n_parts, w);
-      vis_tile<TR>(parts[p], w - tile_start[p], lane, c, false, 0u);
+      vis_tile<TR>(parts[p], w - tile_start[p], lane, sum, status_bits, false, 0u);
     }
   }
-  vis_flush_counters(cnt, status, lane, c);
+  vis_flush_counters(cnt, status, lane, sum, status_bits);
 }
 
 // The free-space walk over all parts' tiles (as visibility_walk_kernel; parts
@@ -735,12 +713,7 @@ static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint
     }
     P.total_tiles = total;
   }
-  P.self_nodes = self_bvh->nodes;
-  P.self_tris = self_bvh->tris;
-  P.self_nt = self_bvh->nt;
-  P.cage_nodes = cage_bvh->nodes;
-  P.cage_tris = cage_bvh->tris;
-  P.cage_nt = cage_bvh->nt;
+  P.mesh = tile_mesh(ctx, self_bvh, cage_bvh);
   // Large calls first clear what they can with the cage's free-space grid
   // (built at the top of this call): a walk kernel, then the traversal.
   if (use_grid && cage_bvh->free_lb && P.total_tiles > 0) {
@@ -999,12 +972,7 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
       }
       P.total_tiles = n >= 2 ? t : 0ull;
     }
-    P.self_nodes = self_bvhs[p]->nodes;
-    P.self_tris = self_bvhs[p]->tris;
-    P.self_nt = self_bvhs[p]->nt;
-    P.cage_nodes = cage_bvhs[p]->nodes;
-    P.cage_tris = cage_bvhs[p]->tris;
-    P.cage_nt = cage_bvhs[p]->nt;
+    P.mesh = tile_mesh(ctx, self_bvhs[p], cage_bvhs[p]);
     const visacd_bvh* cb = cage_bvhs[p];
     if (any_grid && cb->free_lb && part_pairs[p] >= kFreeGridMinPairs) {
       P.cage_free.lb = cb->free_lb;
