@@ -272,10 +272,8 @@ __global__ void node_layout_kernel(const int2* __restrict__ child,
   }
 }
 
-// The one-launch build (order.cu). Host input was checked by the caller, so
-// nothing has to come back; device input is checked by the kernel.
-static int bvh_build_fast(visacd_ctx* ctx, const float* dv, int32_t nv, const uint32_t* dt, int32_t nt, bool check,
-                          visacd_bvh* b) {
+int bvh_prepare(visacd_ctx* ctx, const float* dv, int32_t nv, const uint32_t* dt, int32_t nt, char* scratch,
+                visacd_bvh** out, OrderJob& j) {
   const int n_int = nt > 1 ? nt - 1 : 1;
   const size_t o_tris = ((size_t)n_int * 64 + 255) & ~size_t(255);
   const size_t o_head = o_tris + (((size_t)nt * 48 + 255) & ~size_t(255));
@@ -285,34 +283,67 @@ static int bvh_build_fast(visacd_ctx* ctx, const float* dv, int32_t nv, const ui
     set_error("bvh_build: device allocation failed");
     return VISACD_ERR_NO_MEMORY;
   }
+  visacd_bvh* b = new visacd_bvh();
+  b->device = ctx->device;
+  b->nt = nt;
+  b->nv = nv;
+  b->ctx = ctx;
   b->stream = ctx->stream;
   b->nodes = reinterpret_cast<float4*>(mem);
   b->tris = reinterpret_cast<float4*>(mem + o_tris);
   b->head = mem + o_head;
-  VTRY(ensure_slot(ctx, kSlotTmpTris, order_scratch(nt, true)));
-  OrderJob j = {};
+  j = {};
   j.verts = dv;
   j.tris = dt;
   j.nv = nv;
   j.n = nt;
   j.bits = morton_bits(nt);
   j.head = reinterpret_cast<BvhHead*>(b->head);
+  j.nodes = b->nodes;
   j.leaves = b->tris;
-  order_carve(j, slot<char>(ctx, kSlotTmpTris));
-  VTRY(order_run(ctx, &j, 1));
-  VTRY(order_nodes(ctx, j, b->nodes));
+  order_carve(j, scratch);
   // Every step down the tree lengthens the common prefix of (code, position).
   int len = 0;
   while ((1 << len) < nt) ++len;
   b->depth = 3 * j.bits + len;
-  if (!check) return VISACD_OK;
-  BvhHead* h = nullptr;
-  VTRY(pinned(ctx, sizeof(BvhHead), (void**)&h));
-  VCUDA(cudaMemcpyAsync(h, b->head, sizeof(BvhHead), cudaMemcpyDeviceToHost, ctx->stream));
-  VCUDA(stream_wait(ctx));
-  VCHECK(!h->bad, VISACD_ERR_INVALID_ARG, "bvh_build: a triangle references a vertex index >= %d", nv);
-  memcpy(b->tri_bounds, h->tb, sizeof(b->tri_bounds));
-  b->head_read = true;
+  ctx->bvhs.push_back(b);
+  *out = b;
+  return VISACD_OK;
+}
+
+// The one-launch build (order.cu). Host input was checked by the caller, so
+// nothing has to come back; device input is checked by the kernel.
+static int bvh_build_fast(visacd_ctx* ctx, const float* dv, int32_t nv, const uint32_t* dt, int32_t nt, bool check,
+                          visacd_bvh** out) {
+  VTRY(ensure_slot(ctx, kSlotTmpTris, order_scratch(nt, true)));
+  visacd_bvh* b = nullptr;
+  OrderJob j;
+  VTRY(bvh_prepare(ctx, dv, nv, dt, nt, slot<char>(ctx, kSlotTmpTris), &b, j));
+  int rc = order_run(ctx, &j, 1);
+  if (rc == VISACD_OK) rc = order_nodes(ctx, &j, 1);
+  if (rc == VISACD_OK && check) {
+    BvhHead* h = nullptr;
+    rc = pinned(ctx, sizeof(BvhHead), (void**)&h);
+    if (rc == VISACD_OK) {
+      cudaError_t e = cudaMemcpyAsync(h, b->head, sizeof(BvhHead), cudaMemcpyDeviceToHost, ctx->stream);
+      if (e == cudaSuccess) e = stream_wait(ctx);
+      if (e != cudaSuccess) {
+        set_error("bvh_build: %s", cudaGetErrorString(e));
+        rc = VISACD_ERR_CUDA;
+      } else if (h->bad) {
+        set_error("bvh_build: a triangle references a vertex index >= %d", nv);
+        rc = VISACD_ERR_INVALID_ARG;
+      } else {
+        memcpy(b->tri_bounds, h->tb, sizeof(b->tri_bounds));
+        b->head_read = true;
+      }
+    }
+  }
+  if (rc != VISACD_OK) {
+    visacd_bvh_destroy(b);
+    return rc;
+  }
+  *out = b;
   return VISACD_OK;
 }
 
@@ -365,16 +396,8 @@ int bvh_build(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* t
     dt = slot<uint32_t>(ctx, kSlotBuildTris);
   }
   if (nt <= kOrderMax) {
-    const int rc = bvh_build_fast(ctx, dv, nv, dt, nt, device_ptrs != 0, b);
-    if (rc != VISACD_OK) {
-      if (b->nodes) cudaFreeAsync(b->nodes, ctx->stream);
-      delete b;
-      return rc;
-    }
-    b->ctx = ctx;
-    ctx->bvhs.push_back(b);
-    *out = b;
-    return VISACD_OK;
+    delete b;
+    return bvh_build_fast(ctx, dv, nv, dt, nt, device_ptrs != 0, out);
   }
   const int n_int = nt - 1;
   // Scratch: centroids, keys x2, vals x2, child, parents, boxes, visits, counters.

@@ -314,6 +314,8 @@ inline int morton_bits(int64_t n) {
 // Exclusive scan of n uint32 counts into uint64 offsets (device), total also
 // written to offsets[n]. Uses ctx scan scratch.
 int exclusive_scan_u32_to_u64(visacd_ctx* ctx, const uint32_t* in, uint64_t* out, int64_t n);
+// The same over the numbers of set bits of n words.
+int exclusive_scan_bits(visacd_ctx* ctx, const uint32_t* words, uint64_t* out, int64_t n);
 
 // Stable LSD radix sort of (key, value) pairs on the device. key_bits selects
 // how many low bits of the key take part (multiple of 8). Results land in

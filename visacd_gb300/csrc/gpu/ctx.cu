@@ -249,6 +249,8 @@ __device__ __forceinline__ uint64_t block_exclusive_scan_u64(uint64_t v, uint64_
   return before + x - v;
 }
 
+// POPC: the scanned counts are the set bits of the input words.
+template <bool POPC>
 __global__ void scan_blocks_kernel(const uint32_t* __restrict__ in, int64_t n,
                                    uint64_t* __restrict__ block_sums) {
   int64_t base = (int64_t)blockIdx.x * kScanTile;
@@ -256,7 +258,7 @@ __global__ void scan_blocks_kernel(const uint32_t* __restrict__ in, int64_t n,
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     int64_t i = base + (int64_t)k * kScanThreads + threadIdx.x;
-    if (i < n) s += in[i];
+    if (i < n) s += POPC ? (uint32_t)__popc(in[i]) : in[i];
   }
   uint64_t total;
   block_exclusive_scan_u64(s, &total);
@@ -276,6 +278,7 @@ __global__ void scan_top_kernel(uint64_t* __restrict__ block_sums, int64_t nb) {
   if (threadIdx.x == 0) block_sums[nb] = carry;
 }
 
+template <bool POPC>
 __global__ void scan_add_kernel(const uint32_t* __restrict__ in, int64_t n,
                                 const uint64_t* __restrict__ block_sums,
                                 uint64_t* __restrict__ out, int64_t nb) {
@@ -287,6 +290,7 @@ __global__ void scan_add_kernel(const uint32_t* __restrict__ in, int64_t n,
   for (int k = 0; k < kScanItems; ++k) {
     int64_t i = base + k;
     v[k] = i < n ? in[i] : 0u;
+    if (POPC) v[k] = (uint32_t)__popc(v[k]);
     s += v[k];
   }
   uint64_t total;
@@ -304,6 +308,7 @@ __global__ void scan_add_kernel(const uint32_t* __restrict__ in, int64_t n,
 // the tiles in order with a running carry.
 constexpr int64_t kScanSingle = 4 * kScanTile;
 
+template <bool POPC>
 __global__ void scan_single_kernel(const uint32_t* __restrict__ in, int64_t n, uint64_t* __restrict__ out) {
   uint64_t carry = 0;
   for (int64_t t0 = 0; t0 < n; t0 += kScanTile) {
@@ -314,6 +319,7 @@ __global__ void scan_single_kernel(const uint32_t* __restrict__ in, int64_t n, u
     for (int k = 0; k < kScanItems; ++k) {
       const int64_t i = base + k;
       v[k] = i < n ? in[i] : 0u;
+      if (POPC) v[k] = (uint32_t)__popc(v[k]);
       s += v[k];
     }
     uint64_t total;
@@ -329,9 +335,10 @@ __global__ void scan_single_kernel(const uint32_t* __restrict__ in, int64_t n, u
   if (threadIdx.x == 0) out[n] = carry;
 }
 
-int exclusive_scan_u32_to_u64(visacd_ctx* ctx, const uint32_t* in, uint64_t* out, int64_t n) {
+template <bool POPC>
+static int exclusive_scan(visacd_ctx* ctx, const uint32_t* in, uint64_t* out, int64_t n) {
   if (n <= kScanSingle) {
-    VLAUNCH(ctx, kKScanAdd, 1, kScanThreads, 0, scan_single_kernel, in, n, out);
+    VLAUNCH(ctx, kKScanAdd, 1, kScanThreads, 0, scan_single_kernel<POPC>, in, n, out);
     return VISACD_OK;
   }
   int64_t nb = (n + kScanTile - 1) / kScanTile;
@@ -339,10 +346,17 @@ int exclusive_scan_u32_to_u64(visacd_ctx* ctx, const uint32_t* in, uint64_t* out
   VCHECK(nb < (1ll << 31), VISACD_ERR_INVALID_ARG, "scan too large: %lld", (long long)n);
   VTRY(ensure_slot(ctx, kSlotScanScratch, (size_t)(nb + 1) * sizeof(uint64_t)));
   uint64_t* bs = slot<uint64_t>(ctx, kSlotScanScratch);
-  VLAUNCH(ctx, kKScanBlocks, (unsigned)nb, kScanThreads, 0, scan_blocks_kernel, in, n, bs);
+  VLAUNCH(ctx, kKScanBlocks, (unsigned)nb, kScanThreads, 0, scan_blocks_kernel<POPC>, in, n, bs);
   VLAUNCH(ctx, kKScanTop, 1, kScanThreads, 0, scan_top_kernel, bs, nb);
-  VLAUNCH(ctx, kKScanAdd, (unsigned)nb, kScanThreads, 0, scan_add_kernel, in, n, bs, out, nb);
+  VLAUNCH(ctx, kKScanAdd, (unsigned)nb, kScanThreads, 0, scan_add_kernel<POPC>, in, n, bs, out, nb);
   return VISACD_OK;
+}
+
+int exclusive_scan_u32_to_u64(visacd_ctx* ctx, const uint32_t* in, uint64_t* out, int64_t n) {
+  return exclusive_scan<false>(ctx, in, out, n);
+}
+int exclusive_scan_bits(visacd_ctx* ctx, const uint32_t* words, uint64_t* out, int64_t n) {
+  return exclusive_scan<true>(ctx, words, out, n);
 }
 
 // ---------------------------------------------------------------------------

@@ -146,9 +146,11 @@ __device__ __forceinline__ void order_leaves(const OrderJob& J, int g, float ama
 
 // The leaves of a job a cluster sorted: one block per group (inside the
 // cluster the groups would run one after another, 6.6 us each).
-__global__ void __launch_bounds__(kOrderThreads) order_leaves_kernel(const __grid_constant__ OrderJob J) {
+// blockIdx.y: the job.
+__global__ void __launch_bounds__(kOrderThreads) order_leaves_kernel(const __grid_constant__ OrderArgs A) {
   __shared__ float sum[kOrderWarps][6];
-  order_leaves(J, (int)blockIdx.x, J.head->amax, sum);
+  const OrderJob& J = A.job[blockIdx.y];
+  if ((int)blockIdx.x * 1024 < J.n && J.n > kOrderSmall) order_leaves(J, (int)blockIdx.x, J.head->amax, sum);
 }
 
 __global__ void __launch_bounds__(kOrderThreads) order_kernel(const __grid_constant__ OrderArgs A) {
@@ -501,8 +503,10 @@ __device__ __forceinline__ int key_delta(const uint32_t* __restrict__ k, int n, 
 
 // Internal node i of Karras (2012): its range from the common-prefix lengths,
 // its split, both children's boxes and the traversal record, one thread each.
-__global__ void __launch_bounds__(128) order_nodes_kernel(const __grid_constant__ OrderJob J,
-                                                          float4* __restrict__ nodes) {
+// blockIdx.y: the job.
+__global__ void __launch_bounds__(128) order_nodes_kernel(const __grid_constant__ OrderArgs A) {
+  const OrderJob& J = A.job[blockIdx.y];
+  float4* __restrict__ nodes = J.nodes;
   const int n = J.n;
   const uint32_t* __restrict__ keys = J.k0;
   if (n == 1) {  // one internal node whose two children are that leaf
@@ -606,11 +610,18 @@ int order_run(visacd_ctx* ctx, const OrderJob* jobs, int n_jobs) {
   return VISACD_OK;
 }
 
-int order_nodes(visacd_ctx* ctx, const OrderJob& j, float4* nodes) {
-  if (j.n > kOrderSmall)
-    VLAUNCH(ctx, kKNodeLayout, (unsigned)((j.n + 1023) / 1024), kOrderThreads, 0, order_leaves_kernel, j);
-  VLAUNCH(ctx, kKKarras, grid_for(j.n > 1 ? j.n - 1 : 1, 128, 32LL * ctx->sm_count), 128, 0, order_nodes_kernel, j,
-          nodes);
+int order_nodes(visacd_ctx* ctx, const OrderJob* jobs, int n_jobs) {
+  OrderArgs a;
+  int most = 0;
+  for (int k = 0; k < n_jobs; ++k) {
+    a.job[k] = jobs[k];
+    most = std::max(most, jobs[k].n);
+  }
+  if (most > kOrderSmall)
+    VLAUNCH(ctx, kKNodeLayout, dim3((unsigned)((most + 1023) / 1024), (unsigned)n_jobs), kOrderThreads, 0,
+            order_leaves_kernel, a);
+  VLAUNCH(ctx, kKKarras, dim3(grid_for(most > 1 ? most - 1 : 1, 128, 32LL * ctx->sm_count), (unsigned)n_jobs), 128, 0,
+          order_nodes_kernel, a);
   return VISACD_OK;
 }
 

@@ -28,6 +28,7 @@ struct OrderJob {
   float* part;           // scratch: cluster x 16
   // Triangle jobs: the leaves in order and the box tables of order_box.
   BvhHead* head;
+  float4* nodes;                   // 4 (n - 1)
   float4* leaves;                  // 3 n
   float *box, *pre, *suf;          // 6 n: leaf boxes; unions from / to the ends of each run of 32 leaves
   float *bpre, *bsuf;              // 6 per run: unions from / to the ends of each group of 32 runs
@@ -46,7 +47,13 @@ void order_carve(OrderJob& j, char* base);
 // Enqueues the jobs (each at most kOrderMax primitives, at least one).
 int order_run(visacd_ctx* ctx, const OrderJob* jobs, int n_jobs);
 
-// Karras hierarchy and node records of a finished triangle job.
-int order_nodes(visacd_ctx* ctx, const OrderJob& j, float4* nodes);
+// Karras hierarchies and node records of finished triangle jobs (OrderJob::nodes).
+int order_nodes(visacd_ctx* ctx, const OrderJob* jobs, int n_jobs);
+
+// A one-launch build of a BVH over device input (1 to kOrderMax triangles): its
+// memory and its job, for order_run and order_nodes. The handle is registered
+// with the context; `scratch` holds order_scratch(nt, true) bytes.
+int bvh_prepare(visacd_ctx* ctx, const float* dv, int32_t nv, const uint32_t* dt, int32_t nt, char* scratch,
+                visacd_bvh** out, OrderJob& job);
 
 }  // namespace vgpu

@@ -41,6 +41,10 @@ namespace vgpu {
 // cage's free-space grid: below this the grid costs about what the walk saves.
 constexpr int64_t kFreeGridMinPairs = 1 << 22;
 
+// Pairs up to which a call emits and sends its edges without waiting for
+// their number (128 KB of room; the wait it saves is about 15 us).
+constexpr int64_t kFewPairs = 1 << 14;
+
 struct VisParams {
   const float* pts;
   int32_t n;
@@ -460,13 +464,6 @@ __global__ void new_rows_kernel(const uint32_t* __restrict__ perm, const uint32_
 }
 
 // ---- bitset compaction ----------------------------------------------------
-__global__ void bit_popc_kernel(const uint32_t* __restrict__ bits, int64_t nw,
-                                uint32_t* __restrict__ counts) {
-  for (int64_t w = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; w < nw;
-       w += (int64_t)gridDim.x * blockDim.x)
-    counts[w] = __popc(bits[w]);
-}
-
 __global__ void bit_emit_kernel(const uint32_t* __restrict__ bits, int64_t nw,
                                 const uint64_t* __restrict__ off, int64_t n,
                                 uint32_t* __restrict__ edges) {
@@ -586,23 +583,26 @@ static size_t points_scratch(const PointOrder* o, int count) {
     if (o[k].n > 1 && o[k].n <= kOrderMax) b += order_scratch(o[k].n, false);
   return b;
 }
+static OrderJob points_job(const PointOrder& q, char* scratch) {
+  OrderJob j = {};
+  j.verts = q.pts;
+  j.nv = j.n = q.n;
+  j.bits = morton_bits(q.n);
+  order_carve(j, scratch);
+  j.v0 = q.perm;
+  j.is_new = q.is_new;
+  j.rows = q.rows;
+  j.rank = q.rank;
+  return j;
+}
 static int points_order(visacd_ctx* ctx, const PointOrder* o, int count, char* scratch, VisCounters* cnt) {
   std::vector<OrderJob> jobs;
   for (int k = 0; k < count; ++k) {
     const PointOrder& q = o[k];
     if (q.n < 2) continue;
     if (q.n <= kOrderMax) {
-      OrderJob j = {};
-      j.verts = q.pts;
-      j.nv = j.n = q.n;
-      j.bits = morton_bits(q.n);
-      order_carve(j, scratch);
+      jobs.push_back(points_job(q, scratch));
       scratch += order_scratch(q.n, false);
-      j.v0 = q.perm;
-      j.is_new = q.is_new;
-      j.rows = q.rows;
-      j.rank = q.rank;
-      jobs.push_back(j);
       continue;
     }
     VTRY(points_order_large(ctx, q.pts, q.n, cnt, q.perm));
@@ -618,6 +618,18 @@ static int points_order(visacd_ctx* ctx, const PointOrder* o, int count, char* s
     }
   }
   return jobs.empty() ? VISACD_OK : order_run(ctx, jobs.data(), (int)jobs.size());
+}
+
+// Where a single-part call keeps its orders.
+static int order_slots(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint8_t* d_new, PointOrder& o) {
+  VTRY(ensure_slot(ctx, kSlotVisPerm, (size_t)n * 4));
+  o = {d_pts, n, slot<uint32_t>(ctx, kSlotVisPerm), d_new, nullptr, nullptr};
+  if (d_new) {
+    VTRY(ensure_slot(ctx, kSlotVisRank, (size_t)n * 4 + (size_t)n * 4 + 256));
+    o.rows = slot<uint32_t>(ctx, kSlotVisRank);
+    o.rank = reinterpret_cast<int32_t*>(o.rows + ((n + 63) & ~63));
+  }
+  return VISACD_OK;
 }
 
 // Morton order of n device points into perm; synchronizes.
@@ -637,7 +649,8 @@ int vis_morton_order(visacd_ctx* ctx, const float* d_pts, int32_t n, uint32_t* p
 
 static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint8_t* d_new,
                       const visacd_bvh* self_bvh, const visacd_bvh* cage_bvh, int64_t* n_edges,
-                      visacd_vis_stats* stats, int64_t pairs, int32_t n_new) {
+                      visacd_vis_stats* stats, int64_t pairs, int32_t n_new, const PointOrder* ordered,
+                      const uint32_t** few_edges) {
   // The cage's free-space grid, for calls with many pairs (`pairs`: the
   // call's pair count, or a bound of it): built once per cage BVH, before this
   // call's counters take the shared scratch and staging buffers.
@@ -656,16 +669,15 @@ static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint
     return VISACD_OK;
   }
   // Morton order of the points; rows: the new ones in order.
-  VTRY(ensure_slot(ctx, kSlotVisPerm, (size_t)n * 4));
-  uint32_t* perm = slot<uint32_t>(ctx, kSlotVisPerm);
-  PointOrder order = {d_pts, n, perm, d_new, nullptr, nullptr};
-  if (d_new) {
-    VTRY(ensure_slot(ctx, kSlotVisRank, (size_t)n * 4 + (size_t)n * 4 + 256));
-    order.rows = slot<uint32_t>(ctx, kSlotVisRank);
-    order.rank = reinterpret_cast<int32_t*>(order.rows + ((n + 63) & ~63));
+  PointOrder order;
+  if (ordered) {
+    order = *ordered;
+  } else {
+    VTRY(order_slots(ctx, d_pts, n, d_new, order));
+    VTRY(ensure_slot(ctx, kSlotVisOrder, points_scratch(&order, 1)));
+    VTRY(points_order(ctx, &order, 1, slot<char>(ctx, kSlotVisOrder), cnt));
   }
-  VTRY(ensure_slot(ctx, kSlotVisOrder, points_scratch(&order, 1)));
-  VTRY(points_order(ctx, &order, 1, slot<char>(ctx, kSlotVisOrder), cnt));
+  const uint32_t* perm = order.perm;
 
   const int variant = choose_vis_variant(ctx, n, d_new != nullptr, self_bvh, cage_bvh);
   const int TR = kVisVariants[variant].tr, TC = 32 / TR;
@@ -743,27 +755,38 @@ static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint
   P.cnt = cnt;
   P.status = ctx->d_status;
   if (P.total_tiles > 0) VTRY(launch_vis_variant(ctx, variant, P));
-  // Compaction: popcount, scan, emit in linear-pair order.
-  VTRY(ensure_slot(ctx, kSlotWordCounts, (size_t)nw * 4));
+  // Compaction: scan of the words' set bits, emit in linear-pair order.
   VTRY(ensure_slot(ctx, kSlotWordOffsets, (size_t)(nw + 1) * 8));
-  uint32_t* wc = slot<uint32_t>(ctx, kSlotWordCounts);
   uint64_t* wo = slot<uint64_t>(ctx, kSlotWordOffsets);
   const unsigned gw = grid_for(nw, 256, 16LL * ctx->sm_count);
-  VLAUNCH(ctx, kKBitPopc, gw, 256, 0, bit_popc_kernel, P.bitset, nw, wc);
-  VTRY(exclusive_scan_u32_to_u64(ctx, wc, wo, nw));
-  // Counters and the status word in one wait.
+  VTRY(exclusive_scan_bits(ctx, P.bitset, wo, nw));
+  // A call with few pairs has room for all of them as edges: they are emitted,
+  // and sent along with the counters, before their number is known here.
+  const bool few = np <= kFewPairs;
+  if (few) {
+    VTRY(ensure_slot(ctx, kSlotEdgesOut, (size_t)np * 8));
+    VLAUNCH(ctx, kKBitEmit, gw, 256, 0, bit_emit_kernel, P.bitset, nw, wo, (int64_t)n,
+            slot<uint32_t>(ctx, kSlotEdgesOut));
+  }
+  // Counters and the status word (and those edges) in one wait.
   VisCounters* h = nullptr;
   uint32_t* hs = nullptr;
-  VTRY(pinned(ctx, sizeof(VisCounters) + 64, (void**)&h));
-  hs = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(h) + ((sizeof(VisCounters) + 15) & ~size_t(15)));
+  constexpr size_t o_hs = (sizeof(VisCounters) + 15) & ~size_t(15);
+  const bool send = few && few_edges;
+  VTRY(pinned(ctx, o_hs + 64 + (send ? (size_t)np * 8 : 0), (void**)&h));
+  hs = reinterpret_cast<uint32_t*>(reinterpret_cast<char*>(h) + o_hs);
+  if (send) {
+    *few_edges = hs + 16;
+    VCUDA(cudaMemcpyAsync(hs + 16, ctx->buf[kSlotEdgesOut].p, (size_t)np * 8, cudaMemcpyDeviceToHost, ctx->stream));
+  }
   VCUDA(cudaMemcpyAsync(h, cnt, sizeof(VisCounters), cudaMemcpyDeviceToHost, ctx->stream));
   VCUDA(cudaMemcpyAsync(hs, ctx->d_status, sizeof(uint32_t), cudaMemcpyDeviceToHost, ctx->stream));
   VCUDA(stream_wait(ctx));
   const VisCounters hc = *h;
   VTRY(status_result(ctx, *hs, "visibility"));
   const int64_t ne = (int64_t)hc.edges;
-  VTRY(ensure_slot(ctx, kSlotEdgesOut, (size_t)(ne > 0 ? ne : 1) * 8));
-  if (ne > 0) {
+  if (ne > 0 && !few) {
+    VTRY(ensure_slot(ctx, kSlotEdgesOut, (size_t)ne * 8));
     VLAUNCH(ctx, kKBitEmit, gw, 256, 0, bit_emit_kernel, P.bitset, nw, wo, (int64_t)n,
             slot<uint32_t>(ctx, kSlotEdgesOut));
   }
@@ -1022,14 +1045,11 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
   }
   // Compaction over the concatenated bitset.
   const int64_t nw = (int64_t)words;
-  VTRY(ensure_slot(ctx, kSlotWordCounts, (size_t)std::max<int64_t>(nw, 1) * 4));
   VTRY(ensure_slot(ctx, kSlotWordOffsets, (size_t)(nw + 1) * 8));
-  uint32_t* wc = slot<uint32_t>(ctx, kSlotWordCounts);
   uint64_t* wo = slot<uint64_t>(ctx, kSlotWordOffsets);
   const unsigned gw = grid_for(std::max<int64_t>(nw, 1), 256, 16LL * ctx->sm_count);
   if (nw) {
-    VLAUNCH(ctx, kKBitPopc, gw, 256, 0, bit_popc_kernel, bits, nw, wc);
-    VTRY(exclusive_scan_u32_to_u64(ctx, wc, wo, nw));
+    VTRY(exclusive_scan_bits(ctx, bits, wo, nw));
   } else {
     VCUDA(cudaMemsetAsync(wo, 0, 8, ctx->stream));
   }
@@ -1112,7 +1132,55 @@ int visibility_impl(visacd_ctx* ctx, const float* pts, int32_t n, const uint8_t*
       d_new = slot<uint8_t>(ctx, kSlotMask);
     }
   }
-  return vis_device(ctx, d_pts, n, d_new, self_bvh, cage_bvh, n_edges, stats, pairs, n_new);
+  return vis_device(ctx, d_pts, n, d_new, self_bvh, cage_bvh, n_edges, stats, pairs, n_new, nullptr, nullptr);
+}
+
+// compute_intersection_matrix on checked input: the part, its mask and the
+// cage in one upload, both BVHs and the points' order in one launch.
+static int matrix_together(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* tris, int32_t nt,
+                           const uint8_t* is_new, const float* cage_verts, int32_t ncv, const uint32_t* cage_tris,
+                           int32_t nct, visacd_bvh** sb, visacd_bvh** cb, int64_t* n_edges, visacd_vis_stats* stats,
+                           const uint32_t** few_edges) {
+  VCUDA(cudaSetDevice(ctx->device));
+  auto al = [](size_t b) { return (b + 63) & ~size_t(63); };
+  const void* src[5] = {verts, tris, cage_verts, cage_tris, is_new};
+  const size_t bytes[5] = {(size_t)nv * 12, (size_t)nt * 12, (size_t)ncv * 12, (size_t)nct * 12,
+                           is_new ? (size_t)nv : 0};
+  size_t at[5], total = 0;
+  for (int k = 0; k < 5; ++k) {
+    at[k] = total;
+    total += al(bytes[k]);
+  }
+  VTRY(ensure_slot(ctx, kSlotBuildVerts, total));
+  char* d = slot<char>(ctx, kSlotBuildVerts);
+  Stager up(ctx);
+  VTRY(up.reserve(total, 1));
+  for (int k = 0; k < 5; ++k)
+    if (bytes[k]) memcpy(up.host() + at[k], src[k], bytes[k]);
+  VTRY(up.copy(d, total));
+  const float* d_pts = reinterpret_cast<const float*>(d + at[0]);
+  const uint8_t* d_new = is_new ? reinterpret_cast<const uint8_t*>(d + at[4]) : nullptr;
+  OrderJob jobs[3];
+  PointOrder order;
+  VTRY(order_slots(ctx, d_pts, nv, d_new, order));
+  VTRY(ensure_slot(ctx, kSlotTmpTris, order_scratch(nt, true) + order_scratch(nct, true) + order_scratch(nv, false)));
+  char* scratch = slot<char>(ctx, kSlotTmpTris);
+  VTRY(bvh_prepare(ctx, d_pts, nv, reinterpret_cast<const uint32_t*>(d + at[1]), nt, scratch, sb, jobs[0]));
+  scratch += order_scratch(nt, true);
+  VTRY(bvh_prepare(ctx, reinterpret_cast<const float*>(d + at[2]), ncv, reinterpret_cast<const uint32_t*>(d + at[3]),
+                   nct, scratch, cb, jobs[1]));
+  scratch += order_scratch(nct, true);
+  jobs[2] = points_job(order, scratch);
+  VTRY(order_run(ctx, jobs, 3));
+  VTRY(order_nodes(ctx, jobs, 2));
+  int64_t pairs = (int64_t)nv * (nv - 1) / 2;
+  int32_t n_new = -1;
+  if (is_new) {
+    n_new = 0;
+    for (int32_t v = 0; v < nv; ++v) n_new += is_new[v] != 0;
+    pairs -= ((int64_t)nv - n_new) * ((int64_t)nv - n_new - 1) / 2;
+  }
+  return vis_device(ctx, d_pts, nv, d_new, *sb, *cb, n_edges, stats, pairs, n_new, &order, few_edges);
 }
 
 }  // namespace vgpu
@@ -1163,18 +1231,33 @@ extern "C" int visacd_compute_intersection_matrix(
     visacd_vis_stats* stats) {
   VCHECK(ctx && n_edges, VISACD_ERR_INVALID_ARG, "compute_intersection_matrix: null argument");
   visacd_bvh *sb = nullptr, *cb = nullptr;
-  int rc = bvh_build(ctx, verts, nv, tris, nt, 0, &sb);
-  if (rc == VISACD_OK) rc = bvh_build(ctx, cage_verts, ncv, cage_tris, nct, 0, &cb);
-  if (rc == VISACD_OK) {
-    // A BVH over a mesh with no triangles still needs the vertex count check.
-    if (sb->nt == 0) sb->nv = nv;
-    rc = visibility_impl(ctx, verts, nv, is_new, 0, sb, cb, n_edges, stats);
+  const uint32_t* few_edges = nullptr;
+  int rc;
+  // Part and cage of ordinary size: one upload, both builds and the points'
+  // order in one launch. Anything else (and every refusal) one by one.
+  const bool together = verts && tris && cage_verts && cage_tris && nv >= 2 && nv <= kOrderMax && nt >= 1 &&
+                        nt <= kOrderMax && ncv >= 1 && nct >= 1 && nct <= kOrderMax &&
+                        indices_in_range(reinterpret_cast<const int32_t*>(tris), 3LL * nt, nv) &&
+                        indices_in_range(reinterpret_cast<const int32_t*>(cage_tris), 3LL * nct, ncv);
+  if (together) {
+    rc = matrix_together(ctx, verts, nv, tris, nt, is_new, cage_verts, ncv, cage_tris, nct, &sb, &cb, n_edges, stats,
+                         &few_edges);
+  } else {
+    rc = bvh_build(ctx, verts, nv, tris, nt, 0, &sb);
+    if (rc == VISACD_OK) rc = bvh_build(ctx, cage_verts, ncv, cage_tris, nct, 0, &cb);
+    if (rc == VISACD_OK) {
+      // A BVH over a mesh with no triangles still needs the vertex count check.
+      if (sb->nt == 0) sb->nv = nv;
+      rc = visibility_impl(ctx, verts, nv, is_new, 0, sb, cb, n_edges, stats);
+    }
   }
   if (rc == VISACD_OK) {
     if (*n_edges > capacity_edges) {
       set_error("compute_intersection_matrix: %lld edges exceed capacity %lld",
                 (long long)*n_edges, (long long)capacity_edges);
       rc = VISACD_ERR_CAPACITY;
+    } else if (few_edges && (edges_out || *n_edges == 0)) {
+      if (*n_edges) memcpy(edges_out, few_edges, (size_t)*n_edges * 8);
     } else {
       rc = visacd_visibility_edges(ctx, edges_out, capacity_edges);
     }
