@@ -29,8 +29,10 @@
 
 namespace vgpu {
 
+// Two CTAs asked for at every K (K = 4 then keeps four edges' values in
+// registers and still has three resident).
 template <int K>
-__global__ void __launch_bounds__(kScoreThreads, (K <= 4 ? 3 : 2))
+__global__ void __launch_bounds__(kScoreThreads, 2)
     score_planes_kernel(const float4* __restrict__ planes, int32_t P,
                         const EdgeRec* __restrict__ recs, int64_t E, int64_t blocks_per_cta,
                         const unsigned* __restrict__ stats,
@@ -259,7 +261,7 @@ static int launch_score(visacd_ctx* ctx, const float4* planes, int32_t P, const 
   const int per_cta = kScoreThreads * K;
   const int groups = (P + per_cta - 1) / per_cta;
   const int64_t nblocks = (E + kEdgeBlock - 1) / kEdgeBlock;
-  // Aim for ~4 CTAs per SM in total (3 resident for K <= 4, 2 for K = 8, so
+  // Aim for ~4 CTAs per SM in total (2 to 5 resident, fewer for larger K, so
   // the edge slices keep every SM busy to the end); each CTA streams a
   // contiguous run of blocks.
   int64_t target_ctas = 4LL * ctx->sm_count;
