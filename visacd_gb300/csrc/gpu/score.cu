@@ -261,9 +261,9 @@ static int launch_score(visacd_ctx* ctx, const float4* planes, int32_t P, const 
   const int per_cta = kScoreThreads * K;
   const int groups = (P + per_cta - 1) / per_cta;
   const int64_t nblocks = (E + kEdgeBlock - 1) / kEdgeBlock;
-  // Aim for ~4 CTAs per SM in total (2 to 5 resident, fewer for larger K, so
-  // the edge slices keep every SM busy to the end); each CTA streams a
-  // contiguous run of blocks.
+  // Aim for ~4 CTAs per SM in total (registers allow 4 resident for K = 2 and
+  // 2 for K = 4 and 8, so the edge slices keep every SM busy to the end); each
+  // CTA streams a contiguous run of blocks.
   int64_t target_ctas = 4LL * ctx->sm_count;
   int64_t slices = (target_ctas + groups - 1) / groups;
   if (slices > nblocks) slices = nblocks;
