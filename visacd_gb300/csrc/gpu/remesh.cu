@@ -4,19 +4,20 @@
 //
 // Same algorithm and arithmetic as the host restatement (manifold_preprocess in
 // csrc/host/remesh.cpp), so the output mesh is identical bit for bit:
-//  1. sdf_tri_prep_kernel computes each triangle's set-up once (voxel box,
-//     FP32 bounds and planes); the boxes are cut into work items of 1024
-//     voxels; sdf_ub_kernel gives every band voxel an FP32 upper bound of its
-//     distance, then sdf_dist_kernel gives every voxel centre in each
-//     triangle's box grown by the band the exact FP64 point-triangle distance
-//     (rounded to float) unless a lower bound rules it out, combined with
-//     atomicMin (non-negative floats order like their bit patterns).
-//  2. For each axis: sdf_cross_kernel marks, for every ray through voxel
-//     centres (offset by 1.2345679e-6 / 2.3456789e-6 voxels) that crosses a
-//     triangle at x, the first voxel whose centre lies beyond x (XOR toggle);
-//     sdf_parity_kernel runs the prefix parity along each ray and adds a vote
-//     where it is odd. Inside = at least two of the three votes.
-//  3. Surface nets: a vertex per sign-changing cell at the mean of its edge
+//  1. sdf_tri_prep_kernel computes each triangle's set-up once (voxel box, ray
+//     boxes, FP32 bounds and planes).
+//  2. Crossings: sdf_cross_kernel marks, for every ray along an axis through
+//     voxel centres (offset by 1.2345679e-6 / 2.3456789e-6 voxels) that crosses
+//     a triangle at x, the first voxel whose centre lies beyond x (one toggle
+//     bit per axis); sdf_parity_yz_kernel and sdf_inside_kernel run the prefix
+//     parities along the rays. Inside = at least two of the three odd.
+//  3. Distances: sdf_ub_kernel gives the voxels that matter an FP32 upper
+//     bound of their distance, then sdf_dist_kernel the exact FP64
+//     point-triangle distance (rounded to float) unless a lower bound rules
+//     the triangle out, combined with atomicMin (non-negative floats order
+//     like their bit patterns). The boxes are cut into work items of 1024
+//     voxels. Which voxels matter: see class_cut.
+//  4. Surface nets: a vertex per sign-changing cell at the mean of its edge
 //     crossings (cells in linear order, exclusive scan), two triangles per
 //     sign-changing grid edge whose four cells all have vertices (voxels in
 //     linear order, x / y / z edges, exclusive scan).
@@ -35,7 +36,22 @@ struct SdfGrid {
   float fiso;
   double scale;
   float margin;  // FP32 lower-bound margin (voxels): 1e-3 + 1e-6 max |grid coordinate|
+  float cut_out, low_out;  // outside voxels need their exact distance between these (class_cut)
 };
+
+// The output depends on a voxel's exact distance d only where a grid edge
+// joins a voxel with f < iso to one with f >= iso (f = -d for inside voxels, d
+// otherwise); elsewhere only the side counts. So with iso > 0:
+//  * a voxel next to one of the other class needs it (kClassEdge);
+//  * any other inside voxel does not: its neighbours are inside, f <= 0 < iso;
+//  * any other outside voxel needs it for iso - 1 <= d < iso + 1, since the
+//    distances of neighbours differ by at most 1: below, its neighbours are
+//    all on the f < iso side, above all on the other.
+// Elsewhere a voxel keeps the band or its upper bound, both on the right side.
+enum : uint8_t { kClassOut = 0, kClassIn = 1, kClassEdge = 2 };
+__device__ __forceinline__ float class_cut(const SdfGrid& g, uint8_t c) {
+  return (c & kClassEdge) ? 3.0e38f : ((c & kClassIn) ? 0.f : g.cut_out);
+}
 
 __device__ __forceinline__ size_t vid(const SdfGrid& g, int i, int j, int k) {
   return ((size_t)k * g.dim[1] + j) * g.dim[0] + i;
@@ -53,6 +69,18 @@ __device__ __forceinline__ void load_tri(const double* __restrict__ P, const int
 
 __device__ __forceinline__ double min3(double a, double b, double c) { return fmin(fmin(a, b), c); }
 __device__ __forceinline__ double max3(double a, double b, double c) { return fmax(fmax(a, b), c); }
+
+// The rays a triangle covers: its box projected on the grid plane.
+__device__ __forceinline__ bool ray_box(const double (&A)[3], const double (&B)[3], const double (&C)[3],
+                                        const SdfGrid& g, int u, int w, int& u0, int& w0, int& eu, int& ew) {
+  u0 = max(0, (int)floor(min3(A[u], B[u], C[u]) - g.org[u]));
+  const int u1 = min(g.dim[u] - 1, (int)ceil(max3(A[u], B[u], C[u]) - g.org[u]));
+  w0 = max(0, (int)floor(min3(A[w], B[w], C[w]) - g.org[w]));
+  const int w1 = min(g.dim[w] - 1, (int)ceil(max3(A[w], B[w], C[w]) - g.org[w]));
+  eu = u1 - u0 + 1;
+  ew = w1 - w0 + 1;
+  return eu > 0 && ew > 0;
+}
 
 // Lower-bound pre-filter of the exact distance: a voxel whose lower bound
 // (FP32, less twice a margin of 1e-3 voxel plus 1e-6 of the largest grid
@@ -75,6 +103,7 @@ struct SdfTri {
   float4 pl;              // unit normal, offset; w of fe[0] = -1e30 without a plane
   float4 fe[3];           // unit in-plane edge normals, offsets (no vertex beyond)
   int has_plane, pad[3];
+  int ray[3][4];          // per axis: first ray and extents over (u, w); extents 0: none
 };
 
 constexpr int kSdfChunk = 1024;  // box voxels per work item of the distance passes
@@ -128,6 +157,13 @@ __global__ void sdf_tri_prep_kernel(const double* __restrict__ P, const int32_t*
                                 mx * C[0] + my * C[1] + mz * C[2]);
         r.fe[e] = make_float4((float)mx, (float)my, (float)mz, (float)-top);
       }
+    }
+    for (int ax = 0; ax < 3; ++ax) {
+      const int u = (ax + 1) % 3, w = (ax + 2) % 3;
+      int eu, ew;
+      if (!ray_box(A, B, C, g, u, w, r.ray[ax][0], r.ray[ax][1], eu, ew)) eu = ew = 0;
+      r.ray[ax][2] = eu;
+      r.ray[ax][3] = ew;
     }
     out[t] = r;
     chunks[t] = r.ext[0] > 0 ? (uint32_t)((r.ext[0] * r.ext[1] * r.ext[2] + kSdfChunk - 1) / kSdfChunk) : 0u;
@@ -225,7 +261,7 @@ __device__ __forceinline__ float sdf_lower_bound(const SdfTri& r, float qx, floa
 
 __global__ void __launch_bounds__(128) sdf_ub_kernel(const double* __restrict__ P, const int32_t* __restrict__ T,
                                                      SdfItems W, SdfGrid g, const SdfTri* __restrict__ prep,
-                                                     uint32_t* __restrict__ ub) {
+                                                     const uint8_t* __restrict__ cls, uint32_t* __restrict__ ub) {
   long long w0, w1;
   item_range(W, w0, w1);
   int t = w0 < w1 ? item_triangle(W, w0) : 0;
@@ -248,8 +284,10 @@ __global__ void __launch_bounds__(128) sdf_ub_kernel(const double* __restrict__ 
                 k = r.lo[2] + q0 / (r.ext[0] * r.ext[1]);
       const size_t v = vid(g, i, j, k);
       const float qx = (float)(g.org[0] + i), qy = (float)(g.org[1] + j), qz = (float)(g.org[2] + k);
+      const float cut = class_cut(g, cls[v]);
+      if (cut <= 0.f) continue;
       const float lb = sdf_lower_bound(r, qx, qy, qz);
-      const float cur = __uint_as_float(*(volatile const uint32_t*)&ub[v]);
+      const float cur = fminf(cut, __uint_as_float(*(volatile const uint32_t*)&ub[v]));
       if (lb - 2.0f * g.margin >= cur) continue;
       const float qa = fmaxf(fabsf(qx), fmaxf(fabsf(qy), fabsf(qz)));
       const float slack = 64.0f * kSdfU * fmaxf(mabs, qa) + g.margin;
@@ -264,7 +302,8 @@ __global__ void __launch_bounds__(128) sdf_ub_kernel(const double* __restrict__ 
 // instead of the few lanes that pass the filter in each warp.
 __global__ void __launch_bounds__(128) sdf_dist_kernel(const double* __restrict__ P, const int32_t* __restrict__ T,
                                                        SdfItems W, SdfGrid g, const SdfTri* __restrict__ prep,
-                                                       const uint32_t* __restrict__ ub, uint32_t* __restrict__ dist) {
+                                                       const uint8_t* __restrict__ cls, const uint32_t* __restrict__ ub,
+                                                       uint32_t* __restrict__ dist) {
   __shared__ int list[kSdfChunk];
   __shared__ int count;
   const int lane = threadIdx.x & 31;
@@ -293,20 +332,27 @@ __global__ void __launch_bounds__(128) sdf_dist_kernel(const double* __restrict_
         const int i = lo0 + q0 % ex0, j = lo1 + (q0 / ex0) % ex1, k = lo2 + q0 / (ex0 * ex1);
         const size_t v = vid(g, i, j, k);
         const float qx = (float)(g.org[0] + i), qy = (float)(g.org[1] + j), qz = (float)(g.org[2] + k);
-        const float gx = fmaxf(fmaxf(blo0 - qx, qx - bhi0), 0.f);
-        const float gy = fmaxf(fmaxf(blo1 - qy, qy - bhi1), 0.f);
-        const float gz = fmaxf(fmaxf(blo2 - qz, qz - bhi2), 0.f);
-        float lb = sqrtf(gx * gx + gy * gy + gz * gz);
-        if (has_plane) {
-          const float pd = fabsf(pl.x * qx + pl.y * qy + pl.z * qz + pl.w);
-          float se = 0.f;
-          se = fmaxf(se, fe0.x * qx + fe0.y * qy + fe0.z * qz + fe0.w);
-          se = fmaxf(se, fe1.x * qx + fe1.y * qy + fe1.z * qz + fe1.w);
-          se = fmaxf(se, fe2.x * qx + fe2.y * qy + fe2.z * qz + fe2.w);
-          lb = fmaxf(lb, sqrtf(pd * pd + se * se));
+        const uint8_t c = cls[v];
+        const float up = __uint_as_float(ub[v]);
+        float cur = fminf(up, class_cut(g, c));
+        // an outside voxel whose upper bound is this low has no neighbour on
+        // the other side
+        if (c == kClassOut && up < g.low_out) cur = 0.f;
+        if (cur > 0.f) {
+          const float gx = fmaxf(fmaxf(blo0 - qx, qx - bhi0), 0.f);
+          const float gy = fmaxf(fmaxf(blo1 - qy, qy - bhi1), 0.f);
+          const float gz = fmaxf(fmaxf(blo2 - qz, qz - bhi2), 0.f);
+          float lb = sqrtf(gx * gx + gy * gy + gz * gz);
+          if (has_plane) {
+            const float pd = fabsf(pl.x * qx + pl.y * qy + pl.z * qz + pl.w);
+            float se = 0.f;
+            se = fmaxf(se, fe0.x * qx + fe0.y * qy + fe0.z * qz + fe0.w);
+            se = fmaxf(se, fe1.x * qx + fe1.y * qy + fe1.z * qz + fe1.w);
+            se = fmaxf(se, fe2.x * qx + fe2.y * qy + fe2.z * qz + fe2.w);
+            lb = fmaxf(lb, sqrtf(pd * pd + se * se));
+          }
+          keep = lb - 2.0f * g.margin < fminf(cur, __uint_as_float(*(volatile const uint32_t*)&dist[v]));
         }
-        const float cur = fminf(__uint_as_float(*(volatile const uint32_t*)&dist[v]), __uint_as_float(ub[v]));
-        keep = lb - 2.0f * g.margin < cur;
       }
       // warp-aggregated append (at most kSdfChunk entries per item)
       const unsigned m = __ballot_sync(0xffffffffu, keep);
@@ -352,97 +398,136 @@ __device__ __forceinline__ void cross_ray(const double (&A)[3], const double (&B
   gi[ax] = s;
   gi[u] = ku;
   gi[w] = kw;
-  atomicXor(&toggle[vid(g, gi[0], gi[1], gi[2])], 1u);
-}
-
-// The rays a triangle covers: its box projected on the grid plane.
-__device__ __forceinline__ bool ray_box(const double (&A)[3], const double (&B)[3], const double (&C)[3],
-                                        const SdfGrid& g, int u, int w, int& u0, int& w0, int& eu, int& ew) {
-  u0 = max(0, (int)floor(min3(A[u], B[u], C[u]) - g.org[u]));
-  const int u1 = min(g.dim[u] - 1, (int)ceil(max3(A[u], B[u], C[u]) - g.org[u]));
-  w0 = max(0, (int)floor(min3(A[w], B[w], C[w]) - g.org[w]));
-  const int w1 = min(g.dim[w] - 1, (int)ceil(max3(A[w], B[w], C[w]) - g.org[w]));
-  eu = u1 - u0 + 1;
-  ew = w1 - w0 + 1;
-  return eu > 0 && ew > 0;
+  atomicXor(&toggle[vid(g, gi[0], gi[1], gi[2])], 1u << ax);
 }
 
 // Triangles covering at most kCrossSmall rays (nearly all): kCrossLanes lanes
-// each, over its rays. Larger ones (the long triangles of clipped parts' caps,
-// big faces): one block each (sdf_cross_wide_kernel).
+// each, over its rays, blockIdx.y the axis. Bound by the latency of the loads
+// and atomics: all three axes in one launch, with one bit each, and the rays of
+// parities next to each other in x, took crossings and votes from 321 to 116 us
+// on 740,000 voxels. Larger ones (the long triangles of
+// clipped parts' caps, big faces) are listed with their axis and take one block
+// each (sdf_cross_wide_kernel).
 constexpr int kCrossSmall = 32;
 constexpr int kCrossLanes = 8;
 
 __global__ void __launch_bounds__(128) sdf_cross_kernel(const double* __restrict__ P, const int32_t* __restrict__ T,
-                                                        int nt, SdfGrid g, int ax, uint32_t* __restrict__ toggle,
-                                                        int* __restrict__ wide, unsigned* __restrict__ n_wide) {
-  const int u = (ax + 1) % 3, w = (ax + 2) % 3;
+                                                        int nt, SdfGrid g, const SdfTri* __restrict__ prep,
+                                                        uint32_t* __restrict__ toggle, int* __restrict__ wide,
+                                                        unsigned* __restrict__ n_wide) {
+  const int ax = blockIdx.y, u = (ax + 1) % 3, w = (ax + 2) % 3;
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
   const int sub = gid % kCrossLanes;
   const int groups = (gridDim.x * blockDim.x) / kCrossLanes;
   for (int t = gid / kCrossLanes; t < nt; t += groups) {
-    double A[3], B[3], C[3];
-    load_tri(P, T, t, A, B, C);
-    int u0, w0, eu, ew;
-    if (!ray_box(A, B, C, g, u, w, u0, w0, eu, ew)) continue;
-    if (eu * ew > kCrossSmall) {
-      if (sub == 0) wide[atomicAdd(n_wide, 1u)] = t;
+    const int4 r = *reinterpret_cast<const int4*>(prep[t].ray[ax]);
+    const int n = r.z * r.w;
+    if (n > kCrossSmall) {
+      if (sub == 0) wide[atomicAdd(n_wide, 1u)] = 3 * t + ax;
       continue;
     }
-    for (int r = sub; r < eu * ew; r += kCrossLanes)
-      cross_ray(A, B, C, g, ax, u, w, u0 + r % eu, w0 + r / eu, toggle);
+    if (sub >= n) continue;
+    double A[3], B[3], C[3];
+    load_tri(P, T, t, A, B, C);
+    for (int q = sub; q < n; q += kCrossLanes) cross_ray(A, B, C, g, ax, u, w, r.x + q % r.z, r.y + q / r.z, toggle);
   }
 }
 
 __global__ void __launch_bounds__(128) sdf_cross_wide_kernel(const double* __restrict__ P,
-                                                             const int32_t* __restrict__ T, SdfGrid g, int ax,
+                                                             const int32_t* __restrict__ T, SdfGrid g,
+                                                             const SdfTri* __restrict__ prep,
                                                              const int* __restrict__ wide,
                                                              const unsigned* __restrict__ n_wide,
                                                              uint32_t* __restrict__ toggle) {
-  const int u = (ax + 1) % 3, w = (ax + 2) % 3;
   const int nw = (int)*n_wide;
   for (int k = blockIdx.x; k < nw; k += gridDim.x) {
-    const int t = wide[k];
+    const int t = wide[k] / 3, ax = wide[k] % 3, u = (ax + 1) % 3, w = (ax + 2) % 3;
+    const int4 r = *reinterpret_cast<const int4*>(prep[t].ray[ax]);
     double A[3], B[3], C[3];
     load_tri(P, T, t, A, B, C);
-    int u0, w0, eu, ew;
-    if (!ray_box(A, B, C, g, u, w, u0, w0, eu, ew)) continue;
-    for (int r = threadIdx.x; r < eu * ew; r += blockDim.x)
-      cross_ray(A, B, C, g, ax, u, w, u0 + r % eu, w0 + r / eu, toggle);
+    for (int q = threadIdx.x; q < r.z * r.w; q += blockDim.x)
+      cross_ray(A, B, C, g, ax, u, w, r.x + q % r.z, r.y + q / r.z, toggle);
   }
 }
 
-__global__ void sdf_parity_kernel(SdfGrid g, int ax, const uint32_t* __restrict__ toggle,
-                                  uint8_t* __restrict__ votes) {
-  const int u = (ax + 1) % 3, w = (ax + 2) % 3;
-  const int ncol = g.dim[u] * g.dim[w];
+// Prefix parities along y (blockIdx.y 0) and z (1): one thread per ray, rays
+// next to each other in x, eight loads in flight.
+__global__ void __launch_bounds__(64) sdf_parity_yz_kernel(SdfGrid g, const uint32_t* __restrict__ toggle,
+                                                           uint8_t* __restrict__ par_y, uint8_t* __restrict__ par_z) {
+  const int ax = 1 + (int)blockIdx.y;
+  const int ncol = g.dim[0] * (ax == 1 ? g.dim[2] : g.dim[1]), n = ax == 1 ? g.dim[1] : g.dim[2];
+  const size_t stride = ax == 1 ? (size_t)g.dim[0] : (size_t)g.dim[0] * g.dim[1];
+  uint8_t* out = ax == 1 ? par_y : par_z;
   for (int col = blockIdx.x * blockDim.x + threadIdx.x; col < ncol; col += gridDim.x * blockDim.x) {
-    int gi[3];
-    gi[u] = col % g.dim[u];
-    gi[w] = col / g.dim[u];
+    const int i = col % g.dim[0], o = col / g.dim[0];
+    const size_t base = ax == 1 ? vid(g, i, 0, o) : vid(g, i, o, 0);
     uint32_t par = 0;
-    for (int i = 0; i < g.dim[ax]; ++i) {
-      gi[ax] = i;
-      const size_t v = vid(g, gi[0], gi[1], gi[2]);
-      par ^= toggle[v];
-      if (par & 1u) votes[v] += 1;
+    for (int s = 0; s < n; s += 8) {
+      uint32_t t[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) t[q] = s + q < n ? toggle[base + (size_t)(s + q) * stride] >> ax : 0u;
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        par ^= t[q];
+        if (s + q < n) out[base + (size_t)(s + q) * stride] = (uint8_t)(par & 1u);
+      }
     }
   }
 }
 
-__global__ void sdf_field_kernel(const uint32_t* __restrict__ dist, const uint8_t* __restrict__ votes, size_t n,
-                                 float* __restrict__ f) {
+// Prefix parity along x (one warp per row, 32 voxels at a time by ballot) and
+// the class of every voxel: inside when at least two parities are odd.
+__global__ void __launch_bounds__(128) sdf_inside_kernel(SdfGrid g, const uint32_t* __restrict__ toggle,
+                                                         const uint8_t* __restrict__ par_y,
+                                                         const uint8_t* __restrict__ par_z,
+                                                         uint8_t* __restrict__ inside) {
+  const int lane = threadIdx.x & 31;
+  const int rows = g.dim[1] * g.dim[2], warps = (gridDim.x * blockDim.x) >> 5;
+  for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
+    const size_t base = (size_t)r * g.dim[0];
+    uint32_t carry = 0;
+    for (int i0 = 0; i0 < g.dim[0]; i0 += 32) {
+      const int i = i0 + lane;
+      const bool in_grid = i < g.dim[0];
+      const unsigned m = __ballot_sync(0xffffffffu, in_grid && (toggle[base + i] & 1u));
+      const uint32_t px = (carry + __popc(m & (0xffffffffu >> (31 - lane)))) & 1u;
+      if (in_grid) inside[base + i] = px + par_y[base + i] + par_z[base + i] >= 2u ? kClassIn : kClassOut;
+      carry += __popc(m);
+    }
+  }
+}
+
+// Marks voxels with a neighbour of the other class (all: every voxel, when
+// the range of class_cut does not apply), and starts both distance arrays at the
+// band.
+__global__ void sdf_class_kernel(SdfGrid g, const uint8_t* __restrict__ inside, int all, uint32_t band,
+                                 uint8_t* __restrict__ cls, uint32_t* __restrict__ ub, uint32_t* __restrict__ dist) {
+  const size_t n = (size_t)g.dim[0] * g.dim[1] * g.dim[2];
+  const size_t sy = g.dim[0], sz = (size_t)g.dim[0] * g.dim[1];
   for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (size_t)gridDim.x * blockDim.x) {
-    const float d = __uint_as_float(dist[v]);
-    f[v] = votes[v] >= 2 ? -d : d;
+    const int i = (int)(v % g.dim[0]), j = (int)((v / g.dim[0]) % g.dim[1]), k = (int)(v / sz);
+    const uint8_t c = inside[v];
+    const bool edge = all || (i > 0 && inside[v - 1] != c) || (i + 1 < g.dim[0] && inside[v + 1] != c) ||
+                      (j > 0 && inside[v - sy] != c) || (j + 1 < g.dim[1] && inside[v + sy] != c) ||
+                      (k > 0 && inside[v - sz] != c) || (k + 1 < g.dim[2] && inside[v + sz] != c);
+    cls[v] = c | (edge ? kClassEdge : 0);
+    ub[v] = band;
+    dist[v] = band;
+  }
+}
+
+// The field: the exact distance where it was needed (the upper bound is never
+// below it), a value on its side elsewhere.
+__global__ void sdf_field_kernel(const uint32_t* __restrict__ dist, const uint32_t* __restrict__ ub,
+                                 const uint8_t* __restrict__ cls, size_t n, float* __restrict__ f) {
+  for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (size_t)gridDim.x * blockDim.x) {
+    const float d = fminf(__uint_as_float(dist[v]), __uint_as_float(ub[v]));
+    f[v] = (cls[v] & kClassIn) ? -d : d;
   }
 }
 
 __constant__ int kCorner[8][3] = {{0, 0, 0}, {1, 0, 0}, {0, 1, 0}, {1, 1, 0},
                                   {0, 0, 1}, {1, 0, 1}, {0, 1, 1}, {1, 1, 1}};
-__constant__ int kCedge[12][2] = {{0, 1}, {2, 3}, {4, 5}, {6, 7}, {0, 2}, {1, 3},
-                                  {4, 6}, {5, 7}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
-
 __device__ __forceinline__ int corner_values(const SdfGrid& g, const float* __restrict__ f, int i, int j, int k,
                                              float (&cv)[8]) {
   int nin = 0;
@@ -464,35 +549,52 @@ __global__ void sdf_cell_flag_kernel(SdfGrid g, const float* __restrict__ f, uin
   }
 }
 
-__global__ void sdf_cell_vertex_kernel(SdfGrid g, const float* __restrict__ f, const uint32_t* __restrict__ flag,
-                                       const uint64_t* __restrict__ off, int32_t* __restrict__ cell_vertex,
-                                       double* __restrict__ out_v) {
-  const int cx = g.dim[0] - 1, cy = g.dim[1] - 1, cz = g.dim[2] - 1;
-  const size_t n = (size_t)cx * cy * cz;
+// Vertex number of every cell (-1: none) and the cells that have one, in order.
+__global__ void sdf_cell_list_kernel(size_t n, const uint32_t* __restrict__ flag, const uint64_t* __restrict__ off,
+                                     int32_t* __restrict__ cell_vertex, uint32_t* __restrict__ cells) {
   for (size_t c = (size_t)blockIdx.x * blockDim.x + threadIdx.x; c < n; c += (size_t)gridDim.x * blockDim.x) {
-    if (!flag[c]) {
-      cell_vertex[c] = -1;
-      continue;
-    }
+    const bool has = flag[c] != 0;
+    const int vtx = (int)off[c];
+    cell_vertex[c] = has ? vtx : -1;
+    if (has) cells[vtx] = (uint32_t)c;
+  }
+}
+
+// One thread per vertex, over the list, so that FP64 runs with full warps: of
+// the cells themselves only about one in twenty-five has a vertex, and the same
+// arithmetic over all of 740,000 took 189 us; now all seven launches of the
+// cells, quads and field take 89 us.
+__global__ void __launch_bounds__(64) sdf_cell_vertex_kernel(SdfGrid g, const float* __restrict__ f,
+                                                             const uint32_t* __restrict__ cells, size_t n,
+                                                             double* __restrict__ out_v) {
+  const int cx = g.dim[0] - 1, cy = g.dim[1] - 1;
+  for (size_t vtx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; vtx < n; vtx += (size_t)gridDim.x * blockDim.x) {
+    const size_t c = cells[vtx];
     const int i = (int)(c % cx), j = (int)((c / cx) % cy), k = (int)(c / ((size_t)cx * cy));
     float cv[8];
     corner_values(g, f, i, j, k, cv);
     double acc[3] = {0, 0, 0};
     int ncross = 0;
+#pragma unroll
     for (int e = 0; e < 12; ++e) {
-      const int c0 = kCedge[e][0], c1 = kCedge[e][1];
+      // Edges 0-3 run along x, 4-7 along y, 8-11 along z (kCedge).
+      constexpr int kC[12][2] = {{0, 1}, {2, 3}, {4, 5}, {6, 7}, {0, 2}, {1, 3},
+                                 {4, 6}, {5, 7}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
+      const int c0 = kC[e][0], c1 = kC[e][1];
       if ((cv[c0] < g.fiso) == (cv[c1] < g.fiso)) continue;
       const double t = __ddiv_rn((double)__fsub_rn(g.fiso, cv[c0]), (double)__fsub_rn(cv[c1], cv[c0]));
-      for (int a = 0; a < 3; ++a)
-        acc[a] = da(acc[a], da((double)kCorner[c0][a], dm(t, (double)(kCorner[c1][a] - kCorner[c0][a]))));
+#pragma unroll
+      for (int a = 0; a < 3; ++a) {
+        const int s0 = (c0 >> a) & 1, s1 = (c1 >> a) & 1;  // kCorner
+        acc[a] = da(acc[a], da((double)s0, dm(t, (double)(s1 - s0))));
+      }
       ++ncross;
     }
-    const int vtx = (int)off[c];
-    cell_vertex[c] = vtx;
     const int ijk[3] = {i, j, k};
+#pragma unroll
     for (int a = 0; a < 3; ++a) {
       const double m = __ddiv_rn(acc[a], (double)ncross);
-      out_v[3 * (size_t)vtx + a] = __ddiv_rn(da((double)(g.org[a] + ijk[a]), m), g.scale);
+      out_v[3 * vtx + a] = __ddiv_rn(da((double)(g.org[a] + ijk[a]), m), g.scale);
     }
   }
 }
@@ -546,10 +648,6 @@ __global__ void sdf_quad_kernel(SdfGrid g, const float* __restrict__ f, const in
   }
 }
 
-__global__ void sdf_fill_kernel(uint32_t* __restrict__ p, size_t n, uint32_t v) {
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = v;
-}
-
 size_t align256(size_t x) { return (x + 255) & ~size_t(255); }
 
 }  // namespace
@@ -591,6 +689,11 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   for (int a = 0; a < 3; ++a)
     qmax = std::max(qmax, std::max(std::fabs((double)g.org[a]), std::fabs((double)g.org[a] + g.dim[a])));
   g.margin = (float)(1e-3 + 1e-6 * qmax);
+  // The range of class_cut, wider by 0.01 for the rounding of the distances to
+  // float and by the lower bounds' margin; it does not hold for iso <= 0.
+  const bool all_exact = !(iso > 0.0);
+  g.cut_out = (float)(iso + 1.0 + 0.01) + 2.0f * g.margin;
+  g.low_out = (float)(iso - 1.0 - 0.01);
   const size_t nvox = (size_t)g.dim[0] * g.dim[1] * g.dim[2];
   VCHECK(nvox <= ((size_t)1 << 30), VISACD_ERR_CAPACITY, "sdf_remesh: grid of %zu voxels is too large", nvox);
   const size_t ncell = (size_t)(g.dim[0] - 1) * (g.dim[1] - 1) * (g.dim[2] - 1);
@@ -602,20 +705,23 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
     at += align256(bytes);
     return o;
   };
-  const size_t oP = take(P.size() * 8), oT = take(3 * (size_t)nt * 4), oPrep = take((size_t)nt * sizeof(SdfTri)),
-               oWide = take(3 * (size_t)nt * 4), oNWide = take(16), oChunks = take((size_t)nt * 4),
-               oChunkOff = take(((size_t)nt + 1) * 8),
-               oDist = take(nvox * 4),
-               oTog = take(nvox * 4), oVotes = take(nvox), oF = take(nvox * 4), oFlag = take(ncell * 4),
-               oCoff = take((ncell + 1) * 8), oCv = take(ncell * 4), oQcnt = take(nint * 4),
-               oQoff = take((nint + 1) * 8);
+  const size_t oP = take(P.size() * 8), oT = take(3 * (size_t)nt * 4);
+  const size_t upload = at;
+  const size_t oTog = take(nvox * 4), oNWide = take(16);
+  const size_t zero_end = at;
+  const size_t oPrep = take((size_t)nt * sizeof(SdfTri)), oWide = take(3 * (size_t)nt * 4),
+               oChunks = take((size_t)nt * 4), oChunkOff = take(((size_t)nt + 1) * 8), oDist = take(nvox * 4),
+               oUb = take(nvox * 4), oPy = take(nvox), oPz = take(nvox), oIn = take(nvox), oCls = take(nvox),
+               oF = take(nvox * 4), oFlag = take(ncell * 4), oCoff = take((ncell + 1) * 8), oCv = take(ncell * 4),
+               oQcnt = take(nint * 4), oQoff = take((nint + 1) * 8);
   VTRY(ensure_slot(ctx, kSlotSdf, at));
   char* base = slot<char>(ctx, kSlotSdf);
   double* dP = (double*)(base + oP);
   int32_t* dT = (int32_t*)(base + oT);
   uint32_t* dist = (uint32_t*)(base + oDist);
-  uint32_t* tog = (uint32_t*)(base + oTog);
-  uint8_t* votes = (uint8_t*)(base + oVotes);
+  uint32_t *tog = (uint32_t*)(base + oTog), *ub = (uint32_t*)(base + oUb);
+  uint8_t *par_y = (uint8_t*)(base + oPy), *par_z = (uint8_t*)(base + oPz), *inside = (uint8_t*)(base + oIn),
+          *cls = (uint8_t*)(base + oCls);
   float* f = (float*)(base + oF);
   uint32_t* flag = (uint32_t*)(base + oFlag);
   uint64_t* coff = (uint64_t*)(base + oCoff);
@@ -624,59 +730,63 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   uint64_t* qoff = (uint64_t*)(base + oQoff);
   cudaStream_t st = ctx->stream;
   Stager up(ctx);
-  VTRY(up.reserve(P.size() * 8 + 3 * (size_t)nt * 4, 2));
-  VTRY(up.put(dP, P.data(), P.size() * 8));
-  VTRY(up.put(dT, tris, 3 * (size_t)nt * 4));
+  VTRY(up.reserve(upload, 1));
+  std::memcpy(up.host() + oP, P.data(), P.size() * 8);
+  std::memcpy(up.host() + oT, tris, 3 * (size_t)nt * 4);
+  VTRY(up.copy(base, upload));
+  VCUDA(cudaMemsetAsync(base + oTog, 0, zero_end - oTog, st));
   const unsigned gv = grid_for((int64_t)nvox, 256, 16 * (int64_t)ctx->sm_count);
   const float band_f = (float)g.band;
   uint32_t band_bits;
   std::memcpy(&band_bits, &band_f, 4);
-  VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_fill_kernel, dist, nvox, band_bits);
-  VCUDA(cudaMemsetAsync(votes, 0, nvox, st));
   SdfTri* prep = (SdfTri*)(base + oPrep);
   uint32_t* chunks = (uint32_t*)(base + oChunks);
   uint64_t* chunk_off = (uint64_t*)(base + oChunkOff);
-  VLAUNCH(ctx, kKSdfDist, grid_for(nt, 128, 16 * (int64_t)ctx->sm_count), 128, 0, sdf_tri_prep_kernel, dP, dT, nt,
+  VLAUNCH(ctx, kKSdfDist, grid_for(nt, 64, 32 * (int64_t)ctx->sm_count), 64, 0, sdf_tri_prep_kernel, dP, dT, nt,
           g, prep, chunks);
+  // Crossings of all three axes, the triangles covering many rays one block
+  // each, then the parities and classes.
+  int* wide = (int*)(base + oWide);
+  unsigned* n_wide = (unsigned*)(base + oNWide);
+  VLAUNCH(ctx, kKSdfCross, dim3(grid_for((int64_t)kCrossLanes * nt, 128, 16 * (int64_t)ctx->sm_count), 3), 128, 0,
+          sdf_cross_kernel, dP, dT, nt, g, (const SdfTri*)prep, tog, wide, n_wide);
+  VLAUNCH(ctx, kKSdfCross, (unsigned)std::min<int64_t>(3LL * nt, 4 * (int64_t)ctx->sm_count), 128, 0,
+          sdf_cross_wide_kernel, dP, dT, g, (const SdfTri*)prep, (const int*)wide, (const unsigned*)n_wide, tog);
+  VLAUNCH(ctx, kKSdfCross,
+          dim3(grid_for((int64_t)g.dim[0] * std::max(g.dim[1], g.dim[2]), 64, 32 * (int64_t)ctx->sm_count), 2), 64, 0,
+          sdf_parity_yz_kernel, g, (const uint32_t*)tog, par_y, par_z);
+  VLAUNCH(ctx, kKSdfCross, grid_for(32LL * g.dim[1] * g.dim[2], 128, 16 * (int64_t)ctx->sm_count), 128, 0,
+          sdf_inside_kernel, g, (const uint32_t*)tog, (const uint8_t*)par_y, (const uint8_t*)par_z, inside);
+  VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_class_kernel, g, (const uint8_t*)inside, all_exact ? 1 : 0, band_bits, cls, ub,
+          dist);
   VTRY(exclusive_scan_u32_to_u64(ctx, chunks, chunk_off, nt));
   SdfItems items;
   items.off = chunk_off;
   items.nt = nt;
   const unsigned gw = (unsigned)(8 * (int64_t)ctx->sm_count);
-  // First pass: FP32 upper bounds per voxel in the toggle buffer (free until
-  // the crossings), then the exact pass.
-  VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_fill_kernel, tog, nvox, band_bits);
-  VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_ub_kernel, dP, dT, items, g, (const SdfTri*)prep, tog);
-  VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_dist_kernel, dP, dT, items, g, (const SdfTri*)prep, (const uint32_t*)tog,
-          dist);
-  // Per axis: the triangles covering many rays are listed by the first
-  // kernel and done one block each by the second (lists and counts per axis).
-  int* wide = (int*)(base + oWide);
-  unsigned* n_wide = (unsigned*)(base + oNWide);
-  VCUDA(cudaMemsetAsync(n_wide, 0, 16, st));
-  for (int ax = 0; ax < 3; ++ax) {
-    VCUDA(cudaMemsetAsync(tog, 0, nvox * 4, st));
-    VLAUNCH(ctx, kKSdfCross, grid_for((int64_t)kCrossLanes * nt, 128, 16 * (int64_t)ctx->sm_count), 128, 0,
-            sdf_cross_kernel, dP, dT, nt, g, ax, tog, wide + (size_t)ax * nt, n_wide + ax);
-    VLAUNCH(ctx, kKSdfCross, (unsigned)std::min<int64_t>(nt, 4 * (int64_t)ctx->sm_count), 128, 0,
-            sdf_cross_wide_kernel, dP, dT, g, ax, (const int*)(wide + (size_t)ax * nt),
-            (const unsigned*)(n_wide + ax), tog);
-    const int u = (ax + 1) % 3, w = (ax + 2) % 3;
-    VLAUNCH(ctx, kKSdfCross, grid_for((int64_t)g.dim[u] * g.dim[w], 128, 1 << 20), 128, 0, sdf_parity_kernel, g, ax,
-            tog, votes);
-  }
-  VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_field_kernel, dist, votes, nvox, f);
+  // First pass: FP32 upper bounds per voxel, then the exact pass.
+  VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_ub_kernel, dP, dT, items, g, (const SdfTri*)prep, (const uint8_t*)cls, ub);
+  VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_dist_kernel, dP, dT, items, g, (const SdfTri*)prep, (const uint8_t*)cls,
+          (const uint32_t*)ub, dist);
+  VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_field_kernel, (const uint32_t*)dist, (const uint32_t*)ub, (const uint8_t*)cls,
+          nvox, f);
   const unsigned gc = grid_for((int64_t)ncell, 256, 16 * (int64_t)ctx->sm_count);
   VLAUNCH(ctx, kKSdf, gc, 256, 0, sdf_cell_flag_kernel, g, f, flag);
   VTRY(exclusive_scan_u32_to_u64(ctx, flag, coff, (int64_t)ncell));
   const unsigned gq = grid_for((int64_t)nint, 256, 16 * (int64_t)ctx->sm_count);
-  uint64_t totals[2];
+  uint64_t* totals = nullptr;
+  VTRY(pinned(ctx, 2 * sizeof(uint64_t), (void**)&totals));
   VCUDA(cudaMemcpyAsync(&totals[0], coff + ncell, 8, cudaMemcpyDeviceToHost, st));
   VCUDA(stream_wait(ctx));
   VCHECK(totals[0] < (1ull << 31), VISACD_ERR_CAPACITY, "sdf_remesh: too many vertices");
-  VTRY(ensure_slot(ctx, kSlotSdfOut, align256(totals[0] * 24) + 256));
+  // (the vertices, then the list of their cells)
+  VTRY(ensure_slot(ctx, kSlotSdfOut, align256(totals[0] * 24) + totals[0] * 4 + 256));
   double* out_v = slot<double>(ctx, kSlotSdfOut);
-  VLAUNCH(ctx, kKSdf, gc, 256, 0, sdf_cell_vertex_kernel, g, f, flag, coff, cv, out_v);
+  uint32_t* cells = reinterpret_cast<uint32_t*>(slot<char>(ctx, kSlotSdfOut) + align256(totals[0] * 24));
+  VLAUNCH(ctx, kKSdf, gc, 256, 0, sdf_cell_list_kernel, ncell, flag, coff, cv, cells);
+  if (totals[0])
+    VLAUNCH(ctx, kKSdf, grid_for((int64_t)totals[0], 64, 32 * (int64_t)ctx->sm_count), 64, 0, sdf_cell_vertex_kernel,
+            g, f, (const uint32_t*)cells, (size_t)totals[0], out_v);
   VLAUNCH(ctx, kKSdf, gq, 256, 0, sdf_quad_kernel, g, f, cv, qcnt, (const uint64_t*)nullptr,
           (int32_t*)nullptr);
   VTRY(exclusive_scan_u32_to_u64(ctx, qcnt, qoff, (int64_t)nint));
@@ -695,16 +805,20 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
 extern "C" int visacd_sdf_fetch(visacd_ctx* ctx, double* verts, int32_t* tris) {
   VCHECK(ctx, VISACD_ERR_INVALID_ARG, "sdf_fetch: null context");
   VCUDA(cudaSetDevice(ctx->device));
-  if (ctx->sdf_nv > 0) {
-    VCHECK(verts, VISACD_ERR_INVALID_ARG, "sdf_fetch: null vertex buffer");
-    VCUDA(cudaMemcpyAsync(verts, slot<double>(ctx, kSlotSdfOut), (size_t)ctx->sdf_nv * 24, cudaMemcpyDeviceToHost,
-                          ctx->stream));
-  }
-  if (ctx->sdf_nt > 0) {
-    VCHECK(tris, VISACD_ERR_INVALID_ARG, "sdf_fetch: null triangle buffer");
-    VCUDA(cudaMemcpyAsync(tris, slot<int32_t>(ctx, kSlotSdfTris), (size_t)ctx->sdf_nt * 12, cudaMemcpyDeviceToHost,
-                          ctx->stream));
-  }
+  VCHECK(ctx->sdf_nv == 0 || verts, VISACD_ERR_INVALID_ARG, "sdf_fetch: null vertex buffer");
+  VCHECK(ctx->sdf_nt == 0 || tris, VISACD_ERR_INVALID_ARG, "sdf_fetch: null triangle buffer");
+  // Through the pinned buffer (both copies in flight at once, one wait) up to
+  // 64 MiB; larger meshes go straight to the caller's memory.
+  const size_t bv = (size_t)ctx->sdf_nv * 24, bt = (size_t)ctx->sdf_nt * 12;
+  const bool staged = bv + bt <= (64u << 20);
+  char* h = nullptr;
+  if (staged) VTRY(pinned(ctx, bv + bt + 1, (void**)&h));
+  void* hv = staged ? (void*)h : (void*)verts;
+  void* ht = staged ? (void*)(h + bv) : (void*)tris;
+  if (bv) VCUDA(cudaMemcpyAsync(hv, slot<double>(ctx, kSlotSdfOut), bv, cudaMemcpyDeviceToHost, ctx->stream));
+  if (bt) VCUDA(cudaMemcpyAsync(ht, slot<int32_t>(ctx, kSlotSdfTris), bt, cudaMemcpyDeviceToHost, ctx->stream));
   VCUDA(stream_wait(ctx));
+  if (staged && bv) std::memcpy(verts, h, bv);
+  if (staged && bt) std::memcpy(tris, h + bv, bt);
   return VISACD_OK;
 }
