@@ -15,7 +15,7 @@
 //     bound of their distance, then sdf_dist_kernel the exact FP64
 //     point-triangle distance (rounded to float) unless a lower bound rules
 //     the triangle out, combined with atomicMin (non-negative floats order
-//     like their bit patterns). The boxes are cut into work items of 1024
+//     like their bit patterns). The boxes are cut into work items of 256
 //     voxels. Which voxels matter: see class_cut.
 //  4. Surface nets: a vertex per sign-changing cell at the mean of its edge
 //     crossings (cells in linear order, exclusive scan), two triangles per
@@ -37,6 +37,7 @@ struct SdfGrid {
   double scale;
   float margin;  // FP32 lower-bound margin (voxels): 1e-3 + 1e-6 max |grid coordinate|
   float cut_out, low_out;  // outside voxels need their exact distance between these (class_cut)
+  double reach;            // the voxel boxes of triangles are grown by this
 };
 
 // The output depends on a voxel's exact distance d only where a grid edge
@@ -48,7 +49,11 @@ struct SdfGrid {
 //    distances of neighbours differ by at most 1: below, its neighbours are
 //    all on the f < iso side, above all on the other.
 // Elsewhere a voxel keeps the band or its upper bound, both on the right side.
-enum : uint8_t { kClassOut = 0, kClassIn = 1, kClassEdge = 2 };
+// So boxes grown by cut_out instead of the band find every distance that is
+// needed, but those of kClassEdge voxels farther out (a mesh that is not closed):
+// sdf_far_kernel marks these kClassFar and sdf_far_dist_kernel, which does
+// nothing without them, goes over the boxes grown by the band.
+enum : uint8_t { kClassOut = 0, kClassIn = 1, kClassEdge = 2, kClassFar = 4 };
 __device__ __forceinline__ float class_cut(const SdfGrid& g, uint8_t c) {
   return (c & kClassEdge) ? 3.0e38f : ((c & kClassIn) ? 0.f : g.cut_out);
 }
@@ -94,8 +99,8 @@ __device__ __forceinline__ bool ray_box(const double (&A)[3], const double (&B)[
 // normal and m_e the unit in-plane normal of edge e pointing away from the
 // triangle (offset so that no vertex lies beyond it), every triangle point x
 // has |q - x|^2 >= (n.(q - x))^2 + (m_e.(q - x))^2 >= p^2 + s_e^2.
-// Per-triangle set-up of the band distances (one thread per triangle, once):
-// the voxel box grown by the band, the FP32 bounding box, and the FP32 plane
+// Per-triangle set-up of the distances (one thread per triangle, once): the
+// voxel box grown by the reach, the vertices in FP32, the FP32 bounding box, and the FP32 plane
 // and edge planes of the lower bound.
 struct SdfTri {
   int lo[3], ext[3];      // voxel box (ext[0] <= 0: nothing in the grid)
@@ -104,9 +109,16 @@ struct SdfTri {
   float4 fe[3];           // unit in-plane edge normals, offsets (no vertex beyond)
   int has_plane, pad[3];
   int ray[3][4];          // per axis: first ray and extents over (u, w); extents 0: none
+  float v[3][3], vabs;    // vertices in FP32, their largest coordinate
+  int pad2[2];
 };
 
-constexpr int kSdfChunk = 1024;  // box voxels per work item of the distance passes
+constexpr int kSdfChunk = 256;  // box voxels per work item of the distance passes (one warp)
+
+__device__ __forceinline__ void box_range(const SdfGrid& g, int a, double mn, double mx, double by, int& lo, int& ext) {
+  lo = max(0, (int)floor(mn - by) - g.org[a]);
+  ext = min(g.dim[a] - 1, (int)ceil(mx + by) - g.org[a]) - lo + 1;
+}
 
 __global__ void sdf_tri_prep_kernel(const double* __restrict__ P, const int32_t* __restrict__ T, int nt, SdfGrid g,
                                     SdfTri* __restrict__ out, uint32_t* __restrict__ chunks) {
@@ -116,9 +128,7 @@ __global__ void sdf_tri_prep_kernel(const double* __restrict__ P, const int32_t*
     SdfTri r;
     for (int a = 0; a < 3; ++a) {
       const double mn = min3(A[a], B[a], C[a]), mx = max3(A[a], B[a], C[a]);
-      r.lo[a] = max(0, (int)floor(mn - g.band) - g.org[a]);
-      const int hi = min(g.dim[a] - 1, (int)ceil(mx + g.band) - g.org[a]);
-      r.ext[a] = hi - r.lo[a] + 1;
+      box_range(g, a, mn, mx, g.reach, r.lo[a], r.ext[a]);
       r.blo[a] = __double2float_rd(mn);
       r.bhi[a] = __double2float_ru(mx);
     }
@@ -165,16 +175,23 @@ __global__ void sdf_tri_prep_kernel(const double* __restrict__ P, const int32_t*
       r.ray[ax][2] = eu;
       r.ray[ax][3] = ew;
     }
+    r.vabs = 0.f;
+    for (int a = 0; a < 3; ++a) {
+      r.v[0][a] = (float)A[a];
+      r.v[1][a] = (float)B[a];
+      r.v[2][a] = (float)C[a];
+      r.vabs = fmaxf(r.vabs, fmaxf(fabsf(r.v[0][a]), fmaxf(fabsf(r.v[1][a]), fabsf(r.v[2][a]))));
+    }
     out[t] = r;
     chunks[t] = r.ext[0] > 0 ? (uint32_t)((r.ext[0] * r.ext[1] * r.ext[2] + kSdfChunk - 1) / kSdfChunk) : 0u;
   }
 }
 
 // Work items of the distance passes: (triangle, chunk of kSdfChunk voxels of
-// its box), numbered by the scanned chunk counts. Block b takes a contiguous
+// its box), numbered by the scanned chunk counts. Each warp takes a contiguous
 // range of items, so a triangle with a large box (the long triangles of a
-// clipped part's cap) is spread over several blocks instead of holding one
-// while the rest of the grid idles.
+// clipped part's cap) is spread over many warps instead of holding one while
+// the rest of the grid idles.
 struct SdfItems {
   const uint64_t* off;  // nt + 1 scanned chunk counts
   int nt;
@@ -182,10 +199,34 @@ struct SdfItems {
 
 __device__ __forceinline__ void item_range(const SdfItems& W, long long& w0, long long& w1) {
   const long long total = (long long)W.off[W.nt];
-  const long long per = (total + gridDim.x - 1) / gridDim.x;
-  w0 = (long long)blockIdx.x * per;
+  const long long warps = ((long long)gridDim.x * blockDim.x) >> 5;
+  const long long per = (total + warps - 1) / warps;
+  w0 = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * per;
   w1 = min(total, w0 + per);
 }
+
+// Position of a lane in a box walked 32 voxels at a time, x fastest: stepped
+// with carries, as three divisions per voxel cost more than the bounds.
+struct BoxWalk {
+  int i, j, k, e0, e1, si, sj, sk;
+  __device__ __forceinline__ BoxWalk(const int (&ext)[3], int q) : e0(ext[0]), e1(ext[1]) {
+    i = q % e0;
+    j = (q / e0) % e1;
+    k = q / (e0 * e1);
+    si = 32 % e0;
+    sj = (32 / e0) % e1;
+    sk = 32 / (e0 * e1);
+  }
+  __device__ __forceinline__ void step() {
+    i += si;
+    const int ci = i >= e0;
+    i -= ci ? e0 : 0;
+    j += sj + ci;
+    const int cj = j >= e1;
+    j -= cj ? e1 : 0;
+    k += sk + cj;
+  }
+};
 
 // Triangle of item w (off[t] <= w < off[t + 1]).
 __device__ __forceinline__ int item_triangle(const SdfItems& W, long long w) {
@@ -259,53 +300,8 @@ __device__ __forceinline__ float sdf_lower_bound(const SdfTri& r, float qx, floa
   return lb;
 }
 
-__global__ void __launch_bounds__(128) sdf_ub_kernel(const double* __restrict__ P, const int32_t* __restrict__ T,
-                                                     SdfItems W, SdfGrid g, const SdfTri* __restrict__ prep,
+__global__ void __launch_bounds__(128) sdf_ub_kernel(SdfItems W, SdfGrid g, const SdfTri* __restrict__ prep,
                                                      const uint8_t* __restrict__ cls, uint32_t* __restrict__ ub) {
-  long long w0, w1;
-  item_range(W, w0, w1);
-  int t = w0 < w1 ? item_triangle(W, w0) : 0;
-  for (long long w = w0; w < w1; ++w) {
-    while ((long long)W.off[t + 1] <= w) ++t;
-    const SdfTri r = prep[t];
-    double Ad[3], Bd[3], Cd[3];
-    load_tri(P, T, t, Ad, Bd, Cd);
-    const float A[3] = {(float)Ad[0], (float)Ad[1], (float)Ad[2]};
-    const float B[3] = {(float)Bd[0], (float)Bd[1], (float)Bd[2]};
-    const float C[3] = {(float)Cd[0], (float)Cd[1], (float)Cd[2]};
-    // rounding of the vertices to float, of the chosen point and of its
-    // distance: a few units of 2^-24 of the largest coordinate involved
-    float mabs = 0.f;
-    for (int a = 0; a < 3; ++a) mabs = fmaxf(mabs, fmaxf(fabsf(A[a]), fmaxf(fabsf(B[a]), fabsf(C[a]))));
-    const int n = r.ext[0] * r.ext[1] * r.ext[2];
-    const int c0 = (int)(w - (long long)W.off[t]) * kSdfChunk, c1 = min(n, c0 + kSdfChunk);
-    for (int q0 = c0 + threadIdx.x; q0 < c1; q0 += blockDim.x) {
-      const int i = r.lo[0] + q0 % r.ext[0], j = r.lo[1] + (q0 / r.ext[0]) % r.ext[1],
-                k = r.lo[2] + q0 / (r.ext[0] * r.ext[1]);
-      const size_t v = vid(g, i, j, k);
-      const float qx = (float)(g.org[0] + i), qy = (float)(g.org[1] + j), qz = (float)(g.org[2] + k);
-      const float cut = class_cut(g, cls[v]);
-      if (cut <= 0.f) continue;
-      const float lb = sdf_lower_bound(r, qx, qy, qz);
-      const float cur = fminf(cut, __uint_as_float(*(volatile const uint32_t*)&ub[v]));
-      if (lb - 2.0f * g.margin >= cur) continue;
-      const float qa = fmaxf(fabsf(qx), fmaxf(fabsf(qy), fabsf(qz)));
-      const float slack = 64.0f * kSdfU * fmaxf(mabs, qa) + g.margin;
-      atomicMin(&ub[v], __float_as_uint(tri_dist_ub32(qx, qy, qz, A, B, C, slack)));
-    }
-  }
-}
-
-// Each work item (a chunk of kSdfChunk box voxels) is filtered first; the
-// voxels that pass are appended to a shared list and evaluated in FP64 by all
-// threads together, so the FP64 pipe (slow on this part) runs with full warps
-// instead of the few lanes that pass the filter in each warp.
-__global__ void __launch_bounds__(128) sdf_dist_kernel(const double* __restrict__ P, const int32_t* __restrict__ T,
-                                                       SdfItems W, SdfGrid g, const SdfTri* __restrict__ prep,
-                                                       const uint8_t* __restrict__ cls, const uint32_t* __restrict__ ub,
-                                                       uint32_t* __restrict__ dist) {
-  __shared__ int list[kSdfChunk];
-  __shared__ int count;
   const int lane = threadIdx.x & 31;
   long long w0, w1;
   item_range(W, w0, w1);
@@ -313,25 +309,91 @@ __global__ void __launch_bounds__(128) sdf_dist_kernel(const double* __restrict_
   for (long long w = w0; w < w1; ++w) {
     while ((long long)W.off[t + 1] <= w) ++t;
     const SdfTri& r = prep[t];
-    const int ex0 = r.ext[0], ex1 = r.ext[1], ex2 = r.ext[2];
-    const int lo0 = r.lo[0], lo1 = r.lo[1], lo2 = r.lo[2];
-    const float blo0 = r.blo[0], blo1 = r.blo[1], blo2 = r.blo[2];
-    const float bhi0 = r.bhi[0], bhi1 = r.bhi[1], bhi2 = r.bhi[2];
-    const bool has_plane = r.has_plane != 0;
-    const float4 pl = r.pl, fe0 = r.fe[0], fe1 = r.fe[1], fe2 = r.fe[2];
-    double A[3], B[3], C[3];
-    load_tri(P, T, t, A, B, C);
-    const int n = ex0 * ex1 * ex2;
+    // rounding of the vertices to float, of the chosen point and of its
+    // distance: a few units of 2^-24 of the largest coordinate involved
+    const int n = r.ext[0] * r.ext[1] * r.ext[2];
     const int c0 = (int)(w - (long long)W.off[t]) * kSdfChunk, c1 = min(n, c0 + kSdfChunk);
-    if (threadIdx.x == 0) count = 0;
-    __syncthreads();
-    for (int base = c0; base < c1; base += blockDim.x) {
-      const int q0 = base + threadIdx.x;
+    BoxWalk at(r.ext, c0 + lane);
+    for (int q0 = c0 + lane; q0 < c1; q0 += 32, at.step()) {
+      const int i = r.lo[0] + at.i, j = r.lo[1] + at.j, k = r.lo[2] + at.k;
+      const size_t v = vid(g, i, j, k);
+      const float cut = class_cut(g, cls[v]);
+      if (cut <= 0.f) continue;
+      const float qx = (float)(g.org[0] + i), qy = (float)(g.org[1] + j), qz = (float)(g.org[2] + k);
+      const float lb = sdf_lower_bound(r, qx, qy, qz);
+      const float cur = fminf(cut, __uint_as_float(*(volatile const uint32_t*)&ub[v]));
+      if (lb - 2.0f * g.margin >= cur) continue;
+      const float qa = fmaxf(fabsf(qx), fmaxf(fabsf(qy), fabsf(qz)));
+      const float slack = 64.0f * kSdfU * fmaxf(r.vabs, qa) + g.margin;
+      atomicMin(&ub[v], __float_as_uint(tri_dist_ub32(qx, qy, qz, r.v[0], r.v[1], r.v[2], slack)));
+    }
+  }
+}
+
+// The (triangle, voxel) pairs that the lower bound leaves, kept per warp over
+// all of its items and evaluated in FP64 32 at a time: the FP64 pipe, slow on
+// this part, runs with full warps, and no warp waits for another. 20,480
+// triangles, 740,000 voxels: with a list per block and barriers around it, boxes
+// grown by the band and three divisions per voxel this pass took 383 us and the
+// FP32 one 212; with the queue, cut_out and BoxWalk 158 and 83.
+struct PairQueue {
+  int t[64];
+  uint32_t v[64];
+};
+
+// Appends the lanes' pairs (keep) to n and evaluates 32 when there are as many,
+// or what is left (flush).
+__device__ __forceinline__ void queue_pairs(PairQueue& Q, int& n, bool keep, int t, uint32_t v, bool flush,
+                                            const double* __restrict__ P, const int32_t* __restrict__ T,
+                                            const SdfGrid& g, uint32_t* __restrict__ dist) {
+  const int lane = threadIdx.x & 31;
+  const unsigned m = __ballot_sync(0xffffffffu, keep);
+  if (keep) {
+    const int at = n + __popc(m & ((1u << lane) - 1u));
+    Q.t[at] = t;
+    Q.v[at] = v;
+  }
+  n += __popc(m);
+  while (n >= 32 || (flush && n > 0)) {
+    __syncwarp();
+    const int first = n > 32 ? n - 32 : 0;
+    if (first + lane < n) {
+      const uint32_t e = Q.v[first + lane];
+      double A[3], B[3], C[3];
+      load_tri(P, T, Q.t[first + lane], A, B, C);
+      const int i = (int)(e % g.dim[0]), j = (int)((e / g.dim[0]) % g.dim[1]),
+                k = (int)(e / ((uint32_t)g.dim[0] * g.dim[1]));
+      const double q[3] = {(double)(g.org[0] + i), (double)(g.org[1] + j), (double)(g.org[2] + k)};
+      atomicMin(&dist[e], __float_as_uint(__double2float_rn(point_tri_dist(q, A, B, C))));
+    }
+    n = first;
+    __syncwarp();
+  }
+}
+
+__global__ void __launch_bounds__(128) sdf_dist_kernel(const double* __restrict__ P, const int32_t* __restrict__ T,
+                                                       SdfItems W, SdfGrid g, const SdfTri* __restrict__ prep,
+                                                       const uint8_t* __restrict__ cls, const uint32_t* __restrict__ ub,
+                                                       uint32_t* __restrict__ dist) {
+  __shared__ PairQueue queues[4];
+  PairQueue& Q = queues[threadIdx.x >> 5];
+  const int lane = threadIdx.x & 31;
+  int nq = 0;
+  long long w0, w1;
+  item_range(W, w0, w1);
+  int t = w0 < w1 ? item_triangle(W, w0) : 0;
+  for (long long w = w0; w < w1; ++w) {
+    while ((long long)W.off[t + 1] <= w) ++t;
+    const SdfTri& r = prep[t];
+    const int n = r.ext[0] * r.ext[1] * r.ext[2];
+    const int c0 = (int)(w - (long long)W.off[t]) * kSdfChunk, c1 = min(n, c0 + kSdfChunk);
+    BoxWalk at(r.ext, c0 + lane);
+    for (int base = c0; base < c1; base += 32, at.step()) {
       bool keep = false;
-      if (q0 < c1) {
-        const int i = lo0 + q0 % ex0, j = lo1 + (q0 / ex0) % ex1, k = lo2 + q0 / (ex0 * ex1);
-        const size_t v = vid(g, i, j, k);
-        const float qx = (float)(g.org[0] + i), qy = (float)(g.org[1] + j), qz = (float)(g.org[2] + k);
+      size_t v = 0;
+      if (base + lane < c1) {
+        const int i = r.lo[0] + at.i, j = r.lo[1] + at.j, k = r.lo[2] + at.k;
+        v = vid(g, i, j, k);
         const uint8_t c = cls[v];
         const float up = __uint_as_float(ub[v]);
         float cur = fminf(up, class_cut(g, c));
@@ -339,38 +401,61 @@ __global__ void __launch_bounds__(128) sdf_dist_kernel(const double* __restrict_
         // the other side
         if (c == kClassOut && up < g.low_out) cur = 0.f;
         if (cur > 0.f) {
-          const float gx = fmaxf(fmaxf(blo0 - qx, qx - bhi0), 0.f);
-          const float gy = fmaxf(fmaxf(blo1 - qy, qy - bhi1), 0.f);
-          const float gz = fmaxf(fmaxf(blo2 - qz, qz - bhi2), 0.f);
-          float lb = sqrtf(gx * gx + gy * gy + gz * gz);
-          if (has_plane) {
-            const float pd = fabsf(pl.x * qx + pl.y * qy + pl.z * qz + pl.w);
-            float se = 0.f;
-            se = fmaxf(se, fe0.x * qx + fe0.y * qy + fe0.z * qz + fe0.w);
-            se = fmaxf(se, fe1.x * qx + fe1.y * qy + fe1.z * qz + fe1.w);
-            se = fmaxf(se, fe2.x * qx + fe2.y * qy + fe2.z * qz + fe2.w);
-            lb = fmaxf(lb, sqrtf(pd * pd + se * se));
-          }
+          const float lb = sdf_lower_bound(r, (float)(g.org[0] + i), (float)(g.org[1] + j), (float)(g.org[2] + k));
           keep = lb - 2.0f * g.margin < fminf(cur, __uint_as_float(*(volatile const uint32_t*)&dist[v]));
         }
       }
-      // warp-aggregated append (at most kSdfChunk entries per item)
-      const unsigned m = __ballot_sync(0xffffffffu, keep);
-      int at = 0;
-      if (lane == 0 && m) at = atomicAdd(&count, __popc(m));
-      at = __shfl_sync(0xffffffffu, at, 0);
-      if (keep) list[at + __popc(m & ((1u << lane) - 1u))] = q0;
+      queue_pairs(Q, nq, keep, t, (uint32_t)v, w == w1 - 1 && base + 32 >= c1, P, T, g, dist);
     }
-    __syncthreads();
-    const int nc = count;
-    for (int e = threadIdx.x; e < nc; e += blockDim.x) {
-      const int q0 = list[e];
-      const int i = lo0 + q0 % ex0, j = lo1 + (q0 / ex0) % ex1, k = lo2 + q0 / (ex0 * ex1);
-      const double q[3] = {(double)(g.org[0] + i), (double)(g.org[1] + j), (double)(g.org[2] + k)};
-      const float d = __double2float_rn(point_tri_dist(q, A, B, C));
-      atomicMin(&dist[vid(g, i, j, k)], __float_as_uint(d));
+  }
+}
+
+__global__ void sdf_far_kernel(SdfGrid g, size_t n, const uint32_t* __restrict__ dist, const uint32_t* __restrict__ ub,
+                               uint8_t* __restrict__ cls, unsigned* __restrict__ n_far) {
+  for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (size_t)gridDim.x * blockDim.x) {
+    const uint8_t c = cls[v];
+    if (!(c & kClassEdge)) continue;
+    if ((double)fminf(__uint_as_float(dist[v]), __uint_as_float(ub[v])) < g.reach) continue;
+    cls[v] = c | kClassFar;
+    *n_far = 1u;
+  }
+}
+
+// Exact distances of the kClassFar voxels, one warp per triangle.
+__global__ void __launch_bounds__(128) sdf_far_dist_kernel(const double* __restrict__ P, const int32_t* __restrict__ T,
+                                                           int nt, SdfGrid g, const SdfTri* __restrict__ prep,
+                                                           const uint8_t* __restrict__ cls,
+                                                           const unsigned* __restrict__ n_far,
+                                                           uint32_t* __restrict__ dist) {
+  __shared__ PairQueue queues[4];
+  PairQueue& Q = queues[threadIdx.x >> 5];
+  if (*n_far == 0) return;
+  const int lane = threadIdx.x & 31, warps = (gridDim.x * blockDim.x) >> 5;
+  int nq = 0;
+  for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < nt; t += warps) {
+    double A[3], B[3], C[3];
+    load_tri(P, T, t, A, B, C);
+    int lo[3], ext[3];
+#pragma unroll
+    for (int a = 0; a < 3; ++a)
+      box_range(g, a, min3(A[a], B[a], C[a]), max3(A[a], B[a], C[a]), g.band, lo[a], ext[a]);
+    if (ext[0] <= 0 || ext[1] <= 0 || ext[2] <= 0) continue;
+    const SdfTri& r = prep[t];
+    const int n = ext[0] * ext[1] * ext[2];
+    BoxWalk at(ext, lane);
+    for (int base = 0; base < n; base += 32, at.step()) {
+      bool keep = false;
+      size_t v = 0;
+      if (base + lane < n) {
+        const int i = lo[0] + at.i, j = lo[1] + at.j, k = lo[2] + at.k;
+        v = vid(g, i, j, k);
+        if (cls[v] & kClassFar) {
+          const float lb = sdf_lower_bound(r, (float)(g.org[0] + i), (float)(g.org[1] + j), (float)(g.org[2] + k));
+          keep = lb - 2.0f * g.margin < __uint_as_float(*(volatile const uint32_t*)&dist[v]);
+        }
+      }
+      queue_pairs(Q, nq, keep, t, (uint32_t)v, base + 32 >= n, P, T, g, dist);
     }
-    __syncthreads();
   }
 }
 
@@ -562,8 +647,7 @@ __global__ void sdf_cell_list_kernel(size_t n, const uint32_t* __restrict__ flag
 
 // One thread per vertex, over the list, so that FP64 runs with full warps: of
 // the cells themselves only about one in twenty-five has a vertex, and the same
-// arithmetic over all of 740,000 took 189 us; now all seven launches of the
-// cells, quads and field take 89 us.
+// arithmetic over all of 740,000 took 189 us; over the list, 23.
 __global__ void __launch_bounds__(64) sdf_cell_vertex_kernel(SdfGrid g, const float* __restrict__ f,
                                                              const uint32_t* __restrict__ cells, size_t n,
                                                              double* __restrict__ out_v) {
@@ -694,6 +778,7 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   const bool all_exact = !(iso > 0.0);
   g.cut_out = (float)(iso + 1.0 + 0.01) + 2.0f * g.margin;
   g.low_out = (float)(iso - 1.0 - 0.01);
+  g.reach = all_exact ? g.band : std::min(g.band, (double)g.cut_out);
   const size_t nvox = (size_t)g.dim[0] * g.dim[1] * g.dim[2];
   VCHECK(nvox <= ((size_t)1 << 30), VISACD_ERR_CAPACITY, "sdf_remesh: grid of %zu voxels is too large", nvox);
   const size_t ncell = (size_t)(g.dim[0] - 1) * (g.dim[1] - 1) * (g.dim[2] - 1);
@@ -707,7 +792,7 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   };
   const size_t oP = take(P.size() * 8), oT = take(3 * (size_t)nt * 4);
   const size_t upload = at;
-  const size_t oTog = take(nvox * 4), oNWide = take(16);
+  const size_t oTog = take(nvox * 4), oNWide = take(16);  // + the far flag
   const size_t zero_end = at;
   const size_t oPrep = take((size_t)nt * sizeof(SdfTri)), oWide = take(3 * (size_t)nt * 4),
                oChunks = take((size_t)nt * 4), oChunkOff = take(((size_t)nt + 1) * 8), oDist = take(nvox * 4),
@@ -765,9 +850,15 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   items.nt = nt;
   const unsigned gw = (unsigned)(8 * (int64_t)ctx->sm_count);
   // First pass: FP32 upper bounds per voxel, then the exact pass.
-  VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_ub_kernel, dP, dT, items, g, (const SdfTri*)prep, (const uint8_t*)cls, ub);
+  VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_ub_kernel, items, g, (const SdfTri*)prep, (const uint8_t*)cls, ub);
   VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_dist_kernel, dP, dT, items, g, (const SdfTri*)prep, (const uint8_t*)cls,
           (const uint32_t*)ub, dist);
+  if (g.reach < g.band) {
+    unsigned* n_far = n_wide + 1;
+    VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_far_kernel, g, nvox, (const uint32_t*)dist, (const uint32_t*)ub, cls, n_far);
+    VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_far_dist_kernel, dP, dT, nt, g, (const SdfTri*)prep, (const uint8_t*)cls,
+            (const unsigned*)n_far, dist);
+  }
   VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_field_kernel, (const uint32_t*)dist, (const uint32_t*)ub, (const uint8_t*)cls,
           nvox, f);
   const unsigned gc = grid_for((int64_t)ncell, 256, 16 * (int64_t)ctx->sm_count);
