@@ -13,12 +13,14 @@
 //    point of a face, the assignment of points to faces (the first face with
 //    the largest distance above eps) and the stable scatter of each face's
 //    outside list in point order (match-any ranks, so every list keeps the
-//    host's order), the new faces' planes, the final compaction of live faces
-//    in creation order and the orientation fix;
-//  * sequential in lane 0, in the host's order: the depth-first flood fill of
-//    visible faces, the horizon list and its loop order, face creation and
-//    neighbour linking, the centroid sum of the orientation fix and the 2D
-//    monotone chain of coplanar input.
+//    host's order), the new faces with their planes and links, the final
+//    compaction of live faces in creation order and the orientation fix;
+//  * in the host's order, one step after another, by the whole warp: the
+//    depth-first flood fill of visible faces (a face's three neighbours tested
+//    in three lanes), the horizon list and its loop order (the edge that
+//    continues the loop found by a ballot over up to 32 edges in registers);
+//  * sequential: the centroid sum of the orientation fix (a lane per axis) and
+//    the 2D monotone chain of coplanar input.
 // Faces are never reused: the host processes faces in creation order, and
 // face ids here are creation indices, so both visit the same faces in the same
 // order. Outside lists are append-only segments of a per-part pool.
@@ -39,7 +41,10 @@
 namespace vgpu {
 namespace {
 
-constexpr int kHullWarps = 4;  // parts in flight per block, one warp each
+constexpr int kHullShared = 64;  // new faces of a step counted in shared memory (more: in the work region)
+constexpr int kHullStack = 8;    // flood-fill stack entries in shared memory (more: in the work region)
+constexpr int kHullOrphans = 256;  // orphaned points of a step in shared memory (more: in the work region)
+constexpr int kHullPerSm = 16;   // resident parts per SM at most (registers)
 constexpr int kMaxHullMult = 16;  // with at most 2^22 points a part, every capacity fits in int32
 
 enum : int32_t {
@@ -57,6 +62,13 @@ struct D3 {
 };
 struct __align__(16) HPlane {  // unit normal and offset of a face
   double x, y, z, w;
+};
+struct __align__(16) HFace {
+  HPlane plane;
+  int4 tv;    // v0, v1, v2, alive
+  int4 nb;    // neighbour across (v[e], v[e+1]) for e = 0..2, visit stamp
+  int2 outl;  // outside list (start in pool, count)
+  int pad[2];
 };
 __device__ __forceinline__ D3 ld3(const double* P, int i) {
   return {P[3 * (int64_t)i], P[3 * (int64_t)i + 1], P[3 * (int64_t)i + 2]};
@@ -114,6 +126,15 @@ __device__ __forceinline__ void warp_min_first(double& v, int& i) {
     }
   }
 }
+// warp_max_first for values that are positive or -1 (no best yet): such
+// doubles order like their bit patterns, so three integer reductions do.
+__device__ __forceinline__ void warp_max_first_pos(double& v, int& i) {
+  const int hi = __reduce_max_sync(0xffffffffu, __double2hiint(v));
+  const bool a = __double2hiint(v) == hi;
+  const unsigned lo = __reduce_max_sync(0xffffffffu, a ? (unsigned)__double2loint(v) : 0u);
+  i = (int)__reduce_min_sync(0xffffffffu, a && (unsigned)__double2loint(v) == lo ? (unsigned)i : 0x7fffffffu);
+  v = __hiloint2double(hi, (int)lo);
+}
 __device__ __forceinline__ double warp_max(double v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_xor_sync(0xffffffffu, v, o));
@@ -138,18 +159,19 @@ __host__ __device__ inline HullCaps hull_caps(int64_t n, int mult) {
 __host__ __device__ inline int64_t hull_a16(int64_t b) { return (b + 15) & ~(int64_t)15; }
 __host__ __device__ inline int64_t hull_region_bytes(int64_t n, int mult) {
   const HullCaps c = hull_caps(n, mult);
-  return hull_a16(c.faces * 32) + hull_a16(c.faces * 16) * 2 + hull_a16(c.faces * 8) + hull_a16(c.pool * 4) +
+  return c.faces * 80 + hull_a16(c.pool * 4) +
          3 * hull_a16(c.list * 4) + 3 * hull_a16(c.hor * 8) + hull_a16(c.hor * 4) + 2 * hull_a16(n * 4);
 }
 
 namespace {
 
 struct HullWork {
-  HPlane* plane;  // face: unit normal, offset
-  int4* tv;        // face: v0, v1, v2, alive
-  int4* nb;        // face: neighbour across (v[e], v[e+1]) for e = 0..2, visit stamp
-  int2* outl;      // face: outside list (start in pool, count)
-  int* pool;
+  // Faces and pool entries: the first nsf and nsp in shared memory.
+  HFace *gface, *sface;
+  int *gpool, *spool;
+  int nsf, nsp;
+  __device__ __forceinline__ HFace& face(int f) { return (f < nsf ? sface : gface)[f]; }
+  __device__ __forceinline__ int& pool(int k) { return (k < nsp ? spool : gpool)[k]; }
   int* vis;        // visible faces of a step, in flood-fill order
   int* stack;
   int* voff;       // first orphan slot of each visible face
@@ -160,6 +182,12 @@ struct HullWork {
   int* orph;       // orphaned points of a step, in order
   int* obest;      // new face (0-based among the step's) of each orphan, -1 = inside
   HullCaps cap;
+};
+// The working set of one step, while it is small (it nearly always is: a few
+// faces, a few dozen points).
+struct __align__(16) HullShared {
+  HPlane plane[kHullShared];  // the new faces' planes
+  int cnt[kHullShared], orph[kHullOrphans], obest[kHullOrphans], stack[kHullStack];
 };
 
 __device__ HullWork carve(char* base, int64_t n, int mult) {
@@ -172,11 +200,9 @@ __device__ HullWork carve(char* base, int64_t n, int mult) {
     p += hull_a16(bytes);
     return r;
   };
-  w.plane = (HPlane*)take(c.faces * 32);
-  w.tv = (int4*)take(c.faces * 16);
-  w.nb = (int4*)take(c.faces * 16);
-  w.outl = (int2*)take(c.faces * 8);
-  w.pool = (int*)take(c.pool * 4);
+  static_assert(sizeof(HFace) == 80, "hull_region_bytes");
+  w.gface = (HFace*)take(c.faces * 80);
+  w.gpool = (int*)take(c.pool * 4);
   w.vis = (int*)take(c.list * 4);
   w.stack = (int*)take(c.list * 4);
   w.voff = (int*)take(c.list * 4);
@@ -200,11 +226,12 @@ __device__ __forceinline__ void set_comp(int4* p, int e, int x) {
 // largest distance above eps, or nowhere; then every face's outside list is
 // written as one pool segment, in point order. Returns the new pool top, or
 // -1 when the pool is full.
-__device__ int64_t assign_points(const double* P, HullWork& W, const int* pts, int m, int4 skip, int f0, int L,
-                                 double eps, int64_t top, int lane) {
-  // Pass 1: best face of each point, counts per face (outl[f].y).
-  if (lane == 0)
-    for (int q = 0; q < L; ++q) W.outl[f0 + q] = make_int2(0, 0);
+__device__ int64_t assign_points(const double* P, HullWork& W, HullShared& S, const int* pts, int m, int4 skip,
+                                 int f0, int L, double eps, int64_t top, int lane) {
+  // Pass 1: best face of each point, counts per face.
+  int* cnt = L <= kHullShared ? S.cnt : W.fillc;
+  int* obest = m <= kHullOrphans ? S.obest : W.obest;
+  for (int q = lane; q < L; q += 32) cnt[q] = 0;
   __syncwarp();
   for (int base = 0; base < m; base += 32) {
     const int k = base + lane;
@@ -215,45 +242,85 @@ __device__ int64_t assign_points(const double* P, HullWork& W, const int* pts, i
       if (pts || (p != skip.x && p != skip.y && p != skip.z && p != skip.w)) {
         const D3 pp = ld3(P, p);
         double bd = eps;
+#pragma unroll 4
         for (int q = 0; q < L; ++q) {
-          const double d = plane_dist(W.plane[f0 + q], pp);
+          const double d = plane_dist(L <= kHullShared ? S.plane[q] : W.face(f0 + q).plane, pp);
           if (d > bd) {
             bd = d;
             bf = q;
           }
         }
       }
-      W.obest[k] = bf;
+      obest[k] = bf;
     }
     const unsigned mm = __match_any_sync(0xffffffffu, bf);
-    if (bf >= 0 && (__ffs(mm) - 1) == lane) W.outl[f0 + bf].y += __popc(mm);
+    if (bf >= 0 && (__ffs(mm) - 1) == lane) cnt[bf] += __popc(mm);
     __syncwarp();
   }
   // Segment starts.
   int64_t end = top;
-  if (lane == 0) {
-    for (int q = 0; q < L; ++q) {
-      const int c = W.outl[f0 + q].y;
-      W.outl[f0 + q].x = (int)end;
-      W.fillc[q] = (int)end;
-      end += c;
+  for (int base = 0; base < L; base += 32) {
+    const int q = base + lane;
+    const int c = q < L ? cnt[q] : 0;
+    int inc = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += x;
     }
+    if (q < L) {
+      const int at = (int)(end + inc - c);
+      W.face(f0 + q).outl = make_int2(at, c);
+      cnt[q] = at;
+    }
+    end += __shfl_sync(0xffffffffu, inc, 31);
   }
-  end = __shfl_sync(0xffffffffu, end, 0);
   if (end > W.cap.pool) return -1;
   __syncwarp();
   // Pass 2: stable scatter.
   const unsigned lt = lanemask_lt();
   for (int base = 0; base < m; base += 32) {
     const int k = base + lane;
-    const int bf = k < m ? W.obest[k] : -2;
+    const int bf = k < m ? obest[k] : -2;
     const unsigned mm = __match_any_sync(0xffffffffu, bf);
-    if (bf >= 0) W.pool[W.fillc[bf] + __popc(mm & lt)] = pts ? pts[k] : k;
+    if (bf >= 0) W.pool(cnt[bf] + __popc(mm & lt)) = pts ? pts[k] : k;
     __syncwarp();
-    if (bf >= 0 && (__ffs(mm) - 1) == lane) W.fillc[bf] += __popc(mm);
+    if (bf >= 0 && (__ffs(mm) - 1) == lane) cnt[bf] += __popc(mm);
     __syncwarp();
   }
   return end;
+}
+
+// assign_points for a step of at most 32 points (lane k has the k-th, p) and 32
+// faces: the same lists, by one ballot per face.
+__device__ int64_t assign_lanes(const double* P, HullWork& W, const HPlane* planes, int p, int m, int f0, int L,
+                                double eps, int64_t top, int lane) {
+  int bf = -1;
+  if (lane < m) {
+    const D3 pp = ld3(P, p);
+    double bd = eps;
+#pragma unroll 4
+    for (int q = 0; q < L; ++q) {
+      const double d = plane_dist(planes[q], pp);
+      if (d > bd) {
+        bd = d;
+        bf = q;
+      }
+    }
+  }
+  const int kept = __popc(__ballot_sync(0xffffffffu, bf >= 0));
+  if (top + kept > W.cap.pool) return -1;
+  int n = (int)top, at = 0;
+  int2 list = make_int2(0, 0);
+  for (int q = 0; q < L; ++q) {
+    const unsigned b = __ballot_sync(0xffffffffu, bf == q);
+    if (bf == q) at = n + __popc(b & lanemask_lt());
+    if (lane == q) list = make_int2(n, __popc(b));
+    n += __popc(b);
+  }
+  if (bf >= 0) W.pool(at) = p;
+  if (lane < L) W.face(f0 + lane).outl = list;
+  return top + kept;
 }
 
 // Coplanar input: the host's flat_hull (2D monotone chain in the plane, closed
@@ -270,7 +337,7 @@ __device__ int flat_hull(const double* P, int n, HullWork& W, int32_t* tris, int
       ia = i;
     }
   }
-  warp_max_first(bd, ia);
+  warp_max_first_pos(bd, ia);
   if (ia == 0x7fffffff) ia = 0;
   D3 u = sub3(ld3(P, ia), o);
   {
@@ -287,19 +354,20 @@ __device__ int flat_hull(const double* P, int n, HullWork& W, int32_t* tris, int
       ic = i;
     }
   }
-  warp_max_first(bc, ic);
+  warp_max_first_pos(bc, ic);
   if (!(bc > 0)) return kHullOk;
   D3 nrm = cross3(u, sub3(ld3(P, ic), o));
   nrm = div3(nrm, norm3(nrm));
   const D3 v = cross3(nrm, u);
   // Sort (x, y, index) lexicographically by rank counting: rank of i = number
   // of keys below it (keys are distinct through the index).
-  double* qx = reinterpret_cast<double*>(W.plane);
+  // (40 of the face array's 640 bytes per point, and the chain of up to 2n.)
+  double* qx = reinterpret_cast<double*>(W.gface);
   double* qy = qx + n;
-  int* qi = reinterpret_cast<int*>(W.tv);
-  int* h = qi + n;
-  double* kx = reinterpret_cast<double*>(W.nb);  // the unsorted keys
+  double* kx = qy + n;  // the unsorted keys
   double* ky = kx + n;
+  int* qi = reinterpret_cast<int*>(ky + n);
+  int* h = qi + n;
   for (int i = lane; i < n; i += 32) {
     const D3 w = sub3(ld3(P, i), o);
     kx[i] = dot3(w, u);
@@ -352,7 +420,7 @@ __device__ int flat_hull(const double* P, int n, HullWork& W, int32_t* tris, int
 }
 
 // One part: the host's convex_hull(pts, fix_normals) (host/hull.cpp).
-__device__ int hull_one(const double* P, int n, HullWork& W, int fix, int32_t* tris, int& ntri, int lane) {
+__device__ int hull_one(const double* P, int n, HullWork& W, HullShared& S, int fix, int32_t* tris, int& ntri, int lane) {
   ntri = 0;
   if (n < 3) return kHullOk;
   double ext = 0.0;
@@ -408,7 +476,7 @@ __device__ int hull_one(const double* P, int n, HullWork& W, int fix, int32_t* t
       i2 = i;
     }
   }
-  warp_max_first(b2, i2);
+  warp_max_first_pos(b2, i2);
   if (i2 == 0x7fffffff) return kHullOk;  // collinear
   D3 nrm = cross3(sub3(ld3(P, i1), p0), sub3(ld3(P, i2), p0));
   {
@@ -425,7 +493,7 @@ __device__ int hull_one(const double* P, int n, HullWork& W, int fix, int32_t* t
       i3 = i;
     }
   }
-  warp_max_first(b3, i3);
+  warp_max_first_pos(b3, i3);
   if (i3 == 0x7fffffff) return flat_hull(P, n, W, tris, ntri, lane);
   if (dot3(nrm, sub3(ld3(P, i3), p0)) > 0) {
     const int t = i1;
@@ -437,174 +505,269 @@ __device__ int hull_one(const double* P, int n, HullWork& W, int fix, int32_t* t
     const int4 f = lane == 0 ? make_int4(i0, i1, i2, 1)
                              : (lane == 1 ? make_int4(i0, i3, i1, 1)
                                           : (lane == 2 ? make_int4(i1, i3, i2, 1) : make_int4(i2, i3, i0, 1)));
-    W.tv[lane] = f;
-    W.plane[lane] = face_plane(P, f.x, f.y, f.z);
+    W.face(lane).tv = f;
+    S.plane[lane] = W.face(lane).plane = face_plane(P, f.x, f.y, f.z);
   }
   __syncwarp();
   if (lane == 0) {
     for (int a = 0; a < 4; ++a) {
       int4 nbv = make_int4(-1, -1, -1, 0);
-      const int4 va = W.tv[a];
+      const int4 va = W.face(a).tv;
       for (int e = 0; e < 3; ++e) {
         const int u = comp(va, e), w = comp(va, (e + 1) % 3);
         for (int b = 0; b < 4; ++b) {
           if (a == b) continue;
-          const int4 vb = W.tv[b];
+          const int4 vb = W.face(b).tv;
           for (int e2 = 0; e2 < 3; ++e2)
             if (comp(vb, e2) == w && comp(vb, (e2 + 1) % 3) == u) set_comp(&nbv, e, b);
         }
       }
-      W.nb[a] = nbv;
+      W.face(a).nb = nbv;
     }
   }
   __syncwarp();
-  int64_t top = assign_points(P, W, nullptr, n, make_int4(i0, i1, i2, i3), 0, 4, eps, 0, lane);
+  int64_t top = assign_points(P, W, S, nullptr, n, make_int4(i0, i1, i2, i3), 0, 4, eps, 0, lane);
   if (top < 0) return kHullPoolCap;
   int nF = 4, cur = 0, iter = 0;
   for (;;) {
     while (cur < nF) {
-      if (W.tv[cur].w && W.outl[cur].y > 0) break;
-      ++cur;
+      const int f = cur + lane;
+      const unsigned m = __ballot_sync(0xffffffffu, f < nF && W.face(f).tv.w && W.face(f).outl.y > 0);
+      if (m) {
+        cur += __ffs(m) - 1;
+        break;
+      }
+      cur += 32;
     }
     if (cur >= nF) break;
     if (++iter > 4 * n + 64) break;
     // Farthest outside point of cur (first in list order among equals).
-    const HPlane pc = W.plane[cur];
-    const int2 ol = W.outl[cur];
+    const HPlane pc = W.face(cur).plane;
+    const int2 ol = W.face(cur).outl;
     double bd = -1.0;
-    int bpos = 0x7fffffff;
+    int bpos = 0x7fffffff, bid = 0;
     for (int k = lane; k < ol.y; k += 32) {
-      const double d = plane_dist(pc, ld3(P, W.pool[ol.x + k]));
+      const int id = W.pool(ol.x + k);
+      const double d = plane_dist(pc, ld3(P, id));
       if (d > bd) {
         bd = d;
         bpos = k;
+        bid = id;
       }
     }
-    warp_max_first(bd, bpos);
+    warp_max_first_pos(bd, bpos);
     if (bpos >= ol.y) return kHullNumeric;
-    const int apex = W.pool[ol.x + bpos];
+    const int apex = __shfl_sync(0xffffffffu, bid, bpos & 31);
     const D3 pa = ld3(P, apex);
-    // Lane 0: flood fill, horizon loop, new faces and links.
-    int st = kHullOk, vn = 0, L = 0, norph = 0;
+    // Flood fill: the stack, the marks and the lists are written by lane 0,
+    // everything else is the same in all lanes. Lane h also keeps horizon edge
+    // h < 32 (end points, face across) and visible face h < 32 (with its outside
+    // list and first orphan).
+    int vn = 0, norph = 0, sp = 1, hn = 0;
+    int hu = -1, hw = -1, hg = -1, vf = 0, vo = 0;
+    int2 vl = make_int2(0, 0);
     if (lane == 0) {
-      int sp = 0, hn = 0;
-      W.stack[sp++] = cur;
-      W.nb[cur].w = iter;
-      while (sp > 0 && st == kHullOk) {
-        const int f = W.stack[--sp];
-        if (vn >= W.cap.list) {
-          st = kHullListCap;
-          break;
+      S.stack[0] = cur;
+      W.face(cur).nb.w = iter;
+    }
+    __syncwarp();
+    while (sp > 0) {
+      --sp;
+      const int f = sp < kHullStack ? S.stack[sp] : W.stack[sp];
+      if (vn >= W.cap.list) return kHullListCap;
+      const HFace& F = W.face(f);
+      const int4 nbf = F.nb, tf = F.tv;
+      const int2 of = F.outl;
+      bool open = false, above = false;
+      if (lane < 3) {
+        const int g = comp(nbf, lane);
+        if (g >= 0) {
+          const HFace& G = W.face(g);
+          open = G.nb.w != iter;
+          above = plane_dist(G.plane, pa) > eps;
         }
+      }
+      const unsigned mo = __ballot_sync(0xffffffffu, open), ma = __ballot_sync(0xffffffffu, open && above);
+      if (lane == 0) {
         W.vis[vn] = f;
         W.voff[vn] = norph;
-        norph += W.outl[f].y - (f == cur ? 1 : 0);
-        ++vn;
-        const int4 nbf = W.nb[f];
-        for (int e = 0; e < 3; ++e) {
-          const int g = comp(nbf, e);
-          if (g < 0 || W.nb[g].w == iter) continue;
-          if (plane_dist(W.plane[g], pa) > eps) {
-            if (sp >= W.cap.list) {
-              st = kHullListCap;
-              break;
-            }
-            W.nb[g].w = iter;
-            W.stack[sp++] = g;
-          } else {
-            if (hn >= W.cap.hor) {
-              st = kHullListCap;
-              break;
-            }
-            const int4 tf = W.tv[f];
-            W.hor[hn] = make_int2(f, e);
-            W.hu[hn] = make_int2(comp(tf, e), comp(tf, (e + 1) % 3));
-            ++hn;
-          }
-        }
       }
-      if (st == kHullOk) {
-        // Order the horizon as a loop (the host's first-unused-match scan).
-        bool ok = hn > 0;
-        if (ok) {
-          W.loop[0] = W.hor[0];
-          int wlast = W.hu[0].y;
-          W.hu[0].x = -1;
-          L = 1;
-          for (int k = 1; k < hn; ++k) {
-            int found = -1;
-            for (int hh = 0; hh < hn; ++hh)
-              if (W.hu[hh].x == wlast) {
-                found = hh;
-                break;
-              }
-            if (found < 0) break;
-            W.loop[L++] = W.hor[found];
-            wlast = W.hu[found].y;
-            W.hu[found].x = -1;
+      if (lane == vn) {
+        vf = f;
+        vo = norph;
+        vl = of;
+      }
+      norph += of.y - (f == cur ? 1 : 0);
+      ++vn;
+#pragma unroll
+      for (int e = 0; e < 3; ++e) {
+        if (!((mo >> e) & 1u)) continue;
+        const int g = comp(nbf, e);
+        if ((ma >> e) & 1u) {
+          // (a face that is a neighbour twice is taken once)
+          if ((e > 0 && ((ma >> 0) & 1u) && nbf.x == g) || (e > 1 && ((ma >> 1) & 1u) && nbf.y == g)) continue;
+          if (sp >= W.cap.list) return kHullListCap;
+          if (lane == 0) {
+            W.face(g).nb.w = iter;
+            if (sp < kHullStack) S.stack[sp] = g;
+            else W.stack[sp] = g;
           }
-          ok = L == hn;
-        }
-        if (!ok) {
-          W.outl[cur].y = 0;  // numerically inconsistent horizon: drop cur's outside set
-          L = 0;
-        } else if (nF + L > W.cap.faces) {
-          st = kHullFaceCap;
+          ++sp;
         } else {
-          for (int k = 0; k < L; ++k) {
-            const int2 fe = W.loop[k];
-            const int4 tf = W.tv[fe.x];
-            const int u = comp(tf, fe.y), w = comp(tf, (fe.y + 1) % 3);
-            const int g = comp(W.nb[fe.x], fe.y);
-            const int nfi = nF + k;
-            W.tv[nfi] = make_int4(u, w, apex, 1);
-            W.nb[nfi] = make_int4(g, nF + (k + 1) % L, nF + (k + L - 1) % L, 0);
-            const int4 tg = W.tv[g];
-            for (int e = 0; e < 3; ++e)
-              if (comp(tg, e) == w && comp(tg, (e + 1) % 3) == u) {
-                set_comp(&W.nb[g], e, nfi);
-                break;
-              }
+          if (hn >= W.cap.hor) return kHullListCap;
+          const int u = comp(tf, e), w = comp(tf, (e + 1) % 3);
+          if (lane == 0) {
+            W.hor[hn] = make_int2(f, e);
+            W.hu[hn] = make_int2(u, w);
           }
+          if (lane == hn) {
+            hu = u;
+            hw = w;
+            hg = g;
+          }
+          ++hn;
         }
       }
+      __syncwarp();
     }
-    st = __shfl_sync(0xffffffffu, st, 0);
-    if (st != kHullOk) return st;
-    L = __shfl_sync(0xffffffffu, L, 0);
-    if (L == 0) {
+    // Order the horizon as a loop (the host's first-unused-match scan). Up to 32
+    // edges: lane k gets edge k of the loop.
+    int L = 0, u = 0, w = 0, g = 0;
+    if (hn > 0 && hn <= 32) {
+      int at = 0, mine = 0;
+      bool unused = lane < hn;
+      for (;;) {
+        if (lane == L) mine = at;
+        if (lane == at) unused = false;
+        if (++L == hn) break;
+        const int wlast = __shfl_sync(0xffffffffu, hw, at);
+        const unsigned m = __ballot_sync(0xffffffffu, unused && hu == wlast);
+        if (!m) break;
+        at = __ffs(m) - 1;
+      }
+      u = __shfl_sync(0xffffffffu, hu, mine);
+      w = __shfl_sync(0xffffffffu, hw, mine);
+      g = __shfl_sync(0xffffffffu, hg, mine);
+    } else if (hn > 32) {
+      if (lane == 0) {
+        W.loop[0] = W.hor[0];
+        int wlast = W.hu[0].y;
+        W.hu[0].x = -1;
+        L = 1;
+        for (int k = 1; k < hn; ++k) {
+          int found = -1;
+          for (int hh = 0; hh < hn; ++hh)
+            if (W.hu[hh].x == wlast) {
+              found = hh;
+              break;
+            }
+          if (found < 0) break;
+          W.loop[L++] = W.hor[found];
+          wlast = W.hu[found].y;
+          W.hu[found].x = -1;
+        }
+      }
+      L = __shfl_sync(0xffffffffu, L, 0);
+    }
+    __syncwarp();
+    if (hn == 0 || L != hn) {
+      if (lane == 0) W.face(cur).outl.y = 0;  // numerically inconsistent horizon: drop cur's outside set
       ++cur;
       __syncwarp();
       continue;
     }
-    vn = __shfl_sync(0xffffffffu, vn, 0);
-    norph = __shfl_sync(0xffffffffu, norph, 0);
-    __syncwarp();
-    // New faces' planes; orphans of the visible faces in order (the apex
-    // skipped); visible faces die.
+    if (nF + L > W.cap.faces) return kHullFaceCap;
+    // New faces and links (the entries written differ between the lanes: each
+    // horizon edge has its own), their normals and lengths.
+    const bool shared_planes = L <= kHullShared;
     for (int k = lane; k < L; k += 32) {
-      const int4 t = W.tv[nF + k];
-      W.plane[nF + k] = face_plane(P, t.x, t.y, t.z);
+      if (L > 32) {
+        const int2 fe = W.loop[k];
+        const HFace& F = W.face(fe.x);
+        u = comp(F.tv, fe.y);
+        w = comp(F.tv, fe.y == 2 ? 0 : fe.y + 1);
+        g = comp(F.nb, fe.y);
+      }
+      const int nfi = nF + k;
+      HFace& N = W.face(nfi);
+      N.tv = make_int4(u, w, apex, 1);
+      N.nb = make_int4(g, k + 1 < L ? nfi + 1 : nF, k > 0 ? nfi - 1 : nF + L - 1, 0);
+      HFace& G = W.face(g);
+      const int4 tg = G.tv;
+      const int e = tg.x == w && tg.y == u ? 0 : (tg.y == w && tg.z == u ? 1 : (tg.z == w && tg.x == u ? 2 : 3));
+      if (e < 3) set_comp(&G.nb, e, nfi);
+      const D3 a = ld3(P, u);
+      const D3 nn = cross3(sub3(ld3(P, w), a), sub3(pa, a));
+      (shared_planes ? S.plane[k] : N.plane) = HPlane{nn.x, nn.y, nn.z, norm3(nn)};
     }
+    __syncwarp();
+    // One division per lane (three in one lane run one after another), then the
+    // offsets: face_plane's values.
+    for (int q = lane; q < 3 * L; q += 32) {
+      HPlane& pl = shared_planes ? S.plane[q / 3] : W.face(nF + q / 3).plane;
+      double* c = &pl.x + q % 3;
+      *c = pl.w > 0 ? __ddiv_rn(*c, pl.w) : 0.0;
+    }
+    __syncwarp();
+    for (int k = lane; k < L; k += 32) {
+      HFace& N = W.face(nF + k);
+      HPlane pl = shared_planes ? S.plane[k] : N.plane;
+      pl.w = dot3(D3{pl.x, pl.y, pl.z}, ld3(P, N.tv.x));
+      if (shared_planes) S.plane[k] = pl;
+      N.plane = pl;
+    }
+    if (norph <= 32 && vn <= 32 && L <= 32) {
+      // An ordinary step: the orphans stay in the lanes.
+      int sel = 0;
+      for (int i = 1; i < vn; ++i)
+        if (lane >= __shfl_sync(0xffffffffu, vo, i)) sel = i;
+      const int sx = __shfl_sync(0xffffffffu, vl.x, sel), so = __shfl_sync(0xffffffffu, vo, sel),
+                sf = __shfl_sync(0xffffffffu, vf, sel);
+      int pid = 0;
+      if (lane < norph) {
+        const int k = lane - so;
+        pid = W.pool(sx + k + (sf == cur && k >= bpos ? 1 : 0));
+      }
+      if (lane < vn) {
+        HFace& F = W.face(vf);
+        F.tv.w = 0;
+        F.outl.y = 0;
+      }
+      __syncwarp();
+      top = assign_lanes(P, W, S.plane, pid, norph, nF, L, eps, top, lane);
+      if (top < 0) return kHullPoolCap;
+      nF += L;
+      ++cur;
+      __syncwarp();
+      continue;
+    }
+    // Orphans of the visible faces in order (the apex skipped); visible faces
+    // die.
+    int* orph = norph <= kHullOrphans ? S.orph : W.orph;
     for (int i = 0; i < vn; ++i) {
-      const int f = W.vis[i];
-      const int2 fl = W.outl[f];
-      const int o0 = W.voff[i];
+      if (i > 0 && (i & 31) == 0 && i + lane < vn) {
+        vf = W.vis[i + lane];
+        vo = W.voff[i + lane];
+        vl = W.face(vf).outl;
+      }
+      const int f = __shfl_sync(0xffffffffu, vf, i & 31);
+      const int o0 = __shfl_sync(0xffffffffu, vo, i & 31);
+      const int2 fl = make_int2(__shfl_sync(0xffffffffu, vl.x, i & 31), __shfl_sync(0xffffffffu, vl.y, i & 31));
       if (f == cur) {
         for (int k = lane; k < fl.y; k += 32)
-          if (k != bpos) W.orph[o0 + (k < bpos ? k : k - 1)] = W.pool[fl.x + k];
+          if (k != bpos) orph[o0 + (k < bpos ? k : k - 1)] = W.pool(fl.x + k);
       } else {
-        for (int k = lane; k < fl.y; k += 32) W.orph[o0 + k] = W.pool[fl.x + k];
+        for (int k = lane; k < fl.y; k += 32) orph[o0 + k] = W.pool(fl.x + k);
       }
     }
     __syncwarp();
     for (int i = lane; i < vn; i += 32) {
-      const int f = W.vis[i];
-      W.tv[f].w = 0;
-      W.outl[f].y = 0;
+      const int f = vn <= 32 ? vf : W.vis[i];
+      W.face(f).tv.w = 0;
+      W.face(f).outl.y = 0;
     }
     __syncwarp();
-    top = assign_points(P, W, W.orph, norph, make_int4(-1, -1, -1, -1), nF, L, eps, top, lane);
+    top = assign_points(P, W, S, orph, norph, make_int4(-1, -1, -1, -1), nF, L, eps, top, lane);
     if (top < 0) return kHullPoolCap;
     nF += L;
     ++cur;
@@ -614,11 +777,11 @@ __device__ int hull_one(const double* P, int n, HullWork& W, int fix, int32_t* t
   int cnt = 0;
   for (int base = 0; base < nF; base += 32) {
     const int f = base + lane;
-    const bool alive = f < nF && W.tv[f].w;
+    const bool alive = f < nF && W.face(f).tv.w;
     const unsigned m = __ballot_sync(0xffffffffu, alive);
     if (cnt + __popc(m) > 2 * n) return kHullOutCap;
     if (alive) {
-      const int4 t = W.tv[f];
+      const int4 t = W.face(f).tv;
       int32_t* o = tris + 3 * (int64_t)(cnt + __popc(m & lanemask_lt()));
       o[0] = t.x;
       o[1] = t.y;
@@ -629,17 +792,13 @@ __device__ int hull_one(const double* P, int n, HullWork& W, int fix, int32_t* t
   ntri = cnt;
   if (fix) {
     // Centroid of all points, summed in index order as the host does.
-    D3 c{0.0, 0.0, 0.0};
-    if (lane == 0) {
-      for (int i = 0; i < n; ++i) {
-        const D3 p = ld3(P, i);
-        c = D3{da(c.x, p.x), da(c.y, p.y), da(c.z, p.z)};
-      }
-      c = div3(c, (double)n);
+    double sum = 0.0;
+    if (lane < 3) {
+#pragma unroll 8
+      for (int i = 0; i < n; ++i) sum = da(sum, P[3 * (int64_t)i + lane]);
+      sum = __ddiv_rn(sum, (double)n);
     }
-    c.x = __shfl_sync(0xffffffffu, c.x, 0);
-    c.y = __shfl_sync(0xffffffffu, c.y, 0);
-    c.z = __shfl_sync(0xffffffffu, c.z, 0);
+    const D3 c{__shfl_sync(0xffffffffu, sum, 0), __shfl_sync(0xffffffffu, sum, 1), __shfl_sync(0xffffffffu, sum, 2)};
     __syncwarp();
     for (int k = lane; k < cnt; k += 32) {
       int32_t* t = tris + 3 * (int64_t)k;
@@ -655,25 +814,60 @@ __device__ int hull_one(const double* P, int n, HullWork& W, int fix, int32_t* t
   return kHullOk;
 }
 
-__global__ void __launch_bounds__(32 * kHullWarps)
+// One part per block of one warp: fewer parts than SMs then have an SM each,
+// with its FP64 pipe. Bound by the one warp's dependent chain (about 9 cycles an
+// instruction, a third of it in the flood fill), not by memory: four warps a
+// block and lane 0 alone on the sequential steps took 106 ms on 10,242 points
+// on their hull, 5.6 ms on 642 and 38 ms on 200 sets of 2,562; this takes 69,
+// 3.6 and 26 (calls). smem: bytes of dynamic shared memory, for the points (up to
+// a quarter), the head of the outside-list pool and the first faces; what does
+// not fit stays in the work region.
+__global__ void __launch_bounds__(32, kHullPerSm)
     hull_kernel(const double* __restrict__ pts, const int64_t* __restrict__ poff, const int32_t* __restrict__ ids,
-                int32_t nj, char* __restrict__ arena, const int64_t* __restrict__ roff, int mult, int fix,
+                int32_t nj, char* __restrict__ arena, const int64_t* __restrict__ roff, int mult, int fix, int smem,
                 int32_t* __restrict__ tris, int32_t* __restrict__ counts, int32_t* __restrict__ pstatus) {
-  const int lane = threadIdx.x & 31;
-  const int nw = gridDim.x * kHullWarps;
-  for (int j = blockIdx.x * kHullWarps + (threadIdx.x >> 5); j < nj; j += nw) {
+  extern __shared__ __align__(16) char hull_smem[];
+  __shared__ HullShared S;
+  const int lane = threadIdx.x;
+  for (int j = blockIdx.x; j < nj; j += gridDim.x) {
     const int part = ids[j];
     const int64_t o = poff[part];
     const int n = (int)(poff[part + 1] - o);
     HullWork W = carve(arena + roff[j], n, mult);
+    const double* P = pts + 3 * o;
+    char* at = hull_smem;
+    int left = smem;
+    if ((int64_t)n * 24 <= left / 4) {
+      double* sp = reinterpret_cast<double*>(at);
+      for (int i = lane; i < 3 * n; i += 32) sp[i] = P[i];
+      P = sp;
+      const int b = (int)hull_a16((int64_t)n * 24);
+      at += b;
+      left -= b;
+    }
+    W.nsp = (int)(min((int64_t)(left / 8), W.cap.pool * 4) / 16 * 4);
+    W.spool = reinterpret_cast<int*>(at);
+    at += 4 * W.nsp;
+    left -= 4 * W.nsp;
+    W.nsf = (int)min((int64_t)(left / 80), W.cap.faces);
+    W.sface = reinterpret_cast<HFace*>(at);
+    __syncwarp();
     int ntri = 0;
-    const int st = hull_one(pts + 3 * o, n, W, fix, tris + 6 * o, ntri, lane);
+    const int st = hull_one(P, n, W, S, fix, tris + 6 * o, ntri, lane);
     if (lane == 0) {
       counts[part] = st == kHullOk ? ntri : 0;
       pstatus[part] = st;
     }
     __syncwarp();
   }
+}
+
+// Dynamic shared memory of a launch of nj parts: an even share of an SM for
+// the parts that will be on one together.
+inline int hull_smem_bytes(int64_t nj, int sm_count) {
+  const int64_t per_sm = std::min<int64_t>(kHullPerSm, (nj + sm_count - 1) / sm_count);
+  const int64_t share = 228 * 1024 / per_sm - 1024 - (int64_t)sizeof(HullShared);  // 1 KiB is the system's
+  return (int)(std::max<int64_t>(0, share) / 16 * 16);
 }
 
 size_t hull_align256(size_t x) { return (x + 255) & ~size_t(255); }
@@ -739,11 +933,13 @@ extern "C" int visacd_convex_hulls(visacd_ctx* ctx, const double* points, const 
     }
     VCUDA(cudaMemcpyAsync(base + oIds, ids.data(), ids.size() * 4, cudaMemcpyHostToDevice, st));
     VCUDA(cudaMemcpyAsync(base + oRoff, roff.data(), roff.size() * 8, cudaMemcpyHostToDevice, st));
-    const unsigned blocks =
-        (unsigned)std::min<int64_t>(((int64_t)ids.size() + kHullWarps - 1) / kHullWarps, 16LL * ctx->sm_count);
-    VLAUNCH(ctx, kKConvexHull, blocks, 32 * kHullWarps, 0, hull_kernel, (const double*)(base + oPts),
+    const unsigned blocks = (unsigned)std::min<int64_t>((int64_t)ids.size(), 64LL * ctx->sm_count);
+    const int smem = hull_smem_bytes((int64_t)ids.size(), ctx->sm_count);
+    VCUDA(cudaFuncSetAttribute(hull_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               227 * 1024 - (int)sizeof(HullShared)));
+    VLAUNCH(ctx, kKConvexHull, blocks, 32, smem, hull_kernel, (const double*)(base + oPts),
             (const int64_t*)(base + oOff), (const int32_t*)(base + oIds), (int32_t)ids.size(), base + oArena,
-            (const int64_t*)(base + oRoff), mult, (int)fix_normals, (int32_t*)(base + oTri),
+            (const int64_t*)(base + oRoff), mult, (int)fix_normals, smem, (int32_t*)(base + oTri),
             (int32_t*)(base + oCnt), (int32_t*)(base + oSt));
     VCUDA(cudaMemcpyAsync(st_now.data(), base + oSt, (size_t)nparts * 4, cudaMemcpyDeviceToHost, st));
     VCUDA(cudaMemcpyAsync(cnt_now.data(), base + oCnt, (size_t)nparts * 4, cudaMemcpyDeviceToHost, st));
