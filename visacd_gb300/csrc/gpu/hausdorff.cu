@@ -11,8 +11,9 @@
 //    meshes get FP32 triangle bounds (box, plane), in four launches plus a scan;
 //  * a two-ring search gives each query an upper bound of its term (the
 //    nearest sample's distance, rounded up); queries with no sample that
-//    close are evaluated one warp each (hhead_kernel);
-//  * the rest skip when their bound does not exceed the running maximum;
+//    close are evaluated one warp each (hterm_kernel);
+//  * of the rest, those with the largest bounds are evaluated first; the others
+//    skip when their bound does not exceed the maximum so far (hselect_kernel);
 //  * k-NN candidates are ranked in FP32 with a proven rounding margin and the
 //    exact 10 chosen in FP64; triangle distances whose FP32 lower bound cannot
 //    lower the minimum are skipped.
@@ -223,7 +224,7 @@ struct HSide {
 // A triangle already seen, or whose FP32 lower bound (box gap or plane
 // distance, minus the rounding margin) is not below the current minimum,
 // cannot lower it and is not evaluated.
-__device__ double query_term(const HSide& S, int qi, float tmargin) {
+__device__ __noinline__ double query_term(const HSide& S, int qi, float tmargin) {
   const double q[3] = {S.Q[3 * (int64_t)qi], S.Q[3 * (int64_t)qi + 1], S.Q[3 * (int64_t)qi + 2]};
   double bd[kKnn];
   int bi[kKnn];
@@ -263,113 +264,129 @@ __device__ double query_term(const HSide& S, int qi, float tmargin) {
   return cmin;
 }
 
-// The smallest not-yet-taken value across the warp's sorted per-lane lists
-// (fd[ptr..]), taken: returns it and its id; ties go to the lower lane.
-__device__ __forceinline__ float warp_take_min(const float (&fd)[kKnnF], const int (&fi)[kKnnF], int nf, int& ptr,
-                                               int& id_out) {
-  const int lane = threadIdx.x & 31;
-  const float mine = ptr < nf ? fd[ptr] : 3.4e38f;
-  float m = mine;
-  for (int o = 16; o; o >>= 1) m = fminf(m, __shfl_xor_sync(0xffffffffu, m, o));
-  const unsigned who = __ballot_sync(0xffffffffu, mine == m && ptr < nf);
-  const int src = who ? __ffs(who) - 1 : 0;
-  int id = ptr < nf ? fi[ptr] : -1;
-  id = __shfl_sync(0xffffffffu, id, src);
-  if (who && lane == src) ++ptr;
-  id_out = who ? id : -1;
-  return who ? m : 3.4e38f;
-}
-
-// query_term for one query by a whole warp (used for the few queries with the
-// largest bounds, which are far from the other surface and walk many rings):
-// the lanes split each ring's cells and each keeps its kKnnF smallest FP32
-// distances, so the warp's kKnnF smallest are exact (a candidate a lane drops
-// has kKnnF smaller ones in that lane alone); a warp tournament takes them in
-// order. Same stop rule, same FP32-to-FP64 selection proof and the same term
-// as query_term; returns false (on all lanes) when the proof fails, and the
-// caller then uses query_term. (These queries are evaluated in full: the
-// nearest sample's distance does not bound the reference formula's minimum
-// when its triangle is degenerate, so it is not used to skip them.)
-constexpr int kTermOk = 0, kTermUnproven = 1, kTermSkipped = 2;
-// r0: the first ring to walk (0: every ring; the rings inside r0 must hold no
-// sample of G).
-
-template <class Prune>
-__device__ int query_term_warp(const HSide& S, int qi, int r0, const Prune& prune, double& term) {
+// The first half of query_term for one query by a whole warp, the ids of its
+// exact 10 nearest samples in order. Lane m < kKnnF holds the m-th smallest FP32
+// distance so far and its sample. A ring is walked as its 8r rows along x, whose
+// samples are contiguous, and the 2 (2r - 1)^2 cells at its two ends, 32 of them
+// at a time; their samples are tested 32 at a time, and those below the last
+// kept distance inserted by ballot and shuffle (sorted lists per lane lie in
+// local memory and leave a long row to one lane: 187 us for a query far from
+// the surface). query_term's stop rule and selection proof; returns false (on
+// all lanes) when the proof fails or the 10th and 11th distances are equal, and
+// the caller then uses query_term, whose order decides which of the two counts.
+// (Queries without a bound are evaluated in full: the nearest sample's distance
+// does not bound the reference formula's minimum when its triangle is
+// degenerate, so it is not used to skip them.)
+__device__ bool query_knn_warp(const HSide& S, int qi, int* ids, int& cnt_out, double& d0_out) {
   const int lane = threadIdx.x & 31;
   const HGrid& G = S.G;
   const double q[3] = {S.Q[3 * (int64_t)qi], S.Q[3 * (int64_t)qi + 1], S.Q[3 * (int64_t)qi + 2]};
-  const int cx = cell_coord(q[0], G.lo[0], G.h, G.dim[0]);
-  const int cy = cell_coord(q[1], G.lo[1], G.h, G.dim[1]);
-  const int cz = cell_coord(q[2], G.lo[2], G.h, G.dim[2]);
+  // The query's cell: one division per lane.
+  const int a = lane % 3;
+  const int ca = cell_coord(a == 0 ? q[0] : (a == 1 ? q[1] : q[2]), a == 0 ? G.lo[0] : (a == 1 ? G.lo[1] : G.lo[2]),
+                            G.h, a == 0 ? G.dim[0] : (a == 1 ? G.dim[1] : G.dim[2]));
+  const int cx = __shfl_sync(0xffffffffu, ca, 0), cy = __shfl_sync(0xffffffffu, ca, 1),
+            cz = __shfl_sync(0xffffffffu, ca, 2);
   const int rmax = max(G.dim[0], max(G.dim[1], G.dim[2]));
   const float qf[3] = {(float)q[0], (float)q[1], (float)q[2]};
   const float hf = (float)G.h;
-  float fd[kKnnF];
-  int fi[kKnnF];
-  int nf = 0;
-  int total = 0;  // candidates seen by the warp
-  float g10 = 3.4e38f;
-  for (int r = r0; r <= rmax; ++r) {
-    const int side = 2 * r + 1;
-    const int cube = side * side * side;
-    int seen = 0;
-    for (int t = lane; t < cube; t += 32) {
-      const int dx = t % side - r, dy = (t / side) % side - r, dz = t / (side * side) - r;
-      if (max(abs(dx), max(abs(dy), abs(dz))) != r) continue;
-      const int x = cx + dx, y = cy + dy, z = cz + dz;
-      if (x < 0 || x >= G.dim[0] || y < 0 || y >= G.dim[1] || z < 0 || z >= G.dim[2]) continue;
-      const int c = (z * G.dim[1] + y) * G.dim[0] + x;
-      for (int k = G.start[c]; k < G.start[c + 1]; ++k) {
-        const float4 sp = G.spts[k];
-        const float ex = sp.x - qf[0], ey = sp.y - qf[1], ez = sp.z - qf[2];
-        const float d2 = ex * ex + ey * ey + ez * ez;
-        ++seen;
-        if (nf < kKnnF || d2 < fd[nf - 1]) {
-          int j = nf < kKnnF ? nf++ : kKnnF - 1;
-          while (j > 0 && fd[j - 1] > d2) {
-            fd[j] = fd[j - 1];
-            fi[j] = fi[j - 1];
-            --j;
+  float myv = 3.4e38f;  // lane m: the m-th kept distance
+  int myid = -1;
+  int nf = 0;           // kept (at most kKnnF)
+  int total = 0;        // candidates seen
+  float last = 3.4e38f;  // the kKnnF-th kept distance
+  for (int r = 0; r <= rmax; ++r) {
+    const int side = 2 * r - 1;
+    const int rows = r > 0 ? 8 * r : 1;
+    const int items = r > 0 ? rows + 2 * side * side : 1;
+    for (int t0 = 0; t0 < items; t0 += 32) {
+      const int t = t0 + lane;
+      int k0 = 0, len = 0;
+      if (t < items) {
+        int dy, dz, x0 = cx - r, x1 = cx + r;
+        if (t < rows) {
+          // the rows at dz = -r, at dz = r (2r + 1 each), then at dy = -r and r
+          const int w = 2 * r + 1;
+          const int u = t - 2 * w;
+          dz = t < w ? -r : (t < 2 * w ? r : (u >> 1) - r + 1);
+          dy = t < w ? t - r : (t < 2 * w ? t - w - r : ((u & 1) ? r : -r));
+        } else {
+          const int u = (t - rows) >> 1;
+          dz = u / side - r + 1;
+          dy = u % side - r + 1;
+          if ((t - rows) & 1) x0 = x1;
+          else x1 = x0;
+        }
+        const int y = cy + dy, z = cz + dz;
+        x0 = max(x0, 0);
+        x1 = min(x1, G.dim[0] - 1);
+        if (x0 <= x1 && y >= 0 && y < G.dim[1] && z >= 0 && z < G.dim[2]) {
+          const int c = (z * G.dim[1] + y) * G.dim[0];
+          k0 = G.start[c + x0];
+          len = G.start[c + x1 + 1] - k0;
+        }
+      }
+      if (!__any_sync(0xffffffffu, len > 0)) continue;
+      int end = len;  // inclusive sums of the lengths
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, end, o);
+        if (lane >= o) end += x;
+      }
+      const int sum = __shfl_sync(0xffffffffu, end, 31);
+      total += sum;
+      for (int p0 = 0; p0 < sum; p0 += 32) {
+        // The item of candidate p: the first whose end lies beyond it.
+        const int p = p0 + lane;
+        int it = 0;
+#pragma unroll
+        for (int o = 16; o; o >>= 1)
+          if (__shfl_sync(0xffffffffu, end, it + o - 1) <= p) it += o;
+        it = min(it, 31);
+        const int k = __shfl_sync(0xffffffffu, k0, it) + p -
+                      (__shfl_sync(0xffffffffu, end, it) - __shfl_sync(0xffffffffu, len, it));
+        float d2 = 0.f;
+        int id = -1;
+        if (p < sum) {
+          const float4 sp = G.spts[k];
+          const float ex = sp.x - qf[0], ey = sp.y - qf[1], ez = sp.z - qf[2];
+          d2 = ex * ex + ey * ey + ez * ez;
+          id = __float_as_int(sp.w);
+        }
+        unsigned m = __ballot_sync(0xffffffffu, id >= 0 && (nf < kKnnF || d2 < last));
+        while (m) {
+          const int src = __ffs(m) - 1;
+          m &= m - 1;
+          const float v = __shfl_sync(0xffffffffu, d2, src);
+          const int vid = __shfl_sync(0xffffffffu, id, src);
+          if (nf == kKnnF && !(v < last)) continue;
+          const int pos = __popc(__ballot_sync(0xffffffffu, lane < nf && myv <= v));
+          const float uv = __shfl_up_sync(0xffffffffu, myv, 1);
+          const int ui = __shfl_up_sync(0xffffffffu, myid, 1);
+          if (nf < kKnnF) ++nf;
+          if (lane < nf && lane >= pos) {
+            myv = lane == pos ? v : uv;
+            myid = lane == pos ? vid : ui;
           }
-          fd[j] = d2;
-          fi[j] = __float_as_int(sp.w);
+          if (nf == kKnnF) last = __shfl_sync(0xffffffffu, myv, kKnnF - 1);
         }
       }
     }
-    for (int o = 16; o; o >>= 1) seen += __shfl_xor_sync(0xffffffffu, seen, o);
-    total += seen;
     if (total >= kKnn) {
-      int ptr = 0, id;
-      float v = 3.4e38f;
-      for (int m = 0; m < kKnn; ++m) v = warp_take_min(fd, fi, nf, ptr, id);
-      g10 = v;
+      const float g10 = __shfl_sync(0xffffffffu, myv, kKnn - 1);
       if (__fadd_ru(__fmul_ru(__fsqrt_ru(g10), 1.0f + 1.0f / 1048576.0f), G.eabs) <=
           __fmul_rd((float)r, hf) * (1.0f - 1e-6f))
         break;
-    }
-  }
-  // The warp's kKnnF smallest (value, id) in order: lane m holds the m-th.
-  float myv = 3.4e38f;
-  int myid = -1;
-  {
-    int ptr = 0;
-    for (int m = 0; m < kKnnF; ++m) {
-      int id;
-      const float v = warp_take_min(fd, fi, nf, ptr, id);
-      if (lane == m) {
-        myv = v;
-        myid = id;
-      }
     }
   }
   // The exact 10 nearest are among these when the kKnnF-th FP32 distance
   // exceeds the 10th by more than twice the bound (or all were kept).
   if (total > kKnnF) {
     const float v16 = __shfl_sync(0xffffffffu, myv, kKnnF - 1);
+    const float g10 = __shfl_sync(0xffffffffu, myv, kKnn - 1);
     const bool ok = __fsqrt_rd(v16) * (1.0f - 1.0f / 1048576.0f) >
                     __fadd_ru(__fadd_ru(__fmul_ru(__fsqrt_ru(g10), 1.0f + 1.0f / 1048576.0f), G.eabs), G.eabs);
-    if (!ok) return kTermUnproven;
+    if (!ok) return false;
   }
   // Exact FP64 distances of the (up to) kKnnF candidates, the 10 nearest kept
   // in order (insertion in candidate order, as query_term).
@@ -379,47 +396,27 @@ __device__ int query_term_warp(const HSide& S, int qi, int r0, const Prune& prun
     const double ex = ds(pp[0], q[0]), ey = ds(pp[1], q[1]), ez = ds(pp[2], q[2]);
     d2 = da(da(dm(ex, ex), dm(ey, ey)), dm(ez, ez));
   }
-  double bd[kKnn];
-  int bi[kKnn];
-  int cnt = 0;
+  if (__any_sync(0xffffffffu, myid >= 0 && !(d2 < DBL_MAX))) return false;  // not finite
+  // Rank of each among them (candidate order between equals); non-negative
+  // doubles order like their bits, and FP64 compares are slow.
+  const unsigned long long key = (unsigned long long)__double_as_longlong(d2);
+  int rank = 0;
+  bool tie = false;
   for (int m = 0; m < kKnnF; ++m) {
-    const double v = __shfl_sync(0xffffffffu, d2, m);
+    const unsigned long long v = __shfl_sync(0xffffffffu, key, m);
     const int id = __shfl_sync(0xffffffffu, myid, m);
-    if (id < 0) continue;
-    if (cnt < kKnn || v < bd[cnt - 1]) {
-      int j = cnt < kKnn ? cnt++ : kKnn - 1;
-      while (j > 0 && bd[j - 1] > v) {
-        bd[j] = bd[j - 1];
-        bi[j] = bi[j - 1];
-        --j;
-      }
-      bd[j] = v;
-      bi[j] = id;
-    }
+    if (id < 0 || m == lane) continue;
+    rank += v < key || (v == key && m < lane);
+    tie |= v == key && m < lane;
   }
-  // Point-triangle distances of the k nearest in parallel (lane j), then the
-  // sequential minimum with the early stop below 1e-14, in order.
-  double dj = DBL_MAX;
-  int which = -1;
-#pragma unroll
-  for (int j = 0; j < kKnn; ++j)
-    if (j == lane && j < cnt) which = bi[j];
-  if (which >= 0) {
-    const int tj = S.ids[which];
-    const int* t = S.mt + 3 * (int64_t)tj;
-    dj = ref_point_tri_dist(q, S.mv + 3 * (int64_t)t[0], S.mv + 3 * (int64_t)t[1], S.mv + 3 * (int64_t)t[2]);
-  }
-  double cmin = DBL_MAX;
-  for (int j = 0; j < cnt; ++j) {
-    const double d = __shfl_sync(0xffffffffu, dj, j);
-    if (d < cmin) {
-      cmin = d;
-      if (cmin < 1e-14) break;
-    }
-  }
-  if (cmin > 10 && cnt > 0) cmin = __dsqrt_rn(bd[0]);
-  term = cmin;
-  return kTermOk;
+  // Equal distances at ranks 9 and 10 (from 0): which one counts is query_term's.
+  const int cand = __popc(__ballot_sync(0xffffffffu, myid >= 0));
+  if (__any_sync(0xffffffffu, myid >= 0 && rank == kKnn && tie)) return false;
+  if (myid >= 0 && rank < kKnn) ids[rank] = myid;
+  d0_out = __shfl_sync(0xffffffffu, d2, max(__ffs(__ballot_sync(0xffffffffu, myid >= 0 && rank == 0)), 1) - 1);
+  cnt_out = min(cand, kKnn);
+  __syncwarp();
+  return true;
 }
 
 // ---- batched evaluation ----------------------------------------------------
@@ -442,6 +439,7 @@ struct HBatch {
   float4* tb;                         // FP32 bounds of all triangles (3 per triangle)
   const double* lower;                // per job: a known lower bound of the job's concavity (volume term)
   unsigned long long* job_max;        // per job: largest term found (double bits)
+  unsigned* job_ub;                   // per job: largest finite upper bound of a term (float bits)
   unsigned long long* gmax;           // largest of the floor, the lower bounds and every term found
   const float* tmargin;               // per job
   int independent;                    // 1: no pruning across jobs
@@ -668,45 +666,121 @@ __global__ void __launch_bounds__(128) hbound_kernel(HBatch H, long long nsamp, 
       }
     }
     if (!proven) farlist[atomicAdd(far, 1u)] = e;
+    else if (__float_as_uint(ub) > *(const volatile unsigned*)(H.job_ub + (s >> 1)))
+      atomicMax(H.job_ub + (s >> 1), __float_as_uint(ub));
     ubs[e] = ub;
     qref[e] = make_int2(s, qi);
   }
 }
 
-// Terms of the queries without a bound (the farlist), one warp each: mostly
-// queries far from the other surface, which walk many rings (and a few near a
-// degenerate triangle); their exact terms raise the maxima that prune the rest.
-__global__ void __launch_bounds__(128) hhead_kernel(HBatch H, const int2* __restrict__ qref,
-                                                    const long long* __restrict__ farlist,
-                                                    const unsigned* __restrict__ far) {
-  const int head = (int)*far;
-  const int warps = (gridDim.x * blockDim.x) >> 5;
-  for (int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < head; w += warps) {
-    const int2 r = qref[farlist[w]];
-    const int job = r.x >> 1;
-    const HSide& S = H.sides[r.x];
-    double term;
-    const int status =
-        query_term_warp(S, r.y, 0, [&](double ub) { return prunable(H, job, ub); }, term);
-    if (status == kTermSkipped) continue;
-    if (status == kTermUnproven) term = query_term(S, r.y, H.tmargin[job]);
-    if ((threadIdx.x & 31) == 0 && term < DBL_MAX) publish(H, job, term);
+// Queries with a bound that a pass evaluates, appended to list: first those
+// whose bound is at least kSeedShare of their job's largest (and, where jobs do
+// not prune one another, every kSeedStep-th), then, against the
+// maxima these and the queries without a bound gave, the others that can still
+// change a used result (prunable).
+// Seeds decide how much the second list holds: 24 sets with 210,014 samples have
+// 3,233 queries with a bound above the final maxima; with the share alone 96,028
+// were listed, with every 64th query too some 27,000. Jobs that prune one another
+// need no such sample: their second list is empty with the share alone.
+constexpr float kSeedShare = 0.9f;
+constexpr int kSeedStep = 64;
+__global__ void __launch_bounds__(256) hselect_kernel(HBatch H, const float* __restrict__ ubs,
+                                                      const int2* __restrict__ qref, long long nsamp, int seeds,
+                                                      unsigned* __restrict__ count, long long* __restrict__ list) {
+  const int lane = threadIdx.x & 31;
+  for (long long e0 = ((long long)blockIdx.x * blockDim.x + threadIdx.x) - lane; e0 < nsamp;
+       e0 += (long long)gridDim.x * blockDim.x) {
+    const long long e = e0 + lane;
+    bool take = false;
+    if (e < nsamp) {
+      const float ub = ubs[e];
+      if (ub < __int_as_float(0x7f800000)) {
+        const int job = qref[e].x >> 1;
+        const bool seed = ub >= kSeedShare * __uint_as_float(H.job_ub[job]) || (H.independent && e % kSeedStep == 0);
+        take = seed == (seeds != 0) && !prunable(H, job, (double)ub);
+      }
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, take);
+    if (!m) continue;
+    unsigned at = 0;
+    if (lane == 0) at = atomicAdd(count, (unsigned)__popc(m));
+    at = __shfl_sync(0xffffffffu, at, 0);
+    if (take) list[at + __popc(m & ((1u << lane) - 1u))] = e;
   }
 }
 
-// Terms of the queries with a bound; a query whose bound cannot change a used
-// result (prunable) is skipped.
-__global__ void __launch_bounds__(128) hquery_kernel(HBatch H, const float* __restrict__ ubs,
-                                                     const int2* __restrict__ qref, long long nsamp) {
-  for (long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x; e < nsamp;
-       e += (long long)gridDim.x * blockDim.x) {
-    const float ub = ubs[e];
-    if (!(ub < __int_as_float(0x7f800000))) continue;  // no bound: evaluated by hhead_kernel
-    const int2 r = qref[e];
-    const int job = r.x >> 1;
-    if (prunable(H, job, (double)ub)) continue;
-    const double cmin = query_term(H.sides[r.x], r.y, H.tmargin[job]);
-    if (DBL_MAX > cmin) publish(H, job, cmin);
+// Terms of the listed queries; a query whose bound no longer matters is skipped.
+// A first launch takes the queries without a bound (mostly far from the other
+// surface, with many rings to walk, and a few near a degenerate triangle) and
+// the seeds, a second one what their maxima leave. On a list longer than the
+// grid's warps a warp finds the nearest samples of two or three queries one after
+// another, then evaluates their triangle distances together (FP64). The list is walked with a
+// stride prime to its length, so that the queries in flight come from all jobs
+// and raise all maxima early. On the 210,014 samples the two launches with their
+// selections take 216 and 277 us; one thread per query in cell order (105,629
+// evaluated) took 905 us, and sorted lists per lane over whole cubes of cells 920
+// us for the 4,221 without a bound.
+__global__ void __launch_bounds__(128) hterm_kernel(HBatch H, const float* __restrict__ ubs,
+                                                    const int2* __restrict__ qref, const long long* __restrict__ list,
+                                                    const unsigned* __restrict__ count) {
+  __shared__ int near_ids[4][3 * kKnn];
+  int* ids = near_ids[threadIdx.x >> 5];
+  const unsigned n = *count;
+  const int lane = threadIdx.x & 31;
+  const unsigned warps = (gridDim.x * blockDim.x) >> 5;
+  const unsigned group = n <= warps ? 1 : (n <= 2 * warps ? 2 : 3);
+  const int mine = min(lane / kKnn, 2), j = lane - kKnn * mine;  // lanes 30, 31: j >= kKnn
+  for (unsigned w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < n; w += group * warps) {
+    int set = 0, qi = 0, cnt = 0;  // of this lane's query
+    double d0 = 0.0;
+    for (int i = 0; i < (int)group; ++i) {
+      const unsigned k = w + (unsigned)i * warps;
+      if (k >= n) break;
+      const long long e = list[(unsigned)((unsigned long long)k * 2654435761ull % n)];
+      const int2 r = qref[e];
+      const int job = r.x >> 1;
+      // (lane 0's view of the maxima: they move while the warp reads them)
+      const float ub = ubs[e];
+      const bool skip = ub < __int_as_float(0x7f800000) && prunable(H, job, (double)ub);
+      if (__shfl_sync(0xffffffffu, (int)skip, 0)) continue;
+      int c = 0;
+      double d = 0.0;
+      if (!query_knn_warp(H.sides[r.x], r.y, ids + kKnn * i, c, d)) {
+        const double term = query_term(H.sides[r.x], r.y, H.tmargin[job]);
+        if (lane == 0 && term < DBL_MAX) publish(H, job, term);
+        continue;
+      }
+      if (mine == i) {
+        set = r.x;
+        qi = r.y;
+        cnt = c;
+        d0 = d;
+      }
+    }
+    double dj = DBL_MAX;
+    if (j < cnt) {
+      const HSide& S = H.sides[set];
+      const double* q = S.Q + 3 * (int64_t)qi;
+      const double qq[3] = {q[0], q[1], q[2]};
+      const int* t = S.mt + 3 * (int64_t)S.ids[ids[kKnn * mine + j]];
+      dj = ref_point_tri_dist(qq, S.mv + 3 * (int64_t)t[0], S.mv + 3 * (int64_t)t[1], S.mv + 3 * (int64_t)t[2]);
+    }
+    // The sequential minimum with the early stop below 1e-14, in order.
+    double cmin = DBL_MAX;
+    bool stop = false;
+#pragma unroll
+    for (int m = 0; m < kKnn; ++m) {
+      const double d = __shfl_sync(0xffffffffu, dj, kKnn * mine + m);
+      if (!stop && d < cmin) {
+        cmin = d;
+        stop = cmin < 1e-14;
+      }
+    }
+    if (j == 0 && cnt > 0) {
+      if (cmin > 10) cmin = __dsqrt_rn(d0);
+      if (cmin < DBL_MAX) publish(H, set >> 1, cmin);
+    }
+    __syncwarp();
   }
 }
 
@@ -806,9 +880,9 @@ extern "C" int visacd_face_hausdorff_batch(visacd_ctx* ctx, int32_t njobs, const
                o_low = carve((size_t)njobs * 8), o_tm = carve((size_t)njobs * 4), o_gm = carve(8),
                o_grids = carve(sizeof(HGrid) * S), o_sides = carve(sizeof(HSide) * S);
   const size_t upload = off;
-  // Zeroed together: job maxima, far count, per-cell counts and fills.
+  // Zeroed together: job maxima and largest bounds, the two lists' counts, per-cell counts and fills.
   const size_t zero_begin = off;
-  const size_t o_jm = carve((size_t)njobs * 8), o_far = carve(8), o_cnt = carve((size_t)(ncell + 1) * 4),
+  const size_t o_jm = carve((size_t)njobs * 8), o_ju = carve((size_t)njobs * 4), o_far = carve(8), o_cnt = carve((size_t)(ncell + 1) * 4),
                o_fill = carve((size_t)ncell * 4);
   const size_t zero_end = off;
   const size_t o_off = carve((size_t)(ncell + 1) * 8), o_cell = carve((size_t)NS * 4),
@@ -873,6 +947,7 @@ extern "C" int visacd_face_hausdorff_batch(visacd_ctx* ctx, int32_t njobs, const
   H.tb = (float4*)(D + o_tb);
   H.lower = (const double*)(D + o_low);
   H.job_max = (unsigned long long*)(D + o_jm);
+  H.job_ub = (unsigned*)(D + o_ju);
   H.gmax = (unsigned long long*)(D + o_gm);
   H.tmargin = (const float*)(D + o_tm);
   H.independent = independent ? 1 : 0;
@@ -889,11 +964,19 @@ extern "C" int visacd_face_hausdorff_batch(visacd_ctx* ctx, int32_t njobs, const
   unsigned* far = (unsigned*)(D + o_far);
   VLAUNCH(ctx, kKHausdorffBound, grid_for(NS, 128, 8LL * ctx->sm_count), 128, 0, hbound_kernel, H, NS,
           (const int*)(D + o_order), (float*)(D + o_ub), (int2*)(D + o_qref), far, (long long*)(D + o_farl));
-  // The queries without a bound one warp each, then the rest with pruning.
-  VLAUNCH(ctx, kKHausdorffHead, grid_for(32LL * NS, 128, 8LL * ctx->sm_count), 128, 0, hhead_kernel, H,
-          (const int2*)(D + o_qref), (const long long*)(D + o_farl), (const unsigned*)far);
-  VLAUNCH(ctx, kKHausdorffQuery, grid_for(NS, 128, 8LL * ctx->sm_count), 128, 0, hquery_kernel, H,
-          (const float*)(D + o_ub), (const int2*)(D + o_qref), NS);
+  // The queries without a bound and the seeds, then what their maxima leave (the
+  // list's second use starts after its first).
+  const float* ubs = (const float*)(D + o_ub);
+  const int2* qref = (const int2*)(D + o_qref);
+  long long* list = (long long*)(D + o_farl);
+  const unsigned gsel = grid_for(NS, 256, 8LL * ctx->sm_count);
+  const unsigned gterm = grid_for(32LL * NS, 128, 8LL * ctx->sm_count);
+  VLAUNCH(ctx, kKHausdorffHead, gsel, 256, 0, hselect_kernel, H, ubs, qref, NS, 1, far, list);
+  VLAUNCH(ctx, kKHausdorffHead, gterm, 128, 0, hterm_kernel, H, ubs, qref, (const long long*)list,
+          (const unsigned*)far);
+  VLAUNCH(ctx, kKHausdorffQuery, gsel, 256, 0, hselect_kernel, H, ubs, qref, NS, 0, far + 1, list);
+  VLAUNCH(ctx, kKHausdorffQuery, gterm, 128, 0, hterm_kernel, H, ubs, qref, (const long long*)list,
+          (const unsigned*)(far + 1));
   double* hres = nullptr;
   VTRY(pinned(ctx, (size_t)njobs * 8, (void**)&hres));
   VCUDA(cudaMemcpyAsync(hres, D + o_jm, (size_t)njobs * 8, cudaMemcpyDeviceToHost, st));
