@@ -17,7 +17,7 @@
 //  2. conflict_kernel (two passes: count, fill): for every pair j < k of valid
 //     candidates, "k is similar to j" — |n_k . n_j| > cos 5 deg and
 //     |d_k - d_j| < 1e-3, the reference's test in its FP64 order — over a
-//     triangle of 256 x 256 tiles, with an FP32 offset pre-filter (a margin
+//     triangle of 256 x 256 tiles, with FP32 offset and dot-product pre-filters (margins
 //     far above the FP32 rounding of the offsets) in front of the FP64 test.
 //     The similar earlier candidates of each k form a CSR list.
 //  3. resolve_kernel (one CTA): the reference keeps candidate k when no kept
@@ -100,44 +100,58 @@ __device__ __forceinline__ void tri_tile(int x, int& kt, int& jt) {
 }
 
 // Pass 0 counts, pass 1 fills the CSR lists of similar earlier candidates.
+// Bound by instruction issue: the offsets are tested four at a time in FP32, what
+// passes by an FP32 dot product (1e-5 below the limit, for unit normals rounded to
+// FP32), and only what passes that in FP64, whose few units would otherwise bound
+// this: nearly every warp has a lane with a pair of close offsets, and seven FP64
+// instructions for it took 91 us a pass over some 11,100 planes (990 tiles).
 template <int PASS>
 __global__ void __launch_bounds__(kCandTile) conflict_kernel(
     const Plane64* __restrict__ planes, const float* __restrict__ d32,
     const uint8_t* __restrict__ state, int32_t D, double normal_eps, uint32_t* __restrict__ count,
     const uint64_t* __restrict__ offset, uint32_t* __restrict__ fill, int32_t* __restrict__ list) {
-  __shared__ Plane64 spl[kCandTile];
-  __shared__ float sd[kCandTile];
-  __shared__ uint8_t sst[kCandTile];
+  __shared__ float4 snorm[kCandTile];
+  __shared__ __align__(16) float sd[kCandTile];  // +inf: no candidate
   int kt, jt;
   tri_tile(blockIdx.x, kt, jt);
   const int j0 = jt * kCandTile;
   const int j = j0 + threadIdx.x;
-  if (j < D) {
-    spl[threadIdx.x] = planes[j];
+  sd[threadIdx.x] = __int_as_float(0x7f800000);
+  if (j < D && state[j] != kInvalid) {
+    const Plane64 p = planes[j];
+    snorm[threadIdx.x] = make_float4((float)p.x, (float)p.y, (float)p.z, 0.f);
     sd[threadIdx.x] = d32[j];
-    sst[threadIdx.x] = state[j];
-  } else {
-    sst[threadIdx.x] = kInvalid;
   }
   __syncthreads();
   const int k = kt * kCandTile + threadIdx.x;
   if (k >= D || state[k] == kInvalid) return;
   const Plane64 pk = planes[k];
-  const float dk = d32[k];
+  const float kx = (float)pk.x, ky = (float)pk.y, kz = (float)pk.z;
+  const float dk = d32[k], near = 1.001e-3f;  // FP32 offsets differ by < 1e-6 from FP64
+  const float eps32 = (float)normal_eps - 1e-5f;
   const int jend = min(kCandTile, k - j0);  // earlier candidates only
   uint32_t c = 0;
-  for (int t = 0; t < jend; ++t) {
-    if (sst[t] == kInvalid) continue;
-    if (!(fabsf(dk - sd[t]) < 1.001e-3f)) continue;  // FP32 offsets differ by < 1e-6 from FP64
-    const Plane64 pj = spl[t];
-    const double dt =
-        fabs(__dadd_rn(__dadd_rn(__dmul_rn(pk.x, pj.x), __dmul_rn(pk.y, pj.y)), __dmul_rn(pk.z, pj.z)));
-    if (dt > normal_eps && fabs(__dsub_rn(pk.w, pj.w)) < 1e-3) {
-      if (PASS == 0) {
-        ++c;
-      } else {
-        const uint32_t pos = atomicAdd(&fill[k], 1u);
-        list[offset[k] + pos] = j0 + t;
+#pragma unroll 2
+  for (int t4 = 0; t4 < jend; t4 += 4) {
+    const float4 d = *reinterpret_cast<const float4*>(sd + t4);
+    const bool n0 = fabsf(dk - d.x) < near, n1 = fabsf(dk - d.y) < near, n2 = fabsf(dk - d.z) < near,
+               n3 = fabsf(dk - d.w) < near;
+    if (!(n0 || n1 || n2 || n3)) continue;
+    for (int u = 0; u < 4; ++u) {
+      const int t = t4 + u;
+      if (t >= jend || !(u == 0 ? n0 : (u == 1 ? n1 : (u == 2 ? n2 : n3)))) continue;
+      const float4 s = snorm[t];
+      if (!(fabsf(kx * s.x + ky * s.y + kz * s.z) > eps32)) continue;
+      const Plane64 pj = planes[j0 + t];
+      const double dt =
+          fabs(__dadd_rn(__dadd_rn(__dmul_rn(pk.x, pj.x), __dmul_rn(pk.y, pj.y)), __dmul_rn(pk.z, pj.z)));
+      if (dt > normal_eps && fabs(__dsub_rn(pk.w, pj.w)) < 1e-3) {
+        if (PASS == 0) {
+          ++c;
+        } else {
+          const uint32_t pos = atomicAdd(&fill[k], 1u);
+          list[offset[k] + pos] = j0 + t;
+        }
       }
     }
   }
@@ -145,10 +159,19 @@ __global__ void __launch_bounds__(kCandTile) conflict_kernel(
 }
 
 // Greedy keep-first resolution in rounds (one CTA). status bit on overrun.
-__global__ void resolve_kernel(const uint64_t* __restrict__ offset, const int32_t* __restrict__ list,
-                               uint8_t* __restrict__ state, int32_t D, unsigned* __restrict__ status) {
+// Up to kResolveShared candidates their states are kept in shared memory: the
+// rounds read them along the lists, and through L2 that took 35 us on some 11,100.
+constexpr int kResolveShared = 32768;
+__global__ void __launch_bounds__(1024) resolve_kernel(const uint64_t* __restrict__ offset,
+                                                       const int32_t* __restrict__ list, uint8_t* __restrict__ state,
+                                                       int32_t D, unsigned* __restrict__ status) {
   __shared__ int undecided;
-  volatile uint8_t* st = state;
+  __shared__ uint8_t sstate[kResolveShared];
+  const bool in_shared = D <= kResolveShared;
+  volatile uint8_t* st = in_shared ? sstate : state;
+  if (in_shared)
+    for (int k = threadIdx.x; k < D; k += blockDim.x) sstate[k] = state[k];
+  __syncthreads();
   bool done = false;
   for (int round = 0; round <= D + 1; ++round) {
     if (threadIdx.x == 0) undecided = 0;
@@ -178,6 +201,10 @@ __global__ void resolve_kernel(const uint64_t* __restrict__ offset, const int32_
       break;
     }
     __syncthreads();
+  }
+  if (in_shared) {
+    __syncthreads();
+    for (int k = threadIdx.x; k < D; k += blockDim.x) state[k] = sstate[k];
   }
   if (!done && threadIdx.x == 0) atomicOr(status, kStatusWorkOverrun);
 }
@@ -342,7 +369,9 @@ __global__ void split_argmax_kernel(const double* __restrict__ scores, const Pla
 // entries, lane l holding the l-th smallest; D maps to an unsigned key with the
 // same order, so (key, edge) compares like (D, edge).
 constexpr int kRefineK = 32;
-constexpr int kRefineTile = 512;  // edges per block step; one warp per proposal
+constexpr int kRefineTile = 512;   // threads of the merge; one warp per proposal
+constexpr int kRefineEdges = 128;  // edges per block step of the first pass
+constexpr int kRefineProps = 8;    // proposals per block of the first pass, one warp each
 constexpr int kLearnedProps = 16;
 constexpr int kRefineSlots = kLearnedProps * kRefineK;
 constexpr int kProbeBase = kLearnedProps + kRefineSlots;  // first probe slot
@@ -367,9 +396,41 @@ __device__ __forceinline__ bool entry_less(unsigned long long ka, int32_t ia, un
   return ka < kb || (ka == kb && ia < ib);
 }
 
+// Lane's entry against the one o lanes away: keeps the smaller (low) or larger.
+__device__ __forceinline__ void entry_exchange(unsigned long long& k, int32_t& i, int o, bool low) {
+  const unsigned long long ok = __shfl_xor_sync(0xffffffffu, k, o);
+  const int32_t oi = __shfl_xor_sync(0xffffffffu, i, o);
+  if (entry_less(ok, oi, k, i) == low) {
+    k = ok;
+    i = oi;
+  }
+}
+// Sorts 32 entries over the lanes (bitonic).
+__device__ __forceinline__ void warp_sort(unsigned long long& k, int32_t& i) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int s = 2; s <= 32; s <<= 1)
+#pragma unroll
+    for (int o = s >> 1; o; o >>= 1) entry_exchange(k, i, o, ((lane & o) == 0) == ((lane & s) == 0));
+}
+// The 32 smallest of two sorted lists, sorted, in (lk, li).
+__device__ __forceinline__ void warp_merge(unsigned long long& lk, int32_t& li, unsigned long long ck, int32_t ci) {
+  const int lane = threadIdx.x & 31;
+  const unsigned long long rk = __shfl_sync(0xffffffffu, ck, 31 - lane);
+  const int32_t ri = __shfl_sync(0xffffffffu, ci, 31 - lane);
+  if (entry_less(rk, ri, lk, li)) {
+    lk = rk;
+    li = ri;
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) entry_exchange(lk, li, o, (lane & o) == 0);
+}
+
 // Offers one candidate per lane to the warp's sorted list (lk, li); all 32
-// lanes call it. A candidate enters when it is below the list's last entry at
-// its turn; the list stays sorted and holds distinct edges.
+// lanes call it. Candidates below the list's last entry enter, one after another
+// up to kOfferInsert (about four shuffle steps each), by a sort and a merge (21
+// such steps) beyond; the list stays sorted and holds distinct edges.
+constexpr int kOfferInsert = 5;
 __device__ __forceinline__ void warp_offer(unsigned long long& lk, int32_t& li, unsigned long long ck,
                                            int32_t ci) {
   const unsigned full = 0xffffffffu;
@@ -377,6 +438,11 @@ __device__ __forceinline__ void warp_offer(unsigned long long& lk, int32_t& li, 
   const unsigned long long tk = __shfl_sync(full, lk, 31);
   const int32_t ti = __shfl_sync(full, li, 31);
   unsigned want = __ballot_sync(full, entry_less(ck, ci, tk, ti));
+  if (__popc(want) > kOfferInsert) {
+    warp_sort(ck, ci);
+    warp_merge(lk, li, ck, ci);
+    return;
+  }
   while (want) {
     const int src = __ffs(want) - 1;
     want &= want - 1;
@@ -398,27 +464,32 @@ __device__ __forceinline__ void warp_offer(unsigned long long& lk, int32_t& li, 
   }
 }
 
-// Pass 1: block b scans edges [b chunk, (b + 1) chunk); warp q keeps
-// proposal q's 32 nearest bisectors of the chunk and writes them to
-// partial[b][q][0..32). The block computes each bisector once per tile.
-__global__ void __launch_bounds__(kRefineTile) refine_partial_kernel(
+// Pass 1: block (b, y) scans edges [b chunk, (b + 1) chunk); warp w keeps the 32
+// nearest bisectors of the chunk to proposal q = kRefineProps y + w and writes
+// them to partial[b][q][0..32). The block computes each bisector once per tile.
+// Bound by FP64 (a division per edge and proposal), so by the SMs it is spread
+// over: 4,661 edges in 10 blocks of 512 edges and 16 proposals took 74 us (and the
+// merge, by insertion, 37); both together now 47.
+__global__ void __launch_bounds__(32 * kRefineProps) refine_partial_kernel(
     const double* __restrict__ verts, const uint32_t* __restrict__ edges, int64_t E,
     const double* __restrict__ props, double half, int64_t chunk, RefineEntry* __restrict__ partial) {
-  __shared__ Plane64 tile[kRefineTile];
-  __shared__ uint8_t valid[kRefineTile];
-  const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ Plane64 tile[kRefineEdges];
+  __shared__ uint8_t valid[kRefineEdges];
+  const int q = blockIdx.y * kRefineProps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const double pa = props[4 * q], pb = props[4 * q + 1], pc = props[4 * q + 2], pd = props[4 * q + 3];
   unsigned long long lk = kNoKey;
   int32_t li = kNoEdge;
   const int64_t begin = (int64_t)blockIdx.x * chunk;
   const int64_t end = min(E, begin + chunk);
-  for (int64_t base = begin; base < end; base += kRefineTile) {
-    const int64_t i = base + threadIdx.x;
-    Plane64 pl = Plane64{0.0, 0.0, 0.0, 0.0};
-    valid[threadIdx.x] = (i < end) && edge_bisector(verts, edges, i, pl);
-    tile[threadIdx.x] = pl;
+  for (int64_t base = begin; base < end; base += kRefineEdges) {
+    if (threadIdx.x < kRefineEdges) {
+      const int64_t i = base + threadIdx.x;
+      Plane64 pl = Plane64{0.0, 0.0, 0.0, 0.0};
+      valid[threadIdx.x] = (i < end) && edge_bisector(verts, edges, i, pl);
+      tile[threadIdx.x] = pl;
+    }
     __syncthreads();
-    for (int j = 0; j < kRefineTile; j += 32) {
+    for (int j = 0; j < kRefineEdges; j += 32) {
       const int t = j + lane;
       unsigned long long ck = kNoKey;
       int32_t ci = kNoEdge;
@@ -451,9 +522,15 @@ __global__ void __launch_bounds__(kRefineTile) refine_merge_kernel(
   const int t = threadIdx.x, q = t >> 5, lane = t & 31;
   unsigned long long lk = kNoKey;
   int32_t li = kNoEdge;
-  for (int b = 0; b < blocks; ++b) {
-    const RefineEntry e = partial[((int64_t)b * kLearnedProps + q) * kRefineK + lane];
-    warp_offer(lk, li, e.key, e.edge);
+  // (each block's list is sorted; four loads in flight)
+  for (int b0 = 0; b0 < blocks; b0 += 4) {
+    RefineEntry e[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      e[u] = b0 + u < blocks ? partial[((int64_t)(b0 + u) * kLearnedProps + q) * kRefineK + lane]
+                             : RefineEntry{kNoKey, kNoEdge, 0};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) warp_merge(lk, li, e[u].key, e[u].edge);
   }
   sel[t] = (lane < per) ? li : kNoEdge;
   __syncthreads();
@@ -875,10 +952,11 @@ extern "C" int visacd_learned_split_search(visacd_lp* lp, const double* verts, i
   VLAUNCH(ctx, kKCandidates, grid_for(3LL * n, 256, 4LL * ctx->sm_count), 256, 0, f64_to_f32_kernel, s.verts,
           pts32, 3LL * n);
 
-  // Refinement blocks: up to two per SM, each a whole number of tiles.
-  const int64_t tiles = (E + kRefineTile - 1) / kRefineTile;
-  const int64_t want = std::min<int64_t>(tiles, 2LL * ctx->sm_count);
-  const int64_t chunk = ((tiles + want - 1) / want) * kRefineTile;
+  // Refinement blocks: up to one per SM over both halves of the proposals (the
+  // merge reads every block's lists in turn), each a whole number of tiles.
+  const int64_t tiles = (E + kRefineEdges - 1) / kRefineEdges;
+  const int64_t want = std::min<int64_t>(tiles, std::max(1, ctx->sm_count * kRefineProps / kLearnedProps));
+  const int64_t chunk = ((tiles + want - 1) / want) * kRefineEdges;
   const int32_t blocks = (int32_t)((E + chunk - 1) / chunk);
   const int32_t P = kProbeBase + probe_slots + n_flat;
   const size_t b_props = 256 * 2, b_partial = align256((size_t)blocks * kRefineSlots * sizeof(RefineEntry)),
@@ -894,7 +972,7 @@ extern "C" int visacd_learned_split_search(visacd_lp* lp, const double* verts, i
   LearnedOut* dout = reinterpret_cast<LearnedOut*>(p + b_props + b_partial + b_o64 + b_o32 + b_nref);
 
   VTRY(lp_propose_device(lp, pts32, n, s.edges, E, center, scale, props));
-  VLAUNCH(ctx, kKLpRefine, blocks, kRefineTile, 0, refine_partial_kernel, s.verts, s.edges, E, props, half,
+  VLAUNCH(ctx, kKLpRefine, dim3(blocks, kLearnedProps / kRefineProps), 32 * kRefineProps, 0, refine_partial_kernel, s.verts, s.edges, E, props, half,
           chunk, partial);
   VLAUNCH(ctx, kKLpRefine, 1, kRefineTile, 0, refine_merge_kernel, partial, blocks, refine_k, s.verts,
           s.edges, L64 + kLearnedProps, L32 + kLearnedProps, nref);
