@@ -416,26 +416,45 @@ __global__ void __launch_bounds__(128, 1) lp_gemm_tc_kernel(const bf16* __restri
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(2 * N));
 }
 
-// Sum of `parts` partial arrays of `count` floats, in order, into out.
-__global__ void lp_sum_parts_kernel(const float* __restrict__ parts, int nparts, int count,
-                                    float* __restrict__ out) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-    float s = 0.f;
-    for (int p = 0; p < nparts; ++p) s += parts[(size_t)p * count + i];
+// Sum of `parts` partial arrays of `count` floats into out, in a fixed order: 32
+// outputs per block of 8 warps, warp w sums parts w, w + 8, ... and the warps'
+// sums are added in order (with one thread per output the serial loop over 293
+// parts of 1,024 took 33 us, and over 256 parts of 64 or 128 25 us).
+__global__ void __launch_bounds__(256) lp_sum_parts_kernel(const float* __restrict__ parts, int nparts, int count,
+                                                           float* __restrict__ out) {
+  __shared__ float sums[8][32];
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + lane;
+  float s = 0.f;
+  if (i < count) {
+#pragma unroll 4
+    for (int p = w; p < nparts; p += 8) s += parts[(size_t)p * count + i];
+  }
+  sums[w][lane] = s;
+  __syncthreads();
+  if (w == 0 && i < count) {
+#pragma unroll
+    for (int k = 1; k < 8; ++k) s += sums[k][lane];
     out[i] = s;
   }
 }
 
-// Column sums of a bf16 [rows x cols] matrix: block j sums rows
-// [j*per, (j+1)*per) of column threadIdx.x into part[j*cols + c].
-__global__ void lp_colsum_kernel(const bf16* __restrict__ X, int rows, int cols, int per,
-                                 float* __restrict__ part) {
-  const int c = threadIdx.x;
-  if (c >= cols) return;
+// Column sums of a bf16 [rows x cols] matrix (cols divides 256): block j sums
+// rows [j*per, (j+1)*per) into part[j*cols + c], 256 / cols rows at a time.
+__global__ void __launch_bounds__(256) lp_colsum_kernel(const bf16* __restrict__ X, int rows, int cols, int per,
+                                                        float* __restrict__ part) {
+  __shared__ float sums[256];
+  const int c = threadIdx.x % cols, g = threadIdx.x / cols, groups = 256 / cols;
   const int r0 = blockIdx.x * per, r1 = min(rows, r0 + per);
   float s = 0.f;
-  for (int r = r0; r < r1; ++r) s += __bfloat162float(X[(size_t)r * cols + c]);
-  part[(size_t)blockIdx.x * cols + c] = s;
+#pragma unroll 8
+  for (int r = r0 + g; r < r1; r += groups) s += __bfloat162float(X[(size_t)r * cols + c]);
+  sums[threadIdx.x] = s;
+  __syncthreads();
+  if (g == 0) {
+    for (int k = 1; k < groups; ++k) s += sums[k * cols + c];
+    part[(size_t)blockIdx.x * cols + c] = s;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -544,97 +563,157 @@ __global__ void lp_planes_kernel(const float* __restrict__ Z, int B, float* __re
 //   loss = sum_l w_l min_q D(q,l) / sum_l w_l + lambda/16 sum_q min_l D(q,l).
 // Writes dZ (bf16, already divided by B) and the part's loss.
 constexpr float kLambda = 0.1f;
-__global__ void lp_loss_kernel(const float* __restrict__ Z, const float* __restrict__ labels,
-                               const float* __restrict__ lw, int B, int L,
-                               bf16* __restrict__ dZ, float* __restrict__ loss) {
-  const int b = blockIdx.x * blockDim.x + threadIdx.x;
-  if (b >= B) return;
-  const float* z = Z + (size_t)b * 64;
-  float nh[kPlanes][3], d[kPlanes], r[kPlanes], gn[kPlanes][3], gd[kPlanes];
-  for (int q = 0; q < kPlanes; ++q) {
-    r[q] = sqrtf(z[4 * q] * z[4 * q] + z[4 * q + 1] * z[4 * q + 1] + z[4 * q + 2] * z[4 * q + 2]) + 1e-12f;
-    for (int a = 0; a < 3; ++a) nh[q][a] = z[4 * q + a] / r[q];
-    d[q] = z[4 * q + 3];
-    gn[q][0] = gn[q][1] = gn[q][2] = gd[q] = 0.f;
-  }
+// One warp per part, lane q (and q + 16 again) holding proposal q; with one thread
+// per part 64 parts filled one block of one SM for 46 us.
+__global__ void __launch_bounds__(32) lp_loss_kernel(const float* __restrict__ Z, const float* __restrict__ labels,
+                                                     const float* __restrict__ lw, int L,
+                                                     bf16* __restrict__ dZ, float* __restrict__ loss) {
+  static_assert(kPlanes == 16, "two halves of a warp");
+  const int b = blockIdx.x, q = threadIdx.x & 15, B = gridDim.x;
+  const float4 z = *reinterpret_cast<const float4*>(Z + (size_t)b * 64 + 4 * q);
+  const float r = sqrtf(z.x * z.x + z.y * z.y + z.z * z.z) + 1e-12f;
+  const float nh[3] = {z.x / r, z.y / r, z.z / r};
+  const float d = z.w;
+  float gn[3] = {0.f, 0.f, 0.f}, gd = 0.f;
   const float* lab = labels + (size_t)b * L * 4;
   const float* w = lw + (size_t)b * L;
   float wsum = 0.f;
   for (int l = 0; l < L; ++l) wsum += w[l];
   const float inv_w = wsum > 0.f ? 1.f / wsum : 0.f;
   float total = 0.f;
-  auto dist = [&](int q, int l, float& sgn) {
-    const float c = nh[q][0] * lab[4 * l] + nh[q][1] * lab[4 * l + 1] + nh[q][2] * lab[4 * l + 2];
-    const float dp = d[q] - lab[4 * l + 3], dm = -d[q] - lab[4 * l + 3];
+  auto dist = [&](int l, float& sgn) {
+    const float c = nh[0] * lab[4 * l] + nh[1] * lab[4 * l + 1] + nh[2] * lab[4 * l + 2];
+    const float dp = d - lab[4 * l + 3], dm = -d - lab[4 * l + 3];
     const float Dp = 2.f - 2.f * c + dp * dp, Dm = 2.f + 2.f * c + dm * dm;
     sgn = Dp <= Dm ? 1.f : -1.f;
     return Dp <= Dm ? Dp : Dm;
   };
   // dD/dn_q = -2 s n_l ; dD/dd_q = 2 (d_q - s d_l)
-  auto add_grad = [&](int q, int l, float sgn, float coef) {
-    for (int a = 0; a < 3; ++a) gn[q][a] += coef * (-2.f * sgn * lab[4 * l + a]);
-    gd[q] += coef * 2.f * (d[q] - sgn * lab[4 * l + 3]);
+  auto add_grad = [&](int l, float sgn, float coef) {
+    for (int a = 0; a < 3; ++a) gn[a] += coef * (-2.f * sgn * lab[4 * l + a]);
+    gd += coef * 2.f * (d - sgn * lab[4 * l + 3]);
   };
+  constexpr float kNone = 3.4e38f;  // no distance (also NaN)
+  float mine = kNone, mine_s = 1.f;  // this proposal's nearest label
+  int mine_l = -1;
   for (int l = 0; l < L; ++l) {
     if (w[l] <= 0.f) continue;
-    int best = 0;
-    float bs = 1.f, bd = 3.4e38f;
-    for (int q = 0; q < kPlanes; ++q) {
-      float s;
-      const float D = dist(q, l, s);
-      if (D < bd) {
-        bd = D;
-        best = q;
-        bs = s;
+    float sgn;
+    const float D = dist(l, sgn);
+    if (D < mine) {
+      mine = D;
+      mine_l = l;
+      mine_s = sgn;
+    }
+    // the label's nearest proposal, the first among equals
+    float bd = D < kNone ? D : kNone;
+    int best = D < kNone ? q : 0;
+#pragma unroll
+    for (int o = 8; o; o >>= 1) {
+      const float od = __shfl_xor_sync(0xffffffffu, bd, o);
+      const int ob = __shfl_xor_sync(0xffffffffu, best, o);
+      if (od < bd || (od == bd && ob < best)) {
+        bd = od;
+        best = ob;
       }
     }
     total += w[l] * inv_w * bd;
-    add_grad(best, l, bs, w[l] * inv_w);
+    if (q == best) add_grad(l, bd < kNone ? sgn : 1.f, w[l] * inv_w);
   }
-  for (int q = 0; q < kPlanes; ++q) {
-    int best = -1;
-    float bs = 1.f, bd = 3.4e38f;
-    for (int l = 0; l < L; ++l) {
-      if (w[l] <= 0.f) continue;
-      float s;
-      const float D = dist(q, l, s);
-      if (D < bd) {
-        bd = D;
-        best = l;
-        bs = s;
-      }
-    }
-    if (best < 0) continue;
-    total += kLambda / kPlanes * bd;
-    add_grad(q, best, bs, kLambda / kPlanes);
+  for (int p = 0; p < kPlanes; ++p) {
+    const float bd = __shfl_sync(0xffffffffu, mine, p);
+    if (__shfl_sync(0xffffffffu, mine_l, p) >= 0) total += kLambda / kPlanes * bd;
   }
-  loss[b] = total;
+  if (mine_l >= 0) add_grad(mine_l, mine_s, kLambda / kPlanes);
+  if (threadIdx.x >= kPlanes) return;
+  if (q == 0) loss[b] = total;
   const float scale = 1.f / (float)B;
-  for (int q = 0; q < kPlanes; ++q) {
-    // through n_hat = n / |n|: dn = (g - n_hat (n_hat . g)) / |n|
-    const float dotg = nh[q][0] * gn[q][0] + nh[q][1] * gn[q][1] + nh[q][2] * gn[q][2];
-    for (int a = 0; a < 3; ++a)
-      dZ[(size_t)b * 64 + 4 * q + a] = __float2bfloat16_rn(scale * (gn[q][a] - nh[q][a] * dotg) / r[q]);
-    dZ[(size_t)b * 64 + 4 * q + 3] = __float2bfloat16_rn(scale * gd[q]);
-  }
+  // through n_hat = n / |n|: dn = (g - n_hat (n_hat . g)) / |n|
+  const float dotg = nh[0] * gn[0] + nh[1] * gn[1] + nh[2] * gn[2];
+  for (int a = 0; a < 3; ++a)
+    dZ[(size_t)b * 64 + 4 * q + a] = __float2bfloat16_rn(scale * (gn[a] - nh[a] * dotg) / r);
+  dZ[(size_t)b * 64 + 4 * q + 3] = __float2bfloat16_rn(scale * gd);
 }
 
-// Gradient through the max-pool: dZ3 is zero except at each (part, channel)'s
-// arg-max row, where it carries dG when the pooled value is positive. Also the
-// layer-3 bias gradient sum_b dG*[G>0] (float32).
-__global__ void lp_pool_backward_kernel(const float* __restrict__ G, const float* __restrict__ dG,
-                                        const int32_t* __restrict__ arg, int B,
-                                        bf16* __restrict__ dZ3, float* __restrict__ db3) {
-  const int c = threadIdx.x;
-  float s = 0.f;
-  for (int b = 0; b < B; ++b) {
-    const int i = b * 256 + c;
-    if (G[i] > 0.f) {
-      dZ3[((size_t)b * kPts + arg[i]) * 256 + c] = __float2bfloat16_rn(dG[i]);
-      s += dG[i];
+// Gradient through the max-pool. It is zero except at each (part, channel)'s
+// arg-max row, where it carries dG when the pooled value is positive, so at most
+// 256 of a part's 2048 rows have any gradient, here and in the layers below. The
+// rows that do (in row order) get the part's slots 0, 1, ... of 256: dZ3 [B*256 x
+// 256] and these rows of the layers' inputs, zeros in the slots left over. The
+// per-edge layers' backward then runs over an eighth of the rows; over all of
+// them (64 parts) its GEMMs and sums took some 340 us, with 67 MB of mostly zeros
+// written once and read twice.
+// Block (b, y) fills slots [64 y, 64 y + 64) of part b; block (B, 0) computes the
+// layer-3 bias gradient sum_b dG*[G>0] (float32, in order).
+constexpr int kSlots = 256;
+__global__ void __launch_bounds__(256) lp_pool_backward_kernel(
+    const float* __restrict__ G, const float* __restrict__ dG, const int32_t* __restrict__ arg, int B,
+    const bf16* __restrict__ A2, const bf16* __restrict__ A1, const bf16* __restrict__ X0, bf16* __restrict__ dZ3,
+    bf16* __restrict__ S2, bf16* __restrict__ S1, bf16* __restrict__ S0, float* __restrict__ db3) {
+  const int b = blockIdx.x, c = threadIdx.x;
+  if (b == B) {
+    if (blockIdx.y != 0) return;
+    float s = 0.f;
+#pragma unroll 8
+    for (int p = 0; p < B; ++p) {
+      const int i = p * 256 + c;
+      if (G[i] > 0.f) s += dG[i];
     }
+    db3[c] = s;
+    return;
   }
-  db3[c] = s;
+  __shared__ uint32_t bits[kPts / 32];
+  __shared__ int before[kPts / 32];
+  __shared__ int rows[kSlots], slot[256];
+  __shared__ uint32_t grad[256];  // bf16 bits of the channel's gradient
+  static_assert(kPts / 32 == 64, "two words per lane");
+  if (c < kPts / 32) bits[c] = 0;
+  rows[c] = -1;
+  __syncthreads();
+  const int i = b * 256 + c;
+  const bool has = G[i] > 0.f;
+  const int row = arg[i];
+  if (has) atomicOr(&bits[row >> 5], 1u << (row & 31));
+  __syncthreads();
+  if (c < 32) {
+    const int n0 = __popc(bits[2 * c]), n1 = __popc(bits[2 * c + 1]);
+    int inc = n0 + n1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int x = __shfl_up_sync(0xffffffffu, inc, o);
+      if (c >= o) inc += x;
+    }
+    before[2 * c] = inc - n0 - n1;
+    before[2 * c + 1] = inc - n1;
+  }
+  __syncthreads();
+  const int sl = has ? before[row >> 5] + __popc(bits[row >> 5] & ((1u << (row & 31)) - 1u)) : -1;
+  if (has) rows[sl] = row;
+  slot[c] = sl;
+  grad[c] = has ? (uint32_t)__bfloat16_as_ushort(__float2bfloat16_rn(dG[i])) : 0u;
+  __syncthreads();
+  const int s0 = blockIdx.y * 64;
+  // dZ3: two channels per store.
+  const int pair = 2 * (c & 127);
+  const int sa = slot[pair], sb = slot[pair + 1];
+  const uint32_t ga = grad[pair], gb = grad[pair + 1] << 16;
+  uint32_t* dz = reinterpret_cast<uint32_t*>(dZ3 + (size_t)b * kSlots * 256) + (c & 127);
+#pragma unroll 4
+  for (int k = s0 + (c >> 7); k < s0 + 64; k += 2)
+    dz[(size_t)k * 128] = (sa == k ? ga : 0u) | (sb == k ? gb : 0u);
+  // The rows of the inputs, 16 bytes a thread: 16 + 8 + 2 pieces per row.
+  static_assert(kIn == 16, "two pieces");
+  for (int t = c; t < 64 * 26; t += 256) {
+    const int k = s0 + t / 26, piece = t % 26;
+    const int width = piece < 16 ? 16 : (piece < 24 ? 8 : 2);
+    const int at = piece < 16 ? piece : (piece < 24 ? piece - 16 : piece - 24);
+    const bf16* src = piece < 16 ? A2 : (piece < 24 ? A1 : X0);
+    bf16* dst = piece < 16 ? S2 : (piece < 24 ? S1 : S0);
+    const int r = rows[k];
+    uint4 v = make_uint4(0, 0, 0, 0);
+    if (r >= 0) v = reinterpret_cast<const uint4*>(src)[((size_t)b * kPts + r) * width + at];
+    reinterpret_cast<uint4*>(dst)[((size_t)b * kSlots + k) * width + at] = v;
+  }
 }
 
 __global__ void lp_adam_kernel(float* __restrict__ p, const float* __restrict__ g, float* __restrict__ m,
@@ -683,12 +762,12 @@ struct visacd_lp {
   int64_t step = 0;
   DevBuf params, params_bf16, grads, adam_m, adam_v;
   DevBuf x0, a1, a2, a3, poolkey, g, gb, arg, a4, a5, z6;
-  DevBuf dz6, dz5, dz4, dg, dz3, dz2, dz1;
+  DevBuf dz6, dz5, dz4, dg, dz3, dz2, dz1, s2, s1, s0;
   DevBuf parts, labels, lw, loss, feats, planes, pts, edges, frame;
   template <class F>
   void each_buf(F f) {
     for (DevBuf* b : {&params, &params_bf16, &grads, &adam_m, &adam_v, &x0, &a1, &a2, &a3, &poolkey, &g, &gb,
-                      &arg, &a4, &a5, &z6, &dz6, &dz5, &dz4, &dg, &dz3, &dz2, &dz1, &parts, &labels, &lw,
+                      &arg, &a4, &a5, &z6, &dz6, &dz5, &dz4, &dg, &dz3, &dz2, &dz1, &s2, &s1, &s0, &parts, &labels, &lw,
                       &loss, &feats, &planes, &pts, &edges, &frame})
       f(*b);
   }
@@ -724,32 +803,37 @@ int gemm(visacd_lp* lp, const bf16* A, int lda, const bf16* B, int ldb, void* C,
   return VISACD_OK;
 }
 
+constexpr int kColRows = 128;   // rows of a partial bias sum
+constexpr int kGradRows = 256;  // rows of a partial weight sum at least
+
 // dW[N x K] = dZ^T X over `rows` rows, split over the rows and summed in order.
 int weight_grad(visacd_lp* lp, const bf16* dZ, int N, const bf16* X, int K, int rows, float* out) {
   visacd_ctx* ctx = lp->ctx;
   const int tiles = ((N + kTM - 1) / kTM) * ((K + kTN - 1) / kTN);
-  int splits = std::max(1, std::min((2 * ctx->sm_count + tiles - 1) / tiles, (rows + kTK - 1) / kTK));
+  int splits = std::max(1, std::min((2 * ctx->sm_count + tiles - 1) / tiles, (rows + kGradRows - 1) / kGradRows));
   int kchunk = (rows + splits - 1) / splits;
   kchunk = (kchunk + kTK - 1) / kTK * kTK;
   splits = (rows + kchunk - 1) / kchunk;
   VCHECK(lp->parts.cap >= (size_t)splits * N * K * sizeof(float), VISACD_ERR_INVALID_ARG,
          "lp: partial-sum buffer too small");
+  if (splits == 1) return gemm<false, false, kEpiStoreF32>(lp, dZ, N, X, K, out, K, N, K, rows, kchunk);
   VTRY((gemm<false, false, kEpiStoreF32>(lp, dZ, N, X, K, lp->parts.p, K, N, K, rows, kchunk)));
-  VLAUNCH(ctx, vgpu::kKLpMisc, vgpu::grid_for((int64_t)N * K, 256, 1024), 256, 0, lp_sum_parts_kernel,
-          P<float>(lp->parts), splits, N * K, out);
+  VLAUNCH(ctx, vgpu::kKLpMisc, (N * K + 31) / 32, 256, 0, lp_sum_parts_kernel, P<float>(lp->parts), splits, N * K,
+          out);
   return VISACD_OK;
 }
 
 // db[N] = column sums of dZ [rows x N], in a fixed order.
 int bias_grad(visacd_lp* lp, const bf16* dZ, int rows, int N, float* out) {
   visacd_ctx* ctx = lp->ctx;
-  const int per = 512;
-  const int blocks = (rows + per - 1) / per;
+  const int blocks = (rows + kColRows - 1) / kColRows;
+  VCHECK(256 % N == 0, VISACD_ERR_INVALID_ARG, "lp: bias width must divide 256");
   VCHECK(lp->parts.cap >= (size_t)blocks * N * sizeof(float), VISACD_ERR_INVALID_ARG,
          "lp: partial-sum buffer too small");
-  VLAUNCH(ctx, vgpu::kKLpMisc, blocks, N, 0, lp_colsum_kernel, dZ, rows, N, per, P<float>(lp->parts));
-  VLAUNCH(ctx, vgpu::kKLpMisc, vgpu::grid_for(N, 256, 64), 256, 0, lp_sum_parts_kernel,
-          P<float>(lp->parts), blocks, N, out);
+  VLAUNCH(ctx, vgpu::kKLpMisc, blocks, 256, 0, lp_colsum_kernel, dZ, rows, N, kColRows,
+          blocks == 1 ? out : P<float>(lp->parts));
+  if (blocks > 1)
+    VLAUNCH(ctx, vgpu::kKLpMisc, (N + 31) / 32, 256, 0, lp_sum_parts_kernel, P<float>(lp->parts), blocks, N, out);
   return VISACD_OK;
 }
 
@@ -773,7 +857,7 @@ int alloc_batch(visacd_lp* lp, int B) {
 }
 
 int alloc_train(visacd_lp* lp, int B) {
-  const size_t rows = (size_t)B * kPts;
+  const size_t rows = (size_t)B * kSlots;
   VTRY(ensure(lp->dz6, (size_t)B * 64 * 2));
   VTRY(ensure(lp->dz5, (size_t)B * 64 * 2));
   VTRY(ensure(lp->dz4, (size_t)B * 128 * 2));
@@ -781,14 +865,17 @@ int alloc_train(visacd_lp* lp, int B) {
   VTRY(ensure(lp->dz3, rows * 256 * 2));
   VTRY(ensure(lp->dz2, rows * 128 * 2));
   VTRY(ensure(lp->dz1, rows * 64 * 2));
+  VTRY(ensure(lp->s2, rows * 128 * 2));
+  VTRY(ensure(lp->s1, rows * 64 * 2));
+  VTRY(ensure(lp->s0, rows * kIn * 2));
   VTRY(ensure(lp->loss, (size_t)B * 4));
   // Partial sums of the split weight gradients (at most 2 x SMs + tiles chunks
   // of <= 64 x 64 tiles... bounded by (2 * SMs + 8) * 256 * 128 floats is more
-  // than enough) and of the bias column sums (rows / 512 blocks x 256).
+  // than enough) and of the bias column sums (kColRows rows a block).
   // Sized once here: a reallocation between stream-ordered launches would free
   // memory a queued kernel still uses.
   const size_t wparts = (size_t)(2 * lp->ctx->sm_count + 8) * 4096 * 8;
-  const size_t bparts = (rows / 512 + 1) * 256;
+  const size_t bparts = (rows / kColRows + 1) * 256;
   VTRY(ensure(lp->parts, std::max(wparts, bparts) * sizeof(float)));
   return VISACD_OK;
 }
@@ -833,11 +920,11 @@ int forward(visacd_lp* lp, int B) {
 // Loss and backward pass after forward(): fills grads (overwritten).
 int backward(visacd_lp* lp, int B, int L) {
   visacd_ctx* ctx = lp->ctx;
-  const int M = B * kPts;
+  const int M = B * kSlots;
   const bf16* W = P<bf16>(lp->params_bf16);
   float* G = P<float>(lp->grads);
-  VLAUNCH(ctx, vgpu::kKLpLoss, vgpu::grid_for(B, 64, 1 << 20), 64, 0, lp_loss_kernel, P<float>(lp->z6),
-          P<float>(lp->labels), P<float>(lp->lw), B, L, P<bf16>(lp->dz6), P<float>(lp->loss));
+  VLAUNCH(ctx, vgpu::kKLpLoss, B, 32, 0, lp_loss_kernel, P<float>(lp->z6), P<float>(lp->labels), P<float>(lp->lw), L,
+          P<bf16>(lp->dz6), P<float>(lp->loss));
   // head
   VTRY(weight_grad(lp, P<bf16>(lp->dz6), 64, P<bf16>(lp->a5), 64, B, G + kOff.w[5]));
   VTRY(bias_grad(lp, P<bf16>(lp->dz6), B, 64, G + kOff.b[5]));
@@ -852,18 +939,18 @@ int backward(visacd_lp* lp, int B, int L) {
   VTRY((gemm<true, false, kEpiStoreF32>(lp, P<bf16>(lp->dz4), 128, W + kOff.w[3], 256, lp->dg.p, 256, B,
                                         256, 128)));
   // max-pool
-  VCUDA(cudaMemsetAsync(lp->dz3.p, 0, (size_t)M * 256 * 2, ctx->stream));
-  VLAUNCH(ctx, vgpu::kKLpPool, 1, 256, 0, lp_pool_backward_kernel, P<float>(lp->g), P<float>(lp->dg),
-          P<int32_t>(lp->arg), B, P<bf16>(lp->dz3), G + kOff.b[2]);
-  // shared per-edge layers
-  VTRY(weight_grad(lp, P<bf16>(lp->dz3), 256, P<bf16>(lp->a2), 128, M, G + kOff.w[2]));
+  VLAUNCH(ctx, vgpu::kKLpPool, dim3(B + 1, kSlots / 64), 256, 0, lp_pool_backward_kernel, P<float>(lp->g),
+          P<float>(lp->dg), P<int32_t>(lp->arg), B, P<bf16>(lp->a2), P<bf16>(lp->a1), P<bf16>(lp->x0),
+          P<bf16>(lp->dz3), P<bf16>(lp->s2), P<bf16>(lp->s1), P<bf16>(lp->s0), G + kOff.b[2]);
+  // shared per-edge layers, over the rows with a gradient
+  VTRY(weight_grad(lp, P<bf16>(lp->dz3), 256, P<bf16>(lp->s2), 128, M, G + kOff.w[2]));
   VTRY((gemm<true, false, kEpiMaskBf16>(lp, P<bf16>(lp->dz3), 256, W + kOff.w[2], 128, lp->dz2.p, 128, M,
-                                        128, 256, 0, nullptr, P<bf16>(lp->a2), 128)));
-  VTRY(weight_grad(lp, P<bf16>(lp->dz2), 128, P<bf16>(lp->a1), 64, M, G + kOff.w[1]));
+                                        128, 256, 0, nullptr, P<bf16>(lp->s2), 128)));
+  VTRY(weight_grad(lp, P<bf16>(lp->dz2), 128, P<bf16>(lp->s1), 64, M, G + kOff.w[1]));
   VTRY(bias_grad(lp, P<bf16>(lp->dz2), M, 128, G + kOff.b[1]));
   VTRY((gemm<true, false, kEpiMaskBf16>(lp, P<bf16>(lp->dz2), 128, W + kOff.w[1], 64, lp->dz1.p, 64, M,
-                                        64, 128, 0, nullptr, P<bf16>(lp->a1), 64)));
-  VTRY(weight_grad(lp, P<bf16>(lp->dz1), 64, P<bf16>(lp->x0), kIn, M, G + kOff.w[0]));
+                                        64, 128, 0, nullptr, P<bf16>(lp->s1), 64)));
+  VTRY(weight_grad(lp, P<bf16>(lp->dz1), 64, P<bf16>(lp->s0), kIn, M, G + kOff.w[0]));
   VTRY(bias_grad(lp, P<bf16>(lp->dz1), M, 64, G + kOff.b[0]));
   return VISACD_OK;
 }
