@@ -285,10 +285,11 @@ __device__ __forceinline__ bool tc_wait(uint32_t bar_addr, uint32_t parity) {
 }
 
 // cp.async of one 128-row X tile into the core-matrix layout (rows past M: zeros).
+template <int kThreads>
 __device__ __forceinline__ void tc_load_x(unsigned char* buf, const bf16* __restrict__ X, int M, int K, int row0,
                                           int tid) {
   const int kg = K / 8, ag = kTcM / 8;
-  for (int c = tid; c < kTcM * kg; c += 128) {
+  for (int c = tid; c < kTcM * kg; c += kThreads) {
     const int r = c / kg, j = c % kg;
     const bool ok = row0 + r < M;
     cp_async16(smem_u32(buf + ((j * ag) + (r >> 3)) * 128 + (r & 7) * 16),
@@ -297,10 +298,21 @@ __device__ __forceinline__ void tc_load_x(unsigned char* buf, const bf16* __rest
   asm volatile("cp.async.commit_group;\n" ::);
 }
 
-__global__ void __launch_bounds__(128, 1) lp_gemm_tc_kernel(const bf16* __restrict__ X, int M, int K,
+// POOL (N = 256, 8 warps): instead of storing Y, the max over each part's rows of
+// every column goes to pool (lp_pool_kernel's keys: value bits, then the lower
+// row). A tile lies in one part; each thread keeps the keys (BF16 bits << 16 |
+// 65535 - row) of its row's 128 columns (warps 0-3 the first half, 4-7 the
+// second) over the CTA's tiles of a part, and the lanes are reduced where the
+// part ends. (One reduction per column and tile took 312 us for 131,072 rows;
+// storing the activations and pooling them in a kernel of its own 64 + 19; this 37.)
+template <bool POOL>
+__global__ void __launch_bounds__(POOL ? 256 : 128, 1) lp_gemm_tc_kernel(const bf16* __restrict__ X, int M, int K,
                                                            const bf16* __restrict__ W, int N,
                                                            const float* __restrict__ bias, bf16* __restrict__ Y,
+                                                           unsigned long long* __restrict__ pool,
                                                            uint32_t* __restrict__ status) {
+  static_assert(kPts % kTcM == 0 && kPts <= 65536, "a tile lies in one part; rows fit 16 bits");
+  constexpr int kThreads = POOL ? 256 : 128;
   extern __shared__ __align__(1024) unsigned char smem[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int ntiles = (M + kTcM - 1) / kTcM;
@@ -320,12 +332,17 @@ __global__ void __launch_bounds__(128, 1) lp_gemm_tc_kernel(const bf16* __restri
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::);
   }
   // W once, then the first X tile.
-  for (int c = tid; c < N * kg; c += 128) {
+  for (int c = tid; c < N * kg; c += kThreads) {
     const int r = c / kg, j = c % kg;
     cp_async16(smem_u32(smem + kTcW + ((j * bg) + (r >> 3)) * 128 + (r & 7) * 16), W + (size_t)r * K + j * 8, true);
   }
-  int t0 = blockIdx.x;
-  if (t0 < ntiles) tc_load_x(smem + kTcX0, X, M, K, t0 * kTcM, tid);
+  // Tiles t0, t0 + step, ...: neighbouring ones with POOL, so that few parts
+  // change on the way.
+  const int step = POOL ? 1 : (int)gridDim.x;
+  const int share = (ntiles + (int)gridDim.x - 1) / (int)gridDim.x;
+  const int t0 = POOL ? (int)blockIdx.x * share : (int)blockIdx.x;
+  const int tend = POOL ? min(ntiles, t0 + share) : ntiles;
+  if (t0 < tend) tc_load_x<kThreads>(smem + kTcX0, X, M, K, t0 * kTcM, tid);
   else asm volatile("cp.async.commit_group;\n" ::);
   asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
   __syncthreads();
@@ -355,9 +372,10 @@ __global__ void __launch_bounds__(128, 1) lp_gemm_tc_kernel(const bf16* __restri
   asm volatile("cp.async.wait_group 0;\n" ::);
   asm volatile("fence.proxy.async.shared::cta;\n" ::);
   __syncthreads();
-  const int nlocal = t0 < ntiles ? (ntiles - 1 - t0) / gridDim.x + 1 : 0;
+  const int nlocal = t0 < tend ? (tend - 1 - t0) / step + 1 : 0;
+  uint32_t best[POOL ? 128 : 1] = {};  // POOL: this row's keys of the warp's columns
   if (nlocal > 0) issue(0);
-  if (nlocal > 1) tc_load_x(smem + kTcX1, X, M, K, (t0 + gridDim.x) * kTcM, tid);
+  if (nlocal > 1) tc_load_x<kThreads>(smem + kTcX1, X, M, K, (t0 + step) * kTcM, tid);
   for (int i = 0; i < nlocal && ok; ++i) {
     // start tile i + 1 while tile i drains
     if (i + 1 < nlocal) {
@@ -372,31 +390,67 @@ __global__ void __launch_bounds__(128, 1) lp_gemm_tc_kernel(const bf16* __restri
     ok = tc_wait((i & 1) ? bar1 : bar0, (uint32_t)((i >> 1) & 1));
     if (!ok) break;
     asm volatile("tcgen05.fence::after_thread_sync;\n" ::);
-    if (i + 2 < nlocal) tc_load_x(smem + ((i & 1) ? kTcX1 : kTcX0), X, M, K, (t0 + (i + 2) * gridDim.x) * kTcM, tid);
-    const int row = (t0 + i * gridDim.x) * kTcM + warp * 32 + lane;
-    const uint32_t acc = tmem + (uint32_t)((i & 1) * N);
-    for (int c0 = 0; c0 < N; c0 += 16) {
-      uint32_t r[16];
-      const uint32_t taddr = acc + ((uint32_t)(warp * 32) << 16) + (uint32_t)c0;
+    if (i + 2 < nlocal) tc_load_x<kThreads>(smem + ((i & 1) ? kTcX1 : kTcX0), X, M, K, (t0 + (i + 2) * step) * kTcM, tid);
+    const int row = (t0 + i * step) * kTcM + (warp & 3) * 32 + lane;
+    const uint32_t acc = tmem + (uint32_t)((i & 1) * N) + ((uint32_t)((warp & 3) * 32) << 16);
+    auto load16 = [&](int c0, uint32_t (&r)[16]) {
       asm volatile(
           "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
           : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
             "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-          : "r"(taddr));
+          : "r"(acc + (uint32_t)c0));
       asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::);
-      if (row < M) {
-        uint32_t o[8];
+    };
+    if constexpr (POOL) {
+      const int h0 = (warp >> 2) * 128;
+      const uint32_t low = 65535u - (uint32_t)(row % kPts);
 #pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          float v0 = __uint_as_float(r[2 * k]) + bias[c0 + 2 * k];
-          float v1 = __uint_as_float(r[2 * k + 1]) + bias[c0 + 2 * k + 1];
-          v0 = v0 > 0.f ? v0 : 0.f;
-          v1 = v1 > 0.f ? v1 : 0.f;
-          o[k] = pack_bf16(v0, v1);
+      for (int c = 0; c < 128; c += 16) {
+        uint32_t r[16];
+        load16(h0 + c, r);
+#pragma unroll
+        for (int k = 0; k < 16; ++k) {
+          const float v = __uint_as_float(r[k]) + bias[h0 + c + k];
+          const uint32_t h = __bfloat16_as_ushort(__float2bfloat16_rn(v > 0.f ? v : 0.f));
+          best[c + k] = max(best[c + k], row < M ? (h << 16) | low : 0u);
         }
-        uint4* dst = reinterpret_cast<uint4*>(Y + (size_t)row * N + c0);
-        dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
-        dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+      }
+      // The part ends (or this CTA's tiles do): its maxima out. Every key is
+      // positive, since its low half is.
+      const int part = (t0 + i * step) * kTcM / kPts;
+      if (i + 1 == nlocal || (t0 + (i + 1) * step) * kTcM / kPts != part) {
+#pragma unroll
+        for (int w = 0; w < 4; ++w) {
+          uint32_t mine = 0;
+#pragma unroll
+          for (int k = 0; k < 32; ++k) {
+            const uint32_t m = __reduce_max_sync(0xffffffffu, best[32 * w + k]);
+            mine = lane == k ? m : mine;
+            best[32 * w + k] = 0;
+          }
+          if (mine)
+            atomicMax(pool + (size_t)part * N + h0 + 32 * w + lane,
+                      ((unsigned long long)(mine & 0xffff0000u) << 32) | (0xFFFFFFFFu - (65535u - (mine & 0xffffu))));
+        }
+      }
+    } else {
+      for (int c0 = 0; c0 < N; c0 += 16) {
+        uint32_t r[16];
+        load16(c0, r);
+        if (row < M) {
+          uint32_t o[8];
+#pragma unroll
+          for (int k = 0; k < 8; ++k) {
+            float v0 = __uint_as_float(r[2 * k]) + bias[c0 + 2 * k];
+            float v1 = __uint_as_float(r[2 * k + 1]) + bias[c0 + 2 * k + 1];
+            v0 = v0 > 0.f ? v0 : 0.f;
+            v1 = v1 > 0.f ? v1 : 0.f;
+            o[k] = pack_bf16(v0, v1);
+          }
+          uint4* dst = reinterpret_cast<uint4*>(Y + (size_t)row * N + c0);
+          dst[0] = make_uint4(o[0], o[1], o[2], o[3]);
+          dst[1] = make_uint4(o[4], o[5], o[6], o[7]);
+        }
       }
     }
     // the accumulator of tile i is read before tile i + 2 reuses it
@@ -843,7 +897,6 @@ int alloc_batch(visacd_lp* lp, int B) {
   VTRY(ensure(lp->x0, rows * kIn * 2));
   VTRY(ensure(lp->a1, rows * 64 * 2));
   VTRY(ensure(lp->a2, rows * 128 * 2));
-  VTRY(ensure(lp->a3, rows * 256 * 2));
   VTRY(ensure(lp->poolkey, (size_t)B * 256 * 8));
   VTRY(ensure(lp->g, (size_t)B * 256 * 4));
   VTRY(ensure(lp->gb, (size_t)B * 256 * 2));
@@ -880,31 +933,46 @@ int alloc_train(visacd_lp* lp, int B) {
   return VISACD_OK;
 }
 
-// Forward pass over x0 (B parts): fills a1..a3, g/gb/arg, a4, a5, z6.
+// Lets both tcgen05 kernels use kTcSmem bytes of shared memory on this device.
+cudaError_t tc_smem() {
+  const cudaError_t e =
+      cudaFuncSetAttribute(lp_gemm_tc_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+  return e != cudaSuccess
+             ? e
+             : cudaFuncSetAttribute(lp_gemm_tc_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem);
+}
+
+// Forward pass over x0 (B parts): fills a1, a2, g/gb/arg, a4, a5, z6 (and a3, the
+// third layer's activations, without tcgen05).
 int forward(visacd_lp* lp, int B) {
   visacd_ctx* ctx = lp->ctx;
   const int M = B * kPts;
   const bf16* W = P<bf16>(lp->params_bf16);
   const float* Pf = P<float>(lp->params);
+  VCUDA(cudaMemsetAsync(lp->poolkey.p, 0, (size_t)B * 256 * 8, ctx->stream));
   if (lp->tcgen05) {
     const bf16* xin[3] = {P<bf16>(lp->x0), P<bf16>(lp->a1), P<bf16>(lp->a2)};
-    bf16* yout[3] = {P<bf16>(lp->a1), P<bf16>(lp->a2), P<bf16>(lp->a3)};
+    bf16* yout[2] = {P<bf16>(lp->a1), P<bf16>(lp->a2)};
     const int tiles = (M + kTcM - 1) / kTcM;
     const int grid = std::max(1, std::min(tiles, ctx->sm_count));
-    for (int l = 0; l < 3; ++l)
-      VLAUNCH(ctx, vgpu::kKLpGemm, grid, 128, kTcSmem, lp_gemm_tc_kernel, xin[l], M, kK[l], W + kOff.w[l], kN[l],
-              Pf + kOff.b[l], yout[l], ctx->d_status);
+    unsigned long long* none = nullptr;
+    for (int l = 0; l < 2; ++l)
+      VLAUNCH(ctx, vgpu::kKLpGemm, grid, 128, kTcSmem, lp_gemm_tc_kernel<false>, xin[l], M, kK[l], W + kOff.w[l], kN[l],
+              Pf + kOff.b[l], yout[l], none, ctx->d_status);
+    static_assert(kN[2] == 256, "the pooling kernel's columns");
+    VLAUNCH(ctx, vgpu::kKLpGemm, grid, 256, kTcSmem, lp_gemm_tc_kernel<true>, xin[2], M, kK[2], W + kOff.w[2], kN[2],
+            Pf + kOff.b[2], (bf16*)nullptr, P<unsigned long long>(lp->poolkey), ctx->d_status);
   } else {
+    VTRY(ensure(lp->a3, (size_t)M * 256 * 2));
     VTRY((gemm<true, true, kEpiBiasReluBf16>(lp, P<bf16>(lp->x0), kIn, W + kOff.w[0], kIn, lp->a1.p, 64, M,
                                              64, kIn, 0, Pf + kOff.b[0])));
     VTRY((gemm<true, true, kEpiBiasReluBf16>(lp, P<bf16>(lp->a1), 64, W + kOff.w[1], 64, lp->a2.p, 128, M,
                                              128, 64, 0, Pf + kOff.b[1])));
     VTRY((gemm<true, true, kEpiBiasReluBf16>(lp, P<bf16>(lp->a2), 128, W + kOff.w[2], 128, lp->a3.p, 256,
                                              M, 256, 128, 0, Pf + kOff.b[2])));
+    VLAUNCH(ctx, vgpu::kKLpPool, dim3(B, 8), 256, 0, lp_pool_kernel, P<bf16>(lp->a3),
+            P<unsigned long long>(lp->poolkey));
   }
-  VCUDA(cudaMemsetAsync(lp->poolkey.p, 0, (size_t)B * 256 * 8, ctx->stream));
-  VLAUNCH(ctx, vgpu::kKLpPool, dim3(B, 8), 256, 0, lp_pool_kernel, P<bf16>(lp->a3),
-          P<unsigned long long>(lp->poolkey));
   VLAUNCH(ctx, vgpu::kKLpPool, vgpu::grid_for(B * 256, 256, 1 << 20), 256, 0, lp_pool_finish_kernel,
           P<unsigned long long>(lp->poolkey), B * 256, P<float>(lp->g), P<bf16>(lp->gb),
           P<int32_t>(lp->arg));
@@ -1026,8 +1094,7 @@ extern "C" int visacd_lp_create(visacd_ctx* ctx, const float* params, uint32_t s
     return fail(VISACD_ERR_CUDA);
   }
   // The forward per-edge layers run on tcgen05 (tensor memory) by default.
-  if ((e = cudaFuncSetAttribute(lp_gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem)) !=
-      cudaSuccess) {
+  if ((e = tc_smem()) != cudaSuccess) {
     vgpu::set_error("lp_create: %s", cudaGetErrorString(e));
     return fail(VISACD_ERR_CUDA);
   }
@@ -1182,7 +1249,7 @@ extern "C" int visacd_lp_set_tcgen05(visacd_lp* lp, int enable) {
   VCHECK(lp->ctx, VISACD_ERR_INVALID_ARG, "lp_set_tcgen05: the proposer's context was destroyed");
   if (enable) {
     VCUDA(cudaSetDevice(lp->ctx->device));
-    VCUDA(cudaFuncSetAttribute(lp_gemm_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kTcSmem));
+    VCUDA(tc_smem());
   }
   lp->tcgen05 = enable != 0;
   return VISACD_OK;
