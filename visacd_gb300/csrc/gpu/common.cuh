@@ -121,6 +121,7 @@ enum CtxSlot {
   kSlotLearned,
   kSlotFreeGrid,
   kSlotVisCleared,
+  kSlotVisReach,
   kSlotConvexHull,
   kSlotCount
 };

@@ -50,6 +50,77 @@ __device__ __forceinline__ float free_bound(const FreeGridView& g, float u, floa
 
 constexpr int kTraceSteps = 32;  // rounds (two grid reads each) before a segment goes to the BVH
 
+// Free reach of the points by direction: the directions are 6 x m x m cells of a
+// cube around the point (axis of the largest component, its sign, and m x m
+// squares of the two other components over it), and reach[cell * n + row] is a
+// length along the axis up to which every segment from the point with a
+// direction in the cell stays free of the cage. Most of a walk's reads are the
+// first, short advances away from the surface, and they are much the same for
+// all segments of a cell, so a table of n x 6 m^2 reaches spares them to n^2 / 2.
+struct FreeReach {
+  const float* reach;  // null: none
+  int m, n;
+  int by_pos;          // rows are sorted positions (else vertex ids)
+};
+
+// Half the width of a cell's squares, with room for the rounding of the
+// components by which a direction is sorted into it (about 2e-6).
+__device__ __forceinline__ float reach_half(int m) { return 1.0f / (float)m + 1e-5f; }
+
+// The reach of point p in a cell. Walking along the cell's middle direction c
+// (largest component 1, length |c|), a point at axis length a of any segment of
+// the cell is within a w of the walk's, w = sqrt(2) reach_half. With Q = lb -
+// margin at the walk's point at a, all of them are free up to the a' with
+// a' w + (a' - a) |c| <= Q. Roundings are directed as in trace_free, whose margin
+// covers the rounding of the walk's points.
+__device__ __forceinline__ float cell_reach(const FreeGridView& g, float px, float py, float pz, int m, int cell) {
+  const int iu = cell % m, iv = (cell / m) % m, face = cell / (m * m);
+  const float u = (float)(2 * iu + 1 - m) / (float)m, v = (float)(2 * iv + 1 - m) / (float)m;
+  const float one = (face & 1) ? -1.f : 1.f;
+  const int axis = face >> 1;
+  const float cx = axis == 0 ? one : (axis == 1 ? v : u), cy = axis == 0 ? u : (axis == 1 ? one : v),
+              cz = axis == 0 ? v : (axis == 1 ? u : one);
+  const float w = __fmul_ru(1.4142137f, reach_half(m));
+  const float c = __fsqrt_ru(__fadd_ru(__fadd_ru(1.f, __fmul_ru(u, u)), __fmul_ru(v, v))) * 1.000001f;
+  const float inv = __frcp_rd(__fadd_ru(w, c));
+  const float u0 = (px - g.ox) * g.inv_h, v0 = (py - g.oy) * g.inv_h, w0 = (pz - g.oz) * g.inv_h;
+  const float du = cx * g.inv_h, dv = cy * g.inv_h, dw = cz * g.inv_h;
+  float a = 0.f;
+  for (int k = 0; k < kTraceSteps; ++k) {
+    const float Q = __fsub_rd(free_bound(g, fmaf(a, du, u0), fmaf(a, dv, v0), fmaf(a, dw, w0)), g.margin);
+    const float next = __fmul_rd(__fadd_rd(Q, __fmul_rd(a, c)), inv);
+    if (!(next > a)) break;
+    const bool slow = next < 1.02f * a;
+    a = next;
+    if (slow) break;
+  }
+  return a * (1.f - 1e-6f);
+}
+
+// The free ends of the segment p -> q (as trace_free) from the table.
+__device__ __forceinline__ void cone_start(const FreeReach& T, int64_t rp, int64_t rq, float dx, float dy, float dz,
+                                           float& t0, float& s0) {
+  const float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
+  const int axis = ax >= ay ? (ax >= az ? 0 : 2) : (ay >= az ? 1 : 2);
+  const float da = axis == 0 ? dx : (axis == 1 ? dy : dz);
+  const float db = axis == 0 ? dy : (axis == 1 ? dz : dx);
+  const float dc = axis == 0 ? dz : (axis == 1 ? dx : dy);
+  const float len = fabsf(da);
+  t0 = 0.f;
+  s0 = 1.f;
+  if (!(len > 1e-30f)) return;
+  const float inv = __frcp_rd(__fmul_ru(len, 1.000001f));
+  const int m = T.m, top = m - 1;
+  const float half = 0.5f * (float)m;
+  const int iu = min(max((int)(fmaf(db, inv, 1.f) * half), 0), top);
+  const int iv = min(max((int)(fmaf(dc, inv, 1.f) * half), 0), top);
+  const int face = 2 * axis + (da < 0.f ? 1 : 0);
+  const int cp = (face * m + iv) * m + iu, cq = ((face ^ 1) * m + (top - iv)) * m + (top - iu);
+  t0 = __fmul_rd(T.reach[(int64_t)cp * T.n + rp], inv);
+  s0 = __fsub_ru(1.f, __fmul_rd(T.reach[(int64_t)cq * T.n + rq], inv));
+}
+
+
 // Free-space walk of the segment p -> q (d = q - p rounded, len its FP32
 // length) through a cage's grid, from both ends at once (two independent
 // chains of dependent reads). The point at t has cell coordinates
@@ -63,13 +134,14 @@ constexpr int kTraceSteps = 32;  // rounds (two grid reads each) before a segmen
 // parts [0, t] and [s, 1] meet: the segment cannot hit the cage. Roundings
 // are directed so that the parts covered are never overstated. `steps`
 // counts the grid reads.
-__device__ __forceinline__ bool trace_free(const FreeGridView& g, float px, float py, float pz, float dx,
-                                           float dy, float dz, float len, unsigned long long& steps) {
+// t0 and s0 > t0: [0, t0] and [s0, 1] are known to be free (cone_start).
+__device__ __forceinline__ bool trace_free(const FreeGridView& g, float px, float py, float pz, float dx, float dy,
+                                           float dz, float len, float t0, float s0, unsigned long long& steps) {
   // 1 / |q - p| rounded down; |q - p| <= len (1 + 17u).
   const float inv_len = __frcp_rd(__fmul_ru(len, 1.000001f));
   const float u0 = (px - g.ox) * g.inv_h, v0 = (py - g.oy) * g.inv_h, w0 = (pz - g.oz) * g.inv_h;
   const float du = dx * g.inv_h, dv = dy * g.inv_h, dw = dz * g.inv_h;
-  float t = 0.f, s = 1.f;
+  float t = t0, s = s0;
   for (int k = 0; k < kTraceSteps; ++k) {
     const float lb0 = free_bound(g, fmaf(t, du, u0), fmaf(t, dv, v0), fmaf(t, dw, w0));
     const float lb1 = free_bound(g, fmaf(s, du, u0), fmaf(s, dv, v0), fmaf(s, dw, w0));

@@ -41,6 +41,18 @@ namespace vgpu {
 // cage's free-space grid: below this the grid costs about what the walk saves.
 constexpr int64_t kFreeGridMinPairs = 1 << 22;
 
+// Tiles a warp of the walk takes at a time (one at a time, its row and column
+// found anew, took 1.14 ms against 0.56 for 1.64 M tiles: the counter's atomics; 4, 8, 16 and 32 at a time with
+// the table below 0.70, 0.67, 0.70 and 0.79), and its resident CTAs per SM
+// (8, 10, 12 and 16: 0.68, 0.67, 0.70 and 0.71).
+constexpr int kWalkRun = 8, kWalkBlocks = 10;
+
+// Cells per side of the cube's faces in a reach table (reach_side): more of them
+// clear more pairs (10,242 points, all pairs: 33.0 of 52.4 M with 4, 46.1 with 8,
+// 50.3 with 16) but take longer to fill; table and walk 0.69 ms with 6, 0.70 with
+// 8, 0.76 with 10, and 1.75 without a table and one tile at a time.
+constexpr int kReachSide = 6;
+
 // Pairs up to which a call emits and sends its edges without waiting for
 // their number (128 KB of room; the wait it saves is about 15 us).
 constexpr int64_t kFewPairs = 1 << 14;
@@ -63,6 +75,7 @@ struct VisParams {
   int64_t ntr;                          // tile rows
   const unsigned long long* row_start;  // triangular mode: first tile of each tile row
   FreeGridView cage_free;               // the cage's free-space grid (lb null: none)
+  FreeReach cage_reach;                 // and the points' reaches in it (reach null: none)
   // After a walk: the tiles with lanes left for the traversal, and per such
   // tile the lanes that are done (no pair, degenerate, or cleared).
   unsigned long long* pend_tiles;       // null: no walk, every tile is traversed
@@ -75,6 +88,12 @@ struct VisParams {
 __device__ __forceinline__ void tile_of(const VisParams& P, unsigned long long w, int64_t& tr,
                                         int64_t& tc, int TR, int TC) {
   if (!P.triangular) {
+    if ((w >> 32) == 0 && P.ntc <= 0xffffffffLL) {  // 64-bit division is a long routine
+      const uint32_t q = (uint32_t)w / (uint32_t)P.ntc;
+      tr = q;
+      tc = (uint32_t)w - q * (uint32_t)P.ntc;
+      return;
+    }
     tr = (int64_t)(w / (unsigned long long)P.ntc);
     tc = (int64_t)(w % (unsigned long long)P.ntc);
     return;
@@ -82,13 +101,15 @@ __device__ __forceinline__ void tile_of(const VisParams& P, unsigned long long w
   if (TR >= TC) {
     // r = TR / TC is an integer and row t holds ntc - r t tiles (never
     // negative: r (ntr - 1) <= ntc), so row t starts at
-    // S(t) = t ntc - r t (t - 1) / 2. Solve S(t) <= w < S(t + 1) in FP64 and
-    // settle the rounding with the exact integers.
-    const int64_t r = TR / TC, ntc = P.ntc;
+    // S(t) = t ntc - r t (t - 1) / 2. S(t) = w at
+    // t = (B - sqrt(B^2 - 8 r w)) / 2r with B = 2 ntc + r, all but the root in
+    // integers; the root in FP32 (off by less than a row for n <= 2^24) and its
+    // rounding settled exactly. In FP64, whose units are few, this bound the
+    // whole walk: 1.5 ms for 1.64 M tiles with hardly a grid read left.
+    const int64_t r = TR / TC, ntc = P.ntc, B = 2 * ntc + r;
     auto S = [&](int64_t t) { return t * ntc - r * t * (t - 1) / 2; };
-    const double b = (double)ntc + 0.5 * (double)r;
-    const double disc = b * b - 2.0 * (double)r * (double)w;
-    int64_t t = (int64_t)((b - sqrt(disc > 0.0 ? disc : 0.0)) / (double)r);
+    const int64_t D = B * B - 8 * r * (int64_t)w;
+    int64_t t = (B - (int64_t)sqrtf(D > 0 ? (float)D : 0.f)) / (2 * r);
     t = t < 0 ? 0 : (t > P.ntr - 1 ? P.ntr - 1 : t);
     while (t > 0 && (unsigned long long)S(t) > w) --t;
     while (t < P.ntr - 1 && (unsigned long long)S(t + 1) <= w) ++t;
@@ -115,8 +136,7 @@ __global__ void tile_row_counts_kernel(int64_t ntr, int64_t ntc, int TR, int TC,
 }
 
 // The pair of `lane` in tile w of P's tile space (original vertex ids i < j),
-// or valid = false. The walk and the traversal kernels share it, so a tile's
-// lane means the same pair in both.
+// or valid = false.
 template <int TR>
 __device__ __forceinline__ bool lane_pair(const VisParams& P, unsigned long long w, int lane, uint32_t& i,
                                           uint32_t& j) {
@@ -145,6 +165,108 @@ __device__ __forceinline__ bool lane_pair(const VisParams& P, unsigned long long
   j = max(oi, oj);
   return valid;
 }
+
+// What a walk kernel counts per lane.
+struct WalkSums {
+  unsigned pairs, deg, cleared;
+  unsigned long long steps;
+};
+
+// Walks `count` tiles of P's tile space from tile w on. Lane l's pair of a tile
+// is lane_pair's; the row's point stays in registers along a tile row, and the
+// next tile is the next of the row or the first of the next row. Tiles with
+// lanes left are listed as base + their number.
+template <int TR>
+__device__ __forceinline__ void walk_tiles(const VisParams& P, unsigned long long w, int count,
+                                           unsigned long long base, int lane, WalkSums& sum,
+                                           unsigned long long* __restrict__ pending,
+                                           unsigned long long* __restrict__ pend_tiles,
+                                           uint32_t* __restrict__ pend_done) {
+  constexpr int TC = 32 / TR;
+  int64_t tr64, tc64;
+  tile_of(P, w, tr64, tc64, TR, TC);
+  int tr = (int)tr64, tc = (int)tc64, row = -1;
+  uint32_t oi = 0;
+  float px = 0.f, py = 0.f, pz = 0.f;
+  for (int k = 0; k < count; ++k) {
+    const int a = tr * TR + lane / TC, b = tc * TC + lane % TC;
+    if (tr != row) {
+      row = tr;
+      if (a < P.nr) {
+        oi = P.rows[a];
+        px = P.pts[3 * (int64_t)oi];
+        py = P.pts[3 * (int64_t)oi + 1];
+        pz = P.pts[3 * (int64_t)oi + 2];
+      }
+    }
+    bool valid = P.triangular ? a < b && b < P.nc : a < P.nr && b < P.nc;
+    uint32_t oj = 0;
+    if (valid) {
+      oj = P.cols[b];
+      if (!P.triangular) valid = oi != oj && (!P.is_new[oj] || P.newrank[oj] > a);
+    }
+    bool done = true;
+    if (valid) {
+      ++sum.pairs;
+      const float dx = __fsub_rn(P.pts[3 * (int64_t)oj], px), dy = __fsub_rn(P.pts[3 * (int64_t)oj + 1], py),
+                  dz = __fsub_rn(P.pts[3 * (int64_t)oj + 2], pz);
+      const float len = seg_length(dx, dy, dz);
+      if (!(len > 0.f)) {  // coincident endpoints (or NaN): never an edge (as in vis_tile)
+        ++sum.deg;
+      } else {
+        float t0 = 0.f, s0 = 1.f;
+        if (P.cage_reach.reach != nullptr) {
+          const bool pos = P.cage_reach.by_pos != 0;
+          cone_start(P.cage_reach, pos ? a : (int64_t)oi, pos ? b : (int64_t)oj, dx, dy, dz, t0, s0);
+        }
+        done = t0 >= s0 || (P.cage_free.lb != nullptr &&
+                            trace_free(P.cage_free, px, py, pz, dx, dy, dz, len, t0, s0, sum.steps));
+        sum.cleared += done;
+      }
+    }
+    const unsigned m = __ballot_sync(0xffffffffu, done);
+    if (lane == 0 && m != 0xffffffffu) {
+      const unsigned long long at = atomicAdd(pending, 1ull);
+      pend_tiles[at] = base + w + k;
+      pend_done[at] = m;
+    }
+    if (++tc >= P.ntc) {
+      ++tr;
+      tc = P.triangular ? tr * TR / TC : 0;
+    }
+  }
+}
+
+__device__ __forceinline__ void walk_flush(VisCounters* __restrict__ cnt, int lane, const WalkSums& sum) {
+  unsigned long long pairs = sum.pairs, deg = sum.deg, cleared = sum.cleared, steps = sum.steps;
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+    deg += __shfl_xor_sync(0xffffffffu, deg, o);
+    cleared += __shfl_xor_sync(0xffffffffu, cleared, o);
+    steps += __shfl_xor_sync(0xffffffffu, steps, o);
+  }
+  if (lane == 0) {
+    if (pairs) atomicAdd(&cnt->pairs, pairs);
+    if (deg) atomicAdd(&cnt->degenerate, deg);
+    if (cleared) atomicAdd(&cnt->certified, cleared);
+    if (steps) atomicAdd(&cnt->trace_steps, steps);
+  }
+}
+
+// The reach table: entry k is point k % n (rows) in cell k / n, so a warp's
+// walks start at neighbouring points in one direction and stay together.
+__global__ void __launch_bounds__(256) visibility_reach_kernel(VisParams P, float* __restrict__ reach) {
+  const FreeReach T = P.cage_reach;
+  const int64_t count = (int64_t)T.n * 6 * T.m * T.m;
+  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < count;
+       k += (int64_t)gridDim.x * blockDim.x) {
+    const int row = (int)(k % T.n);
+    const int64_t v = T.by_pos ? (int64_t)P.rows[row] : row;
+    reach[k] = cell_reach(P.cage_free, P.pts[3 * v], P.pts[3 * v + 1], P.pts[3 * v + 2], T.m, (int)(k / T.n));
+  }
+}
+
 
 // One tile (work item w of P's tile space) for the calling warp: the cage
 // test, then the self test for lanes whose segment leaves the cage, and the
@@ -221,51 +343,18 @@ __global__ void __launch_bounds__(kVisThreads, MINB) visibility_kernel(VisParams
 // traverse.cuh, trace_free). Few registers, so many warps per SM hide the
 // latency of the walk's dependent grid reads.
 template <int TR>
-__global__ void __launch_bounds__(kVisThreads, 16) visibility_walk_kernel(VisParams P) {
+__global__ void __launch_bounds__(kVisThreads, kWalkBlocks) visibility_walk_kernel(VisParams P) {
   const int lane = threadIdx.x & 31;
-  unsigned long long pairs = 0, deg = 0, cleared = 0, steps = 0;
+  WalkSums sum = {};
   for (int guard = 0; guard < (1 << 30); ++guard) {
     unsigned long long w = 0;
-    if (lane == 0) w = atomicAdd(&P.cnt->walk_work, 1ull);
+    if (lane == 0) w = atomicAdd(&P.cnt->walk_work, (unsigned long long)kWalkRun);
     w = __shfl_sync(0xffffffffu, w, 0);
     if (w >= P.total_tiles) break;
-    uint32_t i, j;
-    bool done = true;
-    if (lane_pair<TR>(P, w, lane, i, j)) {
-      ++pairs;
-      const float px = P.pts[3 * (int64_t)i], py = P.pts[3 * (int64_t)i + 1], pz = P.pts[3 * (int64_t)i + 2];
-      const float dx = __fsub_rn(P.pts[3 * (int64_t)j], px), dy = __fsub_rn(P.pts[3 * (int64_t)j + 1], py),
-                  dz = __fsub_rn(P.pts[3 * (int64_t)j + 2], pz);
-      const float len =
-          __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
-      if (!(len > 0.f)) {  // coincident endpoints (or NaN): never an edge (as in vis_tile)
-        ++deg;
-      } else if (trace_free(P.cage_free, px, py, pz, dx, dy, dz, len, steps)) {
-        ++cleared;
-      } else {
-        done = false;
-      }
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, done);
-    if (lane == 0 && m != 0xffffffffu) {
-      const unsigned long long k = atomicAdd(&P.cnt->pending, 1ull);
-      P.pend_tiles[k] = w;
-      P.pend_done[k] = m;
-    }
+    const int count = (int)min((unsigned long long)kWalkRun, P.total_tiles - w);
+    walk_tiles<TR>(P, w, count, 0ull, lane, sum, &P.cnt->pending, P.pend_tiles, P.pend_done);
   }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
-    deg += __shfl_xor_sync(0xffffffffu, deg, o);
-    cleared += __shfl_xor_sync(0xffffffffu, cleared, o);
-    steps += __shfl_xor_sync(0xffffffffu, steps, o);
-  }
-  if (lane == 0) {
-    if (pairs) atomicAdd(&P.cnt->pairs, pairs);
-    if (deg) atomicAdd(&P.cnt->degenerate, deg);
-    if (cleared) atomicAdd(&P.cnt->certified, cleared);
-    if (steps) atomicAdd(&P.cnt->trace_steps, steps);
-  }
+  walk_flush(P.cnt, lane, sum);
 }
 
 // Many parts in one persistent launch: the work items of all parts are
@@ -319,57 +408,28 @@ __global__ void __launch_bounds__(kVisThreads, MINB)
 // without a grid leave every pair to the traversal). Pending tiles are listed
 // by their global number.
 template <int TR>
-__global__ void __launch_bounds__(kVisThreads, 16)
+__global__ void __launch_bounds__(kVisThreads, kWalkBlocks)
     visibility_multi_walk_kernel(const VisParams* __restrict__ parts, int n_parts,
                                  const unsigned long long* __restrict__ tile_start,
                                  unsigned long long total_tiles, VisCounters* __restrict__ cnt,
                                  unsigned long long* __restrict__ pend_tiles, uint32_t* __restrict__ pend_done) {
   const int lane = threadIdx.x & 31;
-  unsigned long long pairs = 0, deg = 0, cleared = 0, steps = 0;
+  WalkSums sum = {};
   for (int guard = 0; guard < (1 << 30); ++guard) {
     unsigned long long w = 0;
-    if (lane == 0) w = atomicAdd(&cnt->walk_work, 1ull);
+    if (lane == 0) w = atomicAdd(&cnt->walk_work, (unsigned long long)kWalkRun);
     w = __shfl_sync(0xffffffffu, w, 0);
     if (w >= total_tiles) break;
-    const int pi = part_of(tile_start, n_parts, w);
-    const VisParams& P = parts[pi];
-    uint32_t i, j;
-    bool done = true;
-    if (lane_pair<TR>(P, w - tile_start[pi], lane, i, j)) {
-      ++pairs;
-      const float px = P.pts[3 * (int64_t)i], py = P.pts[3 * (int64_t)i + 1], pz = P.pts[3 * (int64_t)i + 2];
-      const float dx = __fsub_rn(P.pts[3 * (int64_t)j], px), dy = __fsub_rn(P.pts[3 * (int64_t)j + 1], py),
-                  dz = __fsub_rn(P.pts[3 * (int64_t)j + 2], pz);
-      const float len =
-          __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
-      if (!(len > 0.f)) {
-        ++deg;
-      } else if (P.cage_free.lb != nullptr && trace_free(P.cage_free, px, py, pz, dx, dy, dz, len, steps)) {
-        ++cleared;
-      } else {
-        done = false;
-      }
-    }
-    const unsigned m = __ballot_sync(0xffffffffu, done);
-    if (lane == 0 && m != 0xffffffffu) {
-      const unsigned long long k = atomicAdd(&cnt->pending, 1ull);
-      pend_tiles[k] = w;
-      pend_done[k] = m;
+    const unsigned long long end = min(w + kWalkRun, total_tiles);
+    for (int pi = part_of(tile_start, n_parts, w); w < end; ++pi) {  // the run's parts
+      const unsigned long long part_end = min(end, tile_start[pi + 1]);
+      if (part_end <= w) continue;
+      walk_tiles<TR>(parts[pi], w - tile_start[pi], (int)(part_end - w), tile_start[pi], lane, sum, &cnt->pending,
+                     pend_tiles, pend_done);
+      w = part_end;
     }
   }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) {
-    pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
-    deg += __shfl_xor_sync(0xffffffffu, deg, o);
-    cleared += __shfl_xor_sync(0xffffffffu, cleared, o);
-    steps += __shfl_xor_sync(0xffffffffu, steps, o);
-  }
-  if (lane == 0) {
-    if (pairs) atomicAdd(&cnt->pairs, pairs);
-    if (deg) atomicAdd(&cnt->degenerate, deg);
-    if (cleared) atomicAdd(&cnt->certified, cleared);
-    if (steps) atomicAdd(&cnt->trace_steps, steps);
-  }
+  walk_flush(cnt, lane, sum);
 }
 
 // ---- vertex ordering ------------------------------------------------------
@@ -509,7 +569,7 @@ constexpr int kDefaultVisVariant = 1;
 static int launch_vis_variant(visacd_ctx* ctx, int v, const VisParams& P) {
   const unsigned grid = (unsigned)(ctx->sm_count * kVisVariants[v].minb);
   if (P.pend_tiles != nullptr) {
-    const unsigned wg = (unsigned)(ctx->sm_count * 16);
+    const unsigned wg = (unsigned)(ctx->sm_count * kWalkBlocks);
     switch (kVisVariants[v].tr) {
       case 8: VLAUNCH(ctx, kKVisWalk, wg, kVisThreads, 0, visibility_walk_kernel<8>, P); break;
       case 4: VLAUNCH(ctx, kKVisWalk, wg, kVisThreads, 0, visibility_walk_kernel<4>, P); break;
@@ -647,6 +707,23 @@ int vis_morton_order(visacd_ctx* ctx, const float* d_pts, int32_t n, uint32_t* p
   return VISACD_OK;
 }
 
+// Cells per side of a reach table for n points and a number of pairs: kReachSide,
+// or fewer where the table would have more than a third as many entries as
+// there are pairs (an entry costs about as many reads as a pair's walk without
+// it), or more than 2^28 (1 GiB); below 3 none.
+static int reach_side(int64_t n, int64_t pairs) {
+  const double cells = std::min((double)pairs / 3.0, 268435456.0) / std::max((double)n, 1.0) / 6.0;
+  const int m = (int)std::min((double)kReachSide, std::sqrt(cells));
+  return m < 3 ? 0 : m;
+}
+static size_t reach_entries(int64_t n, int m) { return (size_t)n * 6 * m * m; }
+
+static int launch_reach(visacd_ctx* ctx, const VisParams& P) {
+  VLAUNCH(ctx, kKVisWalk, grid_for((int64_t)reach_entries(P.cage_reach.n, P.cage_reach.m), 256, 16LL * ctx->sm_count),
+          256, 0, visibility_reach_kernel, P, const_cast<float*>(P.cage_reach.reach));
+  return VISACD_OK;
+}
+
 static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint8_t* d_new,
                       const visacd_bvh* self_bvh, const visacd_bvh* cage_bvh, int64_t* n_edges,
                       visacd_vis_stats* stats, int64_t pairs, int32_t n_new, const PointOrder* ordered,
@@ -747,6 +824,12 @@ static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint
       P.cage_free.nx = cb->fg_nx;
       P.cage_free.ny = cb->fg_ny;
       P.cage_free.nz = cb->fg_nz;
+    }
+    // Without room for the table the walk starts at the points.
+    const int m = reach_side(n, pairs);
+    if (m > 0 && ensure_slot(ctx, kSlotVisReach, reach_entries(n, m) * 4) == VISACD_OK) {
+      P.cage_reach = FreeReach{slot<float>(ctx, kSlotVisReach), m, n, P.triangular};
+      VTRY(launch_reach(ctx, P));
     }
   }
   VTRY(ensure_slot(ctx, kSlotBitset, (size_t)nw * 4));
@@ -963,6 +1046,8 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
   VTRY(ensure_slot(ctx, kSlotCounters, sizeof(VisCounters)));
   VisCounters* cnt = slot<VisCounters>(ctx, kSlotCounters);
   std::vector<VisParams> desc(n_parts);
+  std::vector<size_t> reach_at(n_parts, 0);  // of the parts with a reach table
+  size_t reach_total = 0;
   std::vector<unsigned long long> tile_start(n_parts + 1, 0);
   unsigned long long tiles = 0;
   for (int p = 0; p < n_parts; ++p) {
@@ -1009,6 +1094,12 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
       P.cage_free.nx = cb->fg_nx;
       P.cage_free.ny = cb->fg_ny;
       P.cage_free.nz = cb->fg_nz;
+      const int m = reach_side(n, part_pairs[p]);
+      if (m > 0) {
+        P.cage_reach = FreeReach{nullptr, m, n, P.triangular};
+        reach_at[p] = reach_total;
+        reach_total += (reach_entries(n, m) + 63) & ~(size_t)63;
+      }
     }
     P.bitset = bits + word_start[p];
     P.cnt = cnt;
@@ -1017,6 +1108,13 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
     tiles += P.total_tiles;
   }
   tile_start[n_parts] = tiles;
+  // Without room for the tables the walk starts at the points.
+  const bool reaches = reach_total > 0 && ensure_slot(ctx, kSlotVisReach, reach_total * 4) == VISACD_OK;
+  for (int p = 0; p < n_parts; ++p) {
+    if (desc[p].cage_reach.m == 0) continue;
+    if (reaches) desc[p].cage_reach.reach = slot<float>(ctx, kSlotVisReach) + reach_at[p];
+    else desc[p].cage_reach = FreeReach{};
+  }
   {
     VisCounters init;
     memset(&init, 0, sizeof(init));
@@ -1037,7 +1135,9 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
       VTRY(ensure_slot(ctx, kSlotVisCleared, (size_t)tiles * 12 + 256));
       pend = slot<unsigned long long>(ctx, kSlotVisCleared);
       pend_done = reinterpret_cast<uint32_t*>(pend + tiles);
-      VLAUNCH(ctx, kKVisWalk, (unsigned)(ctx->sm_count * 16), kVisThreads, 0, visibility_multi_walk_kernel<8>,
+      for (int p = 0; p < n_parts; ++p)
+        if (desc[p].cage_reach.reach) VTRY(launch_reach(ctx, desc[p]));
+      VLAUNCH(ctx, kKVisWalk, (unsigned)(ctx->sm_count * kWalkBlocks), kVisThreads, 0, visibility_multi_walk_kernel<8>,
               d_desc, n_parts, d_tiles, tiles, cnt, pend, pend_done);
     }
     VLAUNCH(ctx, kKVisibility, (unsigned)(ctx->sm_count * 8), kVisThreads, 0, (visibility_multi_kernel<8, 8>),
