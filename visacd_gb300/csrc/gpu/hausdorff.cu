@@ -795,11 +795,25 @@ size_t al(size_t x) { return (x + 255) & ~size_t(255); }
 // most 160 cells per axis.
 void grid_for_points(const double* x, long long n, HGrid& g) {
   double lo[3] = {1e300, 1e300, 1e300}, hi[3] = {-1e300, -1e300, -1e300};
-  for (long long i = 0; i < n; ++i)
-    for (int a = 0; a < 3; ++a) {
-      lo[a] = std::min(lo[a], x[3 * i + a]);
-      hi[a] = std::max(hi[a], x[3 * i + a]);
-    }
+  auto take = [](double& l, double& h, double v) {
+    l = std::min(l, v);
+    h = std::max(h, v);
+  };
+  // Four points at a time in twelve independent chains.
+  double l12[12], h12[12];
+  for (int k = 0; k < 12; ++k) {
+    l12[k] = 1e300;
+    h12[k] = -1e300;
+  }
+  long long i = 0;
+  for (; i + 4 <= n; i += 4)
+    for (int k = 0; k < 12; ++k) take(l12[k], h12[k], x[3 * i + k]);
+  for (int k = 0; k < 12; ++k) {
+    lo[k % 3] = std::min(lo[k % 3], l12[k]);
+    hi[k % 3] = std::max(hi[k % 3], h12[k]);
+  }
+  for (; i < n; ++i)
+    for (int a = 0; a < 3; ++a) take(lo[a], hi[a], x[3 * i + a]);
   double ext = std::max(hi[0] - lo[0], std::max(hi[1] - lo[1], hi[2] - lo[2]));
   double area_like = 0;
   for (int a = 0; a < 3; ++a) area_like += (hi[a] - lo[a]) * (hi[(a + 1) % 3] - lo[(a + 1) % 3]);

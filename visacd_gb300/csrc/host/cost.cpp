@@ -7,13 +7,14 @@
 // std::discrete_distribution, two std::uniform_real_distribution draws per
 // sample, one extra sample per untouched triangle, all from the process-wide
 // engine, the std::mt19937 sequence, in the reference's order; the draws are
-// made in bulk with the same values, see extract_point_set). The host
+// made in bulk with the same values, see draw_samples). The host
 // nearest-sample search is this
 // project's kd-tree (the reference uses nanoflann); distances to the sampled
 // triangles are the reference's own formula (ref_point_triangle_distance).
 #include <algorithm>
 #include <chrono>
 #include <cmath>
+#include <exception>
 #include <limits>
 #include <numeric>
 #include <queue>
@@ -38,6 +39,7 @@ namespace {
 // distribution's draw for the same p.
 class DiscreteSampler {
  public:
+  DiscreteSampler() = default;
   explicit DiscreteSampler(const std::discrete_distribution<size_t>& d) {
     const auto prob = d.probabilities();
     cp_.resize(prob.size());
@@ -80,16 +82,24 @@ inline Vec3 tri_sample(const Mesh& m, size_t ti, double a, double b) {
 
 }  // namespace
 
-// Engine outputs are taken in bulk: a draw of the triangle distribution takes
-// two outputs (one canonical double; none when there is a single triangle,
-// which std::discrete_distribution returns without drawing), each of the two
-// uniform doubles two, so sample j of the first loop reads a fixed window of
-// the output stream and the samples are computed independently (in parallel
-// for large counts); the untouched triangles then take four outputs each, in
-// index order. Same values as drawing one by one.
-void extract_point_set(const Mesh& m, std::vector<Vec3>& samples, std::vector<int>& tri_ids,
-                       size_t resolution, double base, bool one_per_tri) {
-  if (m.triangles.empty() || m.vertices.empty()) return;
+namespace {
+
+// What the draws from a mesh need before the engine comes in: its triangle
+// distribution and its number of draws. Independent of the engine, so those of
+// several meshes are made in parallel (3.05 M samples of a decomposition 34 ->
+// 24 ms).
+struct SurfaceDraws {
+  const Mesh* mesh = nullptr;
+  size_t resolution = 0;
+  bool regular = false;  // draws by window (else one by one from the distribution)
+  std::discrete_distribution<size_t> pick;
+  DiscreteSampler fast;
+};
+
+SurfaceDraws surface_draws(const Mesh& m, size_t resolution, double base) {
+  SurfaceDraws d;
+  if (m.triangles.empty() || m.vertices.empty()) return d;
+  d.mesh = &m;
   const size_t T = m.triangles.size();
   std::vector<double> areas(T);
   double total = 0;
@@ -99,25 +109,45 @@ void extract_point_set(const Mesh& m, std::vector<Vec3>& samples, std::vector<in
     total += areas[i];
   }
   if (base != 0) resolution = size_t(std::max(1000, int(resolution * (total / base))));
-  std::discrete_distribution<size_t> pick(areas.begin(), areas.end());
+  d.resolution = resolution;
+  d.pick = std::discrete_distribution<size_t>(areas.begin(), areas.end());
+  d.regular = (total > 0 && std::isfinite(total)) || T == 1;
+  if (d.regular) d.fast = DiscreteSampler(d.pick);
+  return d;
+}
+
+// Engine outputs are taken in bulk: a draw of the triangle distribution takes
+// two outputs (one canonical double; none when there is a single triangle,
+// which std::discrete_distribution returns without drawing), each of the two
+// uniform doubles two, so sample j of the first loop reads a fixed window of
+// the output stream and the samples are computed independently (in parallel
+// for large counts); the untouched triangles then take four outputs each, in
+// index order. Same values as drawing one by one.
+void draw_samples(SurfaceDraws& d, std::vector<Vec3>& samples, std::vector<int>& tri_ids, bool one_per_tri) {
+  if (!d.mesh) return;
+  const Mesh& m = *d.mesh;
+  const size_t T = m.triangles.size(), resolution = d.resolution;
   Mt19937& eng = random_engine();
+  thread_local std::vector<uint32_t> w;  // engine outputs
   // Triangles drawn at least once (a bitmap: only membership matters, the
   // untouched ones are visited in index order below).
   std::vector<char> touched(T, 0);
   const size_t b0 = samples.size();
-  if ((total > 0 && std::isfinite(total)) || T == 1) {
+  samples.reserve(b0 + resolution + T);
+  tri_ids.reserve(b0 + resolution + T);
+  if (d.regular) {
     const int per = T == 1 ? 4 : 6;
-    std::vector<uint32_t> w((size_t)per * resolution);
+    w.resize((size_t)per * resolution);
     eng.fill(w.data(), w.size());
     samples.resize(b0 + resolution);
     tri_ids.resize(b0 + resolution);
-    const DiscreteSampler fast(pick);
+    const uint32_t* words = w.data();
 #pragma omp parallel for schedule(static) if (resolution >= 2048)
     for (long j = 0; j < (long)resolution; ++j) {
-      const uint32_t* q = w.data() + (size_t)per * j;
+      const uint32_t* q = words + (size_t)per * j;
       size_t ti = 0;
       if (T > 1) {
-        ti = fast.find(canonical53(q[0], q[1]));
+        ti = d.fast.find(canonical53(q[0], q[1]));
         q += 2;
       }
       samples[b0 + j] = tri_sample(m, ti, canonical53(q[0], q[1]), canonical53(q[2], q[3]));
@@ -128,7 +158,7 @@ void extract_point_set(const Mesh& m, std::vector<Vec3>& samples, std::vector<in
     // Degenerate weights (zero or non-finite total): the distribution itself.
     std::uniform_real_distribution<double> uni(0.0, 1.0);
     for (size_t done = 0; done < resolution; ++done) {
-      const size_t ti = pick(eng);
+      const size_t ti = d.pick(eng);
       const double a = uni(eng);
       const double b = uni(eng);
       samples.push_back(tri_sample(m, ti, a, b));
@@ -140,17 +170,27 @@ void extract_point_set(const Mesh& m, std::vector<Vec3>& samples, std::vector<in
   std::vector<int> rest;
   for (size_t i = 0; i < T; ++i)
     if (!touched[i]) rest.push_back((int)i);
-  std::vector<uint32_t> w(4 * rest.size());
+  w.resize(4 * rest.size());
   eng.fill(w.data(), w.size());
   const size_t b1 = samples.size();
   samples.resize(b1 + rest.size());
   tri_ids.resize(b1 + rest.size());
+  const uint32_t* words = w.data();
 #pragma omp parallel for schedule(static) if (rest.size() >= 2048)
   for (long k = 0; k < (long)rest.size(); ++k) {
-    const uint32_t* q = w.data() + 4 * k;
+    const uint32_t* q = words + 4 * k;
     samples[b1 + k] = tri_sample(m, (size_t)rest[k], canonical53(q[0], q[1]), canonical53(q[2], q[3]));
     tri_ids[b1 + k] = rest[k];
   }
+  if (w.capacity() > ((size_t)1 << 22)) std::vector<uint32_t>().swap(w);  // 16 MB kept at most
+}
+
+}  // namespace
+
+void extract_point_set(const Mesh& m, std::vector<Vec3>& samples, std::vector<int>& tri_ids,
+                       size_t resolution, double base, bool one_per_tri) {
+  SurfaceDraws d = surface_draws(m, resolution, base);
+  draw_samples(d, samples, tri_ids, one_per_tri);
 }
 
 namespace {
@@ -350,12 +390,32 @@ double compute_rv3(const Mesh& c1, const Mesh& c2, const Mesh& ch) {
 }
 
 void sample_hb(const Mesh& a, const Mesh& b, unsigned int resolution, HbSamples& s) {
+  sample_hb_all({&a}, {&b}, resolution, &s);
+}
+
+void sample_hb_all(const std::vector<const Mesh*>& a, const std::vector<const Mesh*>& b, unsigned int resolution,
+                   HbSamples* s) {
   auto& tm = concavity_times();
   const auto t0 = std::chrono::steady_clock::now();
-  extract_point_set(a, s.s1, s.i1, resolution, 1, true);
-  extract_point_set(b, s.s2, s.i2, resolution, 1, true);
+  const long n = (long)a.size();
+  std::vector<SurfaceDraws> d(2 * (size_t)n);
+  std::exception_ptr failed;  // an exception may not leave the parallel region
+#pragma omp parallel for schedule(dynamic, 1) if (n > 1)
+  for (long k = 0; k < 2 * n; ++k) {
+    try {
+      d[k] = surface_draws(k % 2 ? *b[k / 2] : *a[k / 2], resolution, 1);
+    } catch (...) {
+#pragma omp critical
+      failed = std::current_exception();
+    }
+  }
+  if (failed) std::rethrow_exception(failed);
+  for (long i = 0; i < n; ++i) {
+    draw_samples(d[2 * i], s[i].s1, s[i].i1, true);
+    draw_samples(d[2 * i + 1], s[i].s2, s[i].i2, true);
+    tm.samples += (long long)(s[i].s1.size() + s[i].s2.size());
+  }
   tm.sample_ms += std::chrono::duration<double, std::milli>(std::chrono::steady_clock::now() - t0).count();
-  tm.samples += (long long)(s.s1.size() + s.s2.size());
 }
 
 double eval_hb(const Mesh& a, const Mesh& b, const HbSamples& s, double floor) {

@@ -59,6 +59,9 @@ double compute_hb(const Mesh& a, const Mesh& b, unsigned int resolution);
 // when it is >= floor and some value below floor otherwise (the GPU skips the
 // sample terms that cannot reach floor); the host metric is always exact.
 void sample_hb(const Mesh& a, const Mesh& b, unsigned int resolution, HbSamples& s);
+// sample_hb of the pairs a[i], b[i] into s[i], in order (the same draws).
+void sample_hb_all(const std::vector<const Mesh*>& a, const std::vector<const Mesh*>& b, unsigned int resolution,
+                   HbSamples* s);
 double eval_hb(const Mesh& a, const Mesh& b, const HbSamples& s, double floor = 0.0);
 // eval_hb of many pairs in one GPU call: job j is (a[j], b[j], s[j]). With
 // `independent` every value is exact; otherwise, with lower[j] a known lower

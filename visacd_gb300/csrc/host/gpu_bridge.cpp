@@ -369,16 +369,19 @@ std::vector<double> face_hausdorff_batch(const std::vector<const Mesh*>& a, cons
   T.resize(3 * (size_t)toff[2 * J]);
   X.resize(3 * (size_t)soff[2 * J]);
   I.resize((size_t)soff[2 * J]);
-  for (size_t j = 0; j < J; ++j) {
+  double *vd = V.data(), *xd = X.data();
+  int32_t *td = T.data(), *id = I.data();
+#pragma omp parallel for schedule(dynamic, 1) if (J > 1)
+  for (long j = 0; j < (long)J; ++j) {
     const Mesh* m[2] = {a[j], b[j]};
     const std::vector<Vec3>* xs[2] = {&s[j]->s1, &s[j]->s2};
     const std::vector<int>* is[2] = {&s[j]->i1, &s[j]->i2};
     for (int k = 0; k < 2; ++k) {
       const size_t q = 2 * j + k;
-      std::memcpy(V.data() + 3 * voff[q], m[k]->vertices.data(), m[k]->vertices.size() * 24);
-      std::memcpy(T.data() + 3 * toff[q], m[k]->triangles.data(), m[k]->triangles.size() * 12);
-      std::memcpy(X.data() + 3 * soff[q], xs[k]->data(), xs[k]->size() * 24);
-      std::memcpy(I.data() + soff[q], is[k]->data(), is[k]->size() * 4);
+      std::memcpy(vd + 3 * voff[q], m[k]->vertices.data(), m[k]->vertices.size() * 24);
+      std::memcpy(td + 3 * toff[q], m[k]->triangles.data(), m[k]->triangles.size() * 12);
+      std::memcpy(xd + 3 * soff[q], xs[k]->data(), xs[k]->size() * 24);
+      std::memcpy(id + soff[q], is[k]->data(), is[k]->size() * 4);
     }
   }
   check(visacd_face_hausdorff_batch(ctx, (int32_t)J, V.data(), voff.data(), T.data(), toff.data(), X.data(),

@@ -288,10 +288,6 @@ int get_part_with_highest_concavity(const MeshList& parts, double& max_concavity
   const int n = (int)parts.size();
   std::vector<HbSamples> smp(n);
   std::vector<double> c(n);
-  for (int i = 0; i < n; ++i) {
-    c[i] = compute_rv(parts[i], hulls[i]) * 0.3;
-    sample_hb(parts[i], hulls[i], 3000, smp[i]);
-  }
   std::vector<const Mesh*> pa(n), pb(n);
   std::vector<const HbSamples*> ps(n);
   for (int i = 0; i < n; ++i) {
@@ -299,6 +295,9 @@ int get_part_with_highest_concavity(const MeshList& parts, double& max_concavity
     pb[i] = &hulls[i];
     ps[i] = &smp[i];
   }
+#pragma omp parallel for schedule(dynamic, 1) if (n > 1)
+  for (int i = 0; i < n; ++i) c[i] = compute_rv(parts[i], hulls[i]) * 0.3;
+  sample_hb_all(pa, pb, 3000, smp.data());
   const std::vector<double> hb = eval_hb_batch(pa, pb, ps, c, std::max(max_concavity, 0.0), false);
   for (int i = 0; i < n; ++i) c[i] = std::max(c[i], hb[i]);
   int idx = -1;
@@ -317,7 +316,6 @@ double compute_final_concavity(const MeshList& parts, const MeshList& hulls) {
   // get_part_with_highest_concavity.
   const size_t n = parts.size();
   std::vector<HbSamples> smp(n);
-  for (size_t i = 0; i < n; ++i) sample_hb(parts[i], hulls[i], 10000, smp[i]);
   std::vector<const Mesh*> pa(n), pb(n);
   std::vector<const HbSamples*> ps(n);
   for (size_t i = 0; i < n; ++i) {
@@ -325,6 +323,7 @@ double compute_final_concavity(const MeshList& parts, const MeshList& hulls) {
     pb[i] = &hulls[i];
     ps[i] = &smp[i];
   }
+  sample_hb_all(pa, pb, 10000, smp.data());
   const std::vector<double> hb = eval_hb_batch(pa, pb, ps, {}, 0.0, false);
   double h = 0;
   for (size_t i = 0; i < n; ++i)
