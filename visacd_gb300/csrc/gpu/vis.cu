@@ -47,6 +47,11 @@ constexpr int64_t kFreeGridMinPairs = 1 << 22;
 // (8, 10, 12 and 16: 0.68, 0.67, 0.70 and 0.71).
 constexpr int kWalkRun = 8, kWalkBlocks = 10;
 
+// Warps a tile is split over at most (tile_split): with 1, 2, 4, 8 and 16 the
+// traversal of a 162-vertex blob takes 69, 61, 56, 51 and 53 us, of a 128-vertex
+// torus 126, 112, 84, 69 and 67; from some 600 vertices on there are no free warps.
+constexpr int kMaxSplit = 8;
+
 // Cells per side of the cube's faces in a reach table (reach_side): more of them
 // clear more pairs (10,242 points, all pairs: 33.0 of 52.4 M with 4, 46.1 with 8,
 // 50.3 with 16) but take longer to fill; table and walk 0.69 ms with 6, 0.70 with
@@ -312,6 +317,22 @@ __device__ __forceinline__ void vis_flush_counters(VisCounters* cnt, unsigned* s
   }
 }
 
+// Warps a tile is split over: as many (up to 8, four lanes each) as leave all of
+// them resident. A warp runs its lanes' node and leaf tests one after another, so
+// with few tiles the call is one such chain; each warp then takes 32 / split
+// neighbouring pairs of the tile.
+__device__ __forceinline__ int tile_split(unsigned long long tiles) {
+  const unsigned long long warps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+  int split = 1;
+  while (split < kMaxSplit && tiles * (2 * split) <= warps) split *= 2;
+  return split;
+}
+// The lanes that are not part k's of a tile split in `split`.
+__device__ __forceinline__ uint32_t split_others(int split, int k) {
+  const int lanes = 32 / split;
+  return split == 1 ? 0u : ~(((1u << lanes) - 1u) << (k * lanes));
+}
+
 template <int TR, int MINB>
 __global__ void __launch_bounds__(kVisThreads, MINB) visibility_kernel(VisParams P) {
   const int lane = threadIdx.x & 31;
@@ -323,15 +344,18 @@ __global__ void __launch_bounds__(kVisThreads, MINB) visibility_kernel(VisParams
   // After a walk only the tiles it left are traversed (their count is on the
   // device, written by the walk kernel before this launch).
   const unsigned long long items = P.pend_tiles ? P.cnt->pending : P.total_tiles;
+  const int split = tile_split(items);
   for (int guard = 0; guard < (1 << 30); ++guard) {
     unsigned long long w = 0;
     if (lane == 0) w = atomicAdd(&P.cnt->work, 1ull);
     w = __shfl_sync(0xffffffffu, w, 0);
-    if (w >= items) break;
+    if (w >= items * split) break;
+    const uint32_t others = split_others(split, (int)(w % split));
+    w /= split;
     if (P.pend_tiles)
-      vis_tile<TR>(P, P.pend_tiles[w], lane, sum, status_bits, true, P.pend_done[w]);
+      vis_tile<TR>(P, P.pend_tiles[w], lane, sum, status_bits, true, P.pend_done[w] | others);
     else
-      vis_tile<TR>(P, w, lane, sum, status_bits, false, 0u);
+      vis_tile<TR>(P, w, lane, sum, status_bits, false, others);
   }
   vis_flush_counters(P.cnt, P.status, lane, sum, status_bits);
 }
@@ -387,18 +411,21 @@ __global__ void __launch_bounds__(kVisThreads, MINB)
   __syncwarp();
   unsigned status_bits = 0;
   const unsigned long long items = pend_tiles ? cnt->pending : total_tiles;
+  const int split = tile_split(items);
   for (int guard = 0; guard < (1 << 30); ++guard) {
     unsigned long long w = 0;
     if (lane == 0) w = atomicAdd(&cnt->work, 1ull);
     w = __shfl_sync(0xffffffffu, w, 0);
-    if (w >= items) break;
+    if (w >= items * split) break;
+    const uint32_t others = split_others(split, (int)(w % split));
+    w /= split;
     if (pend_tiles) {
       const unsigned long long g = pend_tiles[w];
       const int p = part_of(tile_start, n_parts, g);
-      vis_tile<TR>(parts[p], g - tile_start[p], lane, sum, status_bits, true, pend_done[w]);
+      vis_tile<TR>(parts[p], g - tile_start[p], lane, sum, status_bits, true, pend_done[w] | others);
     } else {
       const int p = part_of(tile_start, n_parts, w);
-      vis_tile<TR>(parts[p], w - tile_start[p], lane, sum, status_bits, false, 0u);
+      vis_tile<TR>(parts[p], w - tile_start[p], lane, sum, status_bits, false, others);
     }
   }
   vis_flush_counters(cnt, status, lane, sum, status_bits);
