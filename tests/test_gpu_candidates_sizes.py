@@ -21,7 +21,7 @@ def _prefix(draws, unique):
 
 
 @pytest.mark.parametrize("level,num,sizes", [
-    (4, 600, (1, 2, 255, 256, 257, 511, 512, 513, 1025)),
+    (4, 600, (1, 2, 255, 256, 257, 511, 512, 513, 1025, 1537, 2305)),
     (6, 8000, (32767, 32768, 32769, 33100)),
 ])
 def test_candidate_counts_at_edges(ctx, orc, level, num, sizes):

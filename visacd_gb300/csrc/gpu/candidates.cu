@@ -129,10 +129,12 @@ __global__ void __launch_bounds__(kCandTile) conflict_kernel(
   const float kx = (float)pk.x, ky = (float)pk.y, kz = (float)pk.z;
   const float dk = d32[k], near = 1.001e-3f;  // FP32 offsets differ by < 1e-6 from FP64
   const float eps32 = (float)normal_eps - 1e-5f;
-  const int jend = min(kCandTile, k - j0);  // earlier candidates only
+  // This block's share of the tile's columns; earlier candidates only.
+  const int share = kCandTile / gridDim.y, jbegin = blockIdx.y * share;
+  const int jend = min(jbegin + share, k - j0);
   uint32_t c = 0;
 #pragma unroll 2
-  for (int t4 = 0; t4 < jend; t4 += 4) {
+  for (int t4 = jbegin; t4 < jend; t4 += 4) {
     const float4 d = *reinterpret_cast<const float4*>(sd + t4);
     const bool n0 = fabsf(dk - d.x) < near, n1 = fabsf(dk - d.y) < near, n2 = fabsf(dk - d.z) < near,
                n3 = fabsf(dk - d.w) < near;
@@ -469,7 +471,7 @@ __device__ __forceinline__ void warp_offer(unsigned long long& lk, int32_t& li, 
 // them to partial[b][q][0..32). The block computes each bisector once per tile.
 // Bound by FP64 (a division per edge and proposal), so by the SMs it is spread
 // over: 4,661 edges in 10 blocks of 512 edges and 16 proposals took 74 us (and the
-// merge, by insertion, 37); both together now 47.
+// merge, by insertion, 37).
 __global__ void __launch_bounds__(32 * kRefineProps) refine_partial_kernel(
     const double* __restrict__ verts, const uint32_t* __restrict__ edges, int64_t E,
     const double* __restrict__ props, double half, int64_t chunk, RefineEntry* __restrict__ partial) {
@@ -509,14 +511,14 @@ __global__ void __launch_bounds__(32 * kRefineProps) refine_partial_kernel(
   partial[((int64_t)blockIdx.x * kLearnedProps + q) * kRefineK + lane] = RefineEntry{lk, li, 0};
 }
 
-// Pass 2 (one block of 16 warps): merges the blocks' lists per proposal,
-// keeps the first `per` entries of each, and writes the union's bisector
-// planes in edge order to out64/out32 [0, n) (zeros in [n, 512)); n to
-// *n_refined.
+// Pass 2 (one block of 16 warps): merges the blocks' lists per proposal, keeps
+// the first `per` entries of each, and writes the union's edges in order to
+// picked [0, n) (kNoEdge in [n, 512)); n to *n_refined. Their planes are FP64 and
+// made by learned_assemble_kernel over several SMs (with them in this one block it
+// took 33 us).
 __global__ void __launch_bounds__(kRefineTile) refine_merge_kernel(
-    const RefineEntry* __restrict__ partial, int32_t blocks, int32_t per,
-    const double* __restrict__ verts, const uint32_t* __restrict__ edges, Plane64* __restrict__ out64,
-    float4* __restrict__ out32, int32_t* __restrict__ n_refined) {
+    const RefineEntry* __restrict__ partial, int32_t blocks, int32_t per, int32_t* __restrict__ picked,
+    int32_t* __restrict__ n_refined) {
   __shared__ int32_t sel[kRefineSlots];
   __shared__ int warp_base[kLearnedProps + 1];
   const int t = threadIdx.x, q = t >> 5, lane = t & 31;
@@ -561,44 +563,37 @@ __global__ void __launch_bounds__(kRefineTile) refine_merge_kernel(
   __syncthreads();
   const int n = warp_base[kLearnedProps];
   if (keep) {
-    const int pos = warp_base[q] + __popc(m & ((1u << lane) - 1u));
-    Plane64 pl = Plane64{0.0, 0.0, 0.0, 0.0};
-    edge_bisector(verts, edges, v, pl);
-    out64[pos] = pl;
-    out32[pos] = make_float4((float)pl.x, (float)pl.y, (float)pl.z, (float)pl.w);
+    picked[warp_base[q] + __popc(m & ((1u << lane) - 1u))] = v;
   }
-  if (t >= n) {
-    out64[t] = Plane64{0.0, 0.0, 0.0, 0.0};
-    out32[t] = make_float4(0.f, 0.f, 0.f, 0.f);
-  }
+  if (t >= n) picked[t] = kNoEdge;
 }
 
-// The scored plane list of the learned search: [0, 16) proposals, [16, 528)
-// refined (written by refine_merge_kernel), [528, 528 + probe_slots) the kept
-// probe candidates (zeros after them), then the F flat planes.
-__global__ void learned_assemble_kernel(const double* __restrict__ props, const Plane64* __restrict__ probe,
+// The scored plane list of the learned search: [0, 16) proposals, [16, 528) the
+// bisectors of the refinement's edges (zeros after them), [528, 528 + probe_slots)
+// the kept probe candidates (zeros after them), then the F flat planes.
+__global__ void learned_assemble_kernel(const double* __restrict__ props, const double* __restrict__ verts,
+                                        const uint32_t* __restrict__ edges, const int32_t* __restrict__ picked,
+                                        const Plane64* __restrict__ probe,
                                         const int32_t* __restrict__ cinfo, int32_t probe_slots,
                                         const double* __restrict__ flat, int32_t F,
                                         Plane64* __restrict__ out64, float4* __restrict__ out32) {
   const int n_probe = cinfo[0];
-  const int total = kLearnedProps + probe_slots + F;
+  const int total = kProbeBase + probe_slots + F;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < total; i += gridDim.x * blockDim.x) {
     Plane64 p = Plane64{0.0, 0.0, 0.0, 0.0};
-    int slot;
     if (i < kLearnedProps) {
       p = Plane64{props[4 * i], props[4 * i + 1], props[4 * i + 2], props[4 * i + 3]};
-      slot = i;
-    } else if (i < kLearnedProps + probe_slots) {
-      const int r = i - kLearnedProps;
-      if (r < n_probe) p = probe[r];
-      slot = kProbeBase + r;
+    } else if (i < kProbeBase) {
+      const int32_t e = picked[i - kLearnedProps];
+      if (e != kNoEdge) edge_bisector(verts, edges, e, p);
+    } else if (i < kProbeBase + probe_slots) {
+      if (i - kProbeBase < n_probe) p = probe[i - kProbeBase];
     } else {
-      const int r = i - kLearnedProps - probe_slots;
+      const int r = i - kProbeBase - probe_slots;
       p = Plane64{flat[4 * r], flat[4 * r + 1], flat[4 * r + 2], flat[4 * r + 3]};
-      slot = kProbeBase + probe_slots + r;
     }
-    out64[slot] = p;
-    out32[slot] = make_float4((float)p.x, (float)p.y, (float)p.z, (float)p.w);
+    out64[i] = p;
+    out32[i] = make_float4((float)p.x, (float)p.y, (float)p.z, (float)p.w);
   }
 }
 
@@ -791,7 +786,10 @@ int generate(visacd_ctx* ctx, const double* verts, int32_t n, const uint32_t* ed
   const int T = (D + kCandTile - 1) / kCandTile;
   const unsigned tiles = (unsigned)(T * (T + 1) / 2);
   const double normal_eps = std::cos(5.0 * M_PI / 180.0);
-  VLAUNCH(ctx, kKCandidates, tiles, kCandTile, 0, conflict_kernel<0>, s.planes, s.d32, s.state, D,
+  // With few tiles their columns are shared out over more blocks (a block walks
+  // its columns one after another).
+  const dim3 conflicts(tiles, tiles * 8 <= (unsigned)ctx->sm_count ? 8 : (tiles * 4 <= (unsigned)ctx->sm_count ? 4 : 1));
+  VLAUNCH(ctx, kKCandidates, conflicts, kCandTile, 0, conflict_kernel<0>, s.planes, s.d32, s.state, D,
           normal_eps, s.count, (const uint64_t*)nullptr, (uint32_t*)nullptr, (int32_t*)nullptr);
   VTRY(exclusive_scan_u32_to_u64(ctx, s.count, s.offset, D));
   // The lists' total size is only known on the device: read it back (one
@@ -804,7 +802,7 @@ int generate(visacd_ctx* ctx, const double* verts, int32_t n, const uint32_t* ed
   VTRY(ensure_slot(ctx, kSlotCandLinks, (size_t)(n_links > 0 ? n_links : 1) * 4));
   int32_t* list = slot<int32_t>(ctx, kSlotCandLinks);
   if (n_links) {
-    VLAUNCH(ctx, kKCandidates, tiles, kCandTile, 0, conflict_kernel<1>, s.planes, s.d32, s.state, D,
+    VLAUNCH(ctx, kKCandidates, conflicts, kCandTile, 0, conflict_kernel<1>, s.planes, s.d32, s.state, D,
             normal_eps, (uint32_t*)nullptr, s.offset, s.fill, list);
   }
   VLAUNCH(ctx, kKCandidates, 1, 1024, 0, resolve_kernel, s.offset, list, s.state, D, ctx->d_status);
@@ -961,7 +959,7 @@ extern "C" int visacd_learned_split_search(visacd_lp* lp, const double* verts, i
   const int32_t P = kProbeBase + probe_slots + n_flat;
   const size_t b_props = 256 * 2, b_partial = align256((size_t)blocks * kRefineSlots * sizeof(RefineEntry)),
                b_o64 = align256((size_t)P * sizeof(Plane64)), b_o32 = align256((size_t)P * sizeof(float4)),
-               b_nref = 256, b_out = align256(sizeof(LearnedOut));
+               b_nref = 256 + 4 * kRefineSlots, b_out = align256(sizeof(LearnedOut));  // the count, then the edges
   VTRY(ensure_slot(ctx, kSlotLearned, b_props + b_partial + b_o64 + b_o32 + b_nref + b_out));
   char* p = slot<char>(ctx, kSlotLearned);
   double* props = reinterpret_cast<double*>(p);
@@ -969,15 +967,16 @@ extern "C" int visacd_learned_split_search(visacd_lp* lp, const double* verts, i
   Plane64* L64 = reinterpret_cast<Plane64*>(p + b_props + b_partial);
   float4* L32 = reinterpret_cast<float4*>(p + b_props + b_partial + b_o64);
   int32_t* nref = reinterpret_cast<int32_t*>(p + b_props + b_partial + b_o64 + b_o32);
+  int32_t* picked = nref + 64;
   LearnedOut* dout = reinterpret_cast<LearnedOut*>(p + b_props + b_partial + b_o64 + b_o32 + b_nref);
 
   VTRY(lp_propose_device(lp, pts32, n, s.edges, E, center, scale, props));
   VLAUNCH(ctx, kKLpRefine, dim3(blocks, kLearnedProps / kRefineProps), 32 * kRefineProps, 0, refine_partial_kernel, s.verts, s.edges, E, props, half,
           chunk, partial);
-  VLAUNCH(ctx, kKLpRefine, 1, kRefineTile, 0, refine_merge_kernel, partial, blocks, refine_k, s.verts,
-          s.edges, L64 + kLearnedProps, L32 + kLearnedProps, nref);
-  VLAUNCH(ctx, kKLpSplit, grid_for(kLearnedProps + probe_slots + n_flat, 256, 64), 256, 0,
-          learned_assemble_kernel, props, s.out64, s.info, probe_slots, s.flat, n_flat, L64, L32);
+  VLAUNCH(ctx, kKLpRefine, 1, kRefineTile, 0, refine_merge_kernel, partial, blocks, refine_k, picked,
+          nref);
+  VLAUNCH(ctx, kKLpSplit, grid_for(P, 32, 4LL * ctx->sm_count), 32, 0, learned_assemble_kernel, props,
+          (const double*)s.verts, (const uint32_t*)s.edges, (const int32_t*)picked, s.out64, s.info, probe_slots, s.flat, n_flat, L64, L32);
 
   VTRY(ensure_slot(ctx, kSlotScores, (size_t)P * 8));
   double* scores = slot<double>(ctx, kSlotScores);
