@@ -459,40 +459,93 @@ __global__ void __launch_bounds__(128) sdf_far_dist_kernel(const double* __restr
   }
 }
 
-// Crossing of one ray (grid column (ku, kw) along axis ax) with a triangle:
-// toggles the first voxel whose centre lies beyond the crossing.
-__device__ __forceinline__ void cross_ray(const double (&A)[3], const double (&B)[3], const double (&C)[3],
+// Crossings of rays (grid column (ku, kw) along axis ax) with triangles. What an
+// FP32 form of the three orientations cannot rule out is kept per warp and
+// evaluated in FP64 32 at a time, as in PairQueue.
+struct RayQueue {
+  int t[64], ku[64], kw[64];
+};
+
+// Crossing of one ray with triangle t: toggles the first voxel whose centre lies
+// beyond the crossing. Component 0, 1, 2 of the vertices: along u, w, ax.
+__device__ __forceinline__ void cross_ray(const double* __restrict__ P, const int32_t* __restrict__ T, int t,
                                           const SdfGrid& g, int ax, int u, int w, int ku, int kw,
                                           uint32_t* __restrict__ toggle) {
+  double V[3][3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) {
+    const double* v = P + 3 * (int64_t)T[3 * (size_t)t + k];
+    V[k][0] = v[u];
+    V[k][1] = v[w];
+    V[k][2] = v[ax];
+  }
+  const double(&A)[3] = V[0], (&B)[3] = V[1], (&C)[3] = V[2];
   const double ou = 1.2345679e-6, ow = 2.3456789e-6;
   const double y = da((double)(g.org[u] + ku), ou), z = da((double)(g.org[w] + kw), ow);
-  const double e0 = ds(dm(ds(B[u], A[u]), ds(z, A[w])), dm(ds(B[w], A[w]), ds(y, A[u])));
-  const double e1 = ds(dm(ds(C[u], B[u]), ds(z, B[w])), dm(ds(C[w], B[w]), ds(y, B[u])));
-  const double e2 = ds(dm(ds(A[u], C[u]), ds(z, C[w])), dm(ds(A[w], C[w]), ds(y, C[u])));
+  const double e0 = ds(dm(ds(B[0], A[0]), ds(z, A[1])), dm(ds(B[1], A[1]), ds(y, A[0])));
+  const double e1 = ds(dm(ds(C[0], B[0]), ds(z, B[1])), dm(ds(C[1], B[1]), ds(y, B[0])));
+  const double e2 = ds(dm(ds(A[0], C[0]), ds(z, C[1])), dm(ds(A[1], C[1]), ds(y, C[0])));
   const bool in = (e0 > 0 && e1 > 0 && e2 > 0) || (e0 < 0 && e1 < 0 && e2 < 0);
   if (!in) return;
   const double sw = da(da(e0, e1), e2);
-  const double x = __ddiv_rn(da(da(dm(e1, A[ax]), dm(e2, B[ax])), dm(e0, C[ax])), sw);
+  const double x = __ddiv_rn(da(da(dm(e1, A[2]), dm(e2, B[2])), dm(e0, C[2])), sw);
   // first voxel s whose centre org + s lies beyond x (integers compare exactly)
-  int s = (int)floor(x - (double)g.org[ax]) + 1;
-  while (s > 0 && (double)(g.org[ax] + s - 1) > x) --s;
-  while (s < g.dim[ax] && !((double)(g.org[ax] + s) > x)) ++s;
+  const int org = g.org[ax], dim = g.dim[ax];
+  int s = (int)floor(x - (double)org) + 1;
+  while (s > 0 && (double)(org + s - 1) > x) --s;
+  while (s < dim && !((double)(org + s) > x)) ++s;
   if (s < 0) s = 0;
-  if (s >= g.dim[ax]) return;
-  int gi[3];
-  gi[ax] = s;
-  gi[u] = ku;
-  gi[w] = kw;
-  atomicXor(&toggle[vid(g, gi[0], gi[1], gi[2])], 1u << ax);
+  if (s >= dim) return;
+  const int gi = ax == 0 ? s : (u == 0 ? ku : kw), gj = ax == 1 ? s : (u == 1 ? ku : kw),
+            gk = ax == 2 ? s : (u == 2 ? ku : kw);
+  atomicXor(&toggle[vid(g, gi, gj, gk)], 1u << ax);
+}
+
+// False when two of the orientations certainly have different signs. Coordinates
+// are off by at most c (rounding to FP32, and the rays' offsets), differences of
+// one triangle's box by twice that; the products' own rounding is far below m's
+// second term.
+__device__ __forceinline__ bool ray_may_cross(const SdfTri& r, const SdfGrid& g, int u, int w, int eu, int ew, int ku,
+                                              int kw) {
+  const float y = (float)(g.org[u] + ku), z = (float)(g.org[w] + kw);
+  const float Au = r.v[0][u], Aw = r.v[0][w], Bu = r.v[1][u], Bw = r.v[1][w], Cu = r.v[2][u], Cw = r.v[2][w];
+  const float c = 8.0f * kSdfU * (r.vabs + fabsf(y) + fabsf(z)) + 5e-6f;
+  const float m = 8.0f * c * (float)(eu + ew + 2) + 1e-6f * (float)(eu + 1) * (float)(ew + 1);
+  const float e0 = (Bu - Au) * (z - Aw) - (Bw - Aw) * (y - Au);
+  const float e1 = (Cu - Bu) * (z - Bw) - (Cw - Bw) * (y - Bu);
+  const float e2 = (Au - Cu) * (z - Cw) - (Aw - Cw) * (y - Cu);
+  return !((e0 < -m || e1 < -m || e2 < -m) && (e0 > m || e1 > m || e2 > m));
+}
+
+__device__ __forceinline__ void queue_rays(RayQueue& Q, int& n, bool keep, int t, int ku, int kw, bool flush,
+                                           const double* __restrict__ P, const int32_t* __restrict__ T,
+                                           const SdfGrid& g, int ax, int u, int w, uint32_t* __restrict__ toggle) {
+  const int lane = threadIdx.x & 31;
+  const unsigned m = __ballot_sync(0xffffffffu, keep);
+  if (keep) {
+    const int at = n + __popc(m & ((1u << lane) - 1u));
+    Q.t[at] = t;
+    Q.ku[at] = ku;
+    Q.kw[at] = kw;
+  }
+  n += __popc(m);
+  while (n >= 32 || (flush && n > 0)) {
+    __syncwarp();
+    const int first = n > 32 ? n - 32 : 0;
+    if (first + lane < n)
+      cross_ray(P, T, Q.t[first + lane], g, ax, u, w, Q.ku[first + lane], Q.kw[first + lane], toggle);
+    n = first;
+    __syncwarp();
+  }
 }
 
 // Triangles covering at most kCrossSmall rays (nearly all): kCrossLanes lanes
-// each, over its rays, blockIdx.y the axis. Bound by the latency of the loads
-// and atomics: all three axes in one launch, with one bit each, and the rays of
-// parities next to each other in x, took crossings and votes from 321 to 116 us
-// on 740,000 voxels. Larger ones (the long triangles of
+// each, over its rays, blockIdx.y the axis. Larger ones (the long triangles of
 // clipped parts' caps, big faces) are listed with their axis and take one block
-// each (sdf_cross_wide_kernel).
+// each (sdf_cross_wide_kernel). All three axes in one launch with one bit each,
+// and the parities' rays next to each other in x, took crossings and votes of
+// 20,480 triangles on 740,000 voxels from 321 to 116 us; of that 82 were this
+// kernel with every ray in FP64 in its own lane, and are 49 now.
 constexpr int kCrossSmall = 32;
 constexpr int kCrossLanes = 8;
 
@@ -500,22 +553,36 @@ __global__ void __launch_bounds__(128) sdf_cross_kernel(const double* __restrict
                                                         int nt, SdfGrid g, const SdfTri* __restrict__ prep,
                                                         uint32_t* __restrict__ toggle, int* __restrict__ wide,
                                                         unsigned* __restrict__ n_wide) {
+  __shared__ RayQueue queues[4];
+  RayQueue& Q = queues[threadIdx.x >> 5];
   const int ax = blockIdx.y, u = (ax + 1) % 3, w = (ax + 2) % 3;
   const int gid = blockIdx.x * blockDim.x + threadIdx.x;
   const int sub = gid % kCrossLanes;
   const int groups = (gridDim.x * blockDim.x) / kCrossLanes;
-  for (int t = gid / kCrossLanes; t < nt; t += groups) {
-    const int4 r = *reinterpret_cast<const int4*>(prep[t].ray[ax]);
-    const int n = r.z * r.w;
+  int nq = 0;
+  for (int t0 = (gid - (int)(threadIdx.x & 31)) / kCrossLanes; t0 < nt; t0 += groups) {  // the warp's first triangle
+    const int t = t0 + (int)(threadIdx.x & 31) / kCrossLanes;
+    int4 r = make_int4(0, 0, 0, 0);
+    if (t < nt) r = *reinterpret_cast<const int4*>(prep[t].ray[ax]);
+    int n = r.z * r.w;
     if (n > kCrossSmall) {
       if (sub == 0) wide[atomicAdd(n_wide, 1u)] = 3 * t + ax;
-      continue;
+      n = 0;
     }
-    if (sub >= n) continue;
-    double A[3], B[3], C[3];
-    load_tri(P, T, t, A, B, C);
-    for (int q = sub; q < n; q += kCrossLanes) cross_ray(A, B, C, g, ax, u, w, r.x + q % r.z, r.y + q / r.z, toggle);
+    const int most = __reduce_max_sync(0xffffffffu, n);
+    for (int q0 = 0; q0 < most; q0 += kCrossLanes) {
+      const int q = q0 + sub;
+      int ku = 0, kw = 0;
+      bool keep = false;
+      if (q < n) {
+        kw = r.y + q / r.z;
+        ku = r.x + q % r.z;
+        keep = ray_may_cross(prep[t], g, u, w, r.z, r.w, ku, kw);
+      }
+      queue_rays(Q, nq, keep, t, ku, kw, false, P, T, g, ax, u, w, toggle);
+    }
   }
+  queue_rays(Q, nq, false, 0, 0, 0, true, P, T, g, ax, u, w, toggle);
 }
 
 __global__ void __launch_bounds__(128) sdf_cross_wide_kernel(const double* __restrict__ P,
@@ -524,14 +591,25 @@ __global__ void __launch_bounds__(128) sdf_cross_wide_kernel(const double* __res
                                                              const int* __restrict__ wide,
                                                              const unsigned* __restrict__ n_wide,
                                                              uint32_t* __restrict__ toggle) {
+  __shared__ RayQueue queues[4];
+  RayQueue& Q = queues[threadIdx.x >> 5];
   const int nw = (int)*n_wide;
   for (int k = blockIdx.x; k < nw; k += gridDim.x) {
     const int t = wide[k] / 3, ax = wide[k] % 3, u = (ax + 1) % 3, w = (ax + 2) % 3;
     const int4 r = *reinterpret_cast<const int4*>(prep[t].ray[ax]);
-    double A[3], B[3], C[3];
-    load_tri(P, T, t, A, B, C);
-    for (int q = threadIdx.x; q < r.z * r.w; q += blockDim.x)
-      cross_ray(A, B, C, g, ax, u, w, r.x + q % r.z, r.y + q / r.z, toggle);
+    const int n = r.z * r.w;
+    int nq = 0;
+    for (int q0 = 0; q0 < n; q0 += blockDim.x) {
+      const int q = q0 + threadIdx.x;
+      int ku = 0, kw = 0;
+      bool keep = false;
+      if (q < n) {
+        kw = r.y + q / r.z;
+        ku = r.x + q % r.z;
+        keep = ray_may_cross(prep[t], g, u, w, r.z, r.w, ku, kw);
+      }
+      queue_rays(Q, nq, keep, t, ku, kw, q0 + (int)blockDim.x >= n, P, T, g, ax, u, w, toggle);
+    }
   }
 }
 
