@@ -307,15 +307,13 @@ def run_ours(args) -> dict:
     # HBM copy and bf16 GEMM only); ncu's L1 / L2 throughput and issue
     # activity of each (profiles/) say what binds them.
     walk_ms, walk_n = ktimes.get("vis_walk", (0.0, 0))
+    reach_ms, reach_n = ktimes.get("vis_reach", (0.0, 0))
     walk_launch_s = walk_ms / max(walk_n, 1) / 1e3
-    # Free-space walk per launch: one point-sampled texture fetch of the bound
-    # grid per step (grid reads, counted by the kernel), and around it the
-    # point (3 FMA), its cell coordinates (3 sub + 3 mul) and the step (sub,
-    # mul, add): 15 FLOP. The texture fetch rate binds it (ncu: L1/TEX is its
-    # busiest unit); the FP32 figure is kept beside it.
+    reach_launch_s = reach_ms / max(reach_n, 1) / 1e3
+    # Free-space walk per launch: the pairs it takes and the grid reads it still
+    # needs (one point-sampled texture fetch each, counted by the kernel) after
+    # the points' tabled reaches. Instruction issue binds it (ncu).
     walk_fetch = walk_reads / walk_launch_s / 1e9 if walk_ms else None
-    walk_flop = 15.0 * walk_reads
-    walk_achieved = walk_flop / walk_launch_s / 1e12 if walk_ms else None
     vis_ms, vis_n = ktimes.get("visibility", (0.0, 0))
     sc_ms, sc_n = ktimes.get("score_planes", (0.0, 0))
     peaks = json.loads((ROOT / "MEASURED_PEAKS.json").read_text()) if (ROOT / "MEASURED_PEAKS.json").exists() else {}
@@ -346,32 +344,26 @@ def run_ours(args) -> dict:
         "gpu_launches": int(launches),
         "kernels_ms_per_step": {k: v[0] / args.steps for k, v in sorted(ktimes.items(), key=lambda kv: -kv[1][0])},
         "kernel_launches": {k: v[1] for k, v in ktimes.items()},
-        "roofline": {"kernel": "visibility_walk_kernel", "bound": "texture-fetch",
-                     "achieved": walk_fetch, "peak": tex_coherent, "unit": "Gfetch/s",
-                     "frac": walk_fetch / tex_coherent if walk_fetch else None,
-                     "frac_of_divergent_fetch_rate": walk_fetch / tex_divergent if walk_fetch else None,
-                     "peak_divergent": tex_divergent,
-                     "fp32_model": {"achieved": walk_achieved, "peak": fp32_peak, "unit": "TFLOP/s",
-                                    "frac": walk_achieved / fp32_peak if walk_achieved else None,
-                                    "work_model": "grid reads x 15 FLOP (point, cell coordinates, step)"},
-                     "traffic": measured_traffic(args.workload, "visibility_walk_kernel"),
-                     "ncu": measured_throughput(args.workload, "visibility_walk_kernel"),
-                     "ms_per_launch": walk_ms / max(walk_n, 1),
-                     "segments_cleared": int(walk_cleared), "grid_reads": int(walk_reads),
-                     "work_model": "grid reads (one point-sampled tex3D<float> fetch each) per launch",
-                     "peak_source": "measured in-process: tex3D<float> point fetches from a cache-resident "
-                                    "32^3 texture, coherent 8x4 texel blocks per warp (peak) and one line per "
-                                    "lane (peak_divergent); HBM peak of measured "
-                                    f"{peaks.get('hbm_gbs')} GB/s not binding (L2-resident grid)"},
-        "roofline_traversal": {"kernel": "visibility_kernel", "bound": "fp32-issue",
-                               "achieved": vis_achieved, "peak": fp32_peak, "unit": "TFLOP/s",
-                               "frac": vis_achieved / fp32_peak if vis_achieved else None,
-                               "traffic": measured_traffic(args.workload, "visibility_kernel"),
-                               "ncu": measured_throughput(args.workload, "visibility_kernel"),
-                               "ms_per_launch": vis_ms / max(vis_n, 1),
-                               "pairs_per_s": n_pairs / (vis_launch_s + walk_launch_s) if vis_ms else None,
-                               "work_model": "packet node visits x 32 lanes x 2 boxes x 12 FLOP + "
-                                             "triangle tests x 60 FLOP (the pairs the walk left)"},
+        "roofline": {"kernel": "visibility_kernel", "bound": "fp32-issue",
+                     "achieved": vis_achieved, "peak": fp32_peak, "unit": "TFLOP/s",
+                     "frac": vis_achieved / fp32_peak if vis_achieved else None,
+                     "traffic": measured_traffic(args.workload, "visibility_kernel"),
+                     "ncu": measured_throughput(args.workload, "visibility_kernel"),
+                     "ms_per_launch": vis_ms / max(vis_n, 1),
+                     "pairs_per_s": n_pairs / (vis_launch_s + walk_launch_s + reach_launch_s) if vis_ms else None,
+                     "work_model": "packet node visits x 32 lanes x 2 boxes x 12 FLOP + "
+                                   "triangle tests x 60 FLOP (the pairs the walk left)",
+                     "peak_source": "measured in-process FP32 FMA rate; HBM peak of measured "
+                                    f"{peaks.get('hbm_gbs')} GB/s not binding (L2-resident BVHs)"},
+        "roofline_walk": {"kernel": "visibility_walk_kernel", "bound": "instruction-issue",
+                          "achieved": n_pairs / walk_launch_s / 1e9 if walk_ms else None, "unit": "Gpairs/s",
+                          "grid_reads_gfetch_per_s": walk_fetch,
+                          "fetch_rate_coherent": tex_coherent, "fetch_rate_divergent": tex_divergent,
+                          "traffic": measured_traffic(args.workload, "visibility_walk_kernel"),
+                          "ncu": measured_throughput(args.workload, "visibility_walk_kernel"),
+                          "ms_per_launch": walk_ms / max(walk_n, 1),
+                          "reach_ms_per_launch": reach_ms / max(reach_n, 1),
+                          "segments_cleared": int(walk_cleared), "grid_reads": int(walk_reads)},
         "roofline_scoring": {"kernel": "score_planes_kernel", "bound": "fp32-issue",
                              "achieved": sc_achieved, "peak": fp32_peak, "unit": "TFLOP/s",
                              "frac": sc_achieved / fp32_peak if sc_achieved else None,

@@ -115,7 +115,8 @@ int visacd_ctx_kernel_times(visacd_ctx* ctx, const char** names, double* total_m
 /* Number of kernel launches issued on this context since creation. */
 int64_t visacd_ctx_launch_count(const visacd_ctx* ctx);
 int visacd_ctx_sm_count(const visacd_ctx* ctx);
-/* The device sort the BVH build and the visibility ordering use: a stable
+/* The device sort of BVH builds and point orders above 131072 primitives
+   (smaller ones sort the same order inside one thread-block cluster): a stable
    sort of (keys[i], vals[i]) by key (keys below 2^key_bits), host arrays
    sorted in place. Up to 512 pairs: a bitonic sort in one CTA's shared
    memory; up to 32768: one CTA running every 8-bit LSD pass; beyond: three

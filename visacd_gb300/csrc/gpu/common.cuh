@@ -219,6 +219,7 @@ enum KernelId {
   kKGridEdt,
   kKGridFinal,
   kKVisWalk,
+  kKVisReach,
   kKConvexHull,
   kKMisc,
   kKCount

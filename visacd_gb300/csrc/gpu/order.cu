@@ -29,8 +29,11 @@ namespace {
 constexpr int kOrderThreads = 1024;
 constexpr int kOrderWarps = kOrderThreads / 32;
 constexpr int kOrderCluster = 8;
-constexpr int kOrderSmall = 2048;  // primitives one CTA serves
-constexpr int kOrderRank = 512;    // of those, ranked by counting instead of sorted
+// Primitives one CTA serves (a build of 1,472 triangles 54 us, with the cluster 57;
+// of 2,048 64 and 63), and of those the ones ranked by counting instead of sorted
+// (400: 33 us, sorted 41; 512: 37 and 43; 688: 46, sorted 45; 1,024: 68 and 49).
+constexpr int kOrderSmall = 2048;
+constexpr int kOrderRank = 512;
 
 struct OrderArgs {
   OrderJob job[kOrderMaxJobs];

@@ -746,7 +746,7 @@ static int reach_side(int64_t n, int64_t pairs) {
 static size_t reach_entries(int64_t n, int m) { return (size_t)n * 6 * m * m; }
 
 static int launch_reach(visacd_ctx* ctx, const VisParams& P) {
-  VLAUNCH(ctx, kKVisWalk, grid_for((int64_t)reach_entries(P.cage_reach.n, P.cage_reach.m), 256, 16LL * ctx->sm_count),
+  VLAUNCH(ctx, kKVisReach, grid_for((int64_t)reach_entries(P.cage_reach.n, P.cage_reach.m), 256, 16LL * ctx->sm_count),
           256, 0, visibility_reach_kernel, P, const_cast<float*>(P.cage_reach.reach));
   return VISACD_OK;
 }
