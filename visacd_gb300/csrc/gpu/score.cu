@@ -238,13 +238,53 @@ static uint32_t score_shape_class(int32_t P, int64_t E) {
 
 static int planes_per_thread(int32_t P);
 
+// How a call is split into CTAs: each takes 256 K planes and a run of `per` edge
+// blocks. The SM with the most CTAs ends last, so the cost is its CTAs times
+// their blocks, times what a block of K planes per thread costs (2^20 edges x
+// 4096 planes take 1.95, 1.71, 1.63 and 1.74 ms with K = 1, 2, 4 and 8), over the
+// share of that rate which few CTAs on an SM reach (a single one 0.70 with K = 1,
+// 0.95 with K = 2, 0.97 with K = 4). 59,183 edges x 2,500 planes take 70 us, 262,144
+// x 592 100, 4,661 x 2,500 14; with about four CTAs per SM and K by the planes alone
+// 106, 141 and 24.
+struct ScoreSplit {
+  int64_t per, slices;
+  double cost;
+};
+static ScoreSplit score_split(int sm_count, int32_t P, int64_t E, int K) {
+  const int64_t groups = (P + (int64_t)kScoreThreads * K - 1) / (kScoreThreads * K);
+  const int64_t nblocks = std::max<int64_t>(1, (E + kEdgeBlock - 1) / kEdgeBlock);
+  const double block = K * (K == 1 ? 1.95 : (K == 2 ? 1.71 : (K == 4 ? 1.63 : 1.74)));
+  ScoreSplit best = {nblocks, 1, 0};
+  // At most 16 CTAs per SM are of use; no fewer blocks per CTA than that gives.
+  const int64_t most = std::max<int64_t>(1, 16LL * sm_count / std::max<int64_t>(groups, 1));
+  for (int64_t per = (nblocks + most - 1) / most; per <= nblocks; per += 1 + per / 16) {
+    const int64_t slices = (nblocks + per - 1) / per;
+    const int64_t ctas = (groups * slices + sm_count - 1) / sm_count;
+    const double share = K == 1   ? (ctas == 1 ? 0.70 : (ctas == 2 ? 0.88 : 1.0))
+                         : ctas == 1 ? (K == 2 ? 0.95 : (K == 4 ? 0.97 : 1.0))
+                                     : 1.0;
+    const double cost = ((double)ctas * per / share + 0.25) * block;
+    if (best.cost == 0 || cost < best.cost) best = {per, slices, cost};
+  }
+  return best;
+}
+
 // Planes per thread of a call: forced, autotuned for its shape class, or the
 // default rule.
 static int choose_score_k(visacd_ctx* ctx, int32_t P, int64_t E) {
   if (ctx->score_k_override) return ctx->score_k_override;
   auto it = ctx->score_tuned.find(score_shape_class(P, E));
   if (it != ctx->score_tuned.end()) return it->second;
-  return planes_per_thread(P);
+  int best = 1;
+  double least = 0;
+  for (int k : {1, 2, 4, 8}) {
+    const double c = score_split(ctx->sm_count, P, E, k).cost;
+    if (least == 0 || c < least) {
+      least = c;
+      best = k;
+    }
+  }
+  return best;
 }
 
 static int planes_per_thread(int32_t P) {
@@ -260,16 +300,8 @@ static int launch_score(visacd_ctx* ctx, const float4* planes, int32_t P, const 
                         unsigned* rcount, unsigned rcap, unsigned* status) {
   const int per_cta = kScoreThreads * K;
   const int groups = (P + per_cta - 1) / per_cta;
-  const int64_t nblocks = (E + kEdgeBlock - 1) / kEdgeBlock;
-  // Aim for ~4 CTAs per SM in total (registers allow 4 resident for K = 2 and
-  // 2 for K = 4 and 8, so the edge slices keep every SM busy to the end); each
-  // CTA streams a contiguous run of blocks.
-  int64_t target_ctas = 4LL * ctx->sm_count;
-  int64_t slices = (target_ctas + groups - 1) / groups;
-  if (slices > nblocks) slices = nblocks;
-  if (slices < 1) slices = 1;
-  int64_t per = (nblocks + slices - 1) / slices;
-  slices = (nblocks + per - 1) / per;
+  const ScoreSplit split = score_split(ctx->sm_count, P, E, K);
+  const int64_t per = split.per, slices = split.slices;
   size_t smem = 2 * kEdgeBlock * sizeof(EdgeRec) + (size_t)K * kScoreThreads * 8;
   static bool configured[9] = {false};
   if (!configured[K]) {
