@@ -236,8 +236,6 @@ static uint32_t score_shape_class(int32_t P, int64_t E) {
   return (uint32_t)lg(P) | ((uint32_t)lg(E) << 8);
 }
 
-static int planes_per_thread(int32_t P);
-
 // How a call is split into CTAs: each takes 256 K planes and a run of `per` edge
 // blocks. The SM with the most CTAs ends last, so the cost is its CTAs times
 // their blocks, times what a block of K planes per thread costs (2^20 edges x
@@ -269,16 +267,12 @@ static ScoreSplit score_split(int sm_count, int32_t P, int64_t E, int K) {
   return best;
 }
 
-// Planes per thread of a call: forced, autotuned for its shape class, or the
-// default rule.
-static int choose_score_k(visacd_ctx* ctx, int32_t P, int64_t E) {
-  if (ctx->score_k_override) return ctx->score_k_override;
-  auto it = ctx->score_tuned.find(score_shape_class(P, E));
-  if (it != ctx->score_tuned.end()) return it->second;
+// The K of least cost.
+static int planes_per_thread(int sm_count, int32_t P, int64_t E) {
   int best = 1;
   double least = 0;
   for (int k : {1, 2, 4, 8}) {
-    const double c = score_split(ctx->sm_count, P, E, k).cost;
+    const double c = score_split(sm_count, P, E, k).cost;
     if (least == 0 || c < least) {
       least = c;
       best = k;
@@ -287,11 +281,13 @@ static int choose_score_k(visacd_ctx* ctx, int32_t P, int64_t E) {
   return best;
 }
 
-static int planes_per_thread(int32_t P) {
-  if (P > 4 * kScoreThreads * 152 / 2) return 8;
-  if (P > 2 * kScoreThreads * 4) return 4;
-  if (P > kScoreThreads * 2) return 2;
-  return 1;
+// Planes per thread of a call: forced, autotuned for its shape class, or the
+// default rule.
+static int choose_score_k(visacd_ctx* ctx, int32_t P, int64_t E) {
+  if (ctx->score_k_override) return ctx->score_k_override;
+  auto it = ctx->score_tuned.find(score_shape_class(P, E));
+  if (it != ctx->score_tuned.end()) return it->second;
+  return planes_per_thread(ctx->sm_count, P, E);
 }
 
 template <int K>
@@ -626,12 +622,8 @@ static int noalloc_launch_score(cudaStream_t st, int sm_count, const float4* pla
                                 unsigned* status) {
   const int per_cta = kScoreThreads * K;
   const int groups = (P + per_cta - 1) / per_cta;
-  const int64_t nblocks = (E + kEdgeBlock - 1) / kEdgeBlock;
-  int64_t slices = (4LL * sm_count + groups - 1) / groups;
-  if (slices > nblocks) slices = nblocks;
-  if (slices < 1) slices = 1;
-  int64_t per = (nblocks + slices - 1) / slices;
-  slices = (nblocks + per - 1) / per;
+  const ScoreSplit split = score_split(sm_count, P, E, K);
+  const int64_t per = split.per, slices = split.slices;
   size_t smem = 2 * kEdgeBlock * sizeof(EdgeRec) + (size_t)K * kScoreThreads * 8;
   VCUDA(cudaFuncSetAttribute(score_planes_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)smem));
@@ -684,7 +676,7 @@ extern "C" int visacd_score_planes_noalloc(const float* d_planes, int32_t P, con
     VCUDA(cudaGetLastError());
     const unsigned rcap = (unsigned)((int64_t)P * ((E + kEdgeBlock - 1) / kEdgeBlock));
     const float4* pl = reinterpret_cast<const float4*>(d_planes);
-    switch (planes_per_thread(P)) {
+    switch (planes_per_thread(sm, P, E)) {
       case 8: VTRY(noalloc_launch_score<8>(st, sm, pl, P, recs, E, cnt->stats, sq, rq, &cnt->recheck_count, rcap, status)); break;
       case 4: VTRY(noalloc_launch_score<4>(st, sm, pl, P, recs, E, cnt->stats, sq, rq, &cnt->recheck_count, rcap, status)); break;
       case 2: VTRY(noalloc_launch_score<2>(st, sm, pl, P, recs, E, cnt->stats, sq, rq, &cnt->recheck_count, rcap, status)); break;
