@@ -330,6 +330,11 @@ __global__ void __launch_bounds__(128) sdf_ub_kernel(SdfItems W, SdfGrid g, cons
   }
 }
 
+// Resident blocks per SM of the two passes, and their grids: one wave, since every
+// warp has its share of the items from the start (with 8 blocks per SM of which 5
+// are resident, 1.6 waves, the exact pass took 24 us more).
+constexpr int kDistBlocks = 6, kUbBlocks = 9;
+
 // The (triangle, voxel) pairs that the lower bound leaves, kept per warp over
 // all of its items and evaluated in FP64 32 at a time: the FP64 pipe, slow on
 // this part, runs with full warps, and no warp waits for another. 20,480
@@ -371,7 +376,7 @@ __device__ __forceinline__ void queue_pairs(PairQueue& Q, int& n, bool keep, int
   }
 }
 
-__global__ void __launch_bounds__(128) sdf_dist_kernel(const double* __restrict__ P, const int32_t* __restrict__ T,
+__global__ void __launch_bounds__(128, kDistBlocks) sdf_dist_kernel(const double* __restrict__ P, const int32_t* __restrict__ T,
                                                        SdfItems W, SdfGrid g, const SdfTri* __restrict__ prep,
                                                        const uint8_t* __restrict__ cls, const uint32_t* __restrict__ ub,
                                                        uint32_t* __restrict__ dist) {
@@ -926,9 +931,9 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   SdfItems items;
   items.off = chunk_off;
   items.nt = nt;
-  const unsigned gw = (unsigned)(8 * (int64_t)ctx->sm_count);
+  const unsigned gw = (unsigned)(kDistBlocks * (int64_t)ctx->sm_count);
   // First pass: FP32 upper bounds per voxel, then the exact pass.
-  VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_ub_kernel, items, g, (const SdfTri*)prep, (const uint8_t*)cls, ub);
+  VLAUNCH(ctx, kKSdfDist, (unsigned)(kUbBlocks * (int64_t)ctx->sm_count), 128, 0, sdf_ub_kernel, items, g, (const SdfTri*)prep, (const uint8_t*)cls, ub);
   VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_dist_kernel, dP, dT, items, g, (const SdfTri*)prep, (const uint8_t*)cls,
           (const uint32_t*)ub, dist);
   if (g.reach < g.band) {
