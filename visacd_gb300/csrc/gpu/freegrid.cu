@@ -111,9 +111,20 @@ __global__ void fg_near_kernel(const float4* __restrict__ tris, int32_t nt, FgPa
     }
     const int sx = c1[0] - c0[0] + 1, sy = c1[1] - c0[1] + 1, sz = c1[2] - c0[2] + 1;
     if (sx <= 0 || sy <= 0 || sz <= 0) continue;
+    // 32 cells at a time, x fastest, stepped with carries (three divisions a cell
+    // cost as much as the bound).
     const int total = sx * sy * sz;
+    const int stx = 32 % sx, sty = (32 / sx) % sy, stz = 32 / (sx * sy);
+    int rx = lane % sx, ry = (lane / sx) % sy, rz = lane / (sx * sy);
     for (int k = lane; k < total; k += 32) {
-      const int ix = c0[0] + k % sx, iy = c0[1] + (k / sx) % sy, iz = c0[2] + k / (sx * sy);
+      const int ix = c0[0] + rx, iy = c0[1] + ry, iz = c0[2] + rz;
+      rx += stx;
+      const int cx = rx >= sx;
+      rx -= cx ? sx : 0;
+      ry += sty + cx;
+      const int cy = ry >= sy;
+      ry -= cy ? sy : 0;
+      rz += stz + cy;
       // The centre exactly as the walk computes it.
       const float x = __fadd_rn(g.ox, __fmul_rn((float)ix + 0.5f, g.h));
       const float y = __fadd_rn(g.oy, __fmul_rn((float)iy + 0.5f, g.h));
