@@ -98,7 +98,7 @@ __device__ __forceinline__ float cell_reach(const FreeGridView& g, float px, flo
 }
 
 // The free ends of the segment p -> q (as trace_free) from the table.
-__device__ __forceinline__ void cone_start(const FreeReach& T, int64_t rp, int64_t rq, float dx, float dy, float dz,
+__device__ __forceinline__ void cone_start(const FreeReach& T, uint32_t rp, uint32_t rq, float dx, float dy, float dz,
                                            float& t0, float& s0) {
   const float ax = fabsf(dx), ay = fabsf(dy), az = fabsf(dz);
   const int axis = ax >= ay ? (ax >= az ? 0 : 2) : (ay >= az ? 1 : 2);
@@ -108,16 +108,19 @@ __device__ __forceinline__ void cone_start(const FreeReach& T, int64_t rp, int64
   const float len = fabsf(da);
   t0 = 0.f;
   s0 = 1.f;
-  if (!(len > 1e-30f)) return;
-  const float inv = __frcp_rd(__fmul_ru(len, 1.000001f));
+  if (!(len > 1e-30f && len < 1e30f)) return;
+  // Below 1 / len: the factor is eight times the hardware reciprocal's error.
+  float inv;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(inv) : "f"(len * 1.000001f));
   const int m = T.m, top = m - 1;
   const float half = 0.5f * (float)m;
   const int iu = min(max((int)(fmaf(db, inv, 1.f) * half), 0), top);
   const int iv = min(max((int)(fmaf(dc, inv, 1.f) * half), 0), top);
   const int face = 2 * axis + (da < 0.f ? 1 : 0);
   const int cp = (face * m + iv) * m + iu, cq = ((face ^ 1) * m + (top - iv)) * m + (top - iu);
-  t0 = __fmul_rd(T.reach[(int64_t)cp * T.n + rp], inv);
-  s0 = __fsub_ru(1.f, __fmul_rd(T.reach[(int64_t)cq * T.n + rq], inv));
+  // (at most 2^28 entries)
+  t0 = __fmul_rd(T.reach[(uint32_t)cp * (uint32_t)T.n + rp], inv);
+  s0 = __fsub_ru(1.f, __fmul_rd(T.reach[(uint32_t)cq * (uint32_t)T.n + rq], inv));
 }
 
 

@@ -215,17 +215,18 @@ __device__ __forceinline__ void walk_tiles(const VisParams& P, unsigned long lon
       ++sum.pairs;
       const float dx = __fsub_rn(P.pts[3 * (int64_t)oj], px), dy = __fsub_rn(P.pts[3 * (int64_t)oj + 1], py),
                   dz = __fsub_rn(P.pts[3 * (int64_t)oj + 2], pz);
-      const float len = seg_length(dx, dy, dz);
-      if (!(len > 0.f)) {  // coincident endpoints (or NaN): never an edge (as in vis_tile)
+      // The square of seg_length, which is positive when its root is.
+      const float sq = __fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz));
+      if (!(sq > 0.f)) {  // coincident endpoints (or NaN): never an edge (as in vis_tile)
         ++sum.deg;
       } else {
         float t0 = 0.f, s0 = 1.f;
         if (P.cage_reach.reach != nullptr) {
           const bool pos = P.cage_reach.by_pos != 0;
-          cone_start(P.cage_reach, pos ? a : (int64_t)oi, pos ? b : (int64_t)oj, dx, dy, dz, t0, s0);
+          cone_start(P.cage_reach, pos ? (uint32_t)a : oi, pos ? (uint32_t)b : oj, dx, dy, dz, t0, s0);
         }
         done = t0 >= s0 || (P.cage_free.lb != nullptr &&
-                            trace_free(P.cage_free, px, py, pz, dx, dy, dz, len, t0, s0, sum.steps));
+                            trace_free(P.cage_free, px, py, pz, dx, dy, dz, __fsqrt_rn(sq), t0, s0, sum.steps));
         sum.cleared += done;
       }
     }
