@@ -88,7 +88,7 @@ typedef struct {
 typedef struct {
   int32_t quantum_exp;    /* edge lengths are summed in units of 2^quantum_exp */
   int32_t argmax;         /* first plane with the maximum score, -1 if P == 0 */
-  int64_t band_blocks;    /* (plane, edge block) pairs re-decided in FP64 */
+  int64_t band_blocks;    /* (plane, edge block) or (vertex, 32 planes) pairs with FP64 decisions */
   int64_t skipped_edges;  /* edges with an out-of-range index or non-finite endpoint */
 } visacd_score_stats;
 

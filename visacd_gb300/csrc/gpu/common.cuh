@@ -220,6 +220,7 @@ enum KernelId {
   kKGridFinal,
   kKVisWalk,
   kKVisReach,
+  kKPlaneSides,
   kKConvexHull,
   kKMisc,
   kKCount

@@ -22,6 +22,9 @@
 //    score_recheck re-decides its band pairs in FP64 — the same FP64
 //    evaluation the oracle uses — so classification equals the FP64 oracle's.
 //  * Sums are integers (order independent), so scores are deterministic.
+//  * Calls with no fewer edges than vertices (visibility edges: 2 to 20 per vertex)
+//    decide each vertex's side of each plane once instead of twice per edge
+//    (plane_sides, score_sides below); the sums are the same integers.
 #include <cstring>
 #include <vector>
 
@@ -225,10 +228,221 @@ struct ScoreCounters {
   unsigned stats[4];                 // max |x|, |y|, |z| (float bits)
   unsigned recheck_count;
   unsigned status;                   // this call's kStatus* bits
-  unsigned pad0[2];
+  unsigned sides_fp64;               // (vertex, 32 planes) groups decided in FP64
+  unsigned pad0;
   unsigned long long skipped;
   int argmax[2];                     // argmax, qexp
 };
+
+// Edges over few vertices. A vertex's side of a plane is the same for all of its
+// edges, so plane_sides_kernel decides it once per (plane, vertex), two bits in words
+// of 32 planes; a value in its rounding band is decided in FP64 there. A CTA of
+// score_sides_kernel keeps one word's sides of all vertices in shared memory. A
+// lane gets its edge's 32 crossings with two logic operations from its two vertices'
+// words; the warp transposes its 32 x 32 bits, so that a lane holds its plane's
+// crossings of 32 edges, and adds up the lengths four edges at a time from tables of
+// the 16 sums that the warp writes for them (the 16 words lie in different banks). Per
+// (plane, edge) that is some 2.3 instructions against ten of score_planes_kernel. Bound by
+// integer issue. Both kernels, against the best K of score_planes_kernel with its
+// re-decision: 59,183 edges x 2,500 planes over 2,562 vertices 80 -> 35 us, 33,370 x
+// 2,500 over 10,242 54 -> 35, 262,144 x 4,096 over 10,242 422 -> 137, 2^20 x 4,096
+// over 24,576 1,647 -> 524. The lane's own plane tested in every edge's word (a
+// broadcast load, a bit test and a predicated add per pair) took 735 for the last,
+// and a CTA that decided its vertices' sides itself 603.
+constexpr int kSidesThreads = 512;
+constexpr int kSidesWarps = kSidesThreads / 32;
+constexpr int kSidesMaxVertices = 24576;  // 192 KB of sides; indices fit 15 bits
+constexpr int64_t kSidesMaxScratch = 1LL << 25;  // groups of 32 planes x vertices: 256 MB
+
+static __global__ void pack_sides_kernel(const float* __restrict__ pts, int32_t n,
+                                         const uint32_t* __restrict__ edges, int64_t E,
+                                         const unsigned* __restrict__ stats, uint32_t* __restrict__ ends,
+                                         uint32_t* __restrict__ lens, unsigned long long* __restrict__ skipped) {
+  const int qexp = quantum_exp_from_cmax_bits(max(stats[0], max(stats[1], stats[2])));
+  unsigned long long nskip = 0;
+  const int64_t padded = (E + 31) & ~31ll;
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < padded;
+       e += (int64_t)gridDim.x * blockDim.x) {
+    const uint2 ij = e < E ? reinterpret_cast<const uint2*>(edges)[e] : make_uint2(0u, 0u);
+    EdgeRec r;
+    const bool ok = edge_record(pts, n, ij, qexp, r) && e < E;
+    ends[e] = ok ? ij.x | (ij.y << 16) : 0u;
+    lens[e] = ok ? r.q : 0u;
+    nskip += e < E && !ok;
+  }
+#pragma unroll
+  for (int o = 16; o; o >>= 1) nskip += __shfl_xor_sync(0xffffffffu, nskip, o);
+  if ((threadIdx.x & 31) == 0 && nskip) atomicAdd(skipped, nskip);
+}
+
+// The sides of two vertices per thread for 32 planes: side[group][vertex] = {above
+// eps, below -eps}, plane k at bit 31 - k. Four FP32 operations and 2.5 integer ones
+// per (plane, vertex).
+constexpr int kSideThreads = 256;
+static __global__ void __launch_bounds__(kSideThreads)
+    plane_sides_kernel(const float4* __restrict__ planes, int32_t P, const float* __restrict__ pts,
+                       int32_t n, int32_t pitch, const unsigned* __restrict__ stats,
+                       uint2* __restrict__ side, unsigned* __restrict__ fp64_groups) {
+  __shared__ float4 pl[32];
+  __shared__ __align__(8) float th[32];  // eps + B
+  __shared__ float width[32];            // the band's width
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int p0 = blockIdx.y * 32;
+  if (tid < 32) {
+    // A plane with a NaN and those past the last: one that has every vertex above it.
+    float4 q = p0 + tid < P ? planes[p0 + tid] : make_float4(0.f, 0.f, 0.f, 1.f);
+    if (isnan(q.x) || isnan(q.y) || isnan(q.z) || isnan(q.w)) q = make_float4(0.f, 0.f, 0.f, 1.f);
+    pl[tid] = q;
+    float nlo, nhi;
+    plane_thresholds(q, stats, nlo, nhi);
+    // Finite coefficients whose bound overflows: every value is decided in FP64.
+    const bool over = isinf(nhi) && isfinite(q.x) && isfinite(q.y) && isfinite(q.z) && isfinite(q.w);
+    th[tid] = -nhi;
+    width[tid] = over ? __int_as_float(-1) : __fsub_rn(-nhi, -nlo);
+  }
+  const int i0 = blockIdx.x * (2 * kSideThreads) + tid;
+  const int i[2] = {min(i0, n - 1), min(i0 + kSideThreads, n - 1)};
+  float x[2], y[2], z[2];
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    x[j] = pts[3 * i[j]];
+    y[j] = pts[3 * i[j] + 1];
+    z[j] = pts[3 * i[j] + 2];
+  }
+  __syncthreads();
+  // The band test is score_planes_kernel's: with d = th - |v|, d < 0 is a certain
+  // side, and d's bits up to those of the band's width need FP64; here the smallest
+  // d of a vertex is held against the widest band of the 32 planes first.
+  const uint32_t widest = __reduce_max_sync(0xffffffffu, __float_as_uint(width[lane]));
+  uint32_t certain[2] = {0, 0}, sign[2] = {0, 0}, dmin[2] = {0xffffffffu, 0xffffffffu};
+#pragma unroll 4
+  for (int k = 0; k < 32; k += 2) {
+    const float4 q0 = pl[k], q1 = pl[k + 1];
+    const float2 t = *reinterpret_cast<const float2*>(&th[k]);
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float v0 = fmaf(q0.x, x[j], fmaf(q0.y, y[j], fmaf(q0.z, z[j], q0.w)));
+      const float v1 = fmaf(q1.x, x[j], fmaf(q1.y, y[j], fmaf(q1.z, z[j], q1.w)));
+      const uint32_t d0 = __float_as_uint(__fsub_rn(t.x, fabsf(v0)));
+      const uint32_t d1 = __float_as_uint(__fsub_rn(t.y, fabsf(v1)));
+      certain[j] = __funnelshift_l(d1, __funnelshift_l(d0, certain[j], 1), 1);
+      sign[j] = __funnelshift_l(__float_as_uint(v1), __funnelshift_l(__float_as_uint(v0), sign[j], 1), 1);
+      dmin[j] = __vimin3_u32(dmin[j], d0, d1);
+    }
+  }
+  unsigned groups = 0;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    if (i0 + j * kSideThreads >= n) continue;
+    uint32_t above = certain[j] & ~sign[j], below = certain[j] & sign[j];
+    if (dmin[j] <= widest) {
+      ++groups;
+      for (int k = 0; k < 32; ++k) {
+        const float4 q = pl[k];
+        const float v = fmaf(q.x, x[j], fmaf(q.y, y[j], fmaf(q.z, z[j], q.w)));
+        if (__float_as_uint(__fsub_rn(th[k], fabsf(v))) <= __float_as_uint(width[k])) {
+          const double w = side_value64(q, x[j], y[j], z[j]), eps = (double)kSideEps;
+          const uint32_t m = 0x80000000u >> k;
+          above = w > eps ? above | m : above & ~m;
+          below = w < -eps ? below | m : below & ~m;
+        }
+      }
+    }
+    side[(int64_t)blockIdx.y * pitch + i[j]] = make_uint2(above, below);
+  }
+  groups = __reduce_add_sync(0xffffffffu, groups);
+  if (lane == 0 && groups) atomicAdd(fp64_groups, groups);
+}
+
+static __global__ void __launch_bounds__(kSidesThreads, 2)
+    score_sides_kernel(const uint2* __restrict__ sides, int32_t pitch, int32_t P,
+                       const uint32_t* __restrict__ ends, const uint32_t* __restrict__ lens, int64_t E,
+                       unsigned long long* __restrict__ score_q, unsigned* __restrict__ status) {
+  extern __shared__ __align__(128) unsigned char smem_raw[];
+  uint2* side = reinterpret_cast<uint2*>(smem_raw);           // pitch x {above, below}
+  __shared__ __align__(512) uint32_t sums[kSidesWarps][128];  // 8 x 16 sums of four lengths
+  __shared__ unsigned long long part[kSidesWarps][32];
+  __shared__ __align__(8) uint64_t bar;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int p0 = blockIdx.y * 32;
+  if (tid == 0) {
+    mbar_init(&bar, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    bulk_load(side, sides + (int64_t)blockIdx.y * pitch, (unsigned)(pitch * sizeof(uint2)), &bar);
+  }
+  __syncthreads();
+  if (__syncthreads_or(!mbar_wait(&bar, 0))) {
+    if (tid == 0) atomicOr(status, kStatusMbarrierTimeout);
+    return;
+  }
+  // Transposition: in the step of distance 2^k a lane keeps half of its bits and
+  // takes the other half from its partner, moved by 2^k.
+  const uint32_t half[5] = {0x55555555u, 0x33333333u, 0x0f0f0f0fu, 0x00ff00ffu, 0x0000ffffu};
+  uint32_t keep[5];
+#pragma unroll
+  for (int k = 0; k < 5; ++k) keep[k] = (lane >> k & 1) ? ~half[k] : half[k];
+  const uint32_t table = smem_u32(&sums[warp][0]);
+  const int64_t step = (int64_t)gridDim.x * kSidesWarps * 32;
+  int64_t e = ((int64_t)blockIdx.x * kSidesWarps + warp) * 32;
+  uint32_t ij = 0;
+  uint4 q = make_uint4(0, 0, 0, 0);
+  if (e < E) {
+    ij = ends[e + lane];
+    q = reinterpret_cast<const uint4*>(lens + e)[lane >> 2];
+  }
+  unsigned long long sum = 0;
+  for (; e < E; e += step) {
+    const uint2 s = side[ij & 0xffffu], t = side[ij >> 16];
+    uint32_t x = (s.x & t.y) | (s.y & t.x);
+    const uint32_t base = ((lane & 1) ? q.z : 0u) + ((lane & 2) ? q.w : 0u);
+    reinterpret_cast<uint4*>(&sums[warp][0])[lane] =
+        make_uint4(base, base + q.x, base + q.y, base + q.x + q.y);
+    if (e + step < E) {
+      ij = ends[e + step + lane];
+      q = reinterpret_cast<const uint4*>(lens + e + step)[lane >> 2];
+    }
+#pragma unroll
+    for (int k = 4; k >= 0; --k) {
+      const uint32_t y = __shfl_xor_sync(0xffffffffu, x, 1 << k);
+      const uint32_t m = __funnelshift_l(y, y, (lane >> k & 1) ? 32 - (1 << k) : 1 << k);
+      x = (x & keep[k]) | (m & ~keep[k]);
+    }
+    __syncwarp();
+    uint32_t add[8];
+#pragma unroll
+    for (int g = 0; g < 8; ++g) {
+      const uint32_t at = ((g ? x >> (4 * g - 2) : x << 2) & 0x3cu) | table;
+      asm volatile("ld.shared.u32 %0, [%1];" : "=r"(add[g]) : "r"(at + 64 * g) : "memory");
+    }
+    sum += ((add[0] + add[1]) + (add[2] + add[3])) + ((add[4] + add[5]) + (add[6] + add[7]));
+    __syncwarp();
+  }
+  part[warp][lane] = sum;
+  __syncthreads();
+  if (tid < 32 && p0 + 31 - tid < P) {  // plane k at bit 31 - k
+    for (int w = 1; w < kSidesWarps; ++w) sum += part[w][tid];
+    if (sum) atomicAdd(&score_q[p0 + 31 - tid], sum);
+  }
+}
+
+// Slices of the edges per group of 32 planes: the SM with the most CTAs ends last,
+// and each CTA loads the sides of all n vertices. In cycles of an SM: 2,500 a CTA,
+// 0.13 a vertex (64 bytes a cycle), 1.35 an edge (5.4 per 32 planes on each of the
+// four schedulers).
+static int sides_slices(int sm_count, int32_t P, int32_t n, int64_t E) {
+  const int64_t groups = (P + 31) / 32;
+  const int64_t most = (E + kSidesThreads - 1) / kSidesThreads;
+  int best = 1;
+  double least = 0;
+  for (int s = 1; s <= 64 && s <= most; ++s) {
+    const double c = (double)((groups * s + sm_count - 1) / sm_count) * (2500.0 + 0.13 * n + 1.35 * (double)E / s);
+    if (least == 0 || c < least) {
+      least = c;
+      best = s;
+    }
+  }
+  return best;
+}
 
 // Shape class of a scoring call: log2 buckets of P and E.
 static uint32_t score_shape_class(int32_t P, int64_t E) {
@@ -311,7 +525,16 @@ static int launch_score(visacd_ctx* ctx, const float4* planes, int32_t P, const 
   return VISACD_OK;
 }
 
-// Core of every scoring entry point. All pointers are device pointers.
+// Whether the sides of the vertices are decided first. At one edge per vertex both
+// ways are equal for many planes (24,576 edges x 2,500 planes 44.9 and 44.9 us, x
+// 4,096 58.1 and 60.8) and this one ahead for few (x 80 16.0 against 21.4; 642 edges
+// 12.0 and 17.3); at two it is 1.3 times as fast. More vertices than shared memory
+// holds, or more sides than the scratch limit, go edge by edge.
+static bool sides_pay(int32_t P, int32_t N, int64_t E) {
+  return N > 0 && N <= kSidesMaxVertices && E >= N && (P + 31LL) / 32 * N <= kSidesMaxScratch;
+}
+
+// Core of every scoring entry point that may allocate. All pointers are device pointers.
 static int score_device(visacd_ctx* ctx, const float* d_planes, int32_t P, const float* d_pts,
                         int32_t N, const uint32_t* d_edges, int64_t E, double* d_scores,
                         float* d_scores_f32, ScoreCounters** d_counters_out, unsigned rcap) {
@@ -326,7 +549,27 @@ static int score_device(visacd_ctx* ctx, const float* d_planes, int32_t P, const
     VLAUNCH(ctx, kKPointStats, grid_for(N, 256, 4LL * ctx->sm_count), 256, 0, point_stats_kernel,
             d_pts, N, cnt->stats);
   }
-  if (E > 0 && P > 0) {
+  if (E > 0 && P > 0 && !ctx->score_k_override && sides_pay(P, N, E)) {
+    const size_t padded = (size_t)((E + 31) & ~31ll);
+    VTRY(ensure_slot(ctx, kSlotEdgePack, padded * 8));
+    uint32_t* ends = slot<uint32_t>(ctx, kSlotEdgePack);
+    uint32_t* lens = ends + padded;
+    VLAUNCH(ctx, kKPackEdges, grid_for(E, 256, 8LL * ctx->sm_count), 256, 0, pack_sides_kernel,
+            d_pts, N, d_edges, E, cnt->stats, ends, lens, &cnt->skipped);
+    const int32_t pitch = (N + 1) & ~1;  // a group's row starts and ends on 16 bytes
+    const unsigned groups = (unsigned)((P + 31) / 32);
+    const float4* pl = reinterpret_cast<const float4*>(d_planes);
+    VTRY(ensure_slot(ctx, kSlotRecheck, (size_t)groups * pitch * sizeof(uint2)));
+    uint2* sides = slot<uint2>(ctx, kSlotRecheck);
+    VLAUNCH(ctx, kKPlaneSides, dim3((unsigned)((N + 2 * kSideThreads - 1) / (2 * kSideThreads)), groups),
+            kSideThreads, 0, plane_sides_kernel, pl, P, d_pts, N, pitch, cnt->stats, sides, &cnt->sides_fp64);
+    const size_t smem = (size_t)pitch * sizeof(uint2);
+    if (smem > 32768)  // beside the static part, past what needs no attribute
+      VCUDA(cudaFuncSetAttribute(score_sides_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kSidesMaxVertices * (int)sizeof(uint2)));
+    VLAUNCH(ctx, kKScore, dim3((unsigned)sides_slices(ctx->sm_count, P, N, E), groups), kSidesThreads, smem,
+            score_sides_kernel, sides, pitch, P, ends, lens, E, sq, &cnt->status);
+  } else if (E > 0 && P > 0) {
     VTRY(ensure_slot(ctx, kSlotEdgePack, (size_t)E * sizeof(EdgeRec)));
     EdgeRec* recs = slot<EdgeRec>(ctx, kSlotEdgePack);
     VLAUNCH(ctx, kKPackEdges, grid_for(E, 256, 8LL * ctx->sm_count), 256, 0, pack_edges_kernel,
@@ -438,7 +681,7 @@ int score_planes_impl(visacd_ctx* ctx, const float* planes, int32_t P, const flo
     if (stats) {
       stats->quantum_exp = hc.argmax[1];
       stats->argmax = hc.argmax[0];
-      stats->band_blocks = hc.recheck_count;
+      stats->band_blocks = (int64_t)hc.recheck_count + hc.sides_fp64;
       stats->skipped_edges = (int64_t)hc.skipped;
     }
   }

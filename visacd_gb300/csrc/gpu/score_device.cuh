@@ -79,6 +79,34 @@ __device__ __forceinline__ float edge_len32(float dx, float dy, float dz) {
   return __fsqrt_rn(s);
 }
 
+// An edge's record; false (a record of zeros) for one with an index out of range or
+// an endpoint that is not finite.
+__device__ __forceinline__ bool edge_record(const float* __restrict__ pts, int32_t n, uint2 ij,
+                                            int qexp, EdgeRec& r) {
+  r.pad = 0;
+  bool ok = ij.x < (uint32_t)n && ij.y < (uint32_t)n;
+  float x1 = 0, y1 = 0, z1 = 0, x2 = 0, y2 = 0, z2 = 0;
+  if (ok) {
+    x1 = pts[3 * (int64_t)ij.x];
+    y1 = pts[3 * (int64_t)ij.x + 1];
+    z1 = pts[3 * (int64_t)ij.x + 2];
+    x2 = pts[3 * (int64_t)ij.y];
+    y2 = pts[3 * (int64_t)ij.y + 1];
+    z2 = pts[3 * (int64_t)ij.y + 2];
+    ok = isfinite(x1) && isfinite(y1) && isfinite(z1) && isfinite(x2) && isfinite(y2) &&
+         isfinite(z2);
+  }
+  if (ok) {
+    float len = edge_len32(__fsub_rn(x2, x1), __fsub_rn(y2, y1), __fsub_rn(z2, z1));
+    r.x1 = x1; r.x2 = x2; r.y1 = y1; r.y2 = y2; r.z1 = z1; r.z2 = z2;
+    r.q = __float2uint_rn(ldexpf(len, -qexp));
+  } else {
+    r.x1 = r.x2 = r.y1 = r.y2 = r.z1 = r.z2 = 0.f;
+    r.q = 0;
+  }
+  return ok;
+}
+
 static __global__ void pack_edges_kernel(const float* __restrict__ pts, int32_t n,
                                   const uint32_t* __restrict__ edges, int64_t E,
                                   const unsigned* __restrict__ stats, EdgeRec* __restrict__ out,
@@ -88,30 +116,8 @@ static __global__ void pack_edges_kernel(const float* __restrict__ pts, int32_t 
   unsigned long long nskip = 0;
   for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < E;
        e += (int64_t)gridDim.x * blockDim.x) {
-    uint2 ij = reinterpret_cast<const uint2*>(edges)[e];
     EdgeRec r;
-    r.pad = 0;
-    bool ok = ij.x < (uint32_t)n && ij.y < (uint32_t)n;
-    float x1 = 0, y1 = 0, z1 = 0, x2 = 0, y2 = 0, z2 = 0;
-    if (ok) {
-      x1 = pts[3 * (int64_t)ij.x];
-      y1 = pts[3 * (int64_t)ij.x + 1];
-      z1 = pts[3 * (int64_t)ij.x + 2];
-      x2 = pts[3 * (int64_t)ij.y];
-      y2 = pts[3 * (int64_t)ij.y + 1];
-      z2 = pts[3 * (int64_t)ij.y + 2];
-      ok = isfinite(x1) && isfinite(y1) && isfinite(z1) && isfinite(x2) && isfinite(y2) &&
-           isfinite(z2);
-    }
-    if (ok) {
-      float len = edge_len32(__fsub_rn(x2, x1), __fsub_rn(y2, y1), __fsub_rn(z2, z1));
-      r.x1 = x1; r.x2 = x2; r.y1 = y1; r.y2 = y2; r.z1 = z1; r.z2 = z2;
-      r.q = __float2uint_rn(ldexpf(len, -qexp));
-    } else {
-      r.x1 = r.x2 = r.y1 = r.y2 = r.z1 = r.z2 = 0.f;
-      r.q = 0;
-      ++nskip;
-    }
+    if (!edge_record(pts, n, reinterpret_cast<const uint2*>(edges)[e], qexp, r)) ++nskip;
     out[e] = r;
   }
 #pragma unroll
