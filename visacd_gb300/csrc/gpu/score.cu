@@ -188,12 +188,14 @@ __global__ void score_finish_kernel(const unsigned long long* __restrict__ score
                                     float* __restrict__ out_f32, int* __restrict__ argmax) {
   unsigned cmax = max(stats[0], max(stats[1], stats[2]));
   int qexp = quantum_exp_from_cmax_bits(cmax);
+  const double unit = ldexp(1.0, qexp);  // the product with it is exact
   const bool lost = (*status & (kStatusMbarrierTimeout | kStatusRecheckOverflow)) != 0u;
   unsigned long long best = 0;
   int best_i = P > 0 ? 0 : -1;
+#pragma unroll 4
   for (int p = threadIdx.x; p < P; p += blockDim.x) {
     unsigned long long v = score_q[p];
-    double s = lost ? __longlong_as_double(0x7ff8000000000000ll) : ldexp((double)v, qexp);
+    double s = lost ? __longlong_as_double(0x7ff8000000000000ll) : (double)v * unit;
     if (out) out[p] = s;
     if (out_f32) out_f32[p] = (float)s;
     if (v > best || (v == best && p < best_i)) {
@@ -201,24 +203,30 @@ __global__ void score_finish_kernel(const unsigned long long* __restrict__ score
       best_i = p;
     }
   }
-  __shared__ unsigned long long sv[1024];
-  __shared__ int si[1024];
-  sv[threadIdx.x] = best;
-  si[threadIdx.x] = best_i;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o; o >>= 1) {
-    if ((int)threadIdx.x < o) {
-      unsigned long long v2 = sv[threadIdx.x + o];
-      int i2 = si[threadIdx.x + o];
-      if (v2 > sv[threadIdx.x] || (v2 == sv[threadIdx.x] && i2 >= 0 && i2 < si[threadIdx.x])) {
-        sv[threadIdx.x] = v2;
-        si[threadIdx.x] = i2;
+  __shared__ unsigned long long sv[32];
+  __shared__ int si[32];
+  for (int pass = 0; pass < 2; ++pass) {
+#pragma unroll
+    for (int o = 16; o; o >>= 1) {
+      const unsigned long long v2 = __shfl_xor_sync(0xffffffffu, best, o);
+      const int i2 = __shfl_xor_sync(0xffffffffu, best_i, o);
+      if (v2 > best || (v2 == best && i2 < best_i)) {
+        best = v2;
+        best_i = i2;
       }
     }
+    if (pass == 1) break;
+    if ((threadIdx.x & 31) == 0) {
+      sv[threadIdx.x >> 5] = best;
+      si[threadIdx.x >> 5] = best_i;
+    }
     __syncthreads();
+    if (threadIdx.x >= 32) return;
+    best = sv[threadIdx.x];
+    best_i = si[threadIdx.x];
   }
   if (threadIdx.x == 0) {
-    argmax[0] = lost ? -2 : si[0];
+    argmax[0] = lost ? -2 : best_i;
     argmax[1] = qexp;
   }
 }
@@ -279,6 +287,15 @@ static __global__ void pack_sides_kernel(const float* __restrict__ pts, int32_t 
 // eps, below -eps}, plane k at bit 31 - k. Four FP32 operations and 2.5 integer ones
 // per (plane, vertex).
 constexpr int kSideThreads = 256;
+constexpr int kSideQueue = 2048;
+
+// Plane k's two bits of a vertex, by FP64.
+__device__ __forceinline__ uint2 decide_side(uint2 w, float4 q, int k, float x, float y, float z) {
+  const double v = side_value64(q, x, y, z), eps = (double)kSideEps;
+  const uint32_t m = 0x80000000u >> k;
+  return make_uint2(v > eps ? w.x | m : w.x & ~m, v < -eps ? w.y | m : w.y & ~m);
+}
+
 static __global__ void __launch_bounds__(kSideThreads)
     plane_sides_kernel(const float4* __restrict__ planes, int32_t P, const float* __restrict__ pts,
                        int32_t n, int32_t pitch, const unsigned* __restrict__ stats,
@@ -286,7 +303,11 @@ static __global__ void __launch_bounds__(kSideThreads)
   __shared__ float4 pl[32];
   __shared__ __align__(8) float th[32];  // eps + B
   __shared__ float width[32];            // the band's width
+  __shared__ uint2 word[2 * kSideThreads];
+  __shared__ uint16_t queue[kSideQueue];
+  __shared__ unsigned queued;
   const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) queued = 0u;
   const int p0 = blockIdx.y * 32;
   if (tid < 32) {
     // A plane with a NaN and those past the last: one that has every vertex above it.
@@ -330,26 +351,48 @@ static __global__ void __launch_bounds__(kSideThreads)
       dmin[j] = __vimin3_u32(dmin[j], d0, d1);
     }
   }
+  // Band values go to a queue, so that full warps decide them in FP64; one that the
+  // queue cannot take is decided by its own lane. A plane through vertices has
+  // several, and lane by lane each cost its warp an FP64 chain: 2,562 vertices x 592
+  // planes through edges 12.4 us, 7.0 with the queue.
   unsigned groups = 0;
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
-    if (i0 + j * kSideThreads >= n) continue;
+    const int il = tid + j * kSideThreads;
     uint32_t above = certain[j] & ~sign[j], below = certain[j] & sign[j];
-    if (dmin[j] <= widest) {
-      ++groups;
-      for (int k = 0; k < 32; ++k) {
-        const float4 q = pl[k];
-        const float v = fmaf(q.x, x[j], fmaf(q.y, y[j], fmaf(q.z, z[j], q.w)));
-        if (__float_as_uint(__fsub_rn(th[k], fabsf(v))) <= __float_as_uint(width[k])) {
-          const double w = side_value64(q, x[j], y[j], z[j]), eps = (double)kSideEps;
-          const uint32_t m = 0x80000000u >> k;
-          above = w > eps ? above | m : above & ~m;
-          below = w < -eps ? below | m : below & ~m;
-        }
-      }
+    word[il] = make_uint2(above, below);
+    if (dmin[j] > widest || i0 + j * kSideThreads >= n) continue;
+    ++groups;
+#pragma unroll 4
+    for (int k = 0; k < 32; ++k) {
+      const float4 q = pl[k];
+      const float v = fmaf(q.x, x[j], fmaf(q.y, y[j], fmaf(q.z, z[j], q.w)));
+      if (__float_as_uint(__fsub_rn(th[k], fabsf(v))) > __float_as_uint(width[k])) continue;
+      const unsigned at = atomicAdd(&queued, 1u);
+      if (at < kSideQueue)
+        queue[at] = (uint16_t)(il << 5 | k);
+      else
+        word[il] = decide_side(word[il], q, k, x[j], y[j], z[j]);
     }
-    side[(int64_t)blockIdx.y * pitch + i[j]] = make_uint2(above, below);
   }
+  __syncthreads();
+  const unsigned m = min(queued, (unsigned)kSideQueue);
+  for (unsigned r = tid; r < m; r += kSideThreads) {
+    const int il = queue[r] >> 5, k = queue[r] & 31;
+    const float* p = pts + 3 * (int64_t)(blockIdx.x * (2 * kSideThreads) + il);
+    const uint2 w = decide_side(make_uint2(0u, 0u), pl[k], k, p[0], p[1], p[2]);
+    const uint32_t keep = ~(0x80000000u >> k);
+    // A band value's bits are clear unless its FP32 side counted as certain.
+    atomicAnd(&word[il].x, keep | w.x);
+    atomicAnd(&word[il].y, keep | w.y);
+    if (w.x) atomicOr(&word[il].x, w.x);
+    if (w.y) atomicOr(&word[il].y, w.y);
+  }
+  if (m) __syncthreads();
+#pragma unroll
+  for (int j = 0; j < 2; ++j)
+    if (i0 + j * kSideThreads < n)
+      side[(int64_t)blockIdx.y * pitch + i0 + j * kSideThreads] = word[tid + j * kSideThreads];
   groups = __reduce_add_sync(0xffffffffu, groups);
   if (lane == 0 && groups) atomicAdd(fp64_groups, groups);
 }
