@@ -250,8 +250,8 @@ struct ScoreCounters {
 // words; the warp transposes its 32 x 32 bits, so that a lane holds its plane's
 // crossings of 32 edges, and adds up the lengths four edges at a time from tables of
 // the 16 sums that the warp writes for them (the 16 words lie in different banks). Per
-// (plane, edge) that is some 2.3 instructions against ten of score_planes_kernel. Bound by
-// integer issue. Both kernels, against the best K of score_planes_kernel with its
+// (plane, edge) that is 2.9 instructions against ten of score_planes_kernel. Bound by
+// the waits for shared memory and integer issue (55 % ALU). Both kernels, against the best K of score_planes_kernel with its
 // re-decision: 59,183 edges x 2,500 planes over 2,562 vertices 80 -> 35 us, 33,370 x
 // 2,500 over 10,242 54 -> 35, 262,144 x 4,096 over 10,242 422 -> 137, 2^20 x 4,096
 // over 24,576 1,647 -> 524. The lane's own plane tested in every edge's word (a
