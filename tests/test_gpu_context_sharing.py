@@ -1,0 +1,40 @@
+"""BVHs used by another context than the one they were built on: a build from
+host arrays is left running on its own context's stream, so whatever reads it
+from another stream has to wait for it first."""
+import numpy as np
+import pytest
+
+from visacd_gb300 import meshgen as mg
+
+pytestmark = pytest.mark.gpu
+
+
+def test_batch_with_a_grid_over_another_contexts_cage(native, ctx):
+    """A part of more than 2^22 pairs, whose cage gets a free-space grid inside the
+    call: the cage is the last of several builds queued on its context when the
+    other context takes it. The edges are those of the traversal alone, in the
+    first call and (with the grid the BVH keeps) in a later one."""
+    v, _ = mg.displaced_blob(5, seed=6)
+    pts = np.ascontiguousarray(v[:3200], np.float32)
+    none = np.zeros((0, 3), np.int32)
+    cage = mg.offset_cage(*mg.displaced_blob(6, seed=6), 0.03)
+    other = native.Context(0)
+    sb = ctx.bvh(pts, none)
+    builds = [other.bvh(*cage) for _ in range(8)]
+    cb = builds[-1]
+    first = ctx.visibility_batch([(pts, sb, cb, None)])[0][0]
+    assert ctx.visibility(pts, sb, cb)[1]["pairs_tested"] == 3200 * 3199 // 2 >= 1 << 22
+    assert ctx.vis_trace_counts()[0] > 0  # the walk is in use
+    later = ctx.visibility_batch([(pts, sb, cb, None)])[0][0]
+    ctx.set_vis_trace(False)
+    try:
+        want = ctx.visibility_batch([(pts, sb, cb, None)])[0][0]
+    finally:
+        ctx.set_vis_trace(True)
+    assert len(want) > 0
+    np.testing.assert_array_equal(first, want)
+    np.testing.assert_array_equal(later, want)
+    for b in builds:
+        b.close()
+    sb.close()
+    other.close()

@@ -971,39 +971,9 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
          "visibility_batch: null argument");
   VCUDA(cudaSetDevice(ctx->device));
   constexpr int TR = 8, TC = 4;
-  // Free-space grids of the large parts' cages (built once per cage BVH),
-  // before this call takes the shared scratch and staging buffers.
-  // A part's pairs: all of them, or (masked) those with a new endpoint.
-  std::vector<int64_t> part_pairs(n_parts, 0);
-  std::vector<int32_t> nr(n_parts, 0);  // new points of the masked parts
-  for (int p = 0; p < n_parts; ++p) {
-    const int64_t n = std::max(n_pts[p], 0);
-    int64_t pairs = n * (n > 0 ? n - 1 : 0) / 2;
-    if (is_new && is_new[p] && pts[p]) {
-      int64_t k = 0;
-      for (int64_t v = 0; v < n; ++v) k += is_new[p][v] != 0;
-      nr[p] = (int32_t)k;
-      pairs -= (n - k) * (n - k - 1) / 2;
-    }
-    part_pairs[p] = pairs;
-  }
-  bool any_grid = false;
-  if (ctx->vis_trace) {
-    for (int p = 0; p < n_parts; ++p) {
-      if (part_pairs[p] >= kFreeGridMinPairs && cage_bvhs[p] && cage_bvhs[p]->ctx && cage_bvhs[p]->nt > 0) {
-        VTRY(free_grid_build(ctx, const_cast<visacd_bvh*>(cage_bvhs[p]), part_pairs[p]));
-        any_grid = any_grid || cage_bvhs[p]->free_lb != nullptr;
-      }
-    }
-  }
-  // Layout of the per-part arrays in one buffer (256-byte aligned pieces).
-  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
-  std::vector<size_t> o_pts(n_parts), o_mask(n_parts), o_perm(n_parts), o_rows(n_parts),
-      o_rank(n_parts);
-  std::vector<int64_t> ntr_tri(n_parts, 0);
-  size_t total = 0;
-  unsigned long long words = 0;
-  std::vector<unsigned long long> word_start(n_parts + 1);
+  // Every part's checks, and the end of its BVHs' builds, come before anything
+  // reads a BVH: a grid is kept for the BVH's life, so one laid from a build that
+  // another context's stream had not finished would lose edges in every later call.
   for (int p = 0; p < n_parts; ++p) {
     const int32_t n = n_pts[p];
     const visacd_bvh* sb = self_bvhs[p];
@@ -1019,6 +989,42 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
            cb->depth, kStack);
     VCHECK(sb->nt == 0 || sb->nv == n, VISACD_ERR_INVALID_ARG,
            "visibility_batch: part %d self BVH has %d vertices, points have %d", p, sb->nv, n);
+  }
+  // Free-space grids of the large parts' cages (built once per cage BVH),
+  // before this call takes the shared scratch and staging buffers.
+  // A part's pairs: all of them, or (masked) those with a new endpoint.
+  std::vector<int64_t> part_pairs(n_parts, 0);
+  std::vector<int32_t> nr(n_parts, 0);  // new points of the masked parts
+  for (int p = 0; p < n_parts; ++p) {
+    const int64_t n = n_pts[p];
+    int64_t pairs = n * (n > 0 ? n - 1 : 0) / 2;
+    if (is_new && is_new[p]) {
+      int64_t k = 0;
+      for (int64_t v = 0; v < n; ++v) k += is_new[p][v] != 0;
+      nr[p] = (int32_t)k;
+      pairs -= (n - k) * (n - k - 1) / 2;
+    }
+    part_pairs[p] = pairs;
+  }
+  bool any_grid = false;
+  if (ctx->vis_trace) {
+    for (int p = 0; p < n_parts; ++p) {
+      if (part_pairs[p] >= kFreeGridMinPairs && cage_bvhs[p]->nt > 0) {
+        VTRY(free_grid_build(ctx, const_cast<visacd_bvh*>(cage_bvhs[p]), part_pairs[p]));
+        any_grid = any_grid || cage_bvhs[p]->free_lb != nullptr;
+      }
+    }
+  }
+  // Layout of the per-part arrays in one buffer (256-byte aligned pieces).
+  auto al = [](size_t b) { return (b + 255) & ~(size_t)255; };
+  std::vector<size_t> o_pts(n_parts), o_mask(n_parts), o_perm(n_parts), o_rows(n_parts),
+      o_rank(n_parts);
+  std::vector<int64_t> ntr_tri(n_parts, 0);
+  size_t total = 0;
+  unsigned long long words = 0;
+  std::vector<unsigned long long> word_start(n_parts + 1);
+  for (int p = 0; p < n_parts; ++p) {
+    const int32_t n = n_pts[p];
     o_pts[p] = total;  total += al((size_t)std::max(n, 1) * 12);
     o_mask[p] = total; total += al((size_t)std::max(n, 1));
     o_perm[p] = total; total += al((size_t)std::max(n, 1) * 4);
