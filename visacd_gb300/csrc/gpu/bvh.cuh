@@ -40,17 +40,26 @@ struct visacd_bvh {
 namespace vgpu {
 
 #ifdef __CUDACC__
-// The record of a node whose children's boxes are (lo xyz, hi xyz): c - e and
-// c + e enclose them (e rounded up).
+// Centre and half extent of [lo, hi] along an axis: c - e and c + e enclose it (e
+// rounded up). An infinite side (a vertex that is not finite) opens the axis both
+// ways: its own centre would be infinite, and c - e or c + e a NaN.
+__device__ __forceinline__ void box_axis(float lo, float hi, float& c, float& e) {
+  c = 0.5f * lo + 0.5f * hi;
+  e = fmaxf(__fsub_ru(hi, c), __fsub_ru(c, lo));
+  if (!(e < INFINITY)) {
+    c = 0.f;
+    e = INFINITY;
+  }
+}
+
+// The record of a node whose children's boxes are (lo xyz, hi xyz).
 __device__ __forceinline__ void node_record(float4* __restrict__ nodes, int64_t i, const float* l, const float* r,
                                             int left, int right) {
   float lc[3], le[3], rc[3], re[3];
 #pragma unroll
   for (int a = 0; a < 3; ++a) {
-    lc[a] = 0.5f * l[a] + 0.5f * l[3 + a];
-    le[a] = fmaxf(__fsub_ru(l[3 + a], lc[a]), __fsub_ru(lc[a], l[a]));
-    rc[a] = 0.5f * r[a] + 0.5f * r[3 + a];
-    re[a] = fmaxf(__fsub_ru(r[3 + a], rc[a]), __fsub_ru(rc[a], r[a]));
+    box_axis(l[a], l[3 + a], lc[a], le[a]);
+    box_axis(r[a], r[3 + a], rc[a], re[a]);
   }
   nodes[4 * i + 0] = make_float4(lc[0], lc[1], lc[2], le[0]);
   nodes[4 * i + 1] = make_float4(le[1], le[2], rc[0], rc[1]);
