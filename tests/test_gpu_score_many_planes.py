@@ -1,0 +1,23 @@
+"""Scoring of very many planes over few vertices, on both sides of the number of
+plane groups that one launch of the kernels by vertex sides can hold."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("N", [8, 512])
+@pytest.mark.parametrize("P", [65535 * 32, 65535 * 32 + 1])
+def test_scores_past_the_grid_limit(ctx, orc, N, P):
+    rng = np.random.default_rng(N + P)
+    planes = rng.normal(size=(P, 4)).astype(np.float32)
+    v = rng.normal(size=(N, 3)).astype(np.float32)
+    e = rng.integers(0, N, (N + 3, 2)).astype(np.uint32)
+    got, st = ctx.score_planes(planes, v, e)
+    # the same planes in calls of a sixteenth, and some of them by the oracle
+    want = np.concatenate([ctx.score_planes(part, v, e)[0] for part in np.array_split(planes, 16)])
+    np.testing.assert_array_equal(got, want)
+    assert st["argmax"] == int(np.argmax(want))
+    some = np.concatenate([np.arange(100), np.arange(P - 100, P)])
+    _, q, qexp, _ = orc.score_planes(planes[some], v, e)
+    np.testing.assert_array_equal(got[some], np.ldexp(q.astype(np.float64), qexp))

@@ -261,6 +261,7 @@ constexpr int kSidesThreads = 512;
 constexpr int kSidesWarps = kSidesThreads / 32;
 constexpr int kSidesMaxVertices = 24576;  // 192 KB of sides; indices fit 15 bits
 constexpr int64_t kSidesMaxScratch = 1LL << 25;  // groups of 32 planes x vertices: 256 MB
+constexpr int64_t kSidesMaxGroups = 65535;       // blocks of a grid in y
 
 static __global__ void pack_sides_kernel(const float* __restrict__ pts, int32_t n,
                                          const uint32_t* __restrict__ edges, int64_t E,
@@ -572,9 +573,11 @@ static int launch_score(visacd_ctx* ctx, const float4* planes, int32_t P, const 
 // ways are equal for many planes (24,576 edges x 2,500 planes 44.9 and 44.9 us, x
 // 4,096 58.1 and 60.8) and this one ahead for few (x 80 16.0 against 21.4; 642 edges
 // 12.0 and 17.3); at two it is 1.3 times as fast. More vertices than shared memory
-// holds, or more sides than the scratch limit, go edge by edge.
+// holds, more sides than the scratch limit, or more groups of 32 planes than a grid
+// has blocks in y (2,097,120 planes) go edge by edge.
 static bool sides_pay(int32_t P, int32_t N, int64_t E) {
-  return N > 0 && N <= kSidesMaxVertices && E >= N && (P + 31LL) / 32 * N <= kSidesMaxScratch;
+  const int64_t groups = (P + 31LL) / 32;
+  return N > 0 && N <= kSidesMaxVertices && E >= N && groups <= kSidesMaxGroups && groups * N <= kSidesMaxScratch;
 }
 
 // Core of every scoring entry point that may allocate. All pointers are device pointers.
