@@ -38,3 +38,17 @@ def test_batch_with_a_grid_over_another_contexts_cage(native, ctx):
         b.close()
     sb.close()
     other.close()
+
+
+@pytest.mark.parametrize("level", [0, 2, 6])
+def test_info_of_a_bvh_whose_context_went(native, ctx, level):
+    mesh = mg.displaced_blob(level, seed=3)
+    other = native.Context(0)
+    kept, asked = other.bvh(*mesh), other.bvh(*mesh)
+    want = asked.info()
+    other.close()
+    assert kept.info() == want and asked.info() == want
+    again = ctx.bvh(*mesh)
+    assert again.info() == want
+    for b in (kept, asked, again):
+        b.close()

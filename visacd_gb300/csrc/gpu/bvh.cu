@@ -496,6 +496,31 @@ int bvh_build(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* t
   return VISACD_OK;
 }
 
+// A one-launch build knows only a bound: the depth is taken from the records
+// when it is asked for, or before they go with their context.
+int bvh_depth(visacd_bvh* m) {
+  if (m->depth_exact || !m->nodes || m->nt <= 0) return VISACD_OK;
+  const int ni = m->nt > 1 ? m->nt - 1 : 1;
+  std::vector<float4> rec((size_t)ni * 4);
+  VCUDA(cudaSetDevice(m->device));
+  VCUDA(cudaMemcpyAsync(rec.data(), m->nodes, (size_t)ni * 64, cudaMemcpyDeviceToHost, m->stream));
+  VCUDA(cudaStreamSynchronize(m->stream));
+  std::vector<std::pair<int, int>> todo(1, {0, 1});
+  int deepest = 0;
+  while (!todo.empty()) {
+    const auto [node, d] = todo.back();
+    todo.pop_back();
+    deepest = std::max(deepest, d);
+    int child[2];
+    memcpy(child, &rec[4 * (size_t)node + 3], sizeof(child));
+    for (int c : child)
+      if (c >= 0) todo.push_back({c, d + 1});
+  }
+  m->depth = deepest;
+  m->depth_exact = true;
+  return VISACD_OK;
+}
+
 void bvh_detach(visacd_bvh* b) {
   if (b->nodes) cudaFreeAsync(b->nodes, b->stream);
   if (b->free_lb) cudaFreeAsync(b->free_lb, b->stream);
@@ -549,29 +574,8 @@ extern "C" int visacd_bvh_info(const visacd_bvh* b, int32_t* n_tris, int32_t* de
   VCHECK(b, VISACD_ERR_INVALID_ARG, "bvh_info: null bvh");
   if (n_tris) *n_tris = b->nt;
   if (depth) {
-    // A one-launch build knows only a bound: the depth is taken from the
-    // records when it is asked for.
     visacd_bvh* m = const_cast<visacd_bvh*>(b);
-    if (!m->depth_exact && m->nodes && m->nt > 0) {
-      const int ni = m->nt > 1 ? m->nt - 1 : 1;
-      std::vector<float4> rec((size_t)ni * 4);
-      VCUDA(cudaSetDevice(m->device));
-      VCUDA(cudaMemcpyAsync(rec.data(), m->nodes, (size_t)ni * 64, cudaMemcpyDeviceToHost, m->stream));
-      VCUDA(cudaStreamSynchronize(m->stream));
-      std::vector<std::pair<int, int>> todo(1, {0, 1});
-      int deepest = 0;
-      while (!todo.empty()) {
-        const auto [node, d] = todo.back();
-        todo.pop_back();
-        deepest = std::max(deepest, d);
-        int child[2];
-        memcpy(child, &rec[4 * (size_t)node + 3], sizeof(child));
-        for (int c : child)
-          if (c >= 0) todo.push_back({c, d + 1});
-      }
-      m->depth = deepest;
-      m->depth_exact = true;
-    }
+    VTRY(bvh_depth(m));
     *depth = m->depth;
   }
   return VISACD_OK;

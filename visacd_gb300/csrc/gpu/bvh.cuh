@@ -79,6 +79,8 @@ int bvh_build(visacd_ctx* ctx, const float* verts, int32_t nv, const uint32_t* t
 // Frees a BVH's device memory when its context goes away (the handle itself
 // stays valid until visacd_bvh_destroy, and is rejected by queries).
 void bvh_detach(visacd_bvh* b);
+// Makes `depth` the tree's exact depth (waits for the stream; once per BVH).
+int bvh_depth(visacd_bvh* b);
 // Reads the BVH's head to the host (waits for the stream; once per BVH).
 int bvh_head(visacd_ctx* ctx, visacd_bvh* b);
 // A build may still be running on its context's stream: a call on another

@@ -741,8 +741,12 @@ extern "C" int visacd_ctx_destroy(visacd_ctx* ctx) {
   if (!ctx) return VISACD_OK;
   cudaSetDevice(ctx->device);
   cudaStreamSynchronize(ctx->stream);
-  // BVHs still alive lose their device memory with their context.
-  for (visacd_bvh* b : ctx->bvhs) bvh_detach(b);
+  // BVHs still alive lose their device memory with their context; what
+  // visacd_bvh_info says of them is kept.
+  for (visacd_bvh* b : ctx->bvhs) {
+    bvh_depth(b);
+    bvh_detach(b);
+  }
   ctx->bvhs.clear();
   if (ctx->grid_tex) cudaDestroyTextureObject(ctx->grid_tex);
   if (ctx->grid_arr) cudaFreeArray(ctx->grid_arr);
