@@ -127,7 +127,9 @@ __global__ void __launch_bounds__(kCandTile) conflict_kernel(
   if (k >= D || state[k] == kInvalid) return;
   const Plane64 pk = planes[k];
   const float kx = (float)pk.x, ky = (float)pk.y, kz = (float)pk.z;
-  const float dk = d32[k], near = 1.001e-3f;  // FP32 offsets differ by < 1e-6 from FP64
+  // Offsets rounded to FP32 are off by 2^-24 of themselves each, both by at most
+  // 1.2e-7 |d_k| together where they are this close.
+  const float dk = d32[k], near = 1.001e-3f + 2.4e-7f * fabsf(dk);
   const float eps32 = (float)normal_eps - 1e-5f;
   // This block's share of the tile's columns; earlier candidates only.
   const int share = kCandTile / gridDim.y, jbegin = blockIdx.y * share;
