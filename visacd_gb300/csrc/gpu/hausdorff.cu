@@ -40,6 +40,8 @@
 namespace vgpu {
 
 constexpr int kKnn = 10;
+constexpr int kMaxCells = 160;  // cells of a grid per axis at most
+constexpr int kPlaceBits = 24;  // of a sample's place, where it is kept with its ring
 constexpr int kBoundRings = 2;  // rings of cells searched for each query's upper bound
 
 struct HGrid {
@@ -271,12 +273,16 @@ __device__ __noinline__ double query_term(const HSide& S, int qi, float tmargin)
 // at a time; their samples are tested 32 at a time, and those below the last
 // kept distance inserted by ballot and shuffle (sorted lists per lane lie in
 // local memory and leave a long row to one lane: 187 us for a query far from
-// the surface). query_term's stop rule and selection proof; returns false (on
-// all lanes) when the proof fails or the 10th and 11th distances are equal, and
-// the caller then uses query_term, whose order decides which of the two counts.
-// (Queries without a bound are evaluated in full: the nearest sample's distance
-// does not bound the reference formula's minimum when its triangle is
-// degenerate, so it is not used to skip them.)
+// the surface). Samples at equal distances are put into query_term's order, which
+// decides which of them counts: by ring, and in a ring by cell, as spts has them.
+// (Left to query_term, ties take a whole warp each at one lane's pace: two lattices
+// of 256 x 256 samples 9.4 ms, 1.5 so; walking the rings in that order
+// instead took 13 % longer for queries far from the surface.) query_term's stop
+// rule and selection proof; returns false (on all lanes) when the proof fails or a
+// distance is not finite, and the caller then uses query_term. (Queries without a
+// bound are evaluated in full: the nearest sample's distance does not bound the
+// reference formula's minimum when its triangle is degenerate, so it is not used
+// to skip them.)
 __device__ bool query_knn_warp(const HSide& S, int qi, int* ids, int& cnt_out, double& d0_out) {
   const int lane = threadIdx.x & 31;
   const HGrid& G = S.G;
@@ -288,10 +294,12 @@ __device__ bool query_knn_warp(const HSide& S, int qi, int* ids, int& cnt_out, d
   const int cx = __shfl_sync(0xffffffffu, ca, 0), cy = __shfl_sync(0xffffffffu, ca, 1),
             cz = __shfl_sync(0xffffffffu, ca, 2);
   const int rmax = max(G.dim[0], max(G.dim[1], G.dim[2]));
+  static_assert(kMaxCells < 1 << (32 - kPlaceBits), "rings beside a place");
+  const bool rings = G.n <= 1 << kPlaceBits;
   const float qf[3] = {(float)q[0], (float)q[1], (float)q[2]};
   const float hf = (float)G.h;
   float myv = 3.4e38f;  // lane m: the m-th kept distance
-  int myid = -1;
+  unsigned myat = ~0u;  // and its sample: place in spts, ring << kPlaceBits above it
   int nf = 0;           // kept (at most kKnnF)
   int total = 0;        // candidates seen
   float last = 3.4e38f;  // the kKnnF-th kept distance
@@ -346,27 +354,26 @@ __device__ bool query_knn_warp(const HSide& S, int qi, int* ids, int& cnt_out, d
         const int k = __shfl_sync(0xffffffffu, k0, it) + p -
                       (__shfl_sync(0xffffffffu, end, it) - __shfl_sync(0xffffffffu, len, it));
         float d2 = 0.f;
-        int id = -1;
         if (p < sum) {
           const float4 sp = G.spts[k];
           const float ex = sp.x - qf[0], ey = sp.y - qf[1], ez = sp.z - qf[2];
           d2 = ex * ex + ey * ey + ez * ez;
-          id = __float_as_int(sp.w);
         }
-        unsigned m = __ballot_sync(0xffffffffu, id >= 0 && (nf < kKnnF || d2 < last));
+        const unsigned place = rings ? (unsigned)r << kPlaceBits | (unsigned)k : (unsigned)k;
+        unsigned m = __ballot_sync(0xffffffffu, p < sum && (nf < kKnnF || d2 < last));
         while (m) {
           const int src = __ffs(m) - 1;
           m &= m - 1;
           const float v = __shfl_sync(0xffffffffu, d2, src);
-          const int vid = __shfl_sync(0xffffffffu, id, src);
+          const unsigned vat = __shfl_sync(0xffffffffu, place, src);
           if (nf == kKnnF && !(v < last)) continue;
           const int pos = __popc(__ballot_sync(0xffffffffu, lane < nf && myv <= v));
           const float uv = __shfl_up_sync(0xffffffffu, myv, 1);
-          const int ui = __shfl_up_sync(0xffffffffu, myid, 1);
+          const unsigned uat = __shfl_up_sync(0xffffffffu, myat, 1);
           if (nf < kKnnF) ++nf;
           if (lane < nf && lane >= pos) {
             myv = lane == pos ? v : uv;
-            myid = lane == pos ? vid : ui;
+            myat = lane == pos ? vat : uat;
           }
           if (nf == kKnnF) last = __shfl_sync(0xffffffffu, myv, kKnnF - 1);
         }
@@ -388,30 +395,44 @@ __device__ bool query_knn_warp(const HSide& S, int qi, int* ids, int& cnt_out, d
                     __fadd_ru(__fadd_ru(__fmul_ru(__fsqrt_ru(g10), 1.0f + 1.0f / 1048576.0f), G.eabs), G.eabs);
     if (!ok) return false;
   }
+  const float prev = __shfl_up_sync(0xffffffffu, myv, 1);
+  if (__any_sync(0xffffffffu, lane > 0 && lane < nf && prev == myv)) {
+    if (!rings) return false;
+    int to = 0;
+    for (int m = 0; m < nf; ++m) {
+      const float v = __shfl_sync(0xffffffffu, myv, m);
+      const unsigned at = __shfl_sync(0xffffffffu, myat, m);
+      to += v < myv || (v == myv && at < myat);
+    }
+    const unsigned own = myat;
+    for (int m = 0; m < nf; ++m) {  // (equal distances change places: only the samples move)
+      const int t = __shfl_sync(0xffffffffu, to, m);
+      const unsigned at = __shfl_sync(0xffffffffu, own, m);
+      if (t == lane) myat = at;
+    }
+  }
+  int myid = -1;
+  if (lane < nf) myid = __float_as_int(G.spts[rings ? myat & ((1u << kPlaceBits) - 1u) : myat].w);
   // Exact FP64 distances of the (up to) kKnnF candidates, the 10 nearest kept
-  // in order (insertion in candidate order, as query_term).
+  // in order (as insertion in candidate order, query_term's, leaves them).
   double d2 = DBL_MAX;
   if (myid >= 0) {
     const double* pp = G.pts + 3 * (int64_t)myid;
     const double ex = ds(pp[0], q[0]), ey = ds(pp[1], q[1]), ez = ds(pp[2], q[2]);
     d2 = da(da(dm(ex, ex), dm(ey, ey)), dm(ez, ez));
   }
-  if (__any_sync(0xffffffffu, myid >= 0 && !(d2 < DBL_MAX))) return false;  // not finite
+  if (__any_sync(0xffffffffu, myid >= 0 && !(myv < 3.4e38f && d2 < DBL_MAX))) return false;  // not finite
   // Rank of each among them (candidate order between equals); non-negative
   // doubles order like their bits, and FP64 compares are slow.
   const unsigned long long key = (unsigned long long)__double_as_longlong(d2);
   int rank = 0;
-  bool tie = false;
   for (int m = 0; m < kKnnF; ++m) {
     const unsigned long long v = __shfl_sync(0xffffffffu, key, m);
     const int id = __shfl_sync(0xffffffffu, myid, m);
     if (id < 0 || m == lane) continue;
     rank += v < key || (v == key && m < lane);
-    tie |= v == key && m < lane;
   }
-  // Equal distances at ranks 9 and 10 (from 0): which one counts is query_term's.
   const int cand = __popc(__ballot_sync(0xffffffffu, myid >= 0));
-  if (__any_sync(0xffffffffu, myid >= 0 && rank == kKnn && tie)) return false;
   if (myid >= 0 && rank < kKnn) ids[rank] = myid;
   d0_out = __shfl_sync(0xffffffffu, d2, max(__ffs(__ballot_sync(0xffffffffu, myid >= 0 && rank == 0)), 1) - 1);
   cnt_out = min(cand, kKnn);
@@ -719,8 +740,10 @@ __global__ void __launch_bounds__(256) hselect_kernel(HBatch H, const float* __r
 // and raise all maxima early. On the 210,014 samples the two launches with their
 // selections take 216 and 277 us; one thread per query in cell order (105,629
 // evaluated) took 905 us, and sorted lists per lane over whole cubes of cells 920
-// us for the 4,221 without a bound.
-__global__ void __launch_bounds__(128) hterm_kernel(HBatch H, const float* __restrict__ ubs,
+// us for the 4,221 without a bound. kTermBlocks blocks an SM: the grid is one wave
+// (with 72 registers, seven resident, far queries take 1.3 times as long).
+constexpr int kTermBlocks = 8;
+__global__ void __launch_bounds__(128, kTermBlocks) hterm_kernel(HBatch H, const float* __restrict__ ubs,
                                                     const int2* __restrict__ qref, const long long* __restrict__ list,
                                                     const unsigned* __restrict__ count) {
   __shared__ int near_ids[4][3 * kKnn];
@@ -818,7 +841,7 @@ void grid_for_points(const double* x, long long n, HGrid& g) {
   double area_like = 0;
   for (int a = 0; a < 3; ++a) area_like += (hi[a] - lo[a]) * (hi[(a + 1) % 3] - lo[(a + 1) % 3]);
   double h = std::sqrt(std::max(area_like, 1e-30) * 2.0 / (double)std::max(n, 1LL));
-  h = std::max(h, ext / 160.0);
+  h = std::max(h, ext / kMaxCells);
   if (!(h > 0)) h = 1.0;
   for (int a = 0; a < 3; ++a) {
     g.lo[a] = lo[a];
@@ -984,7 +1007,7 @@ extern "C" int visacd_face_hausdorff_batch(visacd_ctx* ctx, int32_t njobs, const
   const int2* qref = (const int2*)(D + o_qref);
   long long* list = (long long*)(D + o_farl);
   const unsigned gsel = grid_for(NS, 256, 8LL * ctx->sm_count);
-  const unsigned gterm = grid_for(32LL * NS, 128, 8LL * ctx->sm_count);
+  const unsigned gterm = grid_for(32LL * NS, 128, (int64_t)kTermBlocks * ctx->sm_count);
   VLAUNCH(ctx, kKHausdorffHead, gsel, 256, 0, hselect_kernel, H, ubs, qref, NS, 1, far, list);
   VLAUNCH(ctx, kKHausdorffHead, gterm, 128, 0, hterm_kernel, H, ubs, qref, (const long long*)list,
           (const unsigned*)far);
