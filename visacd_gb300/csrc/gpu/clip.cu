@@ -1194,23 +1194,10 @@ extern "C" int visacd_clip_fetch(visacd_ctx* ctx, int32_t* pos_tris, int32_t* ne
                                  int32_t* border_edges) {
   VCHECK(ctx, VISACD_ERR_INVALID_ARG, "visacd_clip_fetch: null context");
   const visacd_clip_result& r = ctx->clip_out;
-  cudaStream_t st = ctx->stream;
-  // All pieces into the pinned buffer with one wait (a copy straight into
-  // pageable memory waits for itself), then to the caller.
   void* const dst[6] = {pos_tris, neg_tris, pos_map, neg_map, border, border_edges};
+  const void* const src[6] = {ctx->clip_ptrs[0], ctx->clip_ptrs[1], ctx->clip_ptrs[2],
+                              ctx->clip_ptrs[3], ctx->clip_ptrs[4], ctx->clip_ptrs[5]};
   const size_t bytes[6] = {(size_t)r.n_pos * 12, (size_t)r.n_neg * 12,    (size_t)ctx->clip_nv * 4,
                            (size_t)ctx->clip_nv * 4, (size_t)r.n_border * 24, (size_t)r.n_border_edges * 8};
-  size_t at[6], total = 0;
-  for (int k = 0; k < 6; ++k) {
-    at[k] = total;
-    if (dst[k]) total += (bytes[k] + 63) & ~size_t(63);
-  }
-  char* h = nullptr;
-  VTRY(pinned(ctx, total, (void**)&h));
-  for (int k = 0; k < 6; ++k)
-    if (dst[k] && bytes[k]) VCUDA(cudaMemcpyAsync(h + at[k], ctx->clip_ptrs[k], bytes[k], cudaMemcpyDeviceToHost, st));
-  VCUDA(stream_wait(ctx));
-  for (int k = 0; k < 6; ++k)
-    if (dst[k] && bytes[k]) std::memcpy(dst[k], h + at[k], bytes[k]);
-  return VISACD_OK;
+  return fetch(ctx, 6, dst, src, bytes);
 }

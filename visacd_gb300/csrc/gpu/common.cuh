@@ -244,6 +244,16 @@ int status_result(visacd_ctx* ctx, uint32_t status, const char* what);
 // Pinned host staging of at least `bytes`.
 int pinned(visacd_ctx* ctx, size_t bytes, void** out);
 
+// Device-to-host copies of a call's results (null or empty ones are left out), then
+// one wait. Small ones go through the pinned buffer, since a copy into pageable
+// memory waits for itself; large ones straight to the caller's, which over the
+// coherent link needs no second pass by the host: two results of 0.09, 0.38, 1.5
+// and 3.4 MiB together take 22, 40, 117 and 250 us staged and 24, 26, 33 and 43
+// direct, six of 0.15, 0.61, 0.92 and 23 MiB 42, 75, 98 and 1,880 against 84, 92,
+// 95 and 235.
+constexpr size_t kStagedPerCopy = 96 << 10;
+int fetch(visacd_ctx* ctx, int n, void* const* dst, const void* const* src, const size_t* bytes);
+
 // Host-to-device uploads of one call through the context's pinned upload
 // buffer: a host memcpy into pinned memory, then an asynchronous DMA from it,
 // so contexts driven by several host threads do not contend on the driver's

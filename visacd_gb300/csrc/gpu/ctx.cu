@@ -152,6 +152,33 @@ int pinned(visacd_ctx* ctx, size_t bytes, void** out) {
   return VISACD_OK;
 }
 
+int fetch(visacd_ctx* ctx, int n, void* const* dst, const void* const* src, const size_t* bytes) {
+  size_t total = 0;
+  int copies = 0;
+  for (int k = 0; k < n; ++k) {
+    if (!dst[k] || !bytes[k]) continue;
+    total += (bytes[k] + 63) & ~size_t(63);
+    ++copies;
+  }
+  if (!copies) return VISACD_OK;
+  char* h = nullptr;
+  if (total <= copies * kStagedPerCopy) VTRY(pinned(ctx, total, (void**)&h));
+  size_t at = 0;
+  for (int k = 0; k < n; ++k) {
+    if (!dst[k] || !bytes[k]) continue;
+    VCUDA(cudaMemcpyAsync(h ? h + at : dst[k], src[k], bytes[k], cudaMemcpyDeviceToHost, ctx->stream));
+    at += (bytes[k] + 63) & ~size_t(63);
+  }
+  VCUDA(stream_wait(ctx));
+  at = 0;
+  for (int k = 0; h && k < n; ++k) {
+    if (!dst[k] || !bytes[k]) continue;
+    std::memcpy(dst[k], h + at, bytes[k]);
+    at += (bytes[k] + 63) & ~size_t(63);
+  }
+  return VISACD_OK;
+}
+
 int Stager::reserve(size_t total_bytes, int arrays) {
   const size_t need = (total_bytes + 64 * (size_t)(arrays + 1) + 63) & ~size_t(63);
   if (ctx_->h_upload_used + need > ctx_->h_upload_cap) {

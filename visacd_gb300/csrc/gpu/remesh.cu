@@ -1006,18 +1006,8 @@ extern "C" int visacd_sdf_fetch(visacd_ctx* ctx, double* verts, int32_t* tris) {
   VCUDA(cudaSetDevice(ctx->device));
   VCHECK(ctx->sdf_nv == 0 || verts, VISACD_ERR_INVALID_ARG, "sdf_fetch: null vertex buffer");
   VCHECK(ctx->sdf_nt == 0 || tris, VISACD_ERR_INVALID_ARG, "sdf_fetch: null triangle buffer");
-  // Through the pinned buffer (both copies in flight at once, one wait) up to
-  // 64 MiB; larger meshes go straight to the caller's memory.
-  const size_t bv = (size_t)ctx->sdf_nv * 24, bt = (size_t)ctx->sdf_nt * 12;
-  const bool staged = bv + bt <= (64u << 20);
-  char* h = nullptr;
-  if (staged) VTRY(pinned(ctx, bv + bt + 1, (void**)&h));
-  void* hv = staged ? (void*)h : (void*)verts;
-  void* ht = staged ? (void*)(h + bv) : (void*)tris;
-  if (bv) VCUDA(cudaMemcpyAsync(hv, slot<double>(ctx, kSlotSdfOut), bv, cudaMemcpyDeviceToHost, ctx->stream));
-  if (bt) VCUDA(cudaMemcpyAsync(ht, slot<int32_t>(ctx, kSlotSdfTris), bt, cudaMemcpyDeviceToHost, ctx->stream));
-  VCUDA(stream_wait(ctx));
-  if (staged && bv) std::memcpy(verts, h, bv);
-  if (staged && bt) std::memcpy(tris, h + bv, bt);
-  return VISACD_OK;
+  void* const dst[2] = {verts, tris};
+  const void* const src[2] = {slot<double>(ctx, kSlotSdfOut), slot<int32_t>(ctx, kSlotSdfTris)};
+  const size_t bytes[2] = {(size_t)ctx->sdf_nv * 24, (size_t)ctx->sdf_nt * 12};
+  return fetch(ctx, 2, dst, src, bytes);
 }
