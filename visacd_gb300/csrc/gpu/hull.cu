@@ -359,30 +359,38 @@ __device__ int flat_hull(const double* P, int n, HullWork& W, int32_t* tris, int
   D3 nrm = cross3(u, sub3(ld3(P, ic), o));
   nrm = div3(nrm, norm3(nrm));
   const D3 v = cross3(nrm, u);
-  // Sort (x, y, index) lexicographically by rank counting: rank of i = number
-  // of keys below it (keys are distinct through the index).
-  // (40 of the face array's 640 bytes per point, and the chain of up to 2n.)
-  double* qx = reinterpret_cast<double*>(W.gface);
+  // Sort (x, y, index) lexicographically by rank counting: rank of i = number of
+  // keys below it (distinct through the index). The keys are integers of the
+  // doubles' order: four FP64 compares a pair are what bounded this (5,000 points
+  // 73 ms, and 96 with their keys in a cache that the block's shared memory leaves
+  // small; 37 so). They and the sorted points lie in that shared memory where
+  // they fit, else in the face array (36 of its 640 bytes per point); the chain of
+  // up to 2n takes the keys' place.
+  const int64_t shared = 4 * (int64_t)W.nsp + (int64_t)sizeof(HFace) * W.nsf;
+  double* qx = reinterpret_cast<double*>(36 * (int64_t)n <= shared ? (char*)W.spool : (char*)W.gface);
   double* qy = qx + n;
-  double* kx = qy + n;  // the unsorted keys
-  double* ky = kx + n;
+  long long* kx = reinterpret_cast<long long*>(qy + n);
+  long long* ky = kx + n;
   int* qi = reinterpret_cast<int*>(ky + n);
-  int* h = qi + n;
+  int* h = reinterpret_cast<int*>(kx);
+  constexpr long long kSign = 0x7fffffffffffffffll;
   for (int i = lane; i < n; i += 32) {
     const D3 w = sub3(ld3(P, i), o);
-    kx[i] = dot3(w, u);
-    ky[i] = dot3(w, v);
+    const long long x = __double_as_longlong(da(dot3(w, u), 0.0)), y = __double_as_longlong(da(dot3(w, v), 0.0));
+    kx[i] = x ^ (x >> 63 & kSign);
+    ky[i] = y ^ (y >> 63 & kSign);
   }
   __syncwarp();
   for (int i = lane; i < n; i += 32) {
-    const double xi = kx[i], yi = ky[i];
+    const long long xi = kx[i], yi = ky[i];
     int r = 0;
+#pragma unroll 8
     for (int j = 0; j < n; ++j) {
-      const double xj = kx[j], yj = ky[j];
+      const long long xj = kx[j], yj = ky[j];
       r += (xj < xi || (xj == xi && (yj < yi || (yj == yi && j < i)))) ? 1 : 0;
     }
-    qx[r] = xi;
-    qy[r] = yi;
+    qx[r] = __longlong_as_double(xi ^ (xi >> 63 & kSign));
+    qy[r] = __longlong_as_double(yi ^ (yi >> 63 & kSign));
     qi[r] = i;
   }
   __syncwarp();
