@@ -551,6 +551,17 @@ __global__ void new_rows_kernel(const uint32_t* __restrict__ perm, const uint32_
   }
 }
 
+// New points of a mask in device memory, added to *count. What a masked call does
+// follows from it (the pairs, so the grid, the reach table and the tiles).
+__global__ void mask_count_kernel(const uint8_t* __restrict__ is_new, int32_t n,
+                                  unsigned long long* __restrict__ count) {
+  unsigned c = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    c += is_new[i] != 0;
+  c = __reduce_add_sync(0xffffffffu, c);
+  if ((threadIdx.x & 31) == 0 && c) atomicAdd(count, (unsigned long long)c);
+}
+
 // ---- bitset compaction ----------------------------------------------------
 __global__ void bit_emit_kernel(const uint32_t* __restrict__ bits, int64_t nw,
                                 const uint64_t* __restrict__ off, int64_t n,
@@ -757,8 +768,8 @@ static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint
                       visacd_vis_stats* stats, int64_t pairs, int32_t n_new, const PointOrder* ordered,
                       const uint32_t** few_edges) {
   // The cage's free-space grid, for calls with many pairs (`pairs`: the
-  // call's pair count, or a bound of it): built once per cage BVH, before this
-  // call's counters take the shared scratch and staging buffers.
+  // call's pair count): built once per cage BVH, before this call's counters take
+  // the shared scratch and staging buffers.
   const bool use_grid = ctx->vis_trace && n >= 2 && pairs >= kFreeGridMinPairs && cage_bvh->nt > 0;
   if (use_grid) VTRY(free_grid_build(ctx, const_cast<visacd_bvh*>(cage_bvh), pairs));
   VTRY(ensure_slot(ctx, kSlotCounters, sizeof(VisCounters)));
@@ -794,13 +805,6 @@ static int vis_device(visacd_ctx* ctx, const float* d_pts, int32_t n, const uint
   P.nc = n;
   P.ntc = (n + TC - 1) / TC;
   if (d_new) {
-    if (n_new < 0) {  // the mask is on the device: its count with it
-      std::vector<uint8_t> mask((size_t)n);
-      VCUDA(cudaMemcpyAsync(mask.data(), d_new, (size_t)n, cudaMemcpyDeviceToHost, ctx->stream));
-      VCUDA(stream_wait(ctx));
-      n_new = 0;
-      for (uint8_t m : mask) n_new += m != 0;
-    }
     P.rows = order.rows;
     P.nr = n_new;
     P.triangular = 0;
@@ -1245,12 +1249,24 @@ int visibility_impl(visacd_ctx* ctx, const float* pts, int32_t n, const uint8_t*
   const float* d_pts = pts;
   const uint8_t* d_new = is_new;
   int64_t pairs = (int64_t)n * (n > 0 ? n - 1 : 0) / 2;
-  int32_t n_new = -1;
+  int32_t n_new = 0;
   bvh_settle(ctx, self_bvh);
   bvh_settle(ctx, cage_bvh);
-  if (is_new && !device_ptrs) {
+  if (is_new) {
     int64_t k = 0;
-    for (int32_t v = 0; v < n; ++v) k += is_new[v] != 0;
+    if (device_ptrs && n > 0) {
+      VTRY(ensure_slot(ctx, kSlotCounters, sizeof(VisCounters)));
+      unsigned long long* d_rows = &slot<VisCounters>(ctx, kSlotCounters)->n_rows;
+      unsigned long long* h_rows = nullptr;
+      VTRY(pinned(ctx, sizeof(*h_rows), (void**)&h_rows));
+      VCUDA(cudaMemsetAsync(d_rows, 0, sizeof(*d_rows), ctx->stream));
+      VLAUNCH(ctx, kKVisPrep, grid_for(n, 256, 4LL * ctx->sm_count), 256, 0, mask_count_kernel, d_new, n, d_rows);
+      VCUDA(cudaMemcpyAsync(h_rows, d_rows, sizeof(*h_rows), cudaMemcpyDeviceToHost, ctx->stream));
+      VCUDA(stream_wait(ctx));
+      k = (int64_t)*h_rows;
+    } else {
+      for (int32_t v = 0; v < n; ++v) k += is_new[v] != 0;
+    }
     n_new = (int32_t)k;
     pairs -= ((int64_t)n - k) * ((int64_t)n - k - 1) / 2;
   }
@@ -1308,9 +1324,8 @@ static int matrix_together(visacd_ctx* ctx, const float* verts, int32_t nv, cons
   VTRY(order_run(ctx, jobs, 3));
   VTRY(order_nodes(ctx, jobs, 2));
   int64_t pairs = (int64_t)nv * (nv - 1) / 2;
-  int32_t n_new = -1;
+  int32_t n_new = 0;
   if (is_new) {
-    n_new = 0;
     for (int32_t v = 0; v < nv; ++v) n_new += is_new[v] != 0;
     pairs -= ((int64_t)nv - n_new) * ((int64_t)nv - n_new - 1) / 2;
   }
