@@ -57,6 +57,7 @@ __global__ void __launch_bounds__(kVisThreads, 6)
   constexpr int TC = 32 / TR;
   const int lane = threadIdx.x & 31;
   __shared__ unsigned long long sums[kVisThreads / 32][kSums];  // (a batch reports no work counters)
+  __shared__ SegLeaf leaves[kVisThreads / 32];
   unsigned status_bits = 0;
   for (int guard = 0; guard < (1 << 30); ++guard) {
     unsigned long long w = 0;
@@ -90,7 +91,7 @@ __global__ void __launch_bounds__(kVisThreads, 6)
     }
     const bool active = valid && seg_length(__fsub_rn(q.x, p.x), __fsub_rn(q.y, p.y), __fsub_rn(q.z, p.z)) > 0.f;
     if (!__any_sync(0xffffffffu, active)) continue;
-    if (trace_tile(P.mesh, P.pts, i, j, p, q, active, sums[threadIdx.x >> 5], status_bits) == 1u) {
+    if (trace_tile(P.mesh, P.pts, i, j, p, q, active, &leaves[threadIdx.x >> 5], sums[threadIdx.x >> 5], status_bits) == 1u) {
       const int64_t k = row_start(i, P.n) + (int64_t)(j - i - 1);
       atomicOr(&bitset[P.word_begin + (k >> 5)], 1u << (k & 31));
     }

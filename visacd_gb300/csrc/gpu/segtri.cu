@@ -20,7 +20,8 @@ __global__ void seg_tri_kernel(const float* __restrict__ seg, const float* __res
     const float3 p = make_float3(sp[0], sp[1], sp[2]), q = make_float3(sp[3], sp[4], sp[5]);
     const float4 a = make_float4(t[0], t[1], t[2], 0.f), b = make_float4(t[3], t[4], t[5], 0.f),
                  c = make_float4(t[6], t[7], t[8], 0.f);
-    int r = tri_test32(p, q, a, b, c);
+    const float dx = __fsub_rn(q.x, p.x), dy = __fsub_rn(q.y, p.y), dz = __fsub_rn(q.z, p.z);
+    int r = tri_test32(p.x, p.y, p.z, dx, dy, dz, edge_factor(dx, dy, dz), a, b, c);
     if (r == 2) {
       ++rechecks;
       r = tri_recheck(p.x, p.y, p.z, q.x, q.y, q.z, a, b, c) ? 1 : 0;

@@ -158,15 +158,19 @@ __device__ __forceinline__ bool trace_free(const FreeGridView& g, float px, floa
 }
 
 // What the traversal keeps of a lane's segment p -> q (d = q - p rounded): per
-// axis 1 / d, |1 / d| and -p / d. A box test is then three FMAs per axis; the
-// points themselves are read again at the (few) leaf tests, which leaves the
-// registers to the traversal.
+// axis 1 / d, |1 / d| and -p / d in registers, for a box test of three FMAs per
+// axis, and what a leaf test needs in shared memory (two 16-byte reads).
+struct SegLeaf {
+  float4 p[32];  // p, and edge_factor of d
+  float4 d[32];  // d
+};
 struct Seg {
   float ix, iy, iz;
   float ax, ay, az;
   float nx, ny, nz;
   int vi, vj;    // endpoint vertex ids (p = pts[vi], q = pts[vj])
   bool exclude;  // skip triangles incident to vi or vj (self test)
+  SegLeaf* leaf; // the warp's
 };
 
 __device__ __forceinline__ unsigned f2o_v(float f) {
@@ -203,10 +207,11 @@ __device__ __forceinline__ float seg_length(float dx, float dy, float dz) {
   return __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
 }
 
-__device__ __forceinline__ void make_seg(Seg& s, float3 p, float3 q, int vi, int vj) {
-  s.ix = inv_guard(__fsub_rn(q.x, p.x));
-  s.iy = inv_guard(__fsub_rn(q.y, p.y));
-  s.iz = inv_guard(__fsub_rn(q.z, p.z));
+__device__ __forceinline__ void make_seg(Seg& s, float3 p, float3 q, int vi, int vj, SegLeaf* leaf) {
+  const float dx = __fsub_rn(q.x, p.x), dy = __fsub_rn(q.y, p.y), dz = __fsub_rn(q.z, p.z);
+  s.ix = inv_guard(dx);
+  s.iy = inv_guard(dy);
+  s.iz = inv_guard(dz);
   s.ax = fabsf(s.ix);
   s.ay = fabsf(s.iy);
   s.az = fabsf(s.iz);
@@ -216,6 +221,10 @@ __device__ __forceinline__ void make_seg(Seg& s, float3 p, float3 q, int vi, int
   s.vi = vi;
   s.vj = vj;
   s.exclude = true;
+  s.leaf = leaf;
+  // (each lane writes and reads its own)
+  leaf->p[threadIdx.x & 31] = make_float4(p.x, p.y, p.z, edge_factor(dx, dy, dz));
+  leaf->d[threadIdx.x & 31] = make_float4(dx, dy, dz, 0.f);
 }
 
 // Conservative slab test of the segment (t in [0, 1]) against the box with
@@ -370,11 +379,10 @@ static __device__ __noinline__ bool tri_recheck(float ox, float oy, float oz, fl
   return r == 2 ? tri_test64(ox, oy, oz, qx, qy, qz, a, b, c) : r == 1;
 }
 
-// FP32 filter of the segment p -> q: 1 certain hit, 0 certain miss, 2
-// undecided (tri_recheck).
-__device__ __forceinline__ int tri_test32(float3 p, float3 q, float4 a, float4 b, float4 c) {
-  const float ox = p.x, oy = p.y, oz = p.z;
-  const float dx = __fsub_rn(q.x, p.x), dy = __fsub_rn(q.y, p.y), dz = __fsub_rn(q.z, p.z);
+// FP32 filter of the segment p -> p + d (d = q - p rounded, kw = edge_factor of d):
+// 1 certain hit, 0 certain miss, 2 undecided (tri_recheck).
+__device__ __forceinline__ int tri_test32(float ox, float oy, float oz, float dx, float dy, float dz, float kw,
+                                          float4 a, float4 b, float4 c) {
   float Ax = __fsub_rn(a.x, ox), Ay = __fsub_rn(a.y, oy), Az = __fsub_rn(a.z, oz);
   float Bx = __fsub_rn(b.x, ox), By = __fsub_rn(b.y, oy), Bz = __fsub_rn(b.z, oz);
   float Cx = __fsub_rn(c.x, ox), Cy = __fsub_rn(c.y, oy), Cz = __fsub_rn(c.z, oz);
@@ -387,7 +395,7 @@ __device__ __forceinline__ int tri_test32(float3 p, float3 q, float4 a, float4 b
   float Wb = dx * CAx + dy * CAy + dz * CAz;
   float Wc = dx * ABx + dy * ABy + dz * ABz;
   float L2 = L * L;
-  float Ew = edge_factor(dx, dy, dz) * L2;
+  float Ew = kw * L2;
   float mx = max3f(Wa, Wb, Wc), mn = min3f(Wa, Wb, Wc);
   if (mx > Ew && mn < -Ew) return 0;  // edge functions of strictly opposite sign
   bool allpos = mn > Ew, allneg = mx < -Ew;
@@ -416,13 +424,12 @@ __device__ __forceinline__ bool leaf_hit(const float4* __restrict__ tris, int le
     if (ia == s.vi || ia == s.vj || ib == s.vi || ib == s.vj || ic == s.vi || ic == s.vj)
       return false;
   }
-  const float* pp = pts + 3 * (int64_t)s.vi;
-  const float* qq = pts + 3 * (int64_t)s.vj;
-  const float3 p = make_float3(pp[0], pp[1], pp[2]), q = make_float3(qq[0], qq[1], qq[2]);
-  const int r = tri_test32(p, q, a, b, c);
+  const float4 p = s.leaf->p[threadIdx.x & 31], d = s.leaf->d[threadIdx.x & 31];
+  const int r = tri_test32(p.x, p.y, p.z, d.x, d.y, d.z, p.w, a, b, c);
   if (r == 2) {
     ++rechecks;
-    return tri_recheck(p.x, p.y, p.z, q.x, q.y, q.z, a, b, c);
+    const float* q = pts + 3 * (int64_t)s.vj;
+    return tri_recheck(p.x, p.y, p.z, q[0], q[1], q[2], a, b, c);
   }
   return r == 1;
 }
@@ -460,8 +467,8 @@ static __device__ __forceinline__ bool packet_hits(const float4* __restrict__ no
     const int l = lr.x, r = lr.y;
     bool hl, hr;
     if (WIDE) {
-      const float* pp = pts + 3 * (int64_t)s.vi;
-      const float3 p = make_float3(pp[0], pp[1], pp[2]);
+      const float4 o = s.leaf->p[threadIdx.x & 31];
+      const float3 p = make_float3(o.x, o.y, o.z);
       hl = active && box_hit_wide(s, p, n0.x, n0.y, n0.z, n0.w, n1.x, n1.y);
       hr = active && box_hit_wide(s, p, n1.z, n1.w, n2.x, n2.y, n2.z, n2.w);
     } else {
@@ -471,15 +478,15 @@ static __device__ __forceinline__ bool packet_hits(const float4* __restrict__ no
     const unsigned bl = __ballot_sync(full, hl);
     const unsigned br = __ballot_sync(full, hr);
     int next = -1;
-    const bool leaf = (bl && l < 0) || (br && r < 0);
+    // (all of these are the same in every lane)
+    const bool leaf_l = bl && l < 0, leaf_r = br && r < 0, leaf = leaf_l || leaf_r;
     if (leaf) {
       // (one copy of the triangle test: two would cost registers)
 #pragma unroll 1
-      for (int k = 0; k < 2; ++k) {
-        const int child = k ? r : l;
-        if (child < 0 && active && (k ? hr : hl)) {
+      for (int k = leaf_l ? 0 : 1; k < (leaf_r ? 2 : 1); ++k) {
+        if (active && (k ? hr : hl)) {
           ++tri_tests;
-          if (leaf_hit(tris, ~child, s, pts, rechecks)) {
+          if (leaf_hit(tris, ~(k ? r : l), s, pts, rechecks)) {
             hit = true;
             active = false;
           }
@@ -557,12 +564,13 @@ enum { kSumPairs, kSumEdges, kSumSelf, kSumCage, kSumDegenerate, kSumRechecks, k
 // cage, then those that leave it against the part. Few segments leave the
 // cage (most vertex pairs of a part are interior chords, which cross neither
 // surface), so the second test runs for few. Bit 0: hits the cage; bit 1: hits
-// the part as well (1 alone: an edge). sum: the warp's totals.
+// the part as well (1 alone: an edge). leaf, sum: the warp's.
 static __device__ __forceinline__ unsigned trace_tile(const TileMesh& M, const float* __restrict__ pts, uint32_t i,
                                                       uint32_t j, float3 p, float3 q, bool active,
-                                                      unsigned long long* sum, unsigned& status_bits) {
+                                                      SegLeaf* leaf, unsigned long long* sum,
+                                                      unsigned& status_bits) {
   Seg s;
-  make_seg(s, p, q, (int)i, (int)j);
+  make_seg(s, p, q, (int)i, (int)j, leaf);
   unsigned h = 0, rechecks = 0, visits = 0, tests = 0;
   const bool holds[2] = {!active || box_test_holds(p, q, *M.amax[0]), !active || box_test_holds(p, q, *M.amax[1])};
 #pragma unroll 1
