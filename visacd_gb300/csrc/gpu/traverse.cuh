@@ -193,10 +193,9 @@ __device__ __forceinline__ float min3f(float a, float b, float c) {
   return r;
 }
 
-__device__ __forceinline__ float inv_guard(float d) {
-  float ad = fabsf(d);
-  float g = ad < 1e-30f ? copysignf(1e-30f, d) : d;
-  return __frcp_rn(g);
+// 1 / d, with |d| taken as `least` at least.
+__device__ __forceinline__ float inv_guard(float d, float least) {
+  return __frcp_rn(fabsf(d) < least ? copysignf(least, d) : d);
 }
 
 __device__ __forceinline__ float edge_factor(float dx, float dy, float dz) {
@@ -207,11 +206,11 @@ __device__ __forceinline__ float seg_length(float dx, float dy, float dz) {
   return __fsqrt_rn(__fadd_rn(__fadd_rn(__fmul_rn(dx, dx), __fmul_rn(dy, dy)), __fmul_rn(dz, dz)));
 }
 
-__device__ __forceinline__ void make_seg(Seg& s, float3 p, float3 q, int vi, int vj, SegLeaf* leaf) {
+__device__ __forceinline__ void make_seg(Seg& s, float3 p, float3 q, int vi, int vj, float least, SegLeaf* leaf) {
   const float dx = __fsub_rn(q.x, p.x), dy = __fsub_rn(q.y, p.y), dz = __fsub_rn(q.z, p.z);
-  s.ix = inv_guard(dx);
-  s.iy = inv_guard(dy);
-  s.iz = inv_guard(dz);
+  s.ix = inv_guard(dx, least);
+  s.iy = inv_guard(dy, least);
+  s.iz = inv_guard(dz, least);
   s.ax = fabsf(s.ix);
   s.ay = fabsf(s.iy);
   s.az = fabsf(s.iz);
@@ -230,9 +229,11 @@ __device__ __forceinline__ void make_seg(Seg& s, float3 p, float3 q, int vi, int
 // Conservative slab test of the segment (t in [0, 1]) against the box with
 // centre c and half extents e. Leaf boxes are widened by 2^-19 of the mesh's
 // largest |coordinate| M, 32 units of FP32 rounding; with |p|, |q| <= 4 M the
-// test's own error is below 21 units (in position: one of |p| for p / d, one
-// each of the two FMA results, one of |x - p| for 1 / d), so no slack is
-// needed. box_hit_wide serves points farther out.
+// test's own error is at most 24 units (in position: one of |p| for p / d, one
+// each of the two FMA results, of |x - p| for 1 / d and for the rounding of d), so
+// no slack is needed. A component of d below seg_least counts as that: it moves the
+// segment by far less than the widening, so the interval it gives is still too
+// large. box_hit_wide serves points farther out.
 __device__ __forceinline__ bool box_hit(const Seg& s, float cx, float cy, float cz, float ex, float ey, float ez) {
   const float tx = fmaf(cx, s.ix, s.nx), ty = fmaf(cy, s.iy, s.ny), tz = fmaf(cz, s.iz, s.nz);
   const float tn = max3f(fmaf(-ex, s.ax, tx), fmaf(-ey, s.ay, ty), fmaxf(fmaf(-ez, s.az, tz), 0.f));
@@ -249,13 +250,19 @@ __device__ __forceinline__ bool box_hit_wide(const Seg& s, const float3& p, floa
   tf = fmaf(fabsf(tf), 4e-6f, tf);
   return tn <= tf;
 }
-// Whether box_hit serves a segment against a mesh whose largest |coordinate|
-// is amax (also false for coordinates that are not finite).
-__device__ __forceinline__ bool box_test_holds(float3 p, float3 q, float amax) {
+// The least |component| of a segment's direction: its inverse times a coordinate
+// (of 4 M at most) does not overflow.
+__device__ __forceinline__ float seg_least(float amax0, float amax1) {
+  return fmaxf(1e-30f, 1e-37f * fmaxf(amax0, amax1));
+}
+// Whether box_hit serves a segment made with `least` against a mesh whose largest
+// |coordinate| is amax (also false for coordinates that are not finite).
+__device__ __forceinline__ bool box_test_holds(float3 p, float3 q, float amax, float least) {
   const float m = fmaxf(fmaxf(fmaxf(fabsf(p.x), fabsf(p.y)), fmaxf(fabsf(p.z), fabsf(q.x))),
                         fmaxf(fabsf(q.y), fabsf(q.z)));
   // (fmax drops NaNs: those fail the sum)
-  return amax <= 1e7f && m <= 4.f * amax && fabsf(p.x + p.y + p.z + q.x + q.y + q.z) < INFINITY;
+  return amax <= 1e30f && (least <= 1e-30f || least <= 1e-7f * amax) && m <= 4.f * amax &&
+         fabsf(p.x + p.y + p.z + q.x + q.y + q.z) < INFINITY;
 }
 
 // FP64 segment-triangle decision from the FP32 inputs; identical formula to the
@@ -570,9 +577,11 @@ static __device__ __forceinline__ unsigned trace_tile(const TileMesh& M, const f
                                                       SegLeaf* leaf, unsigned long long* sum,
                                                       unsigned& status_bits) {
   Seg s;
-  make_seg(s, p, q, (int)i, (int)j, leaf);
+  const float amax[2] = {*M.amax[0], *M.amax[1]}, least = seg_least(amax[0], amax[1]);
+  make_seg(s, p, q, (int)i, (int)j, least, leaf);
   unsigned h = 0, rechecks = 0, visits = 0, tests = 0;
-  const bool holds[2] = {!active || box_test_holds(p, q, *M.amax[0]), !active || box_test_holds(p, q, *M.amax[1])};
+  const bool holds[2] = {!active || box_test_holds(p, q, amax[0], least),
+                         !active || box_test_holds(p, q, amax[1], least)};
 #pragma unroll 1
   for (int k = 0; k < 2; ++k) {
     s.exclude = k == 1;
