@@ -52,3 +52,20 @@ def test_info_of_a_bvh_whose_context_went(native, ctx, level):
     assert again.info() == want
     for b in (kept, asked, again):
         b.close()
+
+
+def test_info_takes_little_time(ctx):
+    """The depth of 81,920 triangles right after the build, the median of eleven:
+    0.1 ms; 0.86 with the records brought to the host and walked there."""
+    import time
+    mesh = mg.displaced_blob(6, seed=3)
+    took = []
+    for _ in range(11):
+        b = ctx.bvh(*mesh)
+        ctx.synchronize()
+        t0 = time.perf_counter()
+        depth = b.info()[1]
+        took.append(time.perf_counter() - t0)
+        assert 17 <= depth <= 47
+        b.close()
+    assert np.median(took) < 4e-4
