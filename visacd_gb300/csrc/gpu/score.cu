@@ -595,17 +595,18 @@ static int score_device(visacd_ctx* ctx, const float* d_planes, int32_t P, const
     VLAUNCH(ctx, kKPointStats, grid_for(N, 256, 4LL * ctx->sm_count), 256, 0, point_stats_kernel,
             d_pts, N, cnt->stats);
   }
-  if (E > 0 && P > 0 && !ctx->score_k_override && sides_pay(P, N, E)) {
+  const int32_t pitch = N <= kSidesMaxVertices ? (N + 1) & ~1 : 0;  // a group's row of sides: whole 16 bytes
+  const unsigned groups = (unsigned)((P + 31LL) / 32);
+  // Without room for the sides (up to 320 MB) the call goes edge by edge.
+  if (E > 0 && P > 0 && !ctx->score_k_override && sides_pay(P, N, E) &&
+      ensure_slot(ctx, kSlotRecheck, (size_t)groups * pitch * sizeof(uint2)) == VISACD_OK) {
     const size_t padded = (size_t)((E + 31) & ~31ll);
     VTRY(ensure_slot(ctx, kSlotEdgePack, padded * 8));
     uint32_t* ends = slot<uint32_t>(ctx, kSlotEdgePack);
     uint32_t* lens = ends + padded;
     VLAUNCH(ctx, kKPackEdges, grid_for(E, 256, 8LL * ctx->sm_count), 256, 0, pack_sides_kernel,
             d_pts, N, d_edges, E, cnt->stats, ends, lens, &cnt->skipped);
-    const int32_t pitch = (N + 1) & ~1;  // a group's row starts and ends on 16 bytes
-    const unsigned groups = (unsigned)((P + 31) / 32);
     const float4* pl = reinterpret_cast<const float4*>(d_planes);
-    VTRY(ensure_slot(ctx, kSlotRecheck, (size_t)groups * pitch * sizeof(uint2)));
     uint2* sides = slot<uint2>(ctx, kSlotRecheck);
     VLAUNCH(ctx, kKPlaneSides, dim3((unsigned)((N + 2 * kSideThreads - 1) / (2 * kSideThreads)), groups),
             kSideThreads, 0, plane_sides_kernel, pl, P, d_pts, N, pitch, cnt->stats, sides, &cnt->sides_fp64);
