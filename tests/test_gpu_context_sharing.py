@@ -69,3 +69,36 @@ def test_info_takes_little_time(ctx):
         assert 17 <= depth <= 47
         b.close()
     assert np.median(took) < 4e-4
+
+
+@pytest.mark.parametrize("call", ["visibility", "batch", "graph"])
+def test_a_blocking_context_sleeps_through_anothers_build(native, call):
+    """A context that waits blocking (many contexts sharing the cores) also waits so
+    for a build on another context's stream, here behind 0.3 s of other work: the
+    thread's own time is a small part of the wait."""
+    import time
+    torch = pytest.importorskip("torch")
+    stream = torch.cuda.Stream()
+    other, waiting = native.Context(0, stream=stream.cuda_stream), native.Context(0)
+    assert native.lib().visacd_ctx_set_blocking_wait(waiting.handle, 1) == 0
+    pts = mg.displaced_blob(1, seed=2)[0]
+    cage, none = mg.displaced_blob(2, seed=3), np.zeros((0, 3), np.int32)
+    planes = np.array([[1.0, 0, 0, 0]], np.float32)
+    run = {"visibility": lambda a, b: waiting.visibility(pts, a, b)[0],
+           "batch": lambda a, b: waiting.visibility_batch([(pts, a, b, None)])[0][0],
+           "graph": lambda a, b: native.Batch(waiting, [(pts, a, b, planes)]).close()}[call]
+    a, b = other.bvh(pts, none), other.bvh(*cage)
+    want = run(a, b)  # first-call costs
+    with torch.cuda.stream(stream):
+        torch.cuda._sleep(600_000_000)  # a kernel of some 0.3 s
+    c = other.bvh(*cage)
+    t0, c0 = time.perf_counter(), time.thread_time()
+    got = run(a, c)
+    wall, cpu = time.perf_counter() - t0, time.thread_time() - c0
+    np.testing.assert_array_equal(got, want)
+    assert wall > 0.1  # it did wait
+    assert cpu < 0.3 * wall
+    for x in (a, b, c):
+        x.close()
+    waiting.close()
+    other.close()

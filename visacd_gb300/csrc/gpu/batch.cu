@@ -509,8 +509,9 @@ extern "C" int visacd_batch_create(visacd_ctx* ctx, int32_t n_parts, const float
       set_error("batch_create: part %d BVH does not match its points or is too deep", p);
       return fail(VISACD_ERR_INVALID_ARG);
     }
-    bvh_settle(ctx, self_bvhs[p]);
-    bvh_settle(ctx, cage_bvhs[p]);
+    int settled = bvh_settle(ctx, self_bvhs[p]);
+    if (settled == VISACD_OK) settled = bvh_settle(ctx, cage_bvhs[p]);
+    if (settled) return fail(settled);
     BatchPart& P = hp[p];
     memset(&P, 0, sizeof(P));
     P.n = n;

@@ -347,6 +347,17 @@ static int bvh_build_fast(visacd_ctx* ctx, const float* dv, int32_t nv, const ui
   return VISACD_OK;
 }
 
+int bvh_settle(visacd_ctx* ctx, const visacd_bvh* b) {
+  if (!b || !b->ctx || b->stream == ctx->stream) return VISACD_OK;
+  if (ctx->blocking_wait && ctx->wait_event) {
+    VCUDA(cudaEventRecord(ctx->wait_event, b->stream));
+    VCUDA(cudaEventSynchronize(ctx->wait_event));
+  } else {
+    VCUDA(cudaStreamSynchronize(b->stream));
+  }
+  return VISACD_OK;
+}
+
 int bvh_head(visacd_ctx* ctx, visacd_bvh* b) {
   if (b->head_read || !b->head) return VISACD_OK;
   BvhHead* h = nullptr;

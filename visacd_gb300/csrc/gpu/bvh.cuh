@@ -84,10 +84,8 @@ int bvh_depth(visacd_bvh* b);
 // Reads the BVH's head to the host (waits for the stream; once per BVH).
 int bvh_head(visacd_ctx* ctx, visacd_bvh* b);
 // A build may still be running on its context's stream: a call on another
-// stream waits for that one first.
-inline void bvh_settle(visacd_ctx* ctx, const visacd_bvh* b) {
-  if (b && b->ctx && b->stream != ctx->stream) cudaStreamSynchronize(b->stream);
-}
+// stream waits for that one first, in the way its own context waits.
+int bvh_settle(visacd_ctx* ctx, const visacd_bvh* b);
 // Builds the BVH's free-space grid (once; a BVH whose grid would not be
 // usable keeps none), its resolution sized for a call over `pairs` pairs. Uses the context's counter slot and pinned staging
 // buffer (waits for the stream first), so it runs before a call takes them.

@@ -997,10 +997,10 @@ int visibility_multi_impl(visacd_ctx* ctx, int32_t n_parts, const float* const* 
     const visacd_bvh* cb = cage_bvhs[p];
     VCHECK(n >= 0 && (n == 0 || pts[p]) && sb && cb, VISACD_ERR_INVALID_ARG, "visibility_batch: bad part %d", p);
     VCHECK(n <= (1 << 24), VISACD_ERR_INVALID_ARG, "visibility_batch: part %d has n = %d above 2^24", p, n);
-    bvh_settle(ctx, sb);
-    bvh_settle(ctx, cb);
     VCHECK(sb->ctx && cb->ctx && sb->device == ctx->device && cb->device == ctx->device,
            VISACD_ERR_INVALID_ARG, "visibility_batch: part %d BVH is not on this context's device", p);
+    VTRY(bvh_settle(ctx, sb));
+    VTRY(bvh_settle(ctx, cb));
     VCHECK(sb->depth <= kStack && cb->depth <= kStack, VISACD_ERR_INVALID_ARG,
            "visibility_batch: part %d BVH depth %d/%d exceeds the traversal stack (%d)", p, sb->depth,
            cb->depth, kStack);
@@ -1263,8 +1263,8 @@ int visibility_impl(visacd_ctx* ctx, const float* pts, int32_t n, const uint8_t*
   const uint8_t* d_new = is_new;
   int64_t pairs = (int64_t)n * (n > 0 ? n - 1 : 0) / 2;
   int32_t n_new = 0;
-  bvh_settle(ctx, self_bvh);
-  bvh_settle(ctx, cage_bvh);
+  VTRY(bvh_settle(ctx, self_bvh));
+  VTRY(bvh_settle(ctx, cage_bvh));
   if (is_new) {
     int64_t k = 0;
     if (device_ptrs && n > 0) {
