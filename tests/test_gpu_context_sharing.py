@@ -102,3 +102,17 @@ def test_a_blocking_context_sleeps_through_anothers_build(native, call):
         x.close()
     waiting.close()
     other.close()
+
+
+@pytest.mark.parametrize("which", ["part", "cage"])
+def test_a_batch_refuses_a_bvh_whose_context_went(native, ctx, which):
+    v, t = mg.displaced_blob(1, seed=2)
+    cage = mg.offset_cage(v, t, 0.05)
+    other = native.Context(0)
+    a = (other if which == "part" else ctx).bvh(v, t)
+    b = (other if which == "cage" else ctx).bvh(*cage)
+    other.close()
+    with pytest.raises(native.VisacdError):
+        native.Batch(ctx, [(v, a, b, np.array([[1.0, 0, 0, 0]], np.float32))]).close()
+    a.close()
+    b.close()

@@ -504,6 +504,11 @@ extern "C" int visacd_batch_create(visacd_ctx* ctx, int32_t n_parts, const float
       set_error("batch_create: bad part %d", p);
       return fail(VISACD_ERR_INVALID_ARG);
     }
+    if (!self_bvhs[p]->ctx || !cage_bvhs[p]->ctx || self_bvhs[p]->device != ctx->device ||
+        cage_bvhs[p]->device != ctx->device) {
+      set_error("batch_create: part %d BVH is not on this context's device", p);
+      return fail(VISACD_ERR_INVALID_ARG);
+    }
     if (self_bvhs[p]->depth > kStack || cage_bvhs[p]->depth > kStack ||
         (self_bvhs[p]->nt > 0 && self_bvhs[p]->nv != n)) {
       set_error("batch_create: part %d BVH does not match its points or is too deep", p);
