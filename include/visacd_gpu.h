@@ -243,13 +243,17 @@ int visacd_compute_intersection_matrix(visacd_ctx* ctx, const float* verts, int3
 int visacd_score_planes(visacd_ctx* ctx, const float* planes, int32_t P, const float* points,
                         int32_t N, const uint32_t* edges, int64_t E, int device_ptrs,
                         double* scores, visacd_score_stats* stats);
-/* Planes per scoring thread (1, 2, 4 or 8; the scores do not depend on it):
-   visacd_ctx_set_score_k forces one (0: the autotuned choice of the call's
-   shape class if one was measured, else a rule on P). visacd_autotune_scoring
-   times each on this exact call (twice, CUDA events on the context stream),
-   caches the fastest for the call's shape class (log2 buckets of P and E) in
-   the context and reports it; ms_per_k (optional) gets 4 entries. Resets the
-   context's kernel timers. */
+/* Planes per scoring thread (1, 2, 4 or 8; the scores do not depend on it) of the
+   kernel that goes edge by edge. Calls with no fewer edges than vertices decide the
+   vertices' sides first and have no such choice.
+   visacd_ctx_set_score_k forces one, and with it the edge-by-edge kernel (0: the
+   autotuned choice of the call's shape class if one was measured, else a model of
+   the waves of CTAs). visacd_autotune_scoring times each on this exact call (twice,
+   CUDA events on the context stream), caches the fastest for the call's shape class
+   (log2 buckets of P and E) in the context and reports it; ms_per_k (optional) gets
+   4 entries. For a call that can go by vertex sides it times that too, and caches
+   which of the two is faster for the class with N's bucket. Resets the context's
+   kernel timers. */
 int visacd_ctx_set_score_k(visacd_ctx* ctx, int k);
 int visacd_autotune_scoring(visacd_ctx* ctx, const float* planes, int32_t P, const float* points,
                             int32_t N, const uint32_t* edges, int64_t E, int device_ptrs, int* best_k,

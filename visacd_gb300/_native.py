@@ -295,8 +295,9 @@ class Context:
         _check(lib().visacd_ctx_set_score_k(self._h, int(k)), "visacd_ctx_set_score_k")
 
     def autotune_scoring(self, planes, points, edges):
-        """Time 1, 2, 4 and 8 planes per thread on this call, cache the fastest
-        for its shape class: (best, ms per choice)."""
+        """Time 1, 2, 4 and 8 planes per thread on this call and, where it can go
+        that way, vertex sides; cache the fastest for its shape class: (best planes
+        per thread, ms per choice of them)."""
         pl = _f32(planes, 4)
         pt = _f32(points, 3)
         ed = _u32(edges, 2)

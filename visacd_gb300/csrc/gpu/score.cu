@@ -488,10 +488,11 @@ static int sides_slices(int sm_count, int32_t P, int32_t n, int64_t E) {
   return best;
 }
 
-// Shape class of a scoring call: log2 buckets of P and E.
-static uint32_t score_shape_class(int32_t P, int64_t E) {
+// Shape class of a scoring call: log2 buckets of P and E (and of N, where the choice
+// is between vertex sides and edges).
+static uint32_t score_shape_class(int32_t P, int64_t E, int32_t N = 0) {
   auto lg = [](int64_t x) { int r = 0; while (x > 1) { x >>= 1; ++r; } return r; };
-  return (uint32_t)lg(P) | ((uint32_t)lg(E) << 8);
+  return (uint32_t)lg(P) | ((uint32_t)lg(E) << 8) | ((uint32_t)lg(N) << 16);
 }
 
 // How a call is split into CTAs: each takes 256 K planes and a run of `per` edge
@@ -580,6 +581,13 @@ static bool sides_pay(int32_t P, int32_t N, int64_t E) {
   return N > 0 && N <= kSidesMaxVertices && E >= N && groups <= kSidesMaxGroups && groups * N <= kSidesMaxScratch;
 }
 
+// The autotuner's choice for the call's class if it was timed, else sides_pay.
+static bool by_sides(const visacd_ctx* ctx, int32_t P, int32_t N, int64_t E) {
+  if (ctx->score_k_override || !sides_pay(P, N, E)) return false;
+  auto it = ctx->score_tuned_edges.find(score_shape_class(P, E, N));
+  return it == ctx->score_tuned_edges.end() || !it->second;
+}
+
 // Core of every scoring entry point that may allocate. All pointers are device pointers.
 static int score_device(visacd_ctx* ctx, const float* d_planes, int32_t P, const float* d_pts,
                         int32_t N, const uint32_t* d_edges, int64_t E, double* d_scores,
@@ -598,7 +606,7 @@ static int score_device(visacd_ctx* ctx, const float* d_planes, int32_t P, const
   const int32_t pitch = N <= kSidesMaxVertices ? (N + 1) & ~1 : 0;  // a group's row of sides: whole 16 bytes
   const unsigned groups = (unsigned)((P + 31LL) / 32);
   // Without room for the sides (up to 320 MB) the call goes edge by edge.
-  if (E > 0 && P > 0 && !ctx->score_k_override && sides_pay(P, N, E) &&
+  if (E > 0 && P > 0 && by_sides(ctx, P, N, E) &&
       ensure_slot(ctx, kSlotRecheck, (size_t)groups * pitch * sizeof(uint2)) == VISACD_OK) {
     const size_t padded = (size_t)((E + 31) & ~31ll);
     VTRY(ensure_slot(ctx, kSlotEdgePack, padded * 8));
@@ -761,14 +769,18 @@ extern "C" int visacd_autotune_scoring(visacd_ctx* ctx, const float* planes, int
   VCHECK(ctx, VISACD_ERR_INVALID_ARG, "autotune_scoring: null context");
   const int saved_override = ctx->score_k_override;
   const bool saved_timing = ctx->timing;
-  static const int kKs[4] = {1, 2, 4, 8};
+  // Each K edge by edge; then, where the call can go that way, by vertex sides.
+  static const int kKs[5] = {1, 2, 4, 8, 0};
+  const uint32_t both = score_shape_class(P, E, N);
+  const bool sides = E > 0 && P > 0 && sides_pay(P, N, E);
+  ctx->score_tuned_edges.erase(both);
   int best = 0;
-  double best_ms = 1e300;
+  double best_ms = 1e300, best_all = 1e300;  // scoring alone, and with the packing
   int rc = VISACD_OK;
   std::vector<double> scores((size_t)(P > 0 ? P : 1));
-  for (int v = 0; v < 4 && rc == VISACD_OK; ++v) {
+  for (int v = 0; v < (sides ? 5 : 4) && rc == VISACD_OK; ++v) {
     ctx->score_k_override = kKs[v];
-    double ms = 0.0;
+    double ms = 0.0, pack = 0.0;
     for (int rep = 0; rep < 2 && rc == VISACD_OK; ++rep) {
       ctx->timing = true;
       rc = visacd_ctx_reset_times(ctx);
@@ -786,16 +798,25 @@ extern "C" int visacd_autotune_scoring(visacd_ctx* ctx, const float* planes, int
       int64_t cnt[64];
       int nk = 0;
       if (rc == VISACD_OK) rc = visacd_ctx_kernel_times(ctx, names, t, cnt, 64, &nk);
-      ms = 0.0;
-      for (int k = 0; k < nk && k < 64; ++k)
-        if (strcmp(names[k], kernel_name(kKScore)) == 0 || strcmp(names[k], kernel_name(kKScoreRecheck)) == 0)
+      ms = pack = 0.0;
+      for (int k = 0; k < nk && k < 64; ++k) {
+        if (strcmp(names[k], kernel_name(kKScore)) == 0 || strcmp(names[k], kernel_name(kKScoreRecheck)) == 0 ||
+            strcmp(names[k], kernel_name(kKPlaneSides)) == 0)
           ms += t[k];
+        else if (strcmp(names[k], kernel_name(kKPackEdges)) == 0)
+          pack += t[k];
+      }
+    }
+    if (v == 4) {
+      if (rc == VISACD_OK) ctx->score_tuned_edges[both] = best_all < ms + pack;
+      break;
     }
     if (ms_per_k) ms_per_k[v] = ms;
     if (ms < best_ms) {
       best_ms = ms;
       best = kKs[v];
     }
+    best_all = std::min(best_all, ms + pack);
   }
   ctx->score_k_override = saved_override;
   ctx->timing = saved_timing;
