@@ -107,10 +107,17 @@ struct SdfTri {
   float blo[3], bhi[3];   // bounding box rounded outwards
   float4 pl;              // unit normal, offset; w of fe[0] = -1e30 without a plane
   float4 fe[3];           // unit in-plane edge normals, offsets (no vertex beyond)
-  int has_plane, pad[3];
+  int has_plane, irregular, pad[2];
   int ray[3][4];          // per axis: first ray and extents over (u, w); extents 0: none
   float v[3][3], vabs;    // vertices in FP32, their largest coordinate
   int pad2[2];
+};
+
+// What the passes share beside the voxels.
+struct SdfFlags {
+  unsigned n_wide;     // listed triangles of sdf_cross_wide_kernel
+  unsigned n_far;      // whether sdf_far_dist_kernel has work
+  unsigned irregular;  // whether a triangle is irregular
 };
 
 constexpr int kSdfChunk = 256;  // box voxels per work item of the distance passes (one warp)
@@ -121,7 +128,8 @@ __device__ __forceinline__ void box_range(const SdfGrid& g, int a, double mn, do
 }
 
 __global__ void sdf_tri_prep_kernel(const double* __restrict__ P, const int32_t* __restrict__ T, int nt, SdfGrid g,
-                                    SdfTri* __restrict__ out, uint32_t* __restrict__ chunks) {
+                                    SdfTri* __restrict__ out, uint32_t* __restrict__ chunks,
+                                    SdfFlags* __restrict__ flags) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
     double A[3], B[3], C[3];
     load_tri(P, T, t, A, B, C);
@@ -139,6 +147,16 @@ __global__ void sdf_tri_prep_kernel(const double* __restrict__ P, const int32_t*
     double nx = uy * vz - uz * vy, ny = uz * vx - ux * vz, nz = ux * vy - uy * vx;
     const double nl = sqrt(nx * nx + ny * ny + nz * nz);
     r.has_plane = nl > 1e-12;
+    // Irregular: so thin that the exact formula's closest point may be off by 1e-3
+    // voxels or lie outside (its weights are quotients of products of this size, with
+    // an error of some 1e-14 of L^2 (L + band)^2), or NaN. What it gives is the
+    // result, so no bound may spare it: it is evaluated for every voxel of its box,
+    // and bounds nothing; every voxel then needs its distance.
+    const double wx = C[0] - B[0], wy = C[1] - B[1], wz = C[2] - B[2];
+    const double l2 = fmax(fmax(ux * ux + uy * uy + uz * uz, vx * vx + vy * vy + vz * vz), wx * wx + wy * wy + wz * wz);
+    const double len = sqrt(l2), reachable = len + g.band;
+    r.irregular = !(nl * nl >= 1e-11 * l2 * len * reachable * reachable);
+    if (r.irregular) flags->irregular = flags->n_far = 1u;
     r.pl = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int e = 0; e < 3; ++e) r.fe[e] = make_float4(0.f, 0.f, 0.f, -1e30f);
     if (r.has_plane) {
@@ -309,6 +327,7 @@ __global__ void __launch_bounds__(128) sdf_ub_kernel(SdfItems W, SdfGrid g, cons
   for (long long w = w0; w < w1; ++w) {
     while ((long long)W.off[t + 1] <= w) ++t;
     const SdfTri& r = prep[t];
+    if (r.irregular) continue;
     // rounding of the vertices to float, of the chosen point and of its
     // distance: a few units of 2^-24 of the largest coordinate involved
     const int n = r.ext[0] * r.ext[1] * r.ext[2];
@@ -406,7 +425,9 @@ __global__ void __launch_bounds__(128, kDistBlocks) sdf_dist_kernel(const double
         // the other side
         if (c == kClassOut && up < g.low_out) cur = 0.f;
         if (cur > 0.f) {
-          const float lb = sdf_lower_bound(r, (float)(g.org[0] + i), (float)(g.org[1] + j), (float)(g.org[2] + k));
+          const float lb = r.irregular ? -3.0e38f
+                                       : sdf_lower_bound(r, (float)(g.org[0] + i), (float)(g.org[1] + j),
+                                                         (float)(g.org[2] + k));
           keep = lb - 2.0f * g.margin < fminf(cur, __uint_as_float(*(volatile const uint32_t*)&dist[v]));
         }
       }
@@ -462,7 +483,9 @@ __global__ void __launch_bounds__(128, kDistBlocks)
       if (base + lane < c1) {
         const int i = lo[0] + at.i, j = lo[1] + at.j, k = lo[2] + at.k;
         v = vid(g, i, j, k);
-        if (cls[v] & kClassFar) {
+        if (r.irregular) {
+          keep = true;
+        } else if (cls[v] & kClassFar) {
           const float lb = sdf_lower_bound(r, (float)(g.org[0] + i), (float)(g.org[1] + j), (float)(g.org[2] + k));
           keep = lb - 2.0f * g.margin < __uint_as_float(*(volatile const uint32_t*)&dist[v]);
         }
@@ -690,11 +713,13 @@ __global__ void __launch_bounds__(128) sdf_inside_kernel(SdfGrid g, const uint32
   }
 }
 
-// Marks voxels with a neighbour of the other class (all: every voxel, when
-// the range of class_cut does not apply), and starts both distance arrays at the
+// Marks voxels with a neighbour of the other class (all, or a mesh with irregular
+// triangles: every voxel, since the range of class_cut does not apply), and starts both distance arrays at the
 // band.
-__global__ void sdf_class_kernel(SdfGrid g, const uint8_t* __restrict__ inside, int all, uint32_t band,
-                                 uint8_t* __restrict__ cls, uint32_t* __restrict__ ub, uint32_t* __restrict__ dist) {
+__global__ void sdf_class_kernel(SdfGrid g, const uint8_t* __restrict__ inside, int all,
+                                 const SdfFlags* __restrict__ flags, uint32_t band, uint8_t* __restrict__ cls,
+                                 uint32_t* __restrict__ ub, uint32_t* __restrict__ dist) {
+  if (flags->irregular) all = 1;
   const size_t n = (size_t)g.dim[0] * g.dim[1] * g.dim[2];
   const size_t sy = g.dim[0], sz = (size_t)g.dim[0] * g.dim[1];
   for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (size_t)gridDim.x * blockDim.x) {
@@ -900,7 +925,7 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   };
   const size_t oP = take(P.size() * 8), oT = take(3 * (size_t)nt * 4);
   const size_t upload = at;
-  const size_t oTog = take(nvox * 4), oNWide = take(16);  // + the far flag
+  const size_t oTog = take(nvox * 4), oFlags = take(sizeof(SdfFlags));
   const size_t zero_end = at;
   const size_t oPrep = take((size_t)nt * sizeof(SdfTri)), oWide = take(3 * (size_t)nt * 4),
                oChunks = take((size_t)nt * 4), oChunkOff = take(((size_t)nt + 1) * 8), oDist = take(nvox * 4),
@@ -935,12 +960,13 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   SdfTri* prep = (SdfTri*)(base + oPrep);
   uint32_t* chunks = (uint32_t*)(base + oChunks);
   uint64_t* chunk_off = (uint64_t*)(base + oChunkOff);
+  SdfFlags* flags = (SdfFlags*)(base + oFlags);
+  unsigned *n_wide = &flags->n_wide, *n_far = &flags->n_far;
   VLAUNCH(ctx, kKSdfDist, grid_for(nt, 64, 32 * (int64_t)ctx->sm_count), 64, 0, sdf_tri_prep_kernel, dP, dT, nt,
-          g, prep, chunks);
+          g, prep, chunks, flags);
   // Crossings of all three axes, the triangles covering many rays one block
   // each, then the parities and classes.
   int* wide = (int*)(base + oWide);
-  unsigned* n_wide = (unsigned*)(base + oNWide);
   VLAUNCH(ctx, kKSdfCross, dim3(grid_for((int64_t)kCrossLanes * nt, 128, 16 * (int64_t)ctx->sm_count), 3), 128, 0,
           sdf_cross_kernel, dP, dT, nt, g, (const SdfTri*)prep, tog, wide, n_wide);
   VLAUNCH(ctx, kKSdfCross, (unsigned)std::min<int64_t>(3LL * nt, 4 * (int64_t)ctx->sm_count), 128, 0,
@@ -950,8 +976,8 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
           sdf_parity_yz_kernel, g, (const uint32_t*)tog, par_y, par_z);
   VLAUNCH(ctx, kKSdfCross, grid_for(32LL * g.dim[1] * g.dim[2], 128, 16 * (int64_t)ctx->sm_count), 128, 0,
           sdf_inside_kernel, g, (const uint32_t*)tog, (const uint8_t*)par_y, (const uint8_t*)par_z, inside);
-  VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_class_kernel, g, (const uint8_t*)inside, all_exact ? 1 : 0, band_bits, cls, ub,
-          dist);
+  VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_class_kernel, g, (const uint8_t*)inside, all_exact ? 1 : 0,
+          (const SdfFlags*)flags, band_bits, cls, ub, dist);
   VTRY(exclusive_scan_u32_to_u64(ctx, chunks, chunk_off, nt));
   SdfItems items;
   items.off = chunk_off;
@@ -962,7 +988,6 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_dist_kernel, dP, dT, items, g, (const SdfTri*)prep, (const uint8_t*)cls,
           (const uint32_t*)ub, dist);
   if (g.reach < g.band) {
-    unsigned* n_far = n_wide + 1;
     VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_far_kernel, g, nvox, (const uint32_t*)dist, (const uint32_t*)ub, cls, n_far);
     VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_far_dist_kernel, dP, dT, items, g, (const SdfTri*)prep, (const uint8_t*)cls,
             (const unsigned*)n_far, dist);
