@@ -117,6 +117,7 @@ struct SdfTri {
 struct SdfFlags {
   unsigned n_wide;     // listed triangles of sdf_cross_wide_kernel
   unsigned n_far;      // whether sdf_far_dist_kernel has work
+  unsigned n_thin;     // listed triangles of irregular_triangle
   unsigned irregular;  // whether a triangle is irregular
 };
 
@@ -128,7 +129,7 @@ __device__ __forceinline__ void box_range(const SdfGrid& g, int a, double mn, do
 }
 
 __global__ void sdf_tri_prep_kernel(const double* __restrict__ P, const int32_t* __restrict__ T, int nt, SdfGrid g,
-                                    SdfTri* __restrict__ out, uint32_t* __restrict__ chunks,
+                                    SdfTri* __restrict__ out, uint32_t* __restrict__ chunks, int* __restrict__ thin,
                                     SdfFlags* __restrict__ flags) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
     double A[3], B[3], C[3];
@@ -147,16 +148,14 @@ __global__ void sdf_tri_prep_kernel(const double* __restrict__ P, const int32_t*
     double nx = uy * vz - uz * vy, ny = uz * vx - ux * vz, nz = ux * vy - uy * vx;
     const double nl = sqrt(nx * nx + ny * ny + nz * nz);
     r.has_plane = nl > 1e-12;
-    // Irregular: so thin that the exact formula's closest point may be off by 1e-3
-    // voxels or lie outside (its weights are quotients of products of this size, with
-    // an error of some 1e-14 of L^2 (L + band)^2), or NaN. What it gives is the
-    // result, so no bound may spare it: it is evaluated for every voxel of its box,
-    // and bounds nothing; every voxel then needs its distance.
+    // Thin: the exact formula's closest point may be off by 1e-3 voxels or lie outside
+    // (its weights are quotients of products of this size, with an error of some 1e-14
+    // of L^2 (L + band)^2), or be NaN. irregular_triangle looks whether it is.
     const double wx = C[0] - B[0], wy = C[1] - B[1], wz = C[2] - B[2];
     const double l2 = fmax(fmax(ux * ux + uy * uy + uz * uz, vx * vx + vy * vy + vz * vz), wx * wx + wy * wy + wz * wz);
     const double len = sqrt(l2), reachable = len + g.band;
-    r.irregular = !(nl * nl >= 1e-11 * l2 * len * reachable * reachable);
-    if (r.irregular) flags->irregular = flags->n_far = 1u;
+    if (!(nl * nl >= 1e-11 * l2 * len * reachable * reachable)) thin[atomicAdd(&flags->n_thin, 1u)] = t;
+    r.irregular = 0;
     r.pl = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int e = 0; e < 3; ++e) r.fe[e] = make_float4(0.f, 0.f, 0.f, -1e30f);
     if (r.has_plane) {
@@ -316,6 +315,54 @@ __device__ __forceinline__ float sdf_lower_bound(const SdfTri& r, float qx, floa
     lb = fmaxf(lb, sqrtf(pd * pd + se * se));
   }
   return lb;
+}
+
+__device__ __forceinline__ float segment_dist32(const float (&q)[3], const float* a, const float* b) {
+  const float dx = b[0] - a[0], dy = b[1] - a[1], dz = b[2] - a[2];
+  const float px = q[0] - a[0], py = q[1] - a[1], pz = q[2] - a[2];
+  const float k = fminf(fmaxf((px * dx + py * dy + pz * dz) / (dx * dx + dy * dy + dz * dz), 0.f), 1.f);
+  const float ex = px - k * dx, ey = py - k * dy, ez = pz - k * dz;
+  return sqrtf(ex * ex + ey * ey + ez * ez);
+}
+
+// A thin triangle, its part `part` of `parts` by a block: irregular when the exact
+// formula leaves the bounds, or is not the distance to the nearest edge less at most
+// the triangle's height, at some voxel of its box grown by the band. What the formula
+// gives is the result, so an irregular triangle bounds nothing, is evaluated for every
+// voxel of that box, and makes every voxel of the grid take its exact distance (the
+// range of class_cut supposes that neighbours' distances differ by at most 1, with
+// 0.01 to spare). Else it is a triangle like others. Meshes cut by the pipeline hold
+// some thin triangles and hardly an irregular one: with all thin ones taken for
+// irregular a process of a cut bowl took 6 % longer, now the time without the test.
+constexpr double kThinHeight = 2e-3;
+__device__ __noinline__ void irregular_triangle(const double* __restrict__ P, const int32_t* __restrict__ T, int t,
+                                                int part, int parts, const SdfGrid& g, SdfTri* __restrict__ prep,
+                                                SdfFlags* __restrict__ flags) {
+  double A[3], B[3], C[3];
+  load_tri(P, T, t, A, B, C);
+  int lo[3], ext[3];
+#pragma unroll
+  for (int a = 0; a < 3; ++a)
+    box_range(g, a, min3(A[a], B[a], C[a]), max3(A[a], B[a], C[a]), g.band, lo[a], ext[a]);
+  if (ext[0] <= 0 || ext[1] <= 0 || ext[2] <= 0) return;
+  const SdfTri& r = prep[t];
+  const volatile int* found = &r.irregular;
+  const int n = ext[0] * ext[1] * ext[2];
+  for (int k = part * (int)blockDim.x + (int)threadIdx.x; k < n && !*found; k += parts * (int)blockDim.x) {
+    const int i = k % ext[0], j = k / ext[0] % ext[1], l = k / (ext[0] * ext[1]);
+    const float q[3] = {(float)(g.org[0] + lo[0] + i), (float)(g.org[1] + lo[1] + j), (float)(g.org[2] + lo[2] + l)};
+    const double p[3] = {(double)q[0], (double)q[1], (double)q[2]};
+    const float big = kSdfU * fmaxf(r.vabs, fmaxf(fabsf(q[0]), fmaxf(fabsf(q[1]), fabsf(q[2]))));
+    const float edge = fminf(segment_dist32(q, r.v[0], r.v[1]),
+                             fminf(segment_dist32(q, r.v[1], r.v[2]), segment_dist32(q, r.v[2], r.v[0])));
+    const double d = point_tri_dist(p, A, B, C);
+    if (!(fabs(d - (double)edge) <= kThinHeight + (double)(8.0f * big) &&
+          d >= (double)(sdf_lower_bound(r, q[0], q[1], q[2]) - 2.0f * g.margin) &&
+          d <= (double)tri_dist_ub32(q[0], q[1], q[2], r.v[0], r.v[1], r.v[2], 64.0f * big + g.margin))) {
+      prep[t].irregular = 1;
+      flags->irregular = flags->n_far = 1u;
+    }
+  }
 }
 
 __global__ void __launch_bounds__(128) sdf_ub_kernel(SdfItems W, SdfGrid g, const SdfTri* __restrict__ prep,
@@ -693,10 +740,14 @@ __global__ void __launch_bounds__(64) sdf_parity_yz_kernel(SdfGrid g, const uint
 
 // Prefix parity along x (one warp per row, 32 voxels at a time by ballot) and
 // the class of every voxel: inside when at least two parities are odd.
+// Then the thin triangles, all blocks sharing them.
 __global__ void __launch_bounds__(128) sdf_inside_kernel(SdfGrid g, const uint32_t* __restrict__ toggle,
                                                          const uint8_t* __restrict__ par_y,
                                                          const uint8_t* __restrict__ par_z,
-                                                         uint8_t* __restrict__ inside) {
+                                                         uint8_t* __restrict__ inside, const double* __restrict__ P,
+                                                         const int32_t* __restrict__ T, SdfTri* __restrict__ prep,
+                                                         const int* __restrict__ thin, SdfFlags* __restrict__ flags) {
+  const int n_thin = (int)flags->n_thin;
   const int lane = threadIdx.x & 31;
   const int rows = g.dim[1] * g.dim[2], warps = (gridDim.x * blockDim.x) >> 5;
   for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
@@ -711,6 +762,9 @@ __global__ void __launch_bounds__(128) sdf_inside_kernel(SdfGrid g, const uint32
       carry += __popc(m);
     }
   }
+  const int parts = max(1, (int)gridDim.x / max(1, n_thin));
+  for (int k = blockIdx.x; k < n_thin * parts; k += gridDim.x)
+    irregular_triangle(P, T, thin[k / parts], k % parts, parts, g, prep, flags);
 }
 
 // Marks voxels with a neighbour of the other class (all, or a mesh with irregular
@@ -927,7 +981,7 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   const size_t upload = at;
   const size_t oTog = take(nvox * 4), oFlags = take(sizeof(SdfFlags));
   const size_t zero_end = at;
-  const size_t oPrep = take((size_t)nt * sizeof(SdfTri)), oWide = take(3 * (size_t)nt * 4),
+  const size_t oPrep = take((size_t)nt * sizeof(SdfTri)), oWide = take(3 * (size_t)nt * 4), oThin = take((size_t)nt * 4),
                oChunks = take((size_t)nt * 4), oChunkOff = take(((size_t)nt + 1) * 8), oDist = take(nvox * 4),
                oUb = take(nvox * 4), oPy = take(nvox), oPz = take(nvox), oIn = take(nvox), oCls = take(nvox),
                oF = take(nvox * 4), oFlag = take(ncell * 4), oCoff = take((ncell + 1) * 8), oCv = take(ncell * 4),
@@ -961,9 +1015,10 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   uint32_t* chunks = (uint32_t*)(base + oChunks);
   uint64_t* chunk_off = (uint64_t*)(base + oChunkOff);
   SdfFlags* flags = (SdfFlags*)(base + oFlags);
+  int* thin = (int*)(base + oThin);
   unsigned *n_wide = &flags->n_wide, *n_far = &flags->n_far;
   VLAUNCH(ctx, kKSdfDist, grid_for(nt, 64, 32 * (int64_t)ctx->sm_count), 64, 0, sdf_tri_prep_kernel, dP, dT, nt,
-          g, prep, chunks, flags);
+          g, prep, chunks, thin, flags);
   // Crossings of all three axes, the triangles covering many rays one block
   // each, then the parities and classes.
   int* wide = (int*)(base + oWide);
@@ -975,7 +1030,8 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
           dim3(grid_for((int64_t)g.dim[0] * std::max(g.dim[1], g.dim[2]), 64, 32 * (int64_t)ctx->sm_count), 2), 64, 0,
           sdf_parity_yz_kernel, g, (const uint32_t*)tog, par_y, par_z);
   VLAUNCH(ctx, kKSdfCross, grid_for(32LL * g.dim[1] * g.dim[2], 128, 16 * (int64_t)ctx->sm_count), 128, 0,
-          sdf_inside_kernel, g, (const uint32_t*)tog, (const uint8_t*)par_y, (const uint8_t*)par_z, inside);
+          sdf_inside_kernel, g, (const uint32_t*)tog, (const uint8_t*)par_y, (const uint8_t*)par_z, inside,
+          dP, dT, prep, (const int*)thin, flags);
   VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_class_kernel, g, (const uint8_t*)inside, all_exact ? 1 : 0,
           (const SdfFlags*)flags, band_bits, cls, ub, dist);
   VTRY(exclusive_scan_u32_to_u64(ctx, chunks, chunk_off, nt));
