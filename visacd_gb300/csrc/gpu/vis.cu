@@ -181,11 +181,14 @@ struct WalkSums {
 // is lane_pair's; the row's point stays in registers along a tile row, and the
 // next tile is the next of the row or the first of the next row. Tiles with
 // lanes left are listed as base + their number, a run's together with one atomic
-// (18 M pairs in an open soup, nearly all left: 0.20 ms, 0.44 with one a tile).
+// (18 M pairs in an open soup, nearly all left: 0.20 ms, 0.44 with one a tile). The
+// run's done lanes wait in `run` (kWalkRun words of the warp's in shared memory): a
+// register more and visibility_multi_walk_kernel spills (1.82 ms for a bowl's parts,
+// 1.48 so).
 template <int TR>
 __device__ __forceinline__ void walk_tiles(const VisParams& P, unsigned long long w, int count,
                                            unsigned long long base, int lane, WalkSums& sum,
-                                           unsigned long long* __restrict__ pending,
+                                           uint32_t* __restrict__ run, unsigned long long* __restrict__ pending,
                                            unsigned long long* __restrict__ pend_tiles,
                                            uint32_t* __restrict__ pend_done) {
   constexpr int TC = 32 / TR;
@@ -193,7 +196,7 @@ __device__ __forceinline__ void walk_tiles(const VisParams& P, unsigned long lon
   tile_of(P, w, tr64, tc64, TR, TC);
   static_assert(kWalkRun <= 32, "a lane per tile of a run");
   int tr = (int)tr64, tc = (int)tc64, row = -1;
-  uint32_t oi = 0, mask = 0xffffffffu;  // mask: lane k's is the done lanes of tile k
+  uint32_t oi = 0;
   float px = 0.f, py = 0.f, pz = 0.f;
   for (int k = 0; k < count; ++k) {
     const int a = tr * TR + lane / TC, b = tc * TC + lane % TC;
@@ -233,12 +236,14 @@ __device__ __forceinline__ void walk_tiles(const VisParams& P, unsigned long lon
       }
     }
     const unsigned m = __ballot_sync(0xffffffffu, done);
-    if (lane == k) mask = m;
+    if (lane == 0) run[k] = m;
     if (++tc >= P.ntc) {
       ++tr;
       tc = P.triangular ? tr * TR / TC : 0;
     }
   }
+  __syncwarp();
+  const uint32_t mask = lane < count ? run[lane] : 0xffffffffu;
   const unsigned left = __ballot_sync(0xffffffffu, mask != 0xffffffffu);
   if (left) {
     unsigned long long at = 0;
@@ -249,6 +254,7 @@ __device__ __forceinline__ void walk_tiles(const VisParams& P, unsigned long lon
       pend_done[at] = mask;
     }
   }
+  __syncwarp();
 }
 
 __device__ __forceinline__ void walk_flush(VisCounters* __restrict__ cnt, int lane, const WalkSums& sum) {
@@ -383,6 +389,8 @@ __global__ void __launch_bounds__(kVisThreads, MINB) visibility_kernel(VisParams
 template <int TR>
 __global__ void __launch_bounds__(kVisThreads, kWalkBlocks) visibility_walk_kernel(VisParams P) {
   const int lane = threadIdx.x & 31;
+  __shared__ uint32_t runs[kVisThreads / 32][kWalkRun];
+  uint32_t* run = runs[threadIdx.x >> 5];
   WalkSums sum = {};
   for (int guard = 0; guard < (1 << 30); ++guard) {
     unsigned long long w = 0;
@@ -390,7 +398,7 @@ __global__ void __launch_bounds__(kVisThreads, kWalkBlocks) visibility_walk_kern
     w = __shfl_sync(0xffffffffu, w, 0);
     if (w >= P.total_tiles) break;
     const int count = (int)min((unsigned long long)kWalkRun, P.total_tiles - w);
-    walk_tiles<TR>(P, w, count, 0ull, lane, sum, &P.cnt->pending, P.pend_tiles, P.pend_done);
+    walk_tiles<TR>(P, w, count, 0ull, lane, sum, run, &P.cnt->pending, P.pend_tiles, P.pend_done);
   }
   walk_flush(P.cnt, lane, sum);
 }
@@ -455,6 +463,8 @@ __global__ void __launch_bounds__(kVisThreads, kWalkBlocks)
                                  unsigned long long total_tiles, VisCounters* __restrict__ cnt,
                                  unsigned long long* __restrict__ pend_tiles, uint32_t* __restrict__ pend_done) {
   const int lane = threadIdx.x & 31;
+  __shared__ uint32_t runs[kVisThreads / 32][kWalkRun];
+  uint32_t* run = runs[threadIdx.x >> 5];
   WalkSums sum = {};
   for (int guard = 0; guard < (1 << 30); ++guard) {
     unsigned long long w = 0;
@@ -465,8 +475,8 @@ __global__ void __launch_bounds__(kVisThreads, kWalkBlocks)
     for (int pi = part_of(tile_start, n_parts, w); w < end; ++pi) {  // the run's parts
       const unsigned long long part_end = min(end, tile_start[pi + 1]);
       if (part_end <= w) continue;
-      walk_tiles<TR>(parts[pi], w - tile_start[pi], (int)(part_end - w), tile_start[pi], lane, sum, &cnt->pending,
-                     pend_tiles, pend_done);
+      walk_tiles<TR>(parts[pi], w - tile_start[pi], (int)(part_end - w), tile_start[pi], lane, sum, run,
+                     &cnt->pending, pend_tiles, pend_done);
       w = part_end;
     }
   }
