@@ -140,8 +140,8 @@ int visacd_measure_fp32_peak(visacd_ctx* ctx, double* tflops);
 int visacd_measure_tex_peak(visacd_ctx* ctx, double* coherent_gfetch, double* divergent_gfetch);
 
 /* ---- BVH ---------------------------------------------------------------- */
-/* Linear BVH over a triangle mesh: 63-bit Morton codes of triangle centroids,
-   LSD radix sort, Karras (2012) hierarchy, box fit. verts is nv x 3
+/* Linear BVH over a triangle mesh: Morton codes of triangle centroids (30 to 63
+   bits, by the triangle count), LSD radix sort, Karras (2012) hierarchy, box fit. verts is nv x 3
    float32, tris is nt x 3 uint32 (indices < nv, else VISACD_ERR_INVALID_ARG).
    device_ptrs selects host or device input. The BVH keeps the vertex indices
    of every triangle so a visibility query can skip triangles incident to the

@@ -38,7 +38,7 @@ def test_flat_sets_equal_host(native, ctx, kind, count):
 
 
 def test_time_of_a_large_flat_set(ctx):
-    """5,000 points, a third of them repeated: 37 ms of kernel at most, and 69 with FP64
+    """5,000 points, a third of them repeated: 37 ms of kernel at most, and 69 or more with FP64
     compares of keys in a cache that the block's shared memory left small."""
     p = _flat(5000, 1, "normal")
     best = 1e9

@@ -848,7 +848,7 @@ __global__ void __launch_bounds__(64) sdf_cell_vertex_kernel(SdfGrid g, const fl
     int ncross = 0;
 #pragma unroll
     for (int e = 0; e < 12; ++e) {
-      // Edges 0-3 run along x, 4-7 along y, 8-11 along z (kCedge).
+      // Edges 0-3 run along x, 4-7 along y, 8-11 along z, between corners numbered x + 2 y + 4 z.
       constexpr int kC[12][2] = {{0, 1}, {2, 3}, {4, 5}, {6, 7}, {0, 2}, {1, 3},
                                  {4, 6}, {5, 7}, {0, 4}, {1, 5}, {2, 6}, {3, 7}};
       const int c0 = kC[e][0], c1 = kC[e][1];
@@ -856,7 +856,7 @@ __global__ void __launch_bounds__(64) sdf_cell_vertex_kernel(SdfGrid g, const fl
       const double t = __ddiv_rn((double)__fsub_rn(g.fiso, cv[c0]), (double)__fsub_rn(cv[c1], cv[c0]));
 #pragma unroll
       for (int a = 0; a < 3; ++a) {
-        const int s0 = (c0 >> a) & 1, s1 = (c1 >> a) & 1;  // kCorner
+        const int s0 = (c0 >> a) & 1, s1 = (c1 >> a) & 1;
         acc[a] = da(acc[a], da((double)s0, dm(t, (double)(s1 - s0))));
       }
       ++ncross;

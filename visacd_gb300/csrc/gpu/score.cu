@@ -32,8 +32,8 @@
 
 namespace vgpu {
 
-// Two CTAs asked for at every K (K = 4 then keeps four edges' values in
-// registers and still has three resident).
+// Two CTAs asked for at every K: K = 4 then keeps four edges' values in its 82
+// registers, which leaves two resident.
 template <int K>
 __global__ void __launch_bounds__(kScoreThreads, 2)
     score_planes_kernel(const float4* __restrict__ planes, int32_t P,
@@ -502,7 +502,9 @@ static uint32_t score_shape_class(int32_t P, int64_t E, int32_t N = 0) {
 // share of that rate which few CTAs on an SM reach (a single one 0.70 with K = 1,
 // 0.95 with K = 2, 0.97 with K = 4). 59,183 edges x 2,500 planes take 70 us, 262,144
 // x 592 100, 4,661 x 2,500 14; with about four CTAs per SM and K by the planes alone
-// 106, 141 and 24.
+// 106, 141 and 24. Which calls come here: those that sides_pay leaves (fewer edges
+// than vertices, or too many vertices or planes), a forced or autotuned K, and the
+// allocation-free and batched entries, whatever their sizes.
 struct ScoreSplit {
   int64_t per, slices;
   double cost;

@@ -1,5 +1,5 @@
 // Device side of the segment visibility test, shared by the single-part and
-// the batched visibility kernels: segment setup, conservative packed slab test,
+// the batched visibility kernels: segment setup, conservative slab test,
 // FP32 segment-triangle test with its rounding bound, FP64 re-decision, and the
 // warp-packet any-hit traversal (see vis.cu for the design notes).
 #pragma once
