@@ -53,6 +53,13 @@ struct SdfGrid {
 // needed, but those of kClassEdge voxels farther out (a mesh that is not closed):
 // sdf_far_kernel marks these kClassFar and sdf_far_dist_kernel, which does
 // nothing without them, goes over the boxes grown by the band.
+//
+// Thin triangles (SdfTri::thin): the exact formula's closest point may lie off the
+// triangle, or be NaN, and what it gives is the result. So they bound nothing, and the
+// above holds for the other triangles alone; the thin ones are evaluated at every voxel
+// of their boxes grown by the band that is not on its side already (inside and no
+// kClassEdge, or an upper bound below iso - 1). What they bring below iso may have a
+// neighbour whose other distances were not needed: sdf_far_kernel marks that too.
 enum : uint8_t { kClassOut = 0, kClassIn = 1, kClassEdge = 2, kClassFar = 4 };
 __device__ __forceinline__ float class_cut(const SdfGrid& g, uint8_t c) {
   return (c & kClassEdge) ? 3.0e38f : ((c & kClassIn) ? 0.f : g.cut_out);
@@ -107,7 +114,7 @@ struct SdfTri {
   float blo[3], bhi[3];   // bounding box rounded outwards
   float4 pl;              // unit normal, offset; w of fe[0] = -1e30 without a plane
   float4 fe[3];           // unit in-plane edge normals, offsets (no vertex beyond)
-  int has_plane, irregular, pad[2];
+  int has_plane, thin, pad[2];
   int ray[3][4];          // per axis: first ray and extents over (u, w); extents 0: none
   float v[3][3], vabs;    // vertices in FP32, their largest coordinate
   int pad2[2];
@@ -115,13 +122,15 @@ struct SdfTri {
 
 // What the passes share beside the voxels.
 struct SdfFlags {
-  unsigned n_wide;     // listed triangles of sdf_cross_wide_kernel
-  unsigned n_far;      // whether sdf_far_dist_kernel has work
-  unsigned n_thin;     // listed triangles of irregular_triangle
-  unsigned irregular;  // whether a triangle is irregular
+  unsigned n_wide;  // listed triangles of sdf_cross_wide_kernel
+  unsigned n_far;   // whether sdf_far_dist_kernel has work
+  unsigned thin;    // whether a triangle is thin
+  unsigned pad;
 };
 
-constexpr int kSdfChunk = 256;  // box voxels per work item of the distance passes (one warp)
+// Box voxels per work item of the distance passes (one warp); fewer where all of them
+// take the exact formula.
+constexpr int kSdfChunk = 256, kSdfThinChunk = 32;
 
 __device__ __forceinline__ void box_range(const SdfGrid& g, int a, double mn, double mx, double by, int& lo, int& ext) {
   lo = max(0, (int)floor(mn - by) - g.org[a]);
@@ -129,19 +138,12 @@ __device__ __forceinline__ void box_range(const SdfGrid& g, int a, double mn, do
 }
 
 __global__ void sdf_tri_prep_kernel(const double* __restrict__ P, const int32_t* __restrict__ T, int nt, SdfGrid g,
-                                    SdfTri* __restrict__ out, uint32_t* __restrict__ chunks, int* __restrict__ thin,
+                                    SdfTri* __restrict__ out, uint32_t* __restrict__ chunks,
                                     SdfFlags* __restrict__ flags) {
   for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x) {
     double A[3], B[3], C[3];
     load_tri(P, T, t, A, B, C);
     SdfTri r;
-    for (int a = 0; a < 3; ++a) {
-      const double mn = min3(A[a], B[a], C[a]), mx = max3(A[a], B[a], C[a]);
-      box_range(g, a, mn, mx, g.reach, r.lo[a], r.ext[a]);
-      r.blo[a] = __double2float_rd(mn);
-      r.bhi[a] = __double2float_ru(mx);
-    }
-    if (r.ext[0] <= 0 || r.ext[1] <= 0 || r.ext[2] <= 0) r.ext[0] = 0;
     // unit normal and plane offset (FP32 copies; degenerate triangles get none)
     const double ux = B[0] - A[0], uy = B[1] - A[1], uz = B[2] - A[2];
     const double vx = C[0] - A[0], vy = C[1] - A[1], vz = C[2] - A[2];
@@ -150,12 +152,19 @@ __global__ void sdf_tri_prep_kernel(const double* __restrict__ P, const int32_t*
     r.has_plane = nl > 1e-12;
     // Thin: the exact formula's closest point may be off by 1e-3 voxels or lie outside
     // (its weights are quotients of products of this size, with an error of some 1e-14
-    // of L^2 (L + band)^2), or be NaN. irregular_triangle looks whether it is.
+    // of L^2 (L + band)^2), or be NaN.
     const double wx = C[0] - B[0], wy = C[1] - B[1], wz = C[2] - B[2];
     const double l2 = fmax(fmax(ux * ux + uy * uy + uz * uz, vx * vx + vy * vy + vz * vz), wx * wx + wy * wy + wz * wz);
     const double len = sqrt(l2), reachable = len + g.band;
-    if (!(nl * nl >= 1e-11 * l2 * len * reachable * reachable)) thin[atomicAdd(&flags->n_thin, 1u)] = t;
-    r.irregular = 0;
+    r.thin = !(nl * nl >= 1e-11 * l2 * len * reachable * reachable);
+    if (r.thin) flags->thin = 1u;
+    for (int a = 0; a < 3; ++a) {
+      const double mn = min3(A[a], B[a], C[a]), mx = max3(A[a], B[a], C[a]);
+      box_range(g, a, mn, mx, r.thin ? g.band : g.reach, r.lo[a], r.ext[a]);
+      r.blo[a] = __double2float_rd(mn);
+      r.bhi[a] = __double2float_ru(mx);
+    }
+    if (r.ext[0] <= 0 || r.ext[1] <= 0 || r.ext[2] <= 0) r.ext[0] = 0;
     r.pl = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int e = 0; e < 3; ++e) r.fe[e] = make_float4(0.f, 0.f, 0.f, -1e30f);
     if (r.has_plane) {
@@ -200,7 +209,8 @@ __global__ void sdf_tri_prep_kernel(const double* __restrict__ P, const int32_t*
       r.vabs = fmaxf(r.vabs, fmaxf(fabsf(r.v[0][a]), fmaxf(fabsf(r.v[1][a]), fabsf(r.v[2][a]))));
     }
     out[t] = r;
-    chunks[t] = r.ext[0] > 0 ? (uint32_t)((r.ext[0] * r.ext[1] * r.ext[2] + kSdfChunk - 1) / kSdfChunk) : 0u;
+    const int chunk = r.thin ? kSdfThinChunk : kSdfChunk;
+    chunks[t] = r.ext[0] > 0 ? (uint32_t)((r.ext[0] * r.ext[1] * r.ext[2] + chunk - 1) / chunk) : 0u;
   }
 }
 
@@ -317,54 +327,6 @@ __device__ __forceinline__ float sdf_lower_bound(const SdfTri& r, float qx, floa
   return lb;
 }
 
-__device__ __forceinline__ float segment_dist32(const float (&q)[3], const float* a, const float* b) {
-  const float dx = b[0] - a[0], dy = b[1] - a[1], dz = b[2] - a[2];
-  const float px = q[0] - a[0], py = q[1] - a[1], pz = q[2] - a[2];
-  const float k = fminf(fmaxf((px * dx + py * dy + pz * dz) / (dx * dx + dy * dy + dz * dz), 0.f), 1.f);
-  const float ex = px - k * dx, ey = py - k * dy, ez = pz - k * dz;
-  return sqrtf(ex * ex + ey * ey + ez * ez);
-}
-
-// A thin triangle, its part `part` of `parts` by a block: irregular when the exact
-// formula leaves the bounds, or is not the distance to the nearest edge less at most
-// the triangle's height, at some voxel of its box grown by the band. What the formula
-// gives is the result, so an irregular triangle bounds nothing, is evaluated for every
-// voxel of that box, and makes every voxel of the grid take its exact distance (the
-// range of class_cut supposes that neighbours' distances differ by at most 1, with
-// 0.01 to spare). Else it is a triangle like others. Meshes cut by the pipeline hold
-// some thin triangles and hardly an irregular one: with all thin ones taken for
-// irregular a process of a cut bowl took 6 % longer, now the time without the test.
-constexpr double kThinHeight = 2e-3;
-__device__ __noinline__ void irregular_triangle(const double* __restrict__ P, const int32_t* __restrict__ T, int t,
-                                                int part, int parts, const SdfGrid& g, SdfTri* __restrict__ prep,
-                                                SdfFlags* __restrict__ flags) {
-  double A[3], B[3], C[3];
-  load_tri(P, T, t, A, B, C);
-  int lo[3], ext[3];
-#pragma unroll
-  for (int a = 0; a < 3; ++a)
-    box_range(g, a, min3(A[a], B[a], C[a]), max3(A[a], B[a], C[a]), g.band, lo[a], ext[a]);
-  if (ext[0] <= 0 || ext[1] <= 0 || ext[2] <= 0) return;
-  const SdfTri& r = prep[t];
-  const volatile int* found = &r.irregular;
-  const int n = ext[0] * ext[1] * ext[2];
-  for (int k = part * (int)blockDim.x + (int)threadIdx.x; k < n && !*found; k += parts * (int)blockDim.x) {
-    const int i = k % ext[0], j = k / ext[0] % ext[1], l = k / (ext[0] * ext[1]);
-    const float q[3] = {(float)(g.org[0] + lo[0] + i), (float)(g.org[1] + lo[1] + j), (float)(g.org[2] + lo[2] + l)};
-    const double p[3] = {(double)q[0], (double)q[1], (double)q[2]};
-    const float big = kSdfU * fmaxf(r.vabs, fmaxf(fabsf(q[0]), fmaxf(fabsf(q[1]), fabsf(q[2]))));
-    const float edge = fminf(segment_dist32(q, r.v[0], r.v[1]),
-                             fminf(segment_dist32(q, r.v[1], r.v[2]), segment_dist32(q, r.v[2], r.v[0])));
-    const double d = point_tri_dist(p, A, B, C);
-    if (!(fabs(d - (double)edge) <= kThinHeight + (double)(8.0f * big) &&
-          d >= (double)(sdf_lower_bound(r, q[0], q[1], q[2]) - 2.0f * g.margin) &&
-          d <= (double)tri_dist_ub32(q[0], q[1], q[2], r.v[0], r.v[1], r.v[2], 64.0f * big + g.margin))) {
-      prep[t].irregular = 1;
-      flags->irregular = flags->n_far = 1u;
-    }
-  }
-}
-
 __global__ void __launch_bounds__(128) sdf_ub_kernel(SdfItems W, SdfGrid g, const SdfTri* __restrict__ prep,
                                                      const uint8_t* __restrict__ cls, uint32_t* __restrict__ ub) {
   const int lane = threadIdx.x & 31;
@@ -374,7 +336,7 @@ __global__ void __launch_bounds__(128) sdf_ub_kernel(SdfItems W, SdfGrid g, cons
   for (long long w = w0; w < w1; ++w) {
     while ((long long)W.off[t + 1] <= w) ++t;
     const SdfTri& r = prep[t];
-    if (r.irregular) continue;
+    if (r.thin) continue;
     // rounding of the vertices to float, of the chosen point and of its
     // distance: a few units of 2^-24 of the largest coordinate involved
     const int n = r.ext[0] * r.ext[1] * r.ext[2];
@@ -457,7 +419,8 @@ __global__ void __launch_bounds__(128, kDistBlocks) sdf_dist_kernel(const double
     while ((long long)W.off[t + 1] <= w) ++t;
     const SdfTri& r = prep[t];
     const int n = r.ext[0] * r.ext[1] * r.ext[2];
-    const int c0 = (int)(w - (long long)W.off[t]) * kSdfChunk, c1 = min(n, c0 + kSdfChunk);
+    const int chunk = r.thin ? kSdfThinChunk : kSdfChunk;
+    const int c0 = (int)(w - (long long)W.off[t]) * chunk, c1 = min(n, c0 + chunk);
     BoxWalk at(r.ext, c0 + lane);
     for (int base = c0; base < c1; base += 32, at.step()) {
       bool keep = false;
@@ -472,9 +435,9 @@ __global__ void __launch_bounds__(128, kDistBlocks) sdf_dist_kernel(const double
         // the other side
         if (c == kClassOut && up < g.low_out) cur = 0.f;
         if (cur > 0.f) {
-          const float lb = r.irregular ? -3.0e38f
-                                       : sdf_lower_bound(r, (float)(g.org[0] + i), (float)(g.org[1] + j),
-                                                         (float)(g.org[2] + k));
+          const float lb = r.thin ? -3.0e38f
+                                  : sdf_lower_bound(r, (float)(g.org[0] + i), (float)(g.org[1] + j),
+                                                    (float)(g.org[2] + k));
           keep = lb - 2.0f * g.margin < fminf(cur, __uint_as_float(*(volatile const uint32_t*)&dist[v]));
         }
       }
@@ -484,13 +447,23 @@ __global__ void __launch_bounds__(128, kDistBlocks) sdf_dist_kernel(const double
 }
 
 __global__ void sdf_far_kernel(SdfGrid g, size_t n, const uint32_t* __restrict__ dist, const uint32_t* __restrict__ ub,
-                               uint8_t* __restrict__ cls, unsigned* __restrict__ n_far) {
+                               uint8_t* __restrict__ cls, SdfFlags* __restrict__ flags) {
+  const bool thin = flags->thin != 0;
+  const size_t sy = g.dim[0], sz = (size_t)g.dim[0] * g.dim[1];
+  auto field = [&](size_t v) { return fminf(__uint_as_float(dist[v]), __uint_as_float(ub[v])); };
   for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (size_t)gridDim.x * blockDim.x) {
     const uint8_t c = cls[v];
-    if (!(c & kClassEdge)) continue;
-    if ((double)fminf(__uint_as_float(dist[v]), __uint_as_float(ub[v])) < g.reach) continue;
+    if (!(c & kClassEdge) && !(thin && c == kClassOut)) continue;
+    if ((double)field(v) < g.reach) continue;
+    if (!(c & kClassEdge)) {  // (its neighbours are outside too)
+      const int i = (int)(v % sy), j = (int)(v / sy % g.dim[1]), k = (int)(v / sz);
+      if (!((i > 0 && field(v - 1) < g.fiso) || (i + 1 < g.dim[0] && field(v + 1) < g.fiso) ||
+            (j > 0 && field(v - sy) < g.fiso) || (j + 1 < g.dim[1] && field(v + sy) < g.fiso) ||
+            (k > 0 && field(v - sz) < g.fiso) || (k + 1 < g.dim[2] && field(v + sz) < g.fiso)))
+        continue;
+    }
     cls[v] = c | kClassFar;
-    *n_far = 1u;
+    flags->n_far = 1u;
   }
 }
 
@@ -519,8 +492,8 @@ __global__ void __launch_bounds__(128, kDistBlocks)
 #pragma unroll
     for (int x = 0; x < 3; ++x)
       box_range(g, x, min3(A[x], B[x], C[x]), max3(A[x], B[x], C[x]), g.band, lo[x], ext[x]);
-    if (ext[0] <= 0 || ext[1] <= 0 || ext[2] <= 0) return;
     const SdfTri& r = prep[t];
+    if (r.thin || ext[0] <= 0 || ext[1] <= 0 || ext[2] <= 0) return;
     const long long n = ext[0] * ext[1] * ext[2];
     const int c0 = (int)(n * a / items), c1 = (int)(n * b / items);
     BoxWalk at(ext, c0 + lane);
@@ -530,9 +503,7 @@ __global__ void __launch_bounds__(128, kDistBlocks)
       if (base + lane < c1) {
         const int i = lo[0] + at.i, j = lo[1] + at.j, k = lo[2] + at.k;
         v = vid(g, i, j, k);
-        if (r.irregular) {
-          keep = true;
-        } else if (cls[v] & kClassFar) {
+        if (cls[v] & kClassFar) {
           const float lb = sdf_lower_bound(r, (float)(g.org[0] + i), (float)(g.org[1] + j), (float)(g.org[2] + k));
           keep = lb - 2.0f * g.margin < __uint_as_float(*(volatile const uint32_t*)&dist[v]);
         }
@@ -740,14 +711,10 @@ __global__ void __launch_bounds__(64) sdf_parity_yz_kernel(SdfGrid g, const uint
 
 // Prefix parity along x (one warp per row, 32 voxels at a time by ballot) and
 // the class of every voxel: inside when at least two parities are odd.
-// Then the thin triangles, all blocks sharing them.
 __global__ void __launch_bounds__(128) sdf_inside_kernel(SdfGrid g, const uint32_t* __restrict__ toggle,
                                                          const uint8_t* __restrict__ par_y,
                                                          const uint8_t* __restrict__ par_z,
-                                                         uint8_t* __restrict__ inside, const double* __restrict__ P,
-                                                         const int32_t* __restrict__ T, SdfTri* __restrict__ prep,
-                                                         const int* __restrict__ thin, SdfFlags* __restrict__ flags) {
-  const int n_thin = (int)flags->n_thin;
+                                                         uint8_t* __restrict__ inside) {
   const int lane = threadIdx.x & 31;
   const int rows = g.dim[1] * g.dim[2], warps = (gridDim.x * blockDim.x) >> 5;
   for (int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < rows; r += warps) {
@@ -762,18 +729,13 @@ __global__ void __launch_bounds__(128) sdf_inside_kernel(SdfGrid g, const uint32
       carry += __popc(m);
     }
   }
-  const int parts = max(1, (int)gridDim.x / max(1, n_thin));
-  for (int k = blockIdx.x; k < n_thin * parts; k += gridDim.x)
-    irregular_triangle(P, T, thin[k / parts], k % parts, parts, g, prep, flags);
 }
 
-// Marks voxels with a neighbour of the other class (all, or a mesh with irregular
-// triangles: every voxel, since the range of class_cut does not apply), and starts both distance arrays at the
+// Marks voxels with a neighbour of the other class (all: every voxel, when
+// the range of class_cut does not apply), and starts both distance arrays at the
 // band.
-__global__ void sdf_class_kernel(SdfGrid g, const uint8_t* __restrict__ inside, int all,
-                                 const SdfFlags* __restrict__ flags, uint32_t band, uint8_t* __restrict__ cls,
-                                 uint32_t* __restrict__ ub, uint32_t* __restrict__ dist) {
-  if (flags->irregular) all = 1;
+__global__ void sdf_class_kernel(SdfGrid g, const uint8_t* __restrict__ inside, int all, uint32_t band,
+                                 uint8_t* __restrict__ cls, uint32_t* __restrict__ ub, uint32_t* __restrict__ dist) {
   const size_t n = (size_t)g.dim[0] * g.dim[1] * g.dim[2];
   const size_t sy = g.dim[0], sz = (size_t)g.dim[0] * g.dim[1];
   for (size_t v = (size_t)blockIdx.x * blockDim.x + threadIdx.x; v < n; v += (size_t)gridDim.x * blockDim.x) {
@@ -981,8 +943,7 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   const size_t upload = at;
   const size_t oTog = take(nvox * 4), oFlags = take(sizeof(SdfFlags));
   const size_t zero_end = at;
-  const size_t oPrep = take((size_t)nt * sizeof(SdfTri)), oWide = take(3 * (size_t)nt * 4), oThin = take((size_t)nt * 4),
-               oChunks = take((size_t)nt * 4), oChunkOff = take(((size_t)nt + 1) * 8), oDist = take(nvox * 4),
+  const size_t oPrep = take((size_t)nt * sizeof(SdfTri)), oWide = take(3 * (size_t)nt * 4), oChunks = take((size_t)nt * 4), oChunkOff = take(((size_t)nt + 1) * 8), oDist = take(nvox * 4),
                oUb = take(nvox * 4), oPy = take(nvox), oPz = take(nvox), oIn = take(nvox), oCls = take(nvox),
                oF = take(nvox * 4), oFlag = take(ncell * 4), oCoff = take((ncell + 1) * 8), oCv = take(ncell * 4),
                oQcnt = take(nint * 4), oQoff = take((nint + 1) * 8);
@@ -1015,10 +976,9 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   uint32_t* chunks = (uint32_t*)(base + oChunks);
   uint64_t* chunk_off = (uint64_t*)(base + oChunkOff);
   SdfFlags* flags = (SdfFlags*)(base + oFlags);
-  int* thin = (int*)(base + oThin);
   unsigned *n_wide = &flags->n_wide, *n_far = &flags->n_far;
   VLAUNCH(ctx, kKSdfDist, grid_for(nt, 64, 32 * (int64_t)ctx->sm_count), 64, 0, sdf_tri_prep_kernel, dP, dT, nt,
-          g, prep, chunks, thin, flags);
+          g, prep, chunks, flags);
   // Crossings of all three axes, the triangles covering many rays one block
   // each, then the parities and classes.
   int* wide = (int*)(base + oWide);
@@ -1030,10 +990,9 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
           dim3(grid_for((int64_t)g.dim[0] * std::max(g.dim[1], g.dim[2]), 64, 32 * (int64_t)ctx->sm_count), 2), 64, 0,
           sdf_parity_yz_kernel, g, (const uint32_t*)tog, par_y, par_z);
   VLAUNCH(ctx, kKSdfCross, grid_for(32LL * g.dim[1] * g.dim[2], 128, 16 * (int64_t)ctx->sm_count), 128, 0,
-          sdf_inside_kernel, g, (const uint32_t*)tog, (const uint8_t*)par_y, (const uint8_t*)par_z, inside,
-          dP, dT, prep, (const int*)thin, flags);
+          sdf_inside_kernel, g, (const uint32_t*)tog, (const uint8_t*)par_y, (const uint8_t*)par_z, inside);
   VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_class_kernel, g, (const uint8_t*)inside, all_exact ? 1 : 0,
-          (const SdfFlags*)flags, band_bits, cls, ub, dist);
+          band_bits, cls, ub, dist);
   VTRY(exclusive_scan_u32_to_u64(ctx, chunks, chunk_off, nt));
   SdfItems items;
   items.off = chunk_off;
@@ -1044,7 +1003,7 @@ extern "C" int visacd_sdf_remesh(visacd_ctx* ctx, const double* verts, int32_t n
   VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_dist_kernel, dP, dT, items, g, (const SdfTri*)prep, (const uint8_t*)cls,
           (const uint32_t*)ub, dist);
   if (g.reach < g.band) {
-    VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_far_kernel, g, nvox, (const uint32_t*)dist, (const uint32_t*)ub, cls, n_far);
+    VLAUNCH(ctx, kKSdf, gv, 256, 0, sdf_far_kernel, g, nvox, (const uint32_t*)dist, (const uint32_t*)ub, cls, flags);
     VLAUNCH(ctx, kKSdfDist, gw, 128, 0, sdf_far_dist_kernel, dP, dT, items, g, (const SdfTri*)prep, (const uint8_t*)cls,
             (const unsigned*)n_far, dist);
   }
