@@ -181,10 +181,11 @@ struct WalkSums {
 // is lane_pair's; the row's point stays in registers along a tile row, and the
 // next tile is the next of the row or the first of the next row. Tiles with
 // lanes left are listed as base + their number, a run's together with one atomic
-// (18 M pairs in an open soup, nearly all left: 0.20 ms, 0.44 with one a tile). The
-// run's done lanes wait in `run` (kWalkRun words of the warp's in shared memory): a
-// register more and visibility_multi_walk_kernel spills (1.82 ms for a bowl's parts,
-// 1.48 so).
+// (18 M pairs in an open soup, nearly all left: 0.20 ms, 0.44 with one a tile). Their
+// done lanes wait in `run` (kWalkRun words of the warp's in shared memory): in a
+// register more visibility_multi_walk_kernel spills in its loop (1.82 ms for a bowl's
+// parts, 1.50 so). Few tiles are left where the walk pays, so a tile's done lanes are
+// stored only then (a store and a warp barrier for each: 52 M pairs 0.50 ms, 0.48 so).
 template <int TR>
 __device__ __forceinline__ void walk_tiles(const VisParams& P, unsigned long long w, int count,
                                            unsigned long long base, int lane, WalkSums& sum,
@@ -197,6 +198,7 @@ __device__ __forceinline__ void walk_tiles(const VisParams& P, unsigned long lon
   static_assert(kWalkRun <= 32, "a lane per tile of a run");
   int tr = (int)tr64, tc = (int)tc64, row = -1;
   uint32_t oi = 0;
+  unsigned left = 0;  // the tiles with lanes left
   float px = 0.f, py = 0.f, pz = 0.f;
   for (int k = 0; k < count; ++k) {
     const int a = tr * TR + lane / TC, b = tc * TC + lane % TC;
@@ -236,25 +238,26 @@ __device__ __forceinline__ void walk_tiles(const VisParams& P, unsigned long lon
       }
     }
     const unsigned m = __ballot_sync(0xffffffffu, done);
-    if (lane == 0) run[k] = m;
+    if (m != 0xffffffffu) {
+      left |= 1u << k;
+      if (lane == 0) run[k] = m;
+    }
     if (++tc >= P.ntc) {
       ++tr;
       tc = P.triangular ? tr * TR / TC : 0;
     }
   }
-  __syncwarp();
-  const uint32_t mask = lane < count ? run[lane] : 0xffffffffu;
-  const unsigned left = __ballot_sync(0xffffffffu, mask != 0xffffffffu);
   if (left) {
     unsigned long long at = 0;
     if (lane == 0) at = atomicAdd(pending, (unsigned long long)__popc(left));
     at = __shfl_sync(0xffffffffu, at, 0) + __popc(left & ((1u << lane) - 1u));
-    if (mask != 0xffffffffu) {
+    __syncwarp();
+    if (left >> lane & 1u) {
       pend_tiles[at] = base + w + lane;
-      pend_done[at] = mask;
+      pend_done[at] = run[lane];
     }
+    __syncwarp();
   }
-  __syncwarp();
 }
 
 __device__ __forceinline__ void walk_flush(VisCounters* __restrict__ cnt, int lane, const WalkSums& sum) {
