@@ -205,7 +205,8 @@ def run_ours(args) -> dict:
     sb.close()
     cb.close()
     planes = bisector_planes(v, edges0, N_PLANES, seed=1)
-    # Autotune the scoring kernel's planes per thread for this shape class.
+    # Autotune scoring for this shape class: planes per thread of the per-edge kernel,
+    # and whether the kernels by vertex sides are faster still (then the step uses those).
     score_k, score_k_ms = ctx.autotune_scoring(planes, v, edges0)
     d_planes = torch.from_numpy(planes).to(dev)
     d_scores = torch.empty(N_PLANES, dtype=torch.float64, device=dev)
